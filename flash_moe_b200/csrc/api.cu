@@ -105,7 +105,7 @@ int router_front(const void* x, const void* w, void* rm, void* rv, int training,
     rc = launch_gemm_add(xn, w, nullptr, logits, dtype, T, 2 * nk, H, status, stream);
   else
     rc = launch_simt_gemm(xn, H, w, nullptr, nullptr, logits, 2 * static_cast<int64_t>(nk), dtype, 0, T, 2 * nk, H,
-                          stream);
+                          stream, nullptr, /*ordered=*/true);
   if (rc != FMOE_OK) return rc;
   if (logp == nullptr) return FMOE_OK;
   return launch_log_softmax_halves(logits, logp, dtype, T, nk, stream);

@@ -210,10 +210,22 @@ int launch_gemm_swiglu_pair(const void* x, const void* gate_w, const void* up_w,
 int launch_gemm_add_pair(const void* a, const void* b, const float* addend, void* out, int dtype, int64_t M, int N,
                          int K, int32_t* status, cudaStream_t stream, const void* residual = nullptr);
 
-// fp32-FMA GEMM on CUDA cores (simt_gemm.cu): float32 modules and shapes TMA cannot address.
+// the same two GEMMs for few tokens (gemm_sm100_narrow.cu): weight rows on the MMA's 128 rows, K split over a cluster.
+// early_weights: the kernel before this one in the stream is one of a forward's, so the weights cannot be written any
+// more and may be requested before it has finished.
+bool gemm_narrow_preferred(int64_t M, int N, int K, bool swiglu);
+int launch_gemm_swiglu_narrow(const void* x, const void* gate_w, const void* up_w, void* h, int dtype, int64_t M, int I,
+                              int K, bool early_weights, int32_t* status, cudaStream_t stream, void* pre_gate = nullptr,
+                              void* pre_up = nullptr);
+int launch_gemm_add_narrow(const void* a, const void* b, const float* addend, void* out, int dtype, int64_t M, int N,
+                           int K, bool early_weights, int32_t* status, cudaStream_t stream,
+                           const void* residual = nullptr);
+
+// fp32-FMA GEMM on CUDA cores (simt_gemm.cu): float32 modules and shapes TMA cannot address.  `ordered`: every output
+// is one fmaf chain over ascending k (the router's logits, whose last bit decides between experts).
 int launch_simt_gemm(const void* a, int64_t lda, const void* b0, const void* b1, const float* addend, void* out,
                      int64_t ldo, int dtype, int swiglu, int64_t M, int N, int K, cudaStream_t stream,
-                     const void* residual = nullptr);
+                     const void* residual = nullptr, bool ordered = false);
 
 // elementwise.cu
 int launch_log_softmax_halves(const void* logits, void* log_probs, int dtype, int64_t T, int nk, cudaStream_t stream);
