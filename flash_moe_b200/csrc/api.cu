@@ -114,11 +114,13 @@ int router_front(const void* x, const void* w, void* rm, void* rv, int training,
 size_t mlp_ws(int64_t T, int I, int dtype) { return align_up(static_cast<size_t>(T) * I * dtype_size(dtype), 256); }
 
 int mlp_up(const void* x, const void* gw, const void* uw, void* h, int dtype, int64_t T, int H, int I, int32_t* status,
-           cudaStream_t stream, void* pre_gate = nullptr, void* pre_up = nullptr) {
+           cudaStream_t stream, void* pre_gate = nullptr, void* pre_up = nullptr, bool follows_ours = false) {
   const bool tc = is16(dtype) && (H % 8 == 0) && (I % 8 == 0) && aligned16(x) && aligned16(gw) && aligned16(uw);
+  if (tc && gemm_narrow_preferred(T, I, H, true))
+    return launch_gemm_swiglu_narrow(x, gw, uw, h, dtype, T, I, H, follows_ours, status, stream, pre_gate, pre_up);
   if (tc && gemm_pair_supported(T, I, H))
     return launch_gemm_swiglu_pair(x, gw, uw, h, dtype, T, I, H, status, stream, pre_gate, pre_up);
-  if (pre_gate != nullptr || pre_up != nullptr) return FMOE_ERR_UNSUPPORTED;  // only the CTA-pair kernel keeps them
+  if (pre_gate != nullptr || pre_up != nullptr) return FMOE_ERR_UNSUPPORTED;  // only the kernels above keep them
   if (tc) return launch_gemm_swiglu(x, gw, uw, h, dtype, T, I, H, status, stream);
   return launch_simt_gemm(x, H, gw, uw, nullptr, h, I, dtype, 1, T, I, H, stream);
 }
@@ -128,6 +130,8 @@ int mlp_down(const void* h, const void* dw, const float* addend, void* out, int 
              int32_t* status, cudaStream_t stream, const void* residual = nullptr) {
   const bool tc = is16(dtype) && (H % 8 == 0) && (I % 8 == 0) && aligned16(dw) && aligned16(out) &&
                   (addend == nullptr || aligned16(addend)) && (residual == nullptr || aligned16(residual));
+  if (tc && gemm_narrow_preferred(T, H, I, false))  // the up GEMM runs just before: its predecessor is always ours
+    return launch_gemm_add_narrow(h, dw, addend, out, dtype, T, H, I, true, status, stream, residual);
   if (tc && gemm_pair_supported(T, H, I))
     return launch_gemm_add_pair(h, dw, addend, out, dtype, T, H, I, status, stream, residual);
   if (tc) return launch_gemm_add(h, dw, addend, out, dtype, T, H, I, status, stream, residual);

@@ -194,6 +194,21 @@ inline int make_tensor_map(CUtensorMap* m, const void* basep, int dtype, uint64_
   return r == CUDA_SUCCESS ? FMOE_OK : FMOE_ERR_BAD_ARG;
 }
 
+// 2-D 16-bit output written by tiled stores: boxes of box_cols x box_rows elements, no swizzle
+inline int make_tensor_map_out(CUtensorMap* m, const void* basep, int dtype, uint64_t cols, uint64_t rows, uint32_t box_cols,
+                               uint32_t box_rows) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (fn == nullptr) return -static_cast<int>(cudaErrorNotSupported);
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {cols * 2};
+  const cuuint32_t box[2] = {box_cols, box_rows};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUtensorMapDataType dt = dtype == FMOE_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  const CUresult r = fn(m, dt, 2, const_cast<void*>(basep), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? FMOE_OK : FMOE_ERR_BAD_ARG;
+}
+
 // float32 [rows, cols] row-major, boxes of 32 columns (128 bytes) x box_rows rows, 128-byte swizzle: the addend tile of
 // the down GEMM's epilogue
 inline int make_tensor_map_f32(CUtensorMap* m, const void* basep, uint64_t cols, uint64_t rows, uint64_t pitch,

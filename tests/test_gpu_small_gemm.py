@@ -30,3 +30,32 @@ def test_mlp_float32_tiles(T, H, I):
     got = flash_mlp_add(x, wg, wu, wd, addend)
     assert (got.double() - want).norm() <= 2e-6 * want.norm()
     assert torch.equal(got, flash_mlp_add(x, wg, wu, wd, addend))
+
+
+@pytest.mark.parametrize(
+    "T,H,I",
+    [(1, 8, 8), (16, 1024, 4096), (17, 72, 200), (64, 2048, 1024), (129, 128, 8), (257, 256, 1000), (500, 1000, 520),
+     (1100, 512, 2000)],
+)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_mlp_few_tokens(T, H, I, dtype):
+    """Weight-row tiles of 64 and 128 rows, 1 to 256 token columns, K unsplit and split over 2, 4 and 8 CTAs; with the
+    addend, and the pre-activations kept for the backward."""
+    from flash_moe_b200 import check_status
+    from flash_moe_b200.ops.flash_mlp import _mlp_forward, flash_mlp_add
+
+    x, wg, wu, wd, _ = mlp_case(T, H, I, dtype)
+    g, u = x.float() @ wg.float().t(), x.float() @ wu.float().t()
+    h = (torch.nn.functional.silu(g) * u).to(dtype).float()
+    addend = randn((T, H), 5, torch.float32).cuda()
+    ulp = 2.0**-8 if dtype == torch.bfloat16 else 2.0**-11
+    want = h @ wd.float().t() + addend
+    got = flash_mlp_add(x, wg, wu, wd, addend)
+    assert (got.float() - want).norm() <= ulp * want.norm()
+    assert torch.equal(got, flash_mlp_add(x, wg, wu, wd, addend))
+    out, a, b = _mlp_forward(x, wg, wu, wd, save_preacts=True)
+    assert (out.float() - (want - addend)).norm() <= ulp * (want - addend).norm()
+    for kept, ref in ((a, g), (b, u)):
+        if kept is not None:
+            assert (kept.float() - ref).norm() <= ulp * ref.norm()
+    check_status()
