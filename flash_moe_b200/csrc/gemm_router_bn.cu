@@ -64,7 +64,7 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen_tail + 8);
   float2* stats = reinterpret_cast<float2*>(gen_tail + 24);  // (mean, inv_std) per feature, padded to whole k-blocks; 16-byte aligned
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0);  // known to be warp-uniform
   const int lane = threadIdx.x & 31;
   const int m_tile = blockIdx.x % num_m_tiles;
   const int n_tile = blockIdx.x / num_m_tiles;
@@ -145,7 +145,7 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(kFull, *tmem_slot, 0);
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -167,25 +167,30 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = (1u << 4) | (UmmaFmt<T>::v << 7) | (UmmaFmt<T>::v << 10) |
-                                 (static_cast<uint32_t>(BLOCK_N >> 3) << 17) |
-                                 (static_cast<uint32_t>(BLOCK_M >> 4) << 24);
-      bool ok = true;
-      for (int kb = 0; kb < num_k_blocks; ++kb) {
-        const int s = kb % kStages;
-        if (!ptx::mbar_wait_bounded(ready_bar(s), (kb / kStages) & 1u, abort_flag)) { ok = false; break; }
-        ptx::tc_fence_after();
-        const uint64_t da = ptx::umma_desc_kmajor_sw128(a_smem(s));
-        const uint64_t db = ptx::umma_desc_kmajor_sw128(b_smem(s));
+    // ------------------------------------------------------------ MMA issuer (whole-warp loop, see ptx::elect_one)
+    constexpr uint32_t idesc = (1u << 4) | (UmmaFmt<T>::v << 7) | (UmmaFmt<T>::v << 10) |
+                               (static_cast<uint32_t>(BLOCK_N >> 3) << 17) |
+                               (static_cast<uint32_t>(BLOCK_M >> 4) << 24);
+    bool ok = true;
+    int s = 0;
+    uint32_t ph = 0;
+    for (int kb = 0; kb < num_k_blocks; ++kb) {
+      if (!ptx::mbar_wait_bounded(ready_bar(s), ph, abort_flag)) { ok = false; break; }
+      ptx::tc_fence_after();
+      const uint64_t da = ptx::umma_desc_kmajor_sw128(a_smem(s));
+      const uint64_t db = ptx::umma_desc_kmajor_sw128(b_smem(s));
+      if (ptx::elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < BLOCK_K / UMMA_K; ++kk)
           ptx::umma_bf16_ss(tmem_base, da + 2 * kk, db + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
         ptx::umma_commit(empty_bar(s));
       }
-      if (ok) ptx::umma_commit(tfull_bar);
+      if (++s == kStages) {
+        s = 0;
+        ph ^= 1u;
+      }
     }
+    if (ok && ptx::elect_one()) ptx::umma_commit(tfull_bar);
   } else {
     // ------------------------------------------------------------ normalise the x tiles (warps 2..9)
     // Two groups of four warps take alternate k-blocks, so that two tiles are being normalised at any time (one

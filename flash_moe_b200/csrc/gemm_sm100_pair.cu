@@ -53,6 +53,20 @@ struct PairEpi {
 
 using epi::UmmaFmt;
 
+// Order of the tiles: groups of kGroupM row tiles, inside a group column tile by column tile.  The pairs working at one
+// time then cover about 16 x 5 tiles, whose operands stay in L2 until the group is done, instead of 74 row tiles of one
+// column: with more row tiles than fit L2 that order read A from DRAM once per column tile (131072 x 2048 tokens against
+// 11264 gate and up rows: 24 GB per call, now 0.5).
+constexpr int kGroupM = 16;
+__device__ __forceinline__ void tile_coords(int tile, int num_m_tiles, int num_n_tiles, int& m_tile, int& n_tile) {
+  const int per_group = kGroupM * num_n_tiles;
+  const int g = tile / per_group;
+  const int in_group = tile - g * per_group;
+  const int rows = min(kGroupM, num_m_tiles - g * kGroupM);
+  n_tile = in_group / rows;
+  m_tile = g * kGroupM + in_group - n_tile * rows;
+}
+
 template <int EPI, typename T>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB0,
@@ -73,7 +87,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + RING_BYTES + ADDEND_BYTES + (2 * STAGES + 4 + ADDEND_BUFS) * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + RING_BYTES + ADDEND_BYTES + (2 * STAGES + 4 + ADDEND_BUFS) * 8 + 8);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0);  // known to be warp-uniform
   const int lane = threadIdx.x & 31;
   const uint32_t rank = ptx::cluster_ctarank();
   const int pair = blockIdx.x >> 1;
@@ -103,22 +117,23 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   ptx::tc_fence_before();
   ptx::cluster_sync();  // barriers of both CTAs are initialised before anyone signals them
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(kFull, *tmem_slot, 0);
   pdl_wait();  // barriers, tensor memory and tensor maps are ready; the operands come from the kernel before this one
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += npairs) {
-        const int m_tile = tile % num_m_tiles;
-        const int n_tile = tile / num_m_tiles;
-        const int a_row = m_tile * (2 * BLOCK_M) + static_cast<int>(rank) * BLOCK_M;
-        for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1u;
-          if (!ptx::mbar_wait_bounded(empty_bar(s), ph ^ 1u, abort_flag)) { ok = false; break; }
+    // whole-warp loops with one elected issuing lane here and in the MMA warp (see ptx::elect_one)
+    uint32_t it = 0;
+    bool ok = true;
+    int s = 0;
+    uint32_t ph = 0;
+    for (int tile = pair; tile < num_tiles && ok; tile += npairs) {
+      int m_tile, n_tile;
+      tile_coords(tile, num_m_tiles, num_n_tiles, m_tile, n_tile);
+      const int a_row = m_tile * (2 * BLOCK_M) + static_cast<int>(rank) * BLOCK_M;
+      for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
+        if (!ptx::mbar_wait_bounded(empty_bar(s), ph ^ 1u, abort_flag)) { ok = false; break; }
+        if (ptx::elect_one()) {
           if (rank == 0) ptx::mbar_arrive_expect_tx(full_bar(s), 2 * STAGE_BYTES);
           const uint32_t leader_full = ptx::map_to_cta(full_bar(s), 0);
           ptx::tma_load_2d_pair(a_smem(s), &tmA, leader_full, kb * BLOCK_K, a_row);
@@ -131,42 +146,52 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                                   n_tile * BLOCK_N + static_cast<int>(rank) * (BLOCK_N / 2));
           }
         }
+        if (++s == STAGES) {
+          s = 0;
+          ph ^= 1u;
+        }
       }
-      if (!ok && rank == 0) {
-        // gave up: the leader's `full` barriers count the bytes of BOTH CTAs, so once the leader has seen the
-        // stages still in flight complete, neither CTA has a copy on its way; the peer stays until the cluster
-        // barrier of the teardown, which the leader reaches only after this loop
-        const uint32_t first = it > static_cast<uint32_t>(STAGES) ? it - STAGES : 0u;
-        for (uint32_t j = first; j < it; ++j) ptx::mbar_wait_drain(full_bar(j % STAGES), (j / STAGES) & 1u);
-      }
+    }
+    if (!ok && rank == 0) {
+      // gave up: the leader's `full` barriers count the bytes of BOTH CTAs, so once the leader has seen the
+      // stages still in flight complete, neither CTA has a copy on its way; the peer stays until the cluster
+      // barrier of the teardown, which the leader reaches only after this loop
+      const uint32_t first = it > static_cast<uint32_t>(STAGES) ? it - STAGES : 0u;
+      for (uint32_t j = first; j < it; ++j) ptx::mbar_wait_drain(full_bar(j % STAGES), (j / STAGES) & 1u);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       constexpr uint32_t idesc = (1u << 4) | (UmmaFmt<T>::v << 7) | (UmmaFmt<T>::v << 10) |
                                  (static_cast<uint32_t>(BLOCK_N >> 3) << 17) |
                                  (static_cast<uint32_t>((2 * BLOCK_M) >> 4) << 24);
-      uint32_t it = 0, tcount = 0;
+      uint32_t tcount = 0;
       bool ok = true;
+      int s = 0;
+      uint32_t ph = 0;
       for (int tile = pair; tile < num_tiles && ok; tile += npairs, ++tcount) {
         const int acc = tcount & 1u;
         const uint32_t aph = (tcount >> 1) & 1u;
         if (!ptx::mbar_wait_bounded(tempty_bar(acc), aph ^ 1u, abort_flag)) { ok = false; break; }
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BLOCK_N;
-        for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1u;
+        for (int kb = 0; kb < num_k_blocks; ++kb) {
           if (!ptx::mbar_wait_bounded(full_bar(s), ph, abort_flag)) { ok = false; break; }
           ptx::tc_fence_after();
           const uint64_t da = ptx::umma_desc_kmajor_sw128(a_smem(s));
           const uint64_t db = ptx::umma_desc_kmajor_sw128(b_smem(s));
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < BLOCK_K / UMMA_K; ++kk)
-            ptx::umma_bf16_ss_pair(d_tmem, da + 2 * kk, db + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
-          ptx::umma_commit_pair(empty_bar(s), 3);  // frees the slot in both CTAs
+            for (int kk = 0; kk < BLOCK_K / UMMA_K; ++kk)
+              ptx::umma_bf16_ss_pair(d_tmem, da + 2 * kk, db + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
+            ptx::umma_commit_pair(empty_bar(s), 3);  // frees the slot in both CTAs
+          }
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
-        if (ok) ptx::umma_commit_pair(tfull_bar(acc), 3);
+        if (ok && ptx::elect_one()) ptx::umma_commit_pair(tfull_bar(acc), 3);
       }
     }
   } else {
@@ -175,8 +200,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     const int row_in_tile = q * 32 + lane;
     uint32_t tcount = 0;
     for (int tile = pair; tile < num_tiles; tile += npairs, ++tcount) {
-      const int m_tile = tile % num_m_tiles;
-      const int n_tile = tile / num_m_tiles;
+      int m_tile, n_tile;
+      tile_coords(tile, num_m_tiles, num_n_tiles, m_tile, n_tile);
       const int acc = tcount & 1u;
       const uint32_t aph = (tcount >> 1) & 1u;
       // the tile's accumulator is complete when the leader's last commit lands; the ADD epilogue calls this AFTER it
