@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 from typing import Optional
 
 import torch
@@ -67,6 +68,13 @@ class LayerArgs(ctypes.Structure):
     ]
 
 
+# The same layout for struct.pack: one call fills the whole argument block (a store into a ctypes field costs about as much
+# as all of it).  Order: the 19 pointers and sizes up to stage_events, num_tokens, num_experts, the seven int32, the two
+# floats, bn_global_sums, bn_global_count, residual.  Null pointers are 0.
+LAYER_ARGS = struct.Struct("@19Q2q7i2fQqQ")
+assert LAYER_ARGS.size == ctypes.sizeof(LayerArgs)
+
+
 _P = ctypes.c_void_p
 _I = ctypes.c_int
 _L = ctypes.c_int64
@@ -107,6 +115,7 @@ SIGNATURES = {
 }
 
 _lib: Optional[ctypes.CDLL] = None
+_layer_forward = None
 
 
 def lib() -> ctypes.CDLL:
@@ -123,6 +132,10 @@ def lib() -> ctypes.CDLL:
             fn = getattr(handle, name)
             fn.restype = res
             fn.argtypes = args
+        global _layer_forward
+        _layer_forward = handle["fmoe_layer_forward"]  # an object of its own: takes the packed block as bytes
+        _layer_forward.restype = ctypes.c_int
+        _layer_forward.argtypes = [ctypes.c_char_p]
         _lib = handle
     return _lib
 
@@ -155,22 +168,54 @@ def require_cuda(*tensors: torch.Tensor) -> torch.device:
 
 
 def current_stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device_index(device))
+
+
+def device_index(device: torch.device) -> int:
+    return device.index if device.index is not None else torch.cuda.current_device()
 
 
 def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
+def call(name: str, device: torch.device, *args) -> int:
+    """Run a library function whose last argument is the stream on `device` and its current stream.  The CUDA device is
+    only switched when another one is current (a `torch.cuda.device` block costs several microseconds)."""
+    index = device_index(device)
+    fn = getattr(lib(), name)
+    if index == torch._C._cuda_getDevice():
+        return fn(*args, torch._C._cuda_getCurrentRawStream(index))
+    with torch.cuda.device(index):
+        return fn(*args, torch._C._cuda_getCurrentRawStream(index))
+
+
+def layer_forward(device: torch.device, args: bytes) -> int:
+    """fmoe_layer_forward on a block packed with LAYER_ARGS."""
+    fn = _layer_forward or lib() and _layer_forward
+    if device_index(device) == torch._C._cuda_getDevice():
+        return fn(args)
+    with torch.cuda.device(device):
+        return fn(args)
+
+
 # one int32 status word per device; kernels OR error bits into it
 _status = {}
+_status_ptr = {}
 
 
 def status_word(device: torch.device) -> torch.Tensor:
-    key = device.index if device.index is not None else torch.cuda.current_device()
-    if key not in _status:
-        _status[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _status[key]
+    key = device_index(device)
+    w = _status.get(key)
+    if w is None:
+        w = _status[key] = torch.zeros(1, dtype=torch.int32, device=device)
+        _status_ptr[key] = w.data_ptr()
+    return w
+
+
+def status_ptr(device: torch.device) -> int:
+    p = _status_ptr.get(device_index(device))
+    return p if p is not None else status_word(device).data_ptr()
 
 
 def read_status(device=None, clear: bool = True) -> int:

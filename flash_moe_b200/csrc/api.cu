@@ -25,6 +25,57 @@ int device_sm_count() {
   return cache[dev];
 }
 
+namespace {
+struct KernelNote {
+  const void* kern;
+  int dev, threads, smem, value;
+};
+struct KernelNotes {
+  static constexpr int kMax = 64;
+  KernelNote e[kMax];
+  int n = 0;
+  KernelNote* find(const void* kern, int dev, int threads, int smem) {
+    for (int i = 0; i < n; ++i)
+      if (e[i].kern == kern && e[i].dev == dev && e[i].threads == threads && e[i].smem == smem) return &e[i];
+    return nullptr;
+  }
+  void add(const KernelNote& k) {
+    if (n == kMax) n = 0;  // forget and start over: only the time of a query is lost
+    e[n++] = k;
+  }
+};
+}  // namespace
+
+cudaError_t allow_smem_impl(const void* kern, int bytes) {
+  if (bytes <= 48 * 1024) return cudaSuccess;
+  thread_local KernelNotes notes;
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  KernelNote* k = notes.find(kern, dev, 0, 0);
+  if (k != nullptr && k->value >= bytes) return cudaSuccess;
+  err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (err != cudaSuccess) return err;
+  if (k != nullptr) k->value = bytes;
+  else notes.add({kern, dev, 0, 0, bytes});
+  return cudaSuccess;
+}
+
+cudaError_t resident_ctas_impl(const void* kern, int threads, int smem, int* per_sm) {
+  thread_local KernelNotes notes;
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  const KernelNote* k = notes.find(kern, dev, threads, smem);
+  if (k != nullptr) {
+    *per_sm = k->value;
+    return cudaSuccess;
+  }
+  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, threads, static_cast<size_t>(smem));
+  if (err == cudaSuccess) notes.add({kern, dev, threads, smem, *per_sm});
+  return err;
+}
+
 // read on every launch (a getenv costs well under a microsecond), so a process can compare settings: FMOE_PDL is a
 // bit mask of kernel classes (see common.cuh) that are launched with programmatic stream serialisation
 bool pdl_enabled(int kernel_class) {

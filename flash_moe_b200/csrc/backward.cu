@@ -68,7 +68,7 @@ int router_bwd_typed(const void* dscores, const int64_t* idx, void* dlogp, int64
                      cudaStream_t stream) {
   const size_t smem = static_cast<size_t>(k) * 12;
   auto kern = router_bwd_kernel<T>;
-  if (smem > 48 * 1024) FMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  FMOE_CUDA_TRY(allow_smem(kern, static_cast<int>(smem)));
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * 16;
   const int grid = static_cast<int>(ntok < cap ? ntok : cap);
   kern<<<grid, 128, smem, stream>>>(static_cast<const T*>(dscores), idx, static_cast<T*>(dlogp), ntok, nk, k);

@@ -32,6 +32,17 @@ inline int next_pow2(int v) {
 
 int device_sm_count();  // cached per device (api.cu)
 
+// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) and the occupancy query cost a microsecond or more each, in front of
+// every launch: both remember what they did per host thread, device and kernel (api.cu).
+cudaError_t allow_smem_impl(const void* kern, int bytes);
+cudaError_t resident_ctas_impl(const void* kern, int threads, int smem, int* per_sm);
+template <typename K> inline cudaError_t allow_smem(K* kern, int bytes) {
+  return allow_smem_impl(reinterpret_cast<const void*>(kern), bytes);
+}
+template <typename K> inline cudaError_t resident_ctas(K* kern, int threads, int smem, int* per_sm) {
+  return resident_ctas_impl(reinterpret_cast<const void*>(kern), threads, smem, per_sm);
+}
+
 // ---- programmatic dependent launch ----------------------------------------------------------
 // The six kernels of a layer forward run back to back on one stream.  Launched with programmatic stream
 // serialisation, a kernel's CTAs may become resident, and run their set-up (barrier init, tensor-map prefetch, tensor

@@ -642,7 +642,7 @@ int run_scores(const void* rows, const void* table, const int64_t* idx, const vo
       const int xs_stride = ((H + 255) / 256) * 32;  // uint4 per warp, rows padded to 256 columns
       const int smem = 4 * 2 * xs_stride * 16;  // two x-row buffers per warp
       auto kern = expert_scores_mma_kernel<T, 4, false, 2>;
-      if (smem > 48 * 1024) FMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      FMOE_CUDA_TRY(allow_smem(kern, smem));
       FMOE_CUDA_TRY(launch_pdl(4, kern, dim3(grid), dim3(128), smem, stream, 1, static_cast<const T*>(rows),
                                static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, T_, H, N, k, xs_stride,
                                status, act, nullptr, 1, raw_out, 0));
@@ -958,7 +958,7 @@ int run_typed_peer(const void* x, const void* const* down_shards, const void* co
       const int xs_stride = ((H + 255) / 256) * 32;
       const int smem = 4 * 2 * xs_stride * 16;  // two x-row buffers per warp
       auto kern = expert_scores_mma_kernel<T, 4, true, 2>;
-      if (smem > 48 * 1024) FMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      FMOE_CUDA_TRY(allow_smem(kern, smem));
       kern<<<grid, 128, smem, stream>>>(static_cast<const T*>(x), static_cast<const T*>(hot_down), idx,
                                         static_cast<const T*>(gates), w.gs, T_, H, N + hot_rows, k, xs_stride, status,
                                         kActSilu, reinterpret_cast<const T* const*>(down_shards), world, nullptr, N);

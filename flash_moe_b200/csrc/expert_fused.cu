@@ -431,7 +431,7 @@ int launch_fused_nb(const void* x, const void* down, const void* up, const int64
                     float* raw_out, int64_t T_, int H, int64_t N, int k, int act, int32_t* status, cudaStream_t stream) {
   const FusedLayout L = fused_layout(H);
   auto kern = expert_fused_kernel<T, OutT, NB, NS>;
-  FMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total));
+  FMOE_CUDA_TRY(allow_smem(kern, L.total));
   const int sms = device_sm_count();
   const int grid = static_cast<int>(T_ < sms ? T_ : sms);
   kern<<<grid, kThreads, L.total, stream>>>(static_cast<const T*>(x), static_cast<const T*>(down),

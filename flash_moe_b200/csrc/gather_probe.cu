@@ -212,7 +212,7 @@ int launch_gather_probe(const void* table, int64_t num_rows, const int32_t* row_
     if (groups < 2) return FMOE_ERR_UNSUPPORTED;
     const int smem = groups * group_bytes + 2 * kRingMaxGroups * 8 + 64;
     if (mode == 1) {
-      FMOE_CUDA_TRY(cudaFuncSetAttribute(gather_probe_ring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      FMOE_CUDA_TRY(allow_smem(gather_probe_ring_kernel, smem));
       gather_probe_ring_kernel<<<device_sm_count(), 64, smem, stream>>>(static_cast<const uint8_t*>(table), num_rows,
                                                                         row_ids, count, row_bytes, groups, sink, status);
     } else {

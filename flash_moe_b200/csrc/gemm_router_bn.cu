@@ -273,7 +273,7 @@ int launch_bn_gemm(const void* x, const void* w, const float* mean, const float*
   constexpr int kStages = RingDepth<BLOCK_M, BLOCK_N>::v;
   const int smem = kStages * (BLOCK_M * BLOCK_K * 2 + BLOCK_N * BLOCK_K * 2) + (3 * kStages + 1) * 8 + 24 + num_k_blocks * BLOCK_K * 8 + 1024;
   auto kern = router_gemm_bn_kernel<BLOCK_M, BLOCK_N, T>;
-  FMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  FMOE_CUDA_TRY(allow_smem(kern, smem));
   const int num_m_tiles = static_cast<int>((M + BLOCK_M - 1) / BLOCK_M);
   const int num_n_tiles = (N + BLOCK_N - 1) / BLOCK_N;
   FMOE_CUDA_TRY(launch_pdl(1, kern, dim3(num_m_tiles * num_n_tiles), dim3(kThreads), smem, stream, 1, tA, tB, mean, invstd,

@@ -284,7 +284,7 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB0, const CUtensorMap& tB1
            int num_n_tiles, int K, int32_t* status, cudaStream_t stream) {
   using C = Cfg<BLOCK_N>;
   auto kern = gemm_tcgen05_kernel<BLOCK_N, EPI, T>;
-  FMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+  FMOE_CUDA_TRY(allow_smem(kern, C::SMEM_BYTES));
   const int num_m_tiles = static_cast<int>((M + BLOCK_M - 1) / BLOCK_M);
   const int num_k_blocks = (K + BLOCK_K - 1) / BLOCK_K;
   const int64_t tiles = static_cast<int64_t>(num_m_tiles) * num_n_tiles;

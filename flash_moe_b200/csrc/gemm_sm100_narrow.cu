@@ -436,7 +436,7 @@ int launch_plan(const NarrowPlan& p, const void* w0, const void* w1, const void*
   sh.early = early_weights ? 1 : 0;
   const int smem = p.stages * (NB * BLOCK_R * BLOCK_K * 2 + p.bn * BLOCK_K * 2) + sh.xchg_bytes + kBarBytes + 1024;
   auto kern = gemm_narrow_kernel<BLOCK_R, EPI, T>;
-  FMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
+  FMOE_CUDA_TRY(allow_smem(kern, kSmemLimit));
   FMOE_CUDA_TRY(launch_pdl(16, kern, dim3(p.split, (N + BLOCK_R - 1) / BLOCK_R, p.tiles_t), dim3(kThreads), smem, stream,
                            p.split, tW0, tW1, tX, tOut, ep, sh, status));
   return FMOE_OK;

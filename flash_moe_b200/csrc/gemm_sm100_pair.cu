@@ -308,7 +308,7 @@ template <int EPI, typename T>
 int launch_pair(const CUtensorMap& tA, const CUtensorMap& tB0, const CUtensorMap& tB1, const PairEpi& ep, int64_t M,
                 int num_n_tiles, int K, int32_t* status, cudaStream_t stream) {
   auto kern = gemm_tcgen05_pair_kernel<EPI, T>;
-  FMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  FMOE_CUDA_TRY(allow_smem(kern, SMEM_BYTES));
   const int num_m_tiles = static_cast<int>((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M));
   const int num_k_blocks = (K + BLOCK_K - 1) / BLOCK_K;
   const int64_t tiles = static_cast<int64_t>(num_m_tiles) * num_n_tiles;

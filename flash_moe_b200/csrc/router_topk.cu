@@ -800,9 +800,9 @@ int launch_reg_cpl(const void* logp, int64_t T_, int nk, int k, const RouterRegL
                    int64_t* indices, void* gates, int norm, cudaStream_t stream) {
   const int smem = L.cta_bytes + warps * L.warp_bytes;
   auto kern = router_topk_reg_kernel<T, E, CPL>;
-  FMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  FMOE_CUDA_TRY(allow_smem(kern, smem));
   int per_sm = 1;
-  FMOE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem));
+  FMOE_CUDA_TRY(resident_ctas(kern, warps * 32, smem, &per_sm));
   if (per_sm < 1) per_sm = 1;
   const int64_t want = (T_ + warps - 1) / warps;
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * per_sm;
@@ -867,9 +867,9 @@ int launch_smem(const void* logp, int64_t T_, int nk, int k, void* scores, int64
   if (L.cta_bytes + warps * L.warp_bytes > kMaxSmem) return FMOE_ERR_UNSUPPORTED;
   const int smem = L.cta_bytes + warps * L.warp_bytes;
   auto kern = router_topk_smem_kernel<T>;
-  FMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  FMOE_CUDA_TRY(allow_smem(kern, smem));
   int per_sm = 1;
-  FMOE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem));
+  FMOE_CUDA_TRY(resident_ctas(kern, warps * 32, smem, &per_sm));
   if (per_sm < 1) per_sm = 1;
   const int64_t want = (T_ + warps - 1) / warps;
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * per_sm;

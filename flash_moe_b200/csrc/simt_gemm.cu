@@ -163,7 +163,7 @@ int run_sgemm(const float* a, int64_t lda, const float* b0, const float* b1, con
               int64_t M, int N, int K, cudaStream_t stream, const float* residual) {
   using C = SgemmCfg<BM, BN, TM, TN, KG, STAGES, SWIGLU>;
   auto kern = sgemm_kernel<BM, BN, TM, TN, KG, STAGES, SWIGLU>;
-  if (C::SMEM > 48 * 1024) FMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+  FMOE_CUDA_TRY(allow_smem(kern, C::SMEM));
   kern<<<dim3((N + BN - 1) / BN, static_cast<unsigned>((M + BM - 1) / BM)), C::THREADS, C::SMEM, stream>>>(
       a, lda, b0, b1, addend, residual, out, ldo, static_cast<int>(M), N, K);
   FMOE_LAUNCH_CHECK();

@@ -19,6 +19,10 @@ import torch.nn.functional as F
 from .. import _lib
 
 
+# in the order of the argument block of the fused forward
+_WEIGHT_MODULES = ("gate_proj", "up_proj", "down_proj", "router_gate", "down_embed", "up_embed")
+
+
 class FlashMoEConfig:
     """Same six fields and defaults as the reference (flash_moe/modules/flash_moe.py:12-27)."""
 
@@ -95,6 +99,7 @@ class FlashMoE(nn.Module):
         self.overlap_shared_mlp = overlap_shared_mlp
         self._aux_streams: Dict[int, torch.cuda.Stream] = {}
         self._workspaces: Dict[int, torch.Tensor] = {}
+        self._workspace_sizes: Dict[Tuple[int, int], int] = {}
         self.last_indices: Optional[torch.Tensor] = None
         self.last_gates: Optional[torch.Tensor] = None
 
@@ -185,48 +190,59 @@ class FlashMoE(nn.Module):
         block.  The fused path adds it in the epilogue of the last GEMM, so ``residual + layer(x)`` is formed in
         float32 and rounded once; the differentiable path adds it as a separate autograd node.
         """
+        if not hidden_states.is_cuda:
+            _lib.require_cuda(hidden_states)
+        dev = hidden_states.device
         bsz, seq_len, _ = hidden_states.shape
-        dev = _lib.require_cuda(hidden_states)
         if torch.is_grad_enabled() and (hidden_states.requires_grad or any(p.requires_grad for p in self.parameters())):
             if bn_sync_group is not None or stage_timer is not None:
                 raise _lib.FmoeError("bn_sync_group and stage_timer belong to the fused path: call under torch.no_grad()")
             y, router_logits = self._forward_differentiable(hidden_states, return_routing)
             return (y if residual is None else residual + y), router_logits
-        x = hidden_states.reshape(-1, self.hidden_size)
-        if not x.is_contiguous():
-            x = x.contiguous()
+        x = hidden_states if hidden_states.is_contiguous() else hidden_states.contiguous()
         dtype = x.dtype
-        w = self.gate_proj.weight
+        # parameters and buffers straight from the submodules' dictionaries: nn.Module's attribute lookup is most of the
+        # host time of a small forward otherwise
+        mods = self._modules
+        try:
+            weights = [mods[n]._parameters["weight"] for n in _WEIGHT_MODULES]
+        except KeyError:  # parametrised or wrapped submodules compute their weight
+            weights = [getattr(self, n).weight for n in _WEIGHT_MODULES]
+        bn = mods["router_norm"]
+        running_mean, running_var = bn._buffers["running_mean"], bn._buffers["running_var"]
+        w = weights[0]
         if w.dtype != dtype or w.device != dev:
             raise _lib.FmoeError(f"module is {w.dtype} on {w.device}, input is {dtype} on {dev}")
-        T = x.shape[0]
+        T = bsz * seq_len
         H, I, N, nk, k = self.hidden_size, self.intermediate_size, self.num_experts, self.num_keys, self.top_k
+        if x.shape[2] != H:
+            raise _lib.FmoeError(f"the last dimension of hidden_states must be {H}")
         res = None
         if residual is not None:
             if residual.shape != hidden_states.shape or residual.dtype != dtype or residual.device != dev:
                 raise _lib.FmoeError("residual must match hidden_states in shape, dtype and device")
-            res = residual.reshape(-1, H)
-            if not res.is_contiguous():
-                res = res.contiguous()
-        bn = self.router_norm
-        training = bool(self.training) or bn.running_mean is None
+            res = residual.contiguous()
+        training = self.training or running_mean is None
+        momentum = bn.momentum
         if training and T == 1:
             # nn.BatchNorm1d refuses a one-row training batch (its variance is undefined); so does this layer
-            raise ValueError("Expected more than 1 value per channel when training, got input size " + str(list(x.shape)))
-        if bn.momentum is None:
+            raise ValueError("Expected more than 1 value per channel when training, got input size " + str([T, H]))
+        if momentum is None:
             # torch's cumulative moving average: the factor is 1 / (batches seen, this one included)
             seen = int(bn.num_batches_tracked.item()) if bn.num_batches_tracked is not None else 0
             momentum = 1.0 / float(seen + 1)
-        else:
-            momentum = float(bn.momentum)
 
-        y = torch.empty((T, H), device=dev, dtype=dtype)
-        logits = torch.empty((T, 2 * nk), device=dev, dtype=dtype)
+        y = torch.empty_like(x)
+        logits = torch.empty((T, 2, nk), device=dev, dtype=dtype)
         idx = torch.empty((T, k), device=dev, dtype=torch.int64) if return_routing else None
         gates = torch.empty((T, k), device=dev, dtype=dtype) if return_routing else None
-        L = _lib.lib()
         code = _lib.dtype_code(x)
-        ws_bytes = L.fmoe_layer_workspace_bytes(T, H, I, N, nk, k, code)
+        ws_bytes = self._workspace_sizes.get((T, code))
+        if ws_bytes is None:
+            ws_bytes = _lib.lib().fmoe_layer_workspace_bytes(T, H, I, N, nk, k, code)
+            if len(self._workspace_sizes) >= 256:  # callers with ever new token counts
+                self._workspace_sizes.clear()
+            self._workspace_sizes[(T, code)] = ws_bytes
         ws = self._workspace(dev, ws_bytes)
 
         bn_sums, bn_count = None, 0
@@ -234,59 +250,36 @@ class FlashMoE(nn.Module):
             import torch.distributed as dist
 
             bn_sums = torch.empty(2 * H, dtype=torch.float32, device=dev)
-            bws_bytes = L.fmoe_bn_batch_sums_workspace_bytes(H)
+            bws_bytes = _lib.lib().fmoe_bn_batch_sums_workspace_bytes(H)
             bws = torch.empty(bws_bytes, dtype=torch.uint8, device=dev)
-            with torch.cuda.device(dev):
-                _lib.check(L.fmoe_bn_batch_sums(x.data_ptr(), code, T, H, bn_sums.data_ptr(), bws.data_ptr(), bws_bytes,
-                                                _lib.current_stream_ptr(dev)), "fmoe_bn_batch_sums")
+            _lib.check(_lib.call("fmoe_bn_batch_sums", dev, x.data_ptr(), code, T, H, bn_sums.data_ptr(), bws.data_ptr(),
+                                 bws_bytes), "fmoe_bn_batch_sums")
             count = torch.tensor([float(T)], dtype=torch.float64, device=dev)
             dist.all_reduce(bn_sums, group=bn_sync_group)
             dist.all_reduce(count, group=bn_sync_group)
             bn_count = int(count.item())
 
-        with torch.cuda.device(dev):
-            main = torch.cuda.current_stream(dev)
-            aux = self._aux_stream(dev) if self.overlap_shared_mlp else None
-            a = _lib.LayerArgs()
-            a.x = x.data_ptr()
-            a.gate_proj = self.gate_proj.weight.data_ptr()
-            a.up_proj = self.up_proj.weight.data_ptr()
-            a.down_proj = self.down_proj.weight.data_ptr()
-            a.router_gate = self.router_gate.weight.data_ptr()
-            a.down_embed = self.down_embed.weight.data_ptr()
-            a.up_embed = self.up_embed.weight.data_ptr()
-            a.running_mean = _lib.ptr(bn.running_mean)
-            a.running_var = _lib.ptr(bn.running_var)
-            a.y = y.data_ptr()
-            a.router_logits = logits.data_ptr()
-            a.indices_out = _lib.ptr(idx)
-            a.gates_out = _lib.ptr(gates)
-            a.workspace = ws.data_ptr()
-            a.workspace_bytes = ws_bytes
-            a.status = _lib.status_word(dev).data_ptr()
-            a.stream = main.cuda_stream
-            a.aux_stream = aux.cuda_stream if aux is not None else None
-            a.stage_events = stage_timer.c_array() if stage_timer is not None else None
-            a.num_tokens, a.num_experts = T, N
-            a.hidden, a.intermediate, a.num_keys, a.top_k = H, I, nk, k
-            a.dtype = code
-            a.training = int(training)
-            a.norm_topk_prob = int(bool(self.norm_topk_prob))
-            a.bn_momentum = momentum
-            a.bn_eps = float(bn.eps)
-            a.bn_global_sums = _lib.ptr(bn_sums)
-            a.bn_global_count = bn_count
-            a.residual = _lib.ptr(res)
-            rc = L.fmoe_layer_forward(ctypes.byref(a))
-        _lib.check(rc, "fmoe_layer_forward")
+        events = 0
+        if stage_timer is not None:
+            with torch.cuda.device(dev):
+                events = ctypes.cast(stage_timer.c_array(), ctypes.c_void_p).value
+        rc = _lib.layer_forward(dev, _lib.LAYER_ARGS.pack(
+            x.data_ptr(), *[t.data_ptr() for t in weights],
+            0 if running_mean is None else running_mean.data_ptr(), 0 if running_var is None else running_var.data_ptr(),
+            y.data_ptr(), logits.data_ptr(), 0 if idx is None else idx.data_ptr(), 0 if gates is None else gates.data_ptr(),
+            ws.data_ptr(), ws_bytes, _lib.status_ptr(dev), _lib.current_stream_ptr(dev),
+            self._aux_stream(dev).cuda_stream if self.overlap_shared_mlp else 0, events,
+            T, N, H, I, nk, k, code, int(training), int(bool(self.norm_topk_prob)), momentum, bn.eps,
+            0 if bn_sums is None else bn_sums.data_ptr(), bn_count, 0 if res is None else res.data_ptr()))
+        if rc != 0:
+            _lib.check(rc, "fmoe_layer_forward")
         # The side stream is joined back into the calling stream inside the library call, so the
         # input, the outputs and the workspace need no cross-stream bookkeeping afterwards.
-        if training and bn.num_batches_tracked is not None and self.training:
+        if training and self.training and bn.num_batches_tracked is not None:
             bn.num_batches_tracked += 1
         if return_routing:
             self.last_indices, self.last_gates = idx, gates
-        router_logits = logits.view(T, 2, nk).transpose(0, 1)
-        return y.view(bsz, seq_len, H), router_logits
+        return y, logits.transpose(0, 1)
 
 
 class GraphedFlashMoE:

@@ -30,20 +30,14 @@ def _expert_forward(hidden_states, down_weights, up_weights, indices, routing_we
     ws_bytes = L.fmoe_expert_workspace_bytes(T, H, N, k)
     ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dev)
     saved = torch.empty((T, k), device=dev, dtype=torch.float32) if save_scores else None
-    with torch.cuda.device(dev):
-        if save_scores:
-            rc = L.fmoe_expert_forward_saving_scores(
-                x.data_ptr(), d.data_ptr(), u.data_ptr(), idx.data_ptr(), g.data_ptr(), out.data_ptr(), saved.data_ptr(),
-                _lib.dtype_code(x), _lib.DTYPE_CODE[out_dtype], T, H, N, k, ws.data_ptr(), ws_bytes,
-                _lib.status_word(dev).data_ptr(), _lib.current_stream_ptr(dev),
-            )
-        else:
-            rc = L.fmoe_expert_forward(
-                x.data_ptr(), d.data_ptr(), u.data_ptr(), idx.data_ptr(), g.data_ptr(), out.data_ptr(),
-                _lib.dtype_code(x), _lib.DTYPE_CODE[out_dtype], T, H, N, k, ws.data_ptr(), ws_bytes,
-                _lib.status_word(dev).data_ptr(), _lib.current_stream_ptr(dev),
-            )
-    _lib.check(rc, "fmoe_expert_forward")
+    tail = (_lib.dtype_code(x), _lib.DTYPE_CODE[out_dtype], T, H, N, k, ws.data_ptr(), ws_bytes, _lib.status_ptr(dev))
+    rows = (x.data_ptr(), d.data_ptr(), u.data_ptr(), idx.data_ptr(), g.data_ptr(), out.data_ptr())
+    if save_scores:
+        rc = _lib.call("fmoe_expert_forward_saving_scores", dev, *rows, saved.data_ptr(), *tail)
+    else:
+        rc = _lib.call("fmoe_expert_forward", dev, *rows, *tail)
+    if rc:
+        _lib.check(rc, "fmoe_expert_forward")
     return (out, saved) if save_scores else out
 
 
@@ -63,14 +57,11 @@ def _expert_backward(dout, hidden_states, down_weights, up_weights, indices, rou
     L = _lib.lib()
     ws_bytes = L.fmoe_expert_backward_workspace_bytes(T, H, N, k)
     ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
-        rc = L.fmoe_expert_backward(
-            do.data_ptr(), x.data_ptr(), d.data_ptr(), u.data_ptr(), idx.data_ptr(), g.data_ptr(),
-            _lib.ptr(saved_scores), dx.data_ptr(),
-            dd.data_ptr(), du.data_ptr(), dg.data_ptr(), _lib.dtype_code(x), T, H, N, k, ws.data_ptr(), ws_bytes,
-            _lib.status_word(dev).data_ptr(), _lib.current_stream_ptr(dev),
-        )
-    _lib.check(rc, "fmoe_expert_backward")
+    rc = _lib.call("fmoe_expert_backward", dev, do.data_ptr(), x.data_ptr(), d.data_ptr(), u.data_ptr(), idx.data_ptr(),
+                   g.data_ptr(), _lib.ptr(saved_scores), dx.data_ptr(), dd.data_ptr(), du.data_ptr(), dg.data_ptr(),
+                   _lib.dtype_code(x), T, H, N, k, ws.data_ptr(), ws_bytes, _lib.status_ptr(dev))
+    if rc:
+        _lib.check(rc, "fmoe_expert_backward")
     return dx, dd, du, dg
 
 
@@ -93,6 +84,8 @@ class FlashExpertFunc(torch.autograd.Function):
 
 def flash_expert_func(hidden_states, down_weights, up_weights, indices, routing_weights):
     """experts_states[T,H] = sum_j silu(<x, down[idx_j]>) * routing_weights_j * up[idx_j], in hidden_states.dtype."""
+    if not torch.is_grad_enabled():  # an autograd node costs several microseconds of host time
+        return _expert_forward(hidden_states, down_weights, up_weights, indices, routing_weights)
     return FlashExpertFunc.apply(hidden_states, down_weights, up_weights, indices, routing_weights)
 
 
@@ -113,10 +106,8 @@ def combine_partial_rows(rows, slot, num_tokens):
     if slot.shape[1] != num_tokens:
         raise _lib.FmoeError("slot must have one column per token")
     out = torch.empty((num_tokens, rows.shape[1]), device=dev, dtype=torch.float32)
-    with torch.cuda.device(dev):
-        rc = _lib.lib().fmoe_combine_partial_rows(
-            rows.data_ptr(), rows.shape[0], slot.data_ptr(), slot.shape[0], num_tokens, rows.shape[1], out.data_ptr(),
-            _lib.status_word(dev).data_ptr(), _lib.current_stream_ptr(dev))
+    rc = _lib.call("fmoe_combine_partial_rows", dev, rows.data_ptr(), rows.shape[0], slot.data_ptr(), slot.shape[0],
+                   num_tokens, rows.shape[1], out.data_ptr(), _lib.status_ptr(dev))
     _lib.check(rc, "fmoe_combine_partial_rows")
     return out
 

@@ -32,21 +32,16 @@ def _mlp_forward(x, gate_weight, up_weight, down_weight, addend=None, save_preac
         # the fused gate/up GEMM can also store the two pre-activations (its CTA-pair form only)
         a = torch.empty((T, I), device=dev, dtype=x2.dtype)
         b = torch.empty((T, I), device=dev, dtype=x2.dtype)
-        with torch.cuda.device(dev):
-            rc = L.fmoe_mlp_forward_saving_preacts(
-                x2.data_ptr(), wg.data_ptr(), wu.data_ptr(), wd.data_ptr(), out.data_ptr(), a.data_ptr(), b.data_ptr(), code,
-                T, H, I, ws.data_ptr(), ws_bytes, _lib.status_word(dev).data_ptr(), _lib.current_stream_ptr(dev),
-            )
+        rc = _lib.call("fmoe_mlp_forward_saving_preacts", dev, x2.data_ptr(), wg.data_ptr(), wu.data_ptr(), wd.data_ptr(),
+                       out.data_ptr(), a.data_ptr(), b.data_ptr(), code, T, H, I, ws.data_ptr(), ws_bytes, _lib.status_ptr(dev))
         if rc == 0:
             return out.view(*lead, H), a, b
         if rc != _lib.ERR_UNSUPPORTED:
             _lib.check(rc, "fmoe_mlp_forward_saving_preacts")
-    with torch.cuda.device(dev):
-        rc = L.fmoe_mlp_forward(
-            x2.data_ptr(), wg.data_ptr(), wu.data_ptr(), wd.data_ptr(), _lib.ptr(addend), out.data_ptr(), code, T, H, I,
-            ws.data_ptr(), ws_bytes, _lib.status_word(dev).data_ptr(), _lib.current_stream_ptr(dev),
-        )
-    _lib.check(rc, "fmoe_mlp_forward")
+    rc = _lib.call("fmoe_mlp_forward", dev, x2.data_ptr(), wg.data_ptr(), wu.data_ptr(), wd.data_ptr(), _lib.ptr(addend),
+                   out.data_ptr(), code, T, H, I, ws.data_ptr(), ws_bytes, _lib.status_ptr(dev))
+    if rc:
+        _lib.check(rc, "fmoe_mlp_forward")
     return (out.view(*lead, H), None, None) if save_preacts else out.view(*lead, H)
 
 
@@ -58,9 +53,8 @@ def swiglu_backward(dh, a, b, want_h=False):
         raise _lib.FmoeError("dh, a and b must share shape and dtype")
     da, db = torch.empty_like(a), torch.empty_like(b)
     h = torch.empty_like(a) if want_h else None
-    with torch.cuda.device(dev):
-        rc = _lib.lib().fmoe_swiglu_backward(dh.data_ptr(), a.data_ptr(), b.data_ptr(), da.data_ptr(), db.data_ptr(),
-                                             _lib.ptr(h), _lib.dtype_code(a), a.numel(), _lib.current_stream_ptr(dev))
+    rc = _lib.call("fmoe_swiglu_backward", dev, dh.data_ptr(), a.data_ptr(), b.data_ptr(), da.data_ptr(), db.data_ptr(),
+                   _lib.ptr(h), _lib.dtype_code(a), a.numel())
     _lib.check(rc, "fmoe_swiglu_backward")
     return (da, db, h) if want_h else (da, db)
 
@@ -106,6 +100,8 @@ class FlashMLPFunc(torch.autograd.Function):
 
 def flash_mlp_func(x, gate_weight, up_weight, down_weight):
     """(silu(x Wg^T) * (x Wu^T)) Wd^T with the activation fused into the first GEMM's epilogue."""
+    if not torch.is_grad_enabled():  # an autograd node costs several microseconds of host time
+        return _mlp_forward(x, gate_weight, up_weight, down_weight)
     return FlashMLPFunc.apply(x, gate_weight, up_weight, down_weight)
 
 

@@ -26,12 +26,10 @@ def _router_forward(router_logits: torch.Tensor, num_expert_keys: int, num_exper
     scores = torch.empty((T, num_experts_per_tok), device=dev, dtype=lp.dtype)
     indices = torch.empty((T, num_experts_per_tok), device=dev, dtype=torch.int64)
     gates = torch.empty_like(scores) if want_gates else None
-    with torch.cuda.device(dev):
-        rc = _lib.lib().fmoe_router_topk(
-            lp.data_ptr(), _lib.dtype_code(lp), T, num_expert_keys, num_experts_per_tok, scores.data_ptr(),
-            indices.data_ptr(), _lib.ptr(gates), int(bool(norm_topk_prob)), _lib.current_stream_ptr(dev),
-        )
-    _lib.check(rc, "fmoe_router_topk")
+    rc = _lib.call("fmoe_router_topk", dev, lp.data_ptr(), _lib.dtype_code(lp), T, num_expert_keys, num_experts_per_tok,
+                   scores.data_ptr(), indices.data_ptr(), _lib.ptr(gates), int(bool(norm_topk_prob)))
+    if rc:
+        _lib.check(rc, "fmoe_router_topk")
     return (scores, indices, gates) if want_gates else (scores, indices)
 
 
@@ -41,9 +39,8 @@ def _router_backward(dscores, indices, num_expert_keys):
     ds, idx = contiguous(dscores), contiguous(indices)
     T, k = ds.shape
     out = torch.empty((2, T, num_expert_keys), device=dev, dtype=ds.dtype)
-    with torch.cuda.device(dev):
-        rc = _lib.lib().fmoe_router_topk_backward(ds.data_ptr(), idx.data_ptr(), _lib.dtype_code(ds), T, num_expert_keys, k,
-                                                  out.data_ptr(), _lib.current_stream_ptr(dev))
+    rc = _lib.call("fmoe_router_topk_backward", dev, ds.data_ptr(), idx.data_ptr(), _lib.dtype_code(ds), T, num_expert_keys,
+                   k, out.data_ptr())
     _lib.check(rc, "fmoe_router_topk_backward")
     return out
 
@@ -69,6 +66,8 @@ class FlashRouterFunc(torch.autograd.Function):
 
 def flash_router_func(router_logits, num_expert_keys, num_experts_per_tok):
     """(scores[T,k] in the input dtype, indices[T,k] int64) for log-probs ``router_logits[2,T,nk]``."""
+    if not torch.is_grad_enabled():  # an autograd node costs several microseconds of host time
+        return _router_forward(router_logits, num_expert_keys, num_experts_per_tok)
     return FlashRouterFunc.apply(router_logits, num_expert_keys, num_experts_per_tok)
 
 

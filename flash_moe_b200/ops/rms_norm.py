@@ -20,8 +20,6 @@ def rms_norm(x: torch.Tensor, weight: Optional[torch.Tensor] = None, eps: float 
     w = None if weight is None else contiguous(weight)
     out = torch.empty_like(xc)
     rows = xc.numel() // H if H else 0
-    with torch.cuda.device(dev):
-        rc = _lib.lib().fmoe_rms_norm(xc.data_ptr(), _lib.ptr(w), out.data_ptr(), _lib.dtype_code(xc), rows, H, float(eps),
-                                      _lib.current_stream_ptr(dev))
+    rc = _lib.call("fmoe_rms_norm", dev, xc.data_ptr(), _lib.ptr(w), out.data_ptr(), _lib.dtype_code(xc), rows, H, float(eps))
     _lib.check(rc, "fmoe_rms_norm")
     return out
