@@ -4,16 +4,14 @@
 // the arithmetic and the rounding of the stand-alone normalisation pass (xn = T((x - mean) * inv_std), float32
 // inside), so the logits are bit-equal to normalise-then-GEMM while x is read once and xn never exists in memory.
 //
-// One 128 x BLOCK_N tile per CTA, 320 threads:
-//   warp 0 (one lane)  TMA producer: raw 128 x 64 x tile + BLOCK_N x 64 weight tile per stage, 128-byte swizzle;
-//   warps 2..9         normalise the x tile in place (each thread owns 16-byte pieces of fixed features), make the
+// One BLOCK_M x BLOCK_N tile per CTA, 576 threads:
+//   warp 0             TMA producer: raw BLOCK_M x 64 x tile + BLOCK_N x 64 weight tile per stage, 128-byte swizzle;
+//   warps 2..17        normalise the x tile in place (each thread owns 16-byte pieces of fixed features), make the
 //                      writes visible to the tensor core (fence.proxy.async) and arrive on the stage's `ready`;
-//   warp 1 (one lane)  waits for `ready`, issues tcgen05.mma into TMEM, frees the stage with tcgen05.commit;
+//   warp 1             waits for `ready`, issues tcgen05.mma into TMEM, frees the stage with tcgen05.commit;
 //   warps 2..5         epilogue: tcgen05.ld the accumulator (one row per thread), round, store.
 // Columns of x beyond K arrive as zeros from TMA and are normalised with mean 0 / scale 0, so they stay zero.
 // Every wait is bounded; a wait that runs out raises FMOE_STATUS_WAIT_TIMEOUT and the CTA drains and leaves.
-#include <cstdlib>
-
 #include "gemm_epilogue.cuh"
 
 namespace fmoe {
@@ -21,19 +19,22 @@ namespace {
 
 constexpr int BLOCK_K = 64;
 constexpr int UMMA_K = 16;
-constexpr int kXformWarps = 8;
+constexpr int kXformGroups = 4;
+constexpr int kXformWarps = 4 * kXformGroups;
 constexpr int kThreads = (2 + kXformWarps) * 32;
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
 using epi::UmmaFmt;
 
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// ring depth: 8 stages of up to 24 KB, 6 x 32 KB for 128 x 128 tiles, 4 x 48 KB for 256-column tiles
+template <int BLOCK_M, int BLOCK_N> struct RingDepth {
+  static constexpr int v = BLOCK_M == 64 ? 8 : BLOCK_N <= 128 ? 6 : 4;
+};
 
-// ring depth: 6 x 24 KB or 6 x 32 KB stages for 128-column tiles, 4 x 48 KB for 256-column tiles.  Deeper does not
-// help (8 stages measured the same): timestamps taken inside the kernel show the tiles landed and normalised well ahead
-// of the MMA thread, which needs about 700 cycles per k-block (four tcgen05.mma of K = 16 and a commit) whether the
-// tile has 64 or 128 rows - the issue pace of the MMAs, not the operand feed, sets the length of the main loop here.
-template <int BLOCK_M, int BLOCK_N> struct RingDepth { static constexpr int v = BLOCK_N <= 128 ? 6 : 4; };
+// kEarlyTrigger: the next kernel may become resident at once (grids that leave most of the chip idle).  kLateWait: the
+// kernel before this one in the stream works on other data and has itself waited for everything this one reads, so this
+// one runs beside it and waits for it only before it ends (completion stays transitive along the stream).
+enum { kEarlyTrigger = 1, kLateWait = 2 };
 
 // BLOCK_M = 128, or 64 for small problems (twice the CTAs, half the x tile to fetch and normalise per CTA).  With
 // M = 64 the accumulator's row i sits in TMEM lane 32 * (i / 16) + i % 16: each of the four epilogue warps finds 16
@@ -43,7 +44,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const float* __restrict__ mean, const float* __restrict__ invstd,
                       const T* __restrict__ running_mean, const T* __restrict__ running_var, float eps, T* __restrict__ out,
-                      int M, int N, int K, int num_m_tiles, int num_k_blocks, int32_t* status) {
+                      int M, int N, int K, int num_m_tiles, int num_k_blocks, int flags, int32_t* status) {
   constexpr int A_BYTES = BLOCK_M * BLOCK_K * 2;
   constexpr int B_BYTES = BLOCK_N * BLOCK_K * 2;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -69,104 +70,106 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const int m_tile = blockIdx.x % num_m_tiles;
   const int n_tile = blockIdx.x / num_m_tiles;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      ptx::mbar_init(full_bar(s), 1);
-      ptx::mbar_init(ready_bar(s), kXformWarps / 2);  // one group of four warps normalises a k-block
-      ptx::mbar_init(empty_bar(s), 1);
-    }
-    ptx::mbar_init(tfull_bar, 1);
-    *abort_flag = 0;
-    ptx::mbar_fence_init();
-    ptx::prefetch_tensormap(&tmA);
-    ptx::prefetch_tensormap(&tmB);
-  }
-  if (warp == 1) {
-    ptx::tmem_alloc(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), BLOCK_N);
-    ptx::tmem_relinquish();
-  }
-  // everything above is independent of earlier kernels; from here on global memory is read
-  pdl_wait();
-  // the first ring of operand tiles is requested before the statistics are fetched, so that the two cold reads overlap
-  int kb_issued = 0;
-  if (threadIdx.x == 0) {
-    for (; kb_issued < kStages && kb_issued < num_k_blocks; ++kb_issued) {
-      ptx::mbar_arrive_expect_tx(full_bar(kb_issued), STAGE_BYTES);
-      ptx::tma_load_2d(a_smem(kb_issued), &tmA, full_bar(kb_issued), kb_issued * BLOCK_K, m_tile * BLOCK_M);
-      ptx::tma_load_2d(b_smem(kb_issued), &tmB, full_bar(kb_issued), kb_issued * BLOCK_K, n_tile * BLOCK_N);
-    }
-  }
-  // statistics: eval mode straight from the running buffers, training mode from the finalised batch statistics.
-  // One thread fetches the eight features 8 p .. 8 p + 7 of a k-block with vector loads (all of a thread's loads are in
-  // flight together: the buffers are cold, and fetching them one feature at a time took four DRAM round trips), and
-  // writes them as four 16-byte entries: within a k-block the pairs (i, i + 1) of those eight features sit at
-  // [i / 2][p], so the eight 16-byte reads a warp makes for one i cover 128 consecutive bytes instead of one bank group.
-  const bool vec_stats = (running_mean != nullptr)
-                             ? (sizeof(T) == 2 && ((reinterpret_cast<uintptr_t>(running_mean) | reinterpret_cast<uintptr_t>(running_var)) & 15u) == 0)
-                             : (((reinterpret_cast<uintptr_t>(mean) | reinterpret_cast<uintptr_t>(invstd)) & 15u) == 0);
-  for (int ch = threadIdx.x; ch < num_k_blocks * (BLOCK_K / 8); ch += kThreads) {
-    const int c0 = ch * 8;
-    float m[8], sd[8];
-    if (vec_stats && c0 + 8 <= K) {
-      if (running_mean != nullptr) {
-        float v[8];
-        unpack16<T>(ldg16(running_mean + c0), m);
-        unpack16<T>(ldg16(running_var + c0), v);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) sd[i] = 1.0f / sqrtf(v[i] + eps);
-      } else {
-        const float4 m0 = *reinterpret_cast<const float4*>(mean + c0), m1 = *reinterpret_cast<const float4*>(mean + c0 + 4);
-        const float4 s0 = *reinterpret_cast<const float4*>(invstd + c0), s1 = *reinterpret_cast<const float4*>(invstd + c0 + 4);
-        m[0] = m0.x; m[1] = m0.y; m[2] = m0.z; m[3] = m0.w; m[4] = m1.x; m[5] = m1.y; m[6] = m1.z; m[7] = m1.w;
-        sd[0] = s0.x; sd[1] = s0.y; sd[2] = s0.z; sd[3] = s0.w; sd[4] = s1.x; sd[5] = s1.y; sd[6] = s1.z; sd[7] = s1.w;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int c = c0 + i;
-        m[i] = 0.f;
-        sd[i] = 0.f;
-        if (c < K) {
-          if (running_mean != nullptr) {
-            m[i] = to_f32<T>(running_mean[c]);
-            sd[i] = 1.0f / sqrtf(to_f32<T>(running_var[c]) + eps);
-          } else {
-            m[i] = mean[c];
-            sd[i] = invstd[c];
-          }
-        }
-      }
-    }
-    const int kb0 = (c0 / BLOCK_K) * BLOCK_K, pp = (c0 % BLOCK_K) >> 3;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      *reinterpret_cast<float4*>(&stats[kb0 + j * 16 + pp * 2]) = make_float4(m[2 * j], sd[2 * j], m[2 * j + 1], sd[2 * j + 1]);
-  }
-  ptx::tc_fence_before();
-  __syncthreads();
-  ptx::tc_fence_after();
-  const uint32_t tmem_base = __shfl_sync(kFull, *tmem_slot, 0);
-
   if (warp == 0) {
+    if (ptx::elect_one()) {
+      for (int s = 0; s < kStages; ++s) {
+        ptx::mbar_init(full_bar(s), 1);
+        ptx::mbar_init(ready_bar(s), kXformWarps / kXformGroups);  // one group of four warps normalises a k-block
+        ptx::mbar_init(empty_bar(s), 1);
+      }
+      ptx::mbar_init(tfull_bar, 1);
+      *abort_flag = 0;
+      ptx::mbar_fence_init();
+    }
+    __syncwarp();
+    asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");  // the others may use the barriers; no wait here
+    if (ptx::elect_one()) {
+      ptx::prefetch_tensormap(&tmA);
+      ptx::prefetch_tensormap(&tmB);
+    }
+    if ((flags & kLateWait) == 0) pdl_wait();
+    if (flags & kEarlyTrigger) pdl_launch_dependents();
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int kb = kb_issued;
-      bool ok = true;
-      for (; kb < num_k_blocks; ++kb) {
-        const int s = kb % kStages;
-        const uint32_t ph = (kb / kStages) & 1u;
-        if (!ptx::mbar_wait_bounded(empty_bar(s), ph ^ 1u, abort_flag)) { ok = false; break; }
+    bool ok = true;
+    int s = 0, kb = 0;
+    uint32_t ph = 1;
+    for (; kb < num_k_blocks; ++kb) {
+      if (!ptx::mbar_wait_bounded(empty_bar(s), ph, abort_flag)) { ok = false; break; }
+      if (ptx::elect_one()) {
         ptx::mbar_arrive_expect_tx(full_bar(s), STAGE_BYTES);
         ptx::tma_load_2d(a_smem(s), &tmA, full_bar(s), kb * BLOCK_K, m_tile * BLOCK_M);
         ptx::tma_load_2d(b_smem(s), &tmB, full_bar(s), kb * BLOCK_K, n_tile * BLOCK_N);
       }
-      if (!ok) {  // let the copies already issued land before the CTA goes away (bounded)
-        const int first = kb > kStages ? kb - kStages : 0;
-        for (int j = first; j < kb; ++j)
-          ptx::mbar_wait_drain(full_bar(j % kStages), (j / kStages) & 1u);
+      if (++s == kStages) {
+        s = 0;
+        ph ^= 1u;
       }
     }
-  } else if (warp == 1) {
+    if (!ok) {  // let the copies already issued land before the CTA goes away (bounded)
+      const int first = kb > kStages ? kb - kStages : 0;
+      for (int j = first; j < kb; ++j) ptx::mbar_wait_drain(full_bar(j % kStages), (j / kStages) & 1u);
+    }
+  } else {
+    if (warp == 1) {
+      ptx::tmem_alloc(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), BLOCK_N);
+      ptx::tmem_relinquish();
+    }
+    // everything above is independent of earlier kernels; from here on global memory is read
+    if ((flags & kLateWait) == 0) pdl_wait();
+    if (flags & kEarlyTrigger) pdl_launch_dependents();
+    // statistics: eval mode straight from the running buffers, training mode from the finalised batch statistics.
+    // One thread fetches the eight features 8 p .. 8 p + 7 of a k-block with vector loads (all of a thread's loads are in
+    // flight together: the buffers are cold, and fetching them one feature at a time took four DRAM round trips), and
+    // writes them as four 16-byte entries: within a k-block the pairs (i, i + 1) of those eight features sit at
+    // [i / 2][p], so the eight 16-byte reads a warp makes for one i cover 128 consecutive bytes instead of one bank group.
+    const bool vec_stats = (running_mean != nullptr)
+                               ? (sizeof(T) == 2 && ((reinterpret_cast<uintptr_t>(running_mean) | reinterpret_cast<uintptr_t>(running_var)) & 15u) == 0)
+                               : (((reinterpret_cast<uintptr_t>(mean) | reinterpret_cast<uintptr_t>(invstd)) & 15u) == 0);
+    for (int ch = threadIdx.x - 64; ch >= 0 && ch < num_k_blocks * (BLOCK_K / 8); ch += kXformWarps * 32) {
+      const int c0 = ch * 8;
+      float m[8], sd[8];
+      if (vec_stats && c0 + 8 <= K) {
+        if (running_mean != nullptr) {
+          float v[8];
+          unpack16<T>(ldg16(running_mean + c0), m);
+          unpack16<T>(ldg16(running_var + c0), v);
+  #pragma unroll
+          for (int i = 0; i < 8; ++i) sd[i] = 1.0f / sqrtf(v[i] + eps);
+        } else {
+          const float4 m0 = *reinterpret_cast<const float4*>(mean + c0), m1 = *reinterpret_cast<const float4*>(mean + c0 + 4);
+          const float4 s0 = *reinterpret_cast<const float4*>(invstd + c0), s1 = *reinterpret_cast<const float4*>(invstd + c0 + 4);
+          m[0] = m0.x; m[1] = m0.y; m[2] = m0.z; m[3] = m0.w; m[4] = m1.x; m[5] = m1.y; m[6] = m1.z; m[7] = m1.w;
+          sd[0] = s0.x; sd[1] = s0.y; sd[2] = s0.z; sd[3] = s0.w; sd[4] = s1.x; sd[5] = s1.y; sd[6] = s1.z; sd[7] = s1.w;
+        }
+      } else {
+  #pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int c = c0 + i;
+          m[i] = 0.f;
+          sd[i] = 0.f;
+          if (c < K) {
+            if (running_mean != nullptr) {
+              m[i] = to_f32<T>(running_mean[c]);
+              sd[i] = 1.0f / sqrtf(to_f32<T>(running_var[c]) + eps);
+            } else {
+              m[i] = mean[c];
+              sd[i] = invstd[c];
+            }
+          }
+        }
+      }
+      const int kb0 = (c0 / BLOCK_K) * BLOCK_K, pp = (c0 % BLOCK_K) >> 3;
+  #pragma unroll
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float4*>(&stats[kb0 + j * 16 + pp * 2]) = make_float4(m[2 * j], sd[2 * j], m[2 * j + 1], sd[2 * j + 1]);
+    }
+    ptx::tc_fence_before();
+    asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+    ptx::tc_fence_after();
+  }
+  const uint32_t tmem_base = warp == 0 ? 0u : __shfl_sync(kFull, *tmem_slot, 0);
+
+  if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (whole-warp loop, see ptx::elect_one)
     constexpr uint32_t idesc = (1u << 4) | (UmmaFmt<T>::v << 7) | (UmmaFmt<T>::v << 10) |
                                (static_cast<uint32_t>(BLOCK_N >> 3) << 17) |
@@ -191,21 +194,21 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
     }
     if (ok && ptx::elect_one()) ptx::umma_commit(tfull_bar);
-  } else {
-    // ------------------------------------------------------------ normalise the x tiles (warps 2..9)
-    // Two groups of four warps take alternate k-blocks, so that two tiles are being normalised at any time (one
-    // group's load -> arithmetic -> store -> proxy fence -> arrive chain took about 600 cycles per k-block and was the
-    // pace of the whole kernel).  Thread i of a group owns the 16-byte pieces i, i + 128, ... of the BLOCK_M x
-    // 128-byte tile: row (i >> 3) + 16 j, position i & 7.  With the 128-byte swizzle position p of row r holds the
+  } else if (warp >= 2) {
+    // ------------------------------------------------------------ normalise the x tiles (warps 2..17)
+    // Four groups of four warps take the k-blocks in turn, so that four tiles are being normalised at any time: one
+    // group's load -> arithmetic -> store -> proxy fence -> arrive chain takes about 1200 cycles, and with the MMAs
+    // issued from a uniform loop it is the pace of the whole kernel.  Thread i of a group owns the 16-byte
+    // pieces i, i + 128, ... of the BLOCK_M x 128-byte tile: row (i >> 3) + 16 j, position i & 7.  With the 128-byte swizzle position p of row r holds the
     // features 8 * (p ^ (r & 7)) .. + 7 of the k-block, and r & 7 does not depend on j, so one thread always handles the
     // same eight features.
-    constexpr int kGroupThreads = (kXformWarps / 2) * 32;
+    constexpr int kGroupThreads = (kXformWarps / kXformGroups) * 32;
     constexpr int kGroupPieces = BLOCK_M * 8 / kGroupThreads;
-    const int group = (warp - 2) / (kXformWarps / 2);
+    const int group = (warp - 2) / (kXformWarps / kXformGroups);
     const int xt = threadIdx.x - 64 - group * kGroupThreads;
     const int feat0 = 8 * ((xt & 7) ^ ((xt >> 3) & 7));
     bool ok = true;
-    for (int kb = group; kb < num_k_blocks; kb += 2) {
+    for (int kb = group; kb < num_k_blocks; kb += kXformGroups) {
       const int s = kb % kStages;
       float mm[8], ss[8];
 #pragma unroll
@@ -226,7 +229,7 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         for (int i = 0; i < 8; ++i) f[i] = (f[i] - mm[i]) * ss[i];
         tile[xt + kGroupThreads * j] = pack16<T>(f);
       }
-      fence_async_smem();
+      ptx::fence_async_smem();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(ready_bar(s));
     }
@@ -255,6 +258,7 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, BLOCK_N);
   }
+  if (flags & kLateWait) pdl_wait();
   if (threadIdx.x == 0 && *abort_flag != 0 && status != nullptr) atomicOr(status, FMOE_STATUS_WAIT_TIMEOUT);
 }
 
@@ -264,7 +268,8 @@ int make_map(CUtensorMap* m, const void* basep, int dtype, uint64_t cols, uint64
 
 template <int BLOCK_M, int BLOCK_N, typename T>
 int launch_bn_gemm(const void* x, const void* w, const float* mean, const float* invstd, const void* rm, const void* rv,
-                   float eps, void* out, int dtype, int64_t M, int N, int K, int32_t* status, cudaStream_t stream) {
+                   float eps, void* out, int dtype, int64_t M, int N, int K, int flags, int32_t* status,
+                   cudaStream_t stream) {
   CUtensorMap tA, tB;
   int rc;
   if ((rc = make_map(&tA, x, dtype, K, M, BLOCK_M)) != FMOE_OK) return rc;
@@ -278,7 +283,7 @@ int launch_bn_gemm(const void* x, const void* w, const float* mean, const float*
   const int num_n_tiles = (N + BLOCK_N - 1) / BLOCK_N;
   FMOE_CUDA_TRY(launch_pdl(1, kern, dim3(num_m_tiles * num_n_tiles), dim3(kThreads), smem, stream, 1, tA, tB, mean, invstd,
                            static_cast<const T*>(rm), static_cast<const T*>(rv), eps, static_cast<T*>(out),
-                           static_cast<int>(M), N, K, num_m_tiles, num_k_blocks, status));
+                           static_cast<int>(M), N, K, num_m_tiles, num_k_blocks, flags, status));
   return FMOE_OK;
 }
 
@@ -293,7 +298,7 @@ bool router_bn_gemm_supported(int dtype, int64_t M, int N, int K) {
 // Statistics: running_mean / running_var (module dtype, eval mode) when non-null, else mean / invstd (float32 [K]).
 int launch_router_bn_gemm(const void* x, const void* w, const float* mean, const float* invstd,
                           const void* running_mean, const void* running_var, float eps, void* logits, int dtype,
-                          int64_t M, int N, int K, int32_t* status, cudaStream_t stream) {
+                          int64_t M, int N, int K, bool beside_predecessor, int32_t* status, cudaStream_t stream) {
   if (!router_bn_gemm_supported(dtype, M, N, K)) return FMOE_ERR_UNSUPPORTED;
   if (x == nullptr || w == nullptr || logits == nullptr) return FMOE_ERR_BAD_ARG;
   if ((running_mean == nullptr) != (running_var == nullptr)) return FMOE_ERR_BAD_ARG;
@@ -303,16 +308,23 @@ int launch_router_bn_gemm(const void* x, const void* w, const float* mean, const
   const int64_t m_tiles = (M + 127) / 128;
   const int64_t tiles128 = m_tiles * ((N + 127) / 128);
   const bool wide = N > 128 && tiles128 >= 4 * static_cast<int64_t>(device_sm_count());
-  // fewer 128 x 128 tiles than SMs: 64-row tiles put twice as many CTAs to work, each with half the x tile
-  bool small = tiles128 < device_sm_count();
-  if (const char* e = std::getenv("FMOE_BN_TILE")) small = e[0] == '6';  // measurement aid: 64 or 128 rows
+  // fewer 128 x 128 tiles than SMs: 64-row tiles put twice as many CTAs to work, each with half the x tile, and
+  // narrower ones more still while they fit one wave (a CTA pulls its operands at about 62 bytes per clock: at 64 tokens x
+  // 2048 columns, 512 outputs, 16 CTAs of 32 columns instead of 4 of 128)
+  const bool small = tiles128 < device_sm_count();
+  const int64_t m64 = (M + 63) / 64;
+  const int bn64 = m64 * ((N + 31) / 32) <= device_sm_count() ? 32 : m64 * ((N + 63) / 64) <= device_sm_count() ? 64 : 128;
+  const int flags = (small && m64 * ((N + bn64 - 1) / bn64) * 2 <= device_sm_count() ? kEarlyTrigger : 0) |
+                    (beside_predecessor ? kLateWait : 0);
 #define FMOE_BN_GEMM(BM_, BN_)                                                                                       \
   (dtype == FMOE_DTYPE_BF16                                                                                          \
        ? launch_bn_gemm<BM_, BN_, __nv_bfloat16>(x, w, mean, invstd, running_mean, running_var, eps, logits, dtype, M, N, \
-                                                 K, status, stream)                                                  \
+                                                 K, flags, status, stream)                                                  \
        : launch_bn_gemm<BM_, BN_, __half>(x, w, mean, invstd, running_mean, running_var, eps, logits, dtype, M, N, K, \
-                                          status, stream))
+                                          flags, status, stream))
   if (wide) return FMOE_BN_GEMM(128, 256);
+  if (small && bn64 == 32) return FMOE_BN_GEMM(64, 32);
+  if (small && bn64 == 64) return FMOE_BN_GEMM(64, 64);
   if (small) return FMOE_BN_GEMM(64, 128);
   return FMOE_BN_GEMM(128, 128);
 #undef FMOE_BN_GEMM
