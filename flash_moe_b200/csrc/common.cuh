@@ -60,6 +60,18 @@ constexpr int kPdlDefaultMask = 27;
 bool pdl_enabled(int kernel_class);  // api.cu; classes: 1 router GEMM, 2 top-k, 4 scores, 8 accumulate, 16 MLP GEMMs
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Loads of what the predecessor writes, for kernels that do work of their own before pdl_wait(): the compiler may move an
+// ordinary load through a const __restrict__ pointer (or __ldg) in front of the wait, it does not reorder these.
+__device__ __forceinline__ float ld_after_wait(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint16_t ld_after_wait(const uint16_t* p) {
+  uint16_t v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+  return v;
+}
 
 // cudaLaunchKernelEx with the programmatic-serialisation attribute (plus a cluster width when cluster_x > 1)
 template <typename... KArgs, typename... Args>
@@ -212,7 +224,8 @@ bool gemm_router_fused_supported(int nk);
 bool router_bn_gemm_supported(int dtype, int64_t M, int N, int K);
 int launch_router_bn_gemm(const void* x, const void* w, const float* mean, const float* invstd,
                           const void* running_mean, const void* running_var, float eps, void* logits, int dtype,
-                          int64_t M, int N, int K, int32_t* status, cudaStream_t stream);
+                          int64_t M, int N, int K, bool beside_predecessor, int32_t* status, cudaStream_t stream);
+// beside_predecessor: the kernel before it in the stream is one of this forward's that works on other data.
 // CTA-pair (cta_group::2) versions of the two shared-MLP GEMMs (gemm_sm100_pair.cu)
 bool gemm_pair_supported(int64_t M, int N, int K);
 int launch_gemm_swiglu_pair(const void* x, const void* gate_w, const void* up_w, void* h, int dtype, int64_t M, int I,

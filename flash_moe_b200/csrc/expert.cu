@@ -2,20 +2,13 @@
 //   out[t] = sum_j silu(<x[t], D[e_tj]>) * g[t,j] * U[e_tj]
 // (flash_moe/ops/triton/flash_expert.py:13-211, preprocessing :528-577).
 //
-// Two schedules, picked by dtype
-//   A. 16-bit dtypes: no sort.  Scores per token on the tensor cores
-//      (mma.sync, groups of 16 gathered down rows against the token's x row), then the per-token
-//      accumulate of step 3.
-//   B. float32: expert-centric order of the (token, slot) pairs by a
-//      device-side counting sort (histogram with warp-aggregated atomics -> exclusive scan ->
-//      scatter; no host sync; ids outside [0, N) are dropped and flagged), then a scores pass over
-//      the SORTED pairs: a warp walks a contiguous run of pairs, keeps the current expert's down
-//      row in registers (loaded once per run of equal ids with 128-bit loads), gathers each pair's
-//      x row and reduces the dot product in fp32; empty experts cost nothing, a hot expert is
-//      split over many warps.
-//   Both store gs = silu(s) * gate at the pair's (token, slot) position (4 bytes per pair).
-//   3. accumulate pass per token: out[t] = sum_j gs[t,j] * U[e_tj] in fp32 (packed f32x2 FMAs),
-//      fixed slot order, one rounding on store - no atomics, run-to-run deterministic.
+// Per token, no sort, in two passes:
+//   2. scores: gs = silu(<x[t], D[e]>) * gate per (token, slot) - 16-bit tables on the tensor cores (mma.sync, groups of 16
+//      gathered down rows against the token's x row), float32 with FMAs - stored at the pair's position (4 bytes a pair);
+//   3. accumulate: out[t] = sum_j gs[t,j] * U[e_tj] in fp32 (packed f32x2 FMAs), fixed slot order, one rounding on
+//      store - no atomics, run-to-run deterministic.
+// Both have a form for few tokens that spreads one task over the warps of a CTA.  Ids outside [0, N) are skipped and
+// flagged.  16-bit tables of 1 GiB and more take the fused kernel of expert_fused.cu.
 #include <cub/device/device_radix_sort.cuh>
 
 #include <cstdlib>
@@ -30,31 +23,7 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
-// ---------------------------------------------------------------- 1. counting sort
-__global__ void expert_hist_kernel(const int64_t* __restrict__ idx, int64_t P, int64_t N, int* __restrict__ counts,
-                                   int* __restrict__ rank, int32_t* status) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  const int64_t warp_global = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  bool bad = false;
-  for (int64_t base = warp_global * 32; base < P; base += warps_total * 32) {
-    const int64_t p = base + lane;
-    int64_t e = -1;
-    if (p < P) e = idx[p];
-    const bool valid = (p < P) && (e >= 0) && (e < N);
-    if (p < P && !valid && e != -1) bad = true;  // -1 is the empty-slot value: skipped without a flag
-    // lanes holding the same expert id share one atomic; invalid lanes get distinct keys
-    const unsigned key = valid ? static_cast<unsigned>(e) : (0x80000000u | lane);
-    const unsigned peers = __match_any_sync(kFull, key);
-    const int leader = __ffs(peers) - 1;
-    int basecnt = 0;
-    if (valid && lane == leader) basecnt = atomicAdd(&counts[e], __popc(peers));
-    basecnt = __shfl_sync(kFull, basecnt, leader);
-    if (p < P) rank[p] = valid ? basecnt + __popc(peers & ((1u << lane) - 1u)) : -1;
-  }
-  if (bad && status != nullptr) atomicOr(status, FMOE_STATUS_BAD_EXPERT_ID);
-}
-
+// ---------------------------------------------------------------- 1. segment offsets (backward)
 __device__ __forceinline__ int block_reduce_sum(int v, int* sh) {
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(kFull, v, d);
@@ -119,108 +88,6 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const int* __r
     if (first + i < N) offsets[first + i] = run;
     run += item[i];
     if (first + i == N - 1) offsets[N] = run;
-  }
-}
-
-__global__ void expert_scatter_kernel(const int64_t* __restrict__ idx, const int* __restrict__ rank,
-                                      const int* __restrict__ offsets, int64_t P, int* __restrict__ sorted_pair,
-                                      int* __restrict__ sorted_expert) {
-  for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < P;
-       p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int r = rank[p];
-    if (r < 0) continue;
-    const int e = static_cast<int>(idx[p]);
-    const int pos = offsets[e] + r;
-    sorted_pair[pos] = static_cast<int>(p);
-    sorted_expert[pos] = e;
-  }
-}
-
-// ---------------------------------------------------------------- 2. scores over sorted pairs
-// NCH > 0: the row fits NCH 16-byte chunks per lane and the down row is cached in registers.
-// NCH == 0: any H, the down row is re-read (L1-resident) for every pair.
-template <typename T, int NCH>
-__global__ void __launch_bounds__(256) expert_scores_kernel(const T* __restrict__ x, const T* __restrict__ down,
-                                                           const int* __restrict__ sorted_pair,
-                                                           const int* __restrict__ sorted_expert,
-                                                           const int* __restrict__ total_ptr,
-                                                           const T* __restrict__ gates, float* __restrict__ gs, int H,
-                                                           int k, int chunk, int act, float* __restrict__ raw_out) {
-  constexpr int VEC = Vec16<T>::N;
-  constexpr int R = NCH > 0 ? NCH : 1;
-  const int lane = threadIdx.x & 31;
-  const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  const int64_t warp_global = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int total = *total_ptr;
-
-  for (int64_t task = warp_global; task * chunk < total; task += warps_total) {
-    const int pos0 = static_cast<int>(task * chunk);
-    const int pos1 = min(pos0 + chunk, total);
-    int cur_e = -1;
-    float dreg[R][VEC];
-    uint4 xq[R], xn[R];
-    // prefetch the first pair's x row
-    int p_next = sorted_pair[pos0];
-    if (NCH > 0) {
-      const T* xr = x + static_cast<int64_t>(p_next / k) * H;
-#pragma unroll
-      for (int c = 0; c < R; ++c) {
-        const int col = (c * 32 + lane) * VEC;
-        xn[c] = (col < H) ? ldg16(xr + col) : make_uint4(0, 0, 0, 0);
-      }
-    }
-    for (int pos = pos0; pos < pos1; ++pos) {
-      const int p = p_next;
-      const int e = sorted_expert[pos];
-      float acc = 0.f;
-      if (NCH > 0) {
-#pragma unroll
-        for (int c = 0; c < R; ++c) xq[c] = xn[c];
-        if (pos + 1 < pos1) {  // issue the next pair's gather before the math of this one
-          p_next = sorted_pair[pos + 1];
-          const T* xr = x + static_cast<int64_t>(p_next / k) * H;
-#pragma unroll
-          for (int c = 0; c < R; ++c) {
-            const int col = (c * 32 + lane) * VEC;
-            xn[c] = (col < H) ? ldg16(xr + col) : make_uint4(0, 0, 0, 0);
-          }
-        }
-        if (e != cur_e) {  // warp-uniform
-          cur_e = e;
-          const T* dr = down + static_cast<int64_t>(e) * H;
-#pragma unroll
-          for (int c = 0; c < R; ++c) {
-            const int col = (c * 32 + lane) * VEC;
-            const uint4 q = (col < H) ? ldg16(dr + col) : make_uint4(0, 0, 0, 0);
-            unpack16<T>(q, dreg[c]);
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < R; ++c) {
-          float xf[VEC];
-          unpack16<T>(xq[c], xf);
-#pragma unroll
-          for (int i = 0; i < VEC; ++i) acc = fmaf(xf[i], dreg[c][i], acc);
-        }
-      } else {
-        if (pos + 1 < pos1) p_next = sorted_pair[pos + 1];
-        const T* xr = x + static_cast<int64_t>(p / k) * H;
-        const T* dr = down + static_cast<int64_t>(e) * H;
-        for (int col = lane * VEC; col < H; col += 32 * VEC) {
-          float xf[VEC], df[VEC];
-          unpack16<T>(ldg16(xr + col), xf);
-          unpack16<T>(ldg16(dr + col), df);
-#pragma unroll
-          for (int i = 0; i < VEC; ++i) acc = fmaf(xf[i], df[i], acc);
-        }
-      }
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) acc += __shfl_xor_sync(kFull, acc, d);
-      if (lane == 0) {
-        gs[p] = gates != nullptr ? expert_act(acc, act) * to_f32<T>(gates[p]) : acc;  // nullptr: raw dot product
-        if (raw_out != nullptr) raw_out[p] = acc;  // kept for the backward pass
-      }
-    }
   }
 }
 
@@ -392,6 +259,133 @@ __global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* __restr
   if (bad && status != nullptr) atomicOr(status, FMOE_STATUS_BAD_EXPERT_ID);
 }
 
+// ---------------------------------------------------------------- 2c. scores, few tokens
+// One CTA of W warps per (token, group of 16 of its experts), each warp on its own 128-column chunks of the 16 gathered
+// rows; the partial dot products meet in shared memory (added in warp order).  With few tasks the one-warp-per-task kernel
+// above leaves most of the chip idle while a warp pulls 16 whole rows: 64 tokens x 2048 columns, top-32 (128 tasks) took 11.2 us
+// there; both passes of one token x 1024, top-64 (4 tasks) went from 18.7 to 7 us, of 64 tokens from 27.4 to 12.
+template <typename T, int W, bool PEER>
+__global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __restrict__ x, const T* __restrict__ down,
+                                                                    const int64_t* __restrict__ idx,
+                                                                    const T* __restrict__ gates, float* __restrict__ gs,
+                                                                    int64_t tasks, int groups, int H, int64_t N, int k,
+                                                                    int32_t* status, int act, float* __restrict__ raw_out,
+                                                                    const T* const* __restrict__ shards, int world,
+                                                                    int64_t sharded) {
+  __shared__ float part[W][16];
+  pdl_wait();  // ids and gates come from the kernel before this one
+  pdl_launch_dependents();  // the accumulate pass may start gathering: it needs the ids, and only later the scores
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, tq = lane & 3;
+  for (int64_t task = blockIdx.x; task < tasks; task += gridDim.x) {
+    const int64_t t = task / groups;
+    const int j0 = static_cast<int>(task - t * groups) * 16;
+    const int ja = j0 + g, jb = ja + 8;
+    const int64_t ea = ja < k ? idx[t * k + ja] : 0, eb = jb < k ? idx[t * k + jb] : 0;
+    const bool oka = (ja < k) && ea >= 0 && ea < N;
+    const bool okb = (jb < k) && eb >= 0 && eb < N;
+    if (((ja < k && !oka && ea != -1) || (jb < k && !okb && eb != -1)) && status != nullptr)
+      atomicOr(status, FMOE_STATUS_BAD_EXPERT_ID);  // -1: empty slot, no flag
+    const T* ra = table_row<T, PEER>(down, shards, world, oka ? ea : 0, H, sharded) + 8 * tq;
+    const T* rb = table_row<T, PEER>(down, shards, world, okb ? eb : 0, H, sharded) + 8 * tq;
+    const T* rx = x + t * H + 8 * tq;
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int c0 = warp * 128; c0 < H; c0 += W * 128) {
+      uint4 qa[4], qb[4], qx[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int col = c0 + 32 * u;
+        const bool in = col + 8 * tq < H;
+        qa[u] = in ? ldg16(ra + col) : make_uint4(0, 0, 0, 0);
+        qb[u] = in ? ldg16(rb + col) : make_uint4(0, 0, 0, 0);
+        qx[u] = in ? ldg16(rx + col) : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        Mma16816<T>::run(c, qa[u].x, qb[u].x, qa[u].y, qb[u].y, qx[u].x, qx[u].y);
+        Mma16816<T>::run(c, qa[u].z, qb[u].z, qa[u].w, qb[u].w, qx[u].z, qx[u].w);
+      }
+    }
+    if (tq == 0) {
+      part[warp][g] = oka ? c[0] : 0.f;
+      part[warp][g + 8] = okb ? c[2] : 0.f;
+    }
+    __syncthreads();
+    if (threadIdx.x < 16 && j0 + threadIdx.x < k) {
+      float s = 0.f;
+#pragma unroll
+      for (int w = 0; w < W; ++w) s += part[w][threadIdx.x];
+      const int64_t p = t * k + j0 + threadIdx.x;
+      const int64_t e = idx[p];
+      const bool ok = e >= 0 && e < N;
+      gs[p] = gates != nullptr && ok ? expert_act(s, act) * to_f32<T>(gates[p]) : s;  // no gates: the raw dot product
+      if (raw_out != nullptr) raw_out[p] = s;
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------- 2d. scores, float32
+// One warp per (token, 4 of its experts): 16-byte pieces of the four gathered rows and of the token's row, fp32 FMAs, one
+// shuffle reduction.  No sort in front of it (histogram, scan, scatter and a pass over the sorted pairs took 5 launches and
+// 22 us at 256 tokens x 256 columns, top-8; this takes one and 9).
+__global__ void __launch_bounds__(128) expert_scores_f32_kernel(const float* __restrict__ x, const float* __restrict__ down,
+                                                               const int64_t* __restrict__ idx,
+                                                               const float* __restrict__ gates, float* __restrict__ gs,
+                                                               int64_t ntok, int H, int64_t N, int k, int32_t* status,
+                                                               int act, float* __restrict__ raw_out) {
+  constexpr int G = 4;
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  const int64_t warp_global = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int groups = (k + G - 1) / G;
+  bool bad = false;
+  for (int64_t task = warp_global; task < ntok * groups; task += warps_total) {
+    if (task + warps_total >= ntok * groups) pdl_launch_dependents();
+    const int64_t t = task / groups;
+    const int j0 = static_cast<int>(task - t * groups) * G;
+    const float4* rx = reinterpret_cast<const float4*>(x + t * H);
+    const float4* row[G];
+    bool ok[G];
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      const int64_t e = j0 + i < k ? idx[t * k + j0 + i] : -1;
+      ok[i] = e >= 0 && e < N;
+      bad |= !ok[i] && e != -1;
+      row[i] = reinterpret_cast<const float4*>(down + (ok[i] ? e : 0) * H);
+    }
+    float acc[G] = {0.f, 0.f, 0.f, 0.f};
+    const int hv = H >> 2;
+#pragma unroll 2
+    for (int c = lane; c < hv; c += 32) {
+      const float4 v = __ldg(rx + c);
+#pragma unroll
+      for (int i = 0; i < G; ++i) {
+        const float4 d = __ldg(row[i] + c);
+        acc[i] = fmaf(v.x, d.x, acc[i]);
+        acc[i] = fmaf(v.y, d.y, acc[i]);
+        acc[i] = fmaf(v.z, d.z, acc[i]);
+        acc[i] = fmaf(v.w, d.w, acc[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < G; ++i)
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) acc[i] += __shfl_xor_sync(kFull, acc[i], d);
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      if (lane == i && j0 + i < k) {
+        const int64_t p = t * k + j0 + i;
+        const float s = ok[i] ? acc[i] : 0.f;
+        gs[p] = gates != nullptr && ok[i] ? expert_act(s, act) * gates[p] : s;
+        if (raw_out != nullptr) raw_out[p] = s;
+      }
+    }
+  }
+  if (bad && status != nullptr) atomicOr(status, FMOE_STATUS_BAD_EXPERT_ID);
+}
+
 // ---------------------------------------------------------------- 3. per-token accumulate
 // One warp per (token, column block of 32*VEC*NCH elements); 16 x 16 B of gathered rows in flight
 // per lane, packed f32x2 FMAs (two accumulators per instruction).  The launch bound keeps the kernel at 120
@@ -511,6 +505,91 @@ __global__ void __launch_bounds__(128, 4) expert_accum_kernel(const T* __restric
   }
 }
 
+// The same sum for few tokens: a CTA of W warps per (token, block of 32 * VEC columns), each warp on its own batches of 8
+// slots; the W partial sums meet in shared memory and are added in warp order.  The kernel is made resident beside the
+// scores pass (which has itself waited for the ids) and gathers its first batch of rows before it waits for the weights.
+// One token x 1024 columns, top-64: 12.5 us with one warp per 512 columns, 3.8 here; 64 tokens x 2048, top-32: 16.2, 8.6.
+template <typename T, typename OutT, int W, bool PEER>
+__global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __restrict__ up, const int64_t* __restrict__ idx,
+                                                                   const float* __restrict__ gs, OutT* __restrict__ out,
+                                                                   int64_t tasks, int H, int64_t N, int k, int colblocks,
+                                                                   int early, const T* const* __restrict__ shards,
+                                                                   int world, int64_t sharded) {
+  constexpr int VEC = Vec16<T>::N;
+  constexpr int SLOTS = 8;
+  constexpr int COLS = 32 * VEC;
+  __shared__ float part[W][COLS];
+  if (!early) pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  bool waited = !early;
+  for (int64_t task = blockIdx.x; task < tasks; task += gridDim.x) {
+    const int64_t t = task / colblocks;
+    const int col0 = static_cast<int>(task - t * colblocks) * COLS;
+    const bool in = col0 + lane * VEC < H;
+    uint64_t acc[VEC / 2];
+#pragma unroll
+    for (int i = 0; i < VEC / 2; ++i) acc[i] = 0ull;
+    for (int j0 = warp * SLOTS; j0 < k || !waited; j0 += W * SLOTS) {
+      const int j = j0 + (lane & (SLOTS - 1));
+      // ids and rows are read past the L1 cache: an early CTA may find lines of an earlier forward there
+      const int64_t e = j < k ? __ldcg(reinterpret_cast<const long long*>(idx) + t * k + j) : -1;
+      const bool ok = e >= 0 && e < N;
+      const int row = ok ? static_cast<int>(e) : 0;
+      uint4 q[SLOTS];
+#pragma unroll
+      for (int u = 0; u < SLOTS; ++u) {
+        const int r = __shfl_sync(kFull, row, u);
+        q[u] = in ? __ldcg(reinterpret_cast<const uint4*>(table_row<T, PEER>(up, shards, world, r, H, sharded) + col0 + lane * VEC))
+                  : make_uint4(0, 0, 0, 0);
+      }
+      if (!waited) {
+        pdl_wait();
+        waited = true;
+      }
+      const float w = ok ? ld_after_wait(gs + t * k + j) : 0.f;
+#pragma unroll
+      for (int u = 0; u < SLOTS; ++u) {
+        const float wu = __shfl_sync(kFull, w, u);
+        const uint64_t w2 = pack_f32x2(wu, wu);
+        float f[VEC];
+        unpack16<T>(q[u], f);
+#pragma unroll
+        for (int i = 0; i < VEC / 2; ++i) ffma2(acc[i], pack_f32x2(f[2 * i], f[2 * i + 1]), w2);
+      }
+    }
+    if (task + gridDim.x >= tasks) pdl_launch_dependents();
+#pragma unroll
+    for (int i = 0; i < VEC / 2; ++i) {
+      float lo, hi;
+      unpack_f32x2(acc[i], lo, hi);
+      *reinterpret_cast<float2*>(&part[warp][lane * VEC + 2 * i]) = make_float2(lo, hi);
+    }
+    __syncthreads();
+    for (int c = threadIdx.x * 4; c < COLS; c += 32 * W * 4) {
+      if (col0 + c >= H) continue;
+      float4 s = *reinterpret_cast<const float4*>(&part[0][c]);
+#pragma unroll
+      for (int w = 1; w < W; ++w) {
+        const float4 v = *reinterpret_cast<const float4*>(&part[w][c]);
+        s.x += v.x;
+        s.y += v.y;
+        s.z += v.z;
+        s.w += v.w;
+      }
+      OutT* o = out + t * H + col0 + c;
+      if constexpr (sizeof(OutT) == 4) {
+        *reinterpret_cast<float4*>(o) = s;
+      } else {
+        o[0] = from_f32<OutT>(s.x);
+        o[1] = from_f32<OutT>(s.y);
+        o[2] = from_f32<OutT>(s.z);
+        o[3] = from_f32<OutT>(s.w);
+      }
+    }
+    __syncthreads();
+  }
+}
+
 struct ExpertWs {
   int* counts;
   int* offsets;
@@ -543,17 +622,58 @@ ExpertWs carve(void* ws, int64_t T, int64_t N, int k) {
   return w;
 }
 
-template <typename T, int NCH>
-void launch_scores(const void* x, const void* down, const ExpertWs& w, int64_t N, const void* gates, float* gs_out,
-                   int H, int k, int64_t P, cudaStream_t stream, int act, float* raw_out) {
-  const int chunk = 16;
-  const int64_t tasks = (P + chunk - 1) / chunk;
-  const int64_t want = (tasks + 7) / 8;
-  const int64_t cap = static_cast<int64_t>(device_sm_count()) * 8;
-  const int grid = static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
-  expert_scores_kernel<T, NCH><<<grid, 256, 0, stream>>>(static_cast<const T*>(x), static_cast<const T*>(down),
-                                                         w.sorted_pair, w.sorted_expert, w.offsets + N,
-                                                         static_cast<const T*>(gates), gs_out, H, k, chunk, act, raw_out);
+// Few tokens: the largest W in {8, 4} whose CTAs leave no warp without slots; 0 selects the one-warp-per-task kernels.
+// Those keep (SMs x 16) warps busy with several gathers in flight each, so splitting pays below half as many tasks.
+int split_warps(int64_t tasks, int pieces) {
+  if (tasks * 2 > static_cast<int64_t>(device_sm_count()) * 16) return 0;
+  return pieces >= 8 ? 8 : pieces >= 2 ? 4 : 0;
+}
+
+struct PeerTable {  // a table sharded over the GPUs of a node (table_row); no shards: one array
+  const void* const* shards = nullptr;
+  int world = 1;
+  int64_t sharded = 0;
+};
+
+// the scores pass / accumulate pass for few tokens; false: not the shape for it (or, with `rc`, a launch error)
+template <typename T, bool PEER>
+bool try_scores_split(const void* rows, const void* table, const int64_t* idx, const void* gates, float* out, int64_t T_, int H,
+                      int64_t N, int k, int32_t* status, cudaStream_t stream, int act, float* raw_out, const PeerTable& pt,
+                      cudaError_t* rc) {
+  const int groups = (k + 15) / 16;
+  const int64_t tasks = T_ * groups;
+  const int split = split_warps(tasks, (H + 127) / 128);
+  if (split == 0) return false;
+  const int64_t cap = static_cast<int64_t>(device_sm_count()) * (64 / split);
+  auto kern = split == 8 ? expert_scores_split_kernel<T, 8, PEER> : expert_scores_split_kernel<T, 4, PEER>;
+  *rc = launch_pdl(PEER ? 0 : 8, kern, dim3(static_cast<unsigned>(tasks < cap ? tasks : cap)), dim3(32 * split), 0, stream, 1,
+                   static_cast<const T*>(rows), static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, tasks,
+                   groups, H, N, k, status, act, raw_out, reinterpret_cast<const T* const*>(pt.shards), pt.world, pt.sharded);
+  return true;
+}
+
+template <typename T, bool PEER>
+bool try_accum_split(const void* table, const int64_t* idx, const float* coef, void* out, int out_f32, int64_t T_, int H,
+                     int64_t N, int k, bool early, cudaStream_t stream, const PeerTable& pt, cudaError_t* rc) {
+  constexpr int COLS = 32 * Vec16<T>::N;
+  const int split = split_warps(T_ * ((H + 2 * COLS - 1) / (2 * COLS)), (k + 7) / 8);
+  if (split == 0) return false;
+  const int colblocks = (H + COLS - 1) / COLS;
+  const int64_t tasks = T_ * colblocks;
+  const int64_t cap = static_cast<int64_t>(device_sm_count()) * (64 / split);
+  auto go = [&](auto kern, auto* o) {
+    *rc = launch_pdl(PEER ? 0 : 8, kern, dim3(static_cast<unsigned>(tasks < cap ? tasks : cap)), dim3(32 * split), 0, stream, 1,
+                     static_cast<const T*>(table), idx, coef, o, tasks, H, N, k, colblocks, early && !PEER ? 1 : 0,
+                     reinterpret_cast<const T* const*>(pt.shards), pt.world, pt.sharded);
+  };
+  if (out_f32) {
+    if (split == 8) go(expert_accum_split_kernel<T, float, 8, PEER>, static_cast<float*>(out));
+    else go(expert_accum_split_kernel<T, float, 4, PEER>, static_cast<float*>(out));
+  } else {
+    if (split == 8) go(expert_accum_split_kernel<T, T, 8, PEER>, static_cast<T*>(out));
+    else go(expert_accum_split_kernel<T, T, 4, PEER>, static_cast<T*>(out));
+  }
+  return true;
 }
 
 template <typename T, typename OutT, int NCH>
@@ -570,103 +690,61 @@ void launch_accum(const void* up, const int64_t* idx, const float* gs, void* out
                    H, N, k, colblocks, nullptr, 1, 0);  // launch errors surface through the caller's launch check
 }
 
-// 16-bit tables are gathered per token (no sort, tensor-core dot products) whatever their size: measured against
-// the expert-centric order at 2^16 experts x 131072 tokens (3.07 vs 3.94 ms) and at 2^20 experts with Zipf ids
-// (0.54 vs 0.83 ms; uniform ids 1.23 vs 1.16 ms).  float32 takes the expert-centric order.
-// debugging / measurement aid: FMOE_EXPERT_SCHEDULE=token|sorted|fused forces one schedule for 16-bit tables (read
-// once per process; `fused` only where that kernel applies); anything else leaves the default choice
+// debugging / measurement aid: FMOE_EXPERT_SCHEDULE=token|fused forces one schedule for 16-bit tables (read once per
+// process; `fused` only where that kernel applies); anything else leaves the default choice
 int forced_schedule() {
   static const int forced = [] {
     const char* v = std::getenv("FMOE_EXPERT_SCHEDULE");
     if (v == nullptr) return 0;
-    return v[0] == 't' ? 1 : (v[0] == 's' ? 2 : (v[0] == 'f' ? 3 : 0));
+    return v[0] == 't' ? 1 : (v[0] == 'f' ? 3 : 0);
   }();
   return forced;
 }
 
-template <typename T> bool use_token_centric(int64_t N, int H) {
-  if (sizeof(T) != 2) return false;
-  if (forced_schedule() == 1 || forced_schedule() == 2) return forced_schedule() == 1;
-  (void)N;
-  (void)H;
-  return true;
-}
-
-// counting sort of the (token, slot) pairs by expert id: w.offsets[0..N], w.sorted_pair, w.sorted_expert
-int run_sort(const int64_t* idx, int64_t P, int64_t N, const ExpertWs& w, int32_t* status, cudaStream_t stream) {
-  const int sms = device_sm_count();
-  FMOE_CUDA_TRY(cudaMemsetAsync(w.counts, 0, static_cast<size_t>(N) * 4, stream));
-  {
-    const int64_t want = (P + 255) / 256;
-    const int grid = static_cast<int>(want < sms * 8 ? want : sms * 8);
-    expert_hist_kernel<<<grid, 256, 0, stream>>>(idx, P, N, w.counts, w.rank, status);
-    FMOE_LAUNCH_CHECK();
-  }
-  {
-    const int ntiles = static_cast<int>((N + kScanTile - 1) / kScanTile);
-    if (ntiles > 16) {
-      scan_tile_sums_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.counts, N, w.tile_sums);
-      FMOE_LAUNCH_CHECK();
-      scan_apply_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.counts, N, w.tile_sums, w.offsets);
-    } else {
-      scan_apply_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.counts, N, nullptr, w.offsets);
-    }
-    FMOE_LAUNCH_CHECK();
-  }
-  {
-    const int64_t want = (P + 255) / 256;
-    const int grid = static_cast<int>(want < sms * 8 ? want : sms * 8);
-    expert_scatter_kernel<<<grid, 256, 0, stream>>>(idx, w.rank, w.offsets, P, w.sorted_pair, w.sorted_expert);
-    FMOE_LAUNCH_CHECK();
-  }
-  return FMOE_OK;
-}
-
 // per-pair dot products <rows[t], table[e]>: gates != nullptr stores silu(dot) * gate (forward), nullptr the
-// raw dot product.  `sorted` says whether run_sort has filled w for these indices.
+// raw dot product
 template <typename T>
 int run_scores(const void* rows, const void* table, const int64_t* idx, const void* gates, float* out, int64_t T_, int H,
-               int64_t N, int k, const ExpertWs& w, bool sorted, int32_t* status, cudaStream_t stream, int act = 0,
-               float* raw_out = nullptr) {
-  constexpr int VEC = Vec16<T>::N;
-  const int64_t P = T_ * k;
+               int64_t N, int k, int32_t* status, cudaStream_t stream, int act = 0, float* raw_out = nullptr) {
   const int sms = device_sm_count();
-  const int need = (H + 32 * VEC - 1) / (32 * VEC);
-  if (use_token_centric<T>(N, H)) {
-    if constexpr (sizeof(T) == 2) {
-      const int64_t want = (T_ * ((k + 15) / 16) + 3) / 4;
-      // exactly the CTAs that are resident at once (four per SM at 121 registers): every warp walks its tasks with
-      // the next one's ids and x row already in flight, and the work ends evenly (53.7 vs 55.7 us with 16 per SM)
-      const int64_t cap = static_cast<int64_t>(sms) * 4;
-      const int grid = static_cast<int>(want < cap ? want : cap);
-      const int xs_stride = ((H + 255) / 256) * 32;  // uint4 per warp, rows padded to 256 columns
-      const int smem = 4 * 2 * xs_stride * 16;  // two x-row buffers per warp
-      auto kern = expert_scores_mma_kernel<T, 4, false, 2>;
-      FMOE_CUDA_TRY(allow_smem(kern, smem));
-      FMOE_CUDA_TRY(launch_pdl(4, kern, dim3(grid), dim3(128), smem, stream, 1, static_cast<const T*>(rows),
-                               static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, T_, H, N, k, xs_stride,
-                               status, act, nullptr, 1, raw_out, 0));
+  if constexpr (sizeof(T) == 2) {
+    cudaError_t rc = cudaSuccess;
+    if (try_scores_split<T, false>(rows, table, idx, gates, out, T_, H, N, k, status, stream, act, raw_out, PeerTable{}, &rc)) {
+      FMOE_CUDA_TRY(rc);
+      return FMOE_OK;
     }
-    return FMOE_OK;
+    const int64_t want = (T_ * ((k + 15) / 16) + 3) / 4;
+    // exactly the CTAs that are resident at once (four per SM at 121 registers): every warp walks its tasks with
+    // the next one's ids and x row already in flight, and the work ends evenly (53.7 vs 55.7 us with 16 per SM)
+    const int64_t cap = static_cast<int64_t>(sms) * 4;
+    const int grid = static_cast<int>(want < cap ? want : cap);
+    const int xs_stride = ((H + 255) / 256) * 32;  // uint4 per warp, rows padded to 256 columns
+    const int smem = 4 * 2 * xs_stride * 16;  // two x-row buffers per warp
+    auto kern = expert_scores_mma_kernel<T, 4, false, 2>;
+    FMOE_CUDA_TRY(allow_smem(kern, smem));
+    FMOE_CUDA_TRY(launch_pdl(4, kern, dim3(grid), dim3(128), smem, stream, 1, static_cast<const T*>(rows),
+                             static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, T_, H, N, k, xs_stride,
+                             status, act, nullptr, 1, raw_out, 0));
+  } else {
+    const int64_t want = (T_ * ((k + 3) / 4) + 3) / 4;
+    const int64_t cap = static_cast<int64_t>(sms) * 16;
+    FMOE_CUDA_TRY(launch_pdl(8, expert_scores_f32_kernel, dim3(static_cast<unsigned>(want < cap ? want : cap)), dim3(128), 0,
+                             stream, 1, static_cast<const float*>(rows), static_cast<const float*>(table), idx,
+                             static_cast<const float*>(gates), out, T_, H, N, k, status, act, raw_out));
   }
-  if (!sorted) {
-    const int rc = run_sort(idx, P, N, w, status, stream);
-    if (rc != FMOE_OK) return rc;
-  }
-  if (need <= 1) launch_scores<T, 1>(rows, table, w, N, gates, out, H, k, P, stream, act, raw_out);
-  else if (need <= 2) launch_scores<T, 2>(rows, table, w, N, gates, out, H, k, P, stream, act, raw_out);
-  else if (need <= 4) launch_scores<T, 4>(rows, table, w, N, gates, out, H, k, P, stream, act, raw_out);
-  else if (need <= 8) launch_scores<T, 8>(rows, table, w, N, gates, out, H, k, P, stream, act, raw_out);
-  else launch_scores<T, 0>(rows, table, w, N, gates, out, H, k, P, stream, act, raw_out);
-  FMOE_LAUNCH_CHECK();
   return FMOE_OK;
 }
 
 // out[t] = sum_j coef[t,j] * table[idx[t,j]] (float32 accumulation, one rounding)
 template <typename T>
 int run_accum(const void* table, const int64_t* idx, const float* coef, void* out, int out_f32, int64_t T_, int H,
-              int64_t N, int k, cudaStream_t stream) {
+              int64_t N, int k, cudaStream_t stream, bool early = false) {
   constexpr int VEC = Vec16<T>::N;
+  cudaError_t split_rc = cudaSuccess;
+  if (try_accum_split<T, false>(table, idx, coef, out, out_f32, T_, H, N, k, early, stream, PeerTable{}, &split_rc)) {
+    FMOE_CUDA_TRY(split_rc);
+    return FMOE_OK;
+  }
   const int need = (H + 32 * VEC - 1) / (32 * VEC);
 #define FMOE_ACCUM(NCH_)                                                                       \
   do {                                                                                         \
@@ -703,10 +781,12 @@ int run_typed(const void* x, const void* down, const void* up, const int64_t* id
     if (rc != FMOE_OK) return rc;
     return launch_expert_fused(x, down, up, idx, gates, out, dtype, out_f32, T_, H, N, k, act, raw_scores, status, stream);
   }
-  int rc = run_scores<T>(x, down, idx, gates, w.gs, T_, H, N, k, w, false, status, stream, act, raw_scores);
+  int rc = run_scores<T>(x, down, idx, gates, w.gs, T_, H, N, k, status, stream, act, raw_scores);
   if (rc != FMOE_OK) return rc;
   if ((rc = mark_between()) != FMOE_OK) return rc;
-  return run_accum<T>(up, idx, w.gs, out, out_f32, T_, H, N, k, stream);
+  // the accumulate pass may gather rows while the scores pass runs: that pass has waited for the ids (only the kernels
+  // for few tokens, which are launched with programmatic serialisation, let it in early)
+  return run_accum<T>(up, idx, w.gs, out, out_f32, T_, H, N, k, stream, true);
 }
 
 // ---------------------------------------------------------------- backward
@@ -951,7 +1031,13 @@ int run_typed_peer(const void* x, const void* const* down_shards, const void* co
   } else {
     constexpr int VEC = Vec16<T>::N;
     const int sms = device_sm_count();
-    {
+    // the same kernels, at the same sizes, as the unsharded forward: the results are bit-equal
+    const PeerTable pd{down_shards, world, N}, pu{up_shards, world, N};
+    cudaError_t split_rc = cudaSuccess;
+    if (try_scores_split<T, true>(x, hot_down, idx, gates, w.gs, T_, H, N + hot_rows, k, status, stream, kActSilu, nullptr, pd,
+                                  &split_rc)) {
+      FMOE_CUDA_TRY(split_rc);
+    } else {
       const int64_t want = (T_ * ((k + 15) / 16) + 3) / 4;
       const int64_t cap = static_cast<int64_t>(sms) * 16;
       const int grid = static_cast<int>(want < cap ? want : cap);
@@ -963,6 +1049,10 @@ int run_typed_peer(const void* x, const void* const* down_shards, const void* co
                                         static_cast<const T*>(gates), w.gs, T_, H, N + hot_rows, k, xs_stride, status,
                                         kActSilu, reinterpret_cast<const T* const*>(down_shards), world, nullptr, N);
       FMOE_LAUNCH_CHECK();
+    }
+    if (try_accum_split<T, true>(hot_up, idx, w.gs, out, out_f32, T_, H, N + hot_rows, k, false, stream, pu, &split_rc)) {
+      FMOE_CUDA_TRY(split_rc);
+      return FMOE_OK;
     }
     const int need = (H + 32 * VEC - 1) / (32 * VEC);
     const int nch = need <= 1 ? 1 : 2;
@@ -1089,10 +1179,10 @@ int run_backward(const void* dout, const void* x, const void* down, const void* 
                                                   w.fwd.sorted_pair, static_cast<int>(P), 0, key_bits(N), stream));
   }
   if (saved_scores == nullptr) {  // s = <x, D[e]> was not kept by the forward: recompute it
-    rc = run_scores<T>(x, down, idx, nullptr, w.fwd.gs, T_, H, N, k, w.fwd, true, status, stream);
+    rc = run_scores<T>(x, down, idx, nullptr, w.fwd.gs, T_, H, N, k, status, stream);
     if (rc != FMOE_OK) return rc;
   }
-  rc = run_scores<T>(dout, up, idx, nullptr, w.q, T_, H, N, k, w.fwd, true, status, stream);
+  rc = run_scores<T>(dout, up, idx, nullptr, w.q, T_, H, N, k, status, stream);
   if (rc != FMOE_OK) return rc;
   {
     const int64_t want = (P + 255) / 256;

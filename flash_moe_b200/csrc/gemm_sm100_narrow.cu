@@ -113,6 +113,12 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
     __syncwarp();
     asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");  // the others may use the barriers; no wait here
     if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (ptx::elect_one()) {
+      ptx::prefetch_tensormap(&tmW0);
+      ptx::prefetch_tensormap(&tmX);
+      ptx::prefetch_tensormap(&tmOut);
+      if (NB == 2) ptx::prefetch_tensormap(&tmW1);
+    }
     const int first = nkb < sh.stages ? nkb : sh.stages;
     if (sh.early) {
       for (int i = 0; i < first; ++i)
@@ -228,10 +234,12 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
 #pragma unroll
       for (int i = 0; i < COUNT; ++i) {
         const bool in = n_ok && i < lim;
-        ad[i] = (in && ep.addend != nullptr) ? __ldg(ep.addend + o + static_cast<int64_t>(i) * ep.n_valid) : 0.f;
-        rs[i] = (in && ep.residual != nullptr)
-                    ? to_f32<T>(static_cast<const T*>(ep.residual)[o + static_cast<int64_t>(i) * ep.n_valid])
-                    : 0.f;
+        ad[i] = (in && ep.addend != nullptr) ? ld_after_wait(ep.addend + o + static_cast<int64_t>(i) * ep.n_valid) : 0.f;
+        rs[i] = 0.f;
+        if (in && ep.residual != nullptr) {
+          const uint16_t raw = ld_after_wait(static_cast<const uint16_t*>(ep.residual) + o + static_cast<int64_t>(i) * ep.n_valid);
+          rs[i] = to_f32<T>(*reinterpret_cast<const T*>(&raw));
+        }
       }
     }
   };
@@ -367,7 +375,11 @@ int narrow_stages(int rows, int nb, int bn, int split) {
 // (about 62 per clock) or by the MMAs; on top come the fixed start (first operands from memory), the epilogue and, with
 // a split, the exchange of the partial sums.  The constants are a fit to 600 timed combinations of tile and split at 12
 // shapes from 1 to 2048 tokens; the tile it picks is within 6 % of the best of them on average.
-NarrowPlan plan_narrow(int64_t M, int N, int K, int nb) {
+// Up to kSameSplit tokens the split is the one that suits 64 tokens: it decides the order of the sums, and a row's result then
+// does not depend on how many other rows the call has (token shards equal the unsharded batch bit for bit).
+constexpr int kSameSplit = 512;
+NarrowPlan plan_narrow(int64_t M, int N, int K, int nb, int fixed_split = 0) {
+  if (fixed_split == 0 && M <= kSameSplit) return plan_narrow(M, N, K, nb, plan_narrow(64, N, K, nb, -1).split);
   NarrowPlan best;
   const int sms = device_sm_count();
   const int num_kb = (K + BLOCK_K - 1) / BLOCK_K;
@@ -376,6 +388,7 @@ NarrowPlan plan_narrow(int64_t M, int N, int K, int nb) {
     const int row_tiles = (N + rows - 1) / rows;
     for (int64_t tt = t_min; tt <= t_min + 12 && tt * 16 < M + 16; ++tt) {
       for (int split = 1; split <= 8 && split <= num_kb; split *= 2) {
+        if (fixed_split > 0 && split != fixed_split) continue;
         const int unit = split == 8 ? 32 : 16;
         const int bn = static_cast<int>(((M + tt - 1) / tt + unit - 1) / unit * unit);
         const int64_t tiles_t = (M + bn - 1) / bn;

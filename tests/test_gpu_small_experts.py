@@ -1,0 +1,41 @@
+"""Expert passes for few tokens (one task spread over the warps of a CTA) and the float32 scores pass."""
+import pytest
+import torch
+
+from tests.helpers import randn
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize(
+    "T,H,N,k",
+    [(1, 8, 4, 1), (1, 1024, 16384, 64), (3, 136, 50, 17), (64, 2048, 4096, 32), (37, 1000, 300, 9), (590, 512, 1000, 32),
+     (593, 512, 1000, 32)],
+)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_expert_passes_for_few_tokens(T, H, N, k, dtype):
+    """Edges of the split over warps: fewer slots than warps, a group of 17 slots, ragged columns, both sides of the token
+    count at which the one-warp-per-task kernels take over; empty and out-of-range slots."""
+    from flash_moe_b200 import _lib
+    from flash_moe_b200.ops.flash_expert import flash_expert_fp32
+
+    x, d, u = (randn(shape, s, dtype, sc).cuda() for shape, s, sc in (((T, H), 1, 0.5), ((N, H), 2, 0.1), ((N, H), 3, 1.0)))
+    gen = torch.Generator().manual_seed(T + k)
+    idx = torch.randint(0, N, (T, k), generator=gen)
+    idx[0, -1] = -1
+    idx = idx.cuda()
+    gates = torch.softmax(randn((T, k), 4, torch.float32), -1).to(dtype).cuda()
+    ok = (idx >= 0).double()
+    rows = idx.clamp(min=0)
+    want = torch.zeros(T, H, dtype=torch.float64, device="cuda")
+    for j in range(k):
+        s = (x.double() * d[rows[:, j]].double()).sum(-1)
+        want += (torch.nn.functional.silu(s) * gates[:, j].double() * ok[:, j])[:, None] * u[rows[:, j]].double()
+    for _ in range(3):  # back to back: each pass may start beside the one before it
+        got = flash_expert_fp32(x, d, u, idx, gates)
+    assert (got.double() - want).norm() <= 2e-6 * want.norm() + 1e-12
+    assert torch.equal(got, flash_expert_fp32(x, d, u, idx, gates))
+    assert _lib.read_status() == 0
+    idx[0, 0] = N  # skipped and reported
+    flash_expert_fp32(x, d, u, idx, gates)
+    assert _lib.read_status() == _lib.STATUS_BAD_EXPERT_ID
