@@ -18,8 +18,6 @@
 //      gates = exp(score) (and the row renormalisation of flash_moe/modules/flash_moe.py:80-85).
 //
 // One warp owns one token; all scratch lives in shared memory.
-#include <cstdlib>
-
 #include "common.cuh"
 
 namespace fmoe {
@@ -381,9 +379,7 @@ struct RouterRegLayout {
   int nkp, kp, kq, C, Cp;
 };
 
-// CPL > 0: the staircase candidates (at most 32 * CPL of them) stay in registers, CPL per lane, through the threshold
-// search and the emit step, whose loops then have compile-time bounds and no shared-memory round trips between rounds.
-template <typename T, int E, int CPL = 0>
+template <typename T, int E>
 __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int k,
                                                              RouterRegLayout L, T* __restrict__ scores,
                                                              int64_t* __restrict__ indices, T* __restrict__ gates,
@@ -504,28 +500,11 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restric
 
     // 2. staircase candidate scores; track the smallest to narrow the threshold search
     uint32_t cmin = 0xFFFFFFFFu;
-    uint32_t csr[CPL > 0 ? CPL : 1], pqr[CPL > 0 ? CPL : 1];
-    if constexpr (CPL > 0) {
-#pragma unroll
-      for (int j = 0; j < CPL; ++j) {
-        const int c = 32 * j + lane;
-        const bool in = c < C;
-        const uint32_t e = in ? pq[c] : 0u;
-        const uint32_t o = f32_to_ord(round_to<T>(__fadd_rn(sa[e >> 16], sb[e & 0xFFFFu])) + 0.0f);
-        pqr[j] = e;
-        csr[j] = in ? o : 0u;  // 0 is below the key of every float, -inf included
-        if (in) {
-          cs[c] = o;  // the tie search below looks up single cells
-          cmin = min(cmin, o);
-        }
-      }
-    } else {
-      for (int c = lane; c < C; c += 32) {
-        const uint32_t e = pq[c];
-        const uint32_t o = f32_to_ord(round_to<T>(__fadd_rn(sa[e >> 16], sb[e & 0xFFFFu])) + 0.0f);
-        cs[c] = o;
-        cmin = min(cmin, o);
-      }
+    for (int c = lane; c < C; c += 32) {
+      const uint32_t e = pq[c];
+      const uint32_t o = f32_to_ord(round_to<T>(__fadd_rn(sa[e >> 16], sb[e & 0xFFFFu])) + 0.0f);
+      cs[c] = o;
+      cmin = min(cmin, o);
     }
     cmin = __reduce_min_sync(kFull, cmin);
     __syncwarp();
@@ -539,12 +518,7 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restric
       for (int bit = top; bit >= LOW; --bit) {
         const uint32_t trial = tau | (1u << bit);
         int n_ge = 0;
-        if constexpr (CPL > 0) {
-#pragma unroll
-          for (int j = 0; j < CPL; ++j) n_ge += (csr[j] >= trial) ? 1 : 0;
-        } else {
-          for (int c = lane; c < C; c += 32) n_ge += (cs[c] >= trial) ? 1 : 0;
-        }
+        for (int c = lane; c < C; c += 32) n_ge += (cs[c] >= trial) ? 1 : 0;
         n_ge = __reduce_add_sync(kFull, n_ge);
         if (n_ge >= k) tau = trial;
       }
@@ -553,13 +527,15 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restric
 
     // emit everything above tau; collect the staircase candidates equal to tau in the tie list
     int filled = 0, nties = 0;
-    auto emit = [&](int c, uint32_t v, uint32_t e, bool known) {
+    for (int base = 0; base < C; base += 32) {
+      const int c = base + lane;
+      const uint32_t v = (c < C) ? cs[c] : 0u;
       const bool g = (c < C) && (v > tau);
       const bool eq = (c < C) && (v == tau);
       const unsigned bal = __ballot_sync(kFull, g);
       const unsigned beq = __ballot_sync(kFull, eq);
       if (g || eq) {
-        if (!known) e = pq[c];
+        const uint32_t e = pq[c];
         const uint32_t flat = static_cast<uint32_t>(ia[e >> 16]) * static_cast<uint32_t>(nk) + ib[e & 0xFFFFu];
         if (g) {
           const int pos = filled + __popc(bal & ((1u << lane) - 1u));
@@ -571,16 +547,6 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restric
       }
       filled += __popc(bal);
       nties += __popc(beq);
-    };
-    if constexpr (CPL > 0) {
-#pragma unroll
-      for (int j = 0; j < CPL; ++j)
-        if (32 * j < C) emit(32 * j + lane, csr[j], pqr[j], true);
-    } else {
-      for (int base = 0; base < C; base += 32) {
-        const int c = base + lane;
-        emit(c, (c < C) ? cs[c] : 0u, 0u, false);
-      }
     }
     int need = k - filled;
 
@@ -795,11 +761,586 @@ RouterRegLayout make_reg_layout(int nk, int k) {
   return L;
 }
 
-template <typename T, int E, int CPL = 0>
-int launch_reg_cpl(const void* logp, int64_t T_, int nk, int k, const RouterRegLayout& L, int warps, void* scores,
-                   int64_t* indices, void* gates, int norm, cudaStream_t stream) {
+// ------------------------------------------------------------------------------------------
+// 16-bit inputs, num_keys <= 1024, top_k <= 128: the same steps on the few keys that can matter.
+//
+//   1. The 32 lane maxima of each half, sorted (both halves in one packed 16-bit network), give a lower bound on the k-th
+//      largest sum: p maxima of the first half and ceil(k / p) of the second make at least k sums of at least
+//      A_p + B_ceil(k/p); the best p counts.
+//   2. A key whose sum with the other half's maximum stays below the bound is dropped (a superset is kept where rounding
+//      or a non-finite value blurs the test).  What is left - 41 of 128 keys at top-64, 101 of 512 at top-128 for normal
+//      logits - is compacted in index order and sorted.
+//   3. Staircase sums, threshold, ties, winners as above; winners are 32-bit keys (level of the score above the threshold
+//      | inverted flat id) wherever the two fit.
+// ------------------------------------------------------------------------------------------
+struct RouterPrunedLayout {
+  int cta_bytes, warp_bytes;
+  int off_ids, off_win, off_cs, off_tl;
+  int nkp, kp, C, Cp;
+};
+
+constexpr int kPrunedMaxK = 128;  // at most 22 staircase cells per lane stay in registers
+
+// Sorts two key lists (la: na keys, lb: nb keys, in shared memory) descending, 16 lanes and 16 R slots each, and writes
+// values and ids in rank order (first half at 0, second at `stride`); the lists may lie under the values.
+template <typename T, int R>
+__device__ __noinline__ void sort_both_halves(const uint32_t* la, const uint32_t* lb, int na, int nb, float* sv, uint16_t* si,
+                                              int stride, int lane) {
+  using HK = HalfKey<T>;
+  const int l16 = lane & 15;
+  const bool second = lane >= 16;
+  const uint32_t* src = second ? lb : la;
+  const int n = second ? nb : na;
+  uint32_t a[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) a[r] = l16 * R + r < n ? src[l16 * R + r] : 0u;
+  constexpr int N = 16 * R;
+#pragma unroll
+  for (int size = 2; size <= N; size <<= 1) {
+#pragma unroll
+    for (int step = size >> 1; step > 0; step >>= 1) {
+      if (step >= R) {
+        const int ls = step / R;
+        const bool desc = (size == N) || (((l16 * R) & size) == 0);
+        const bool keep_max = ((l16 & ls) == 0) == desc;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const uint32_t other = __shfl_xor_sync(kFull, a[r], ls);
+          a[r] = keep_max ? max(a[r], other) : min(a[r], other);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if ((r & step) == 0) {
+            const bool desc = (size == N) || (size < R ? ((r & size) == 0) : (((l16 * R) & size) == 0));
+            const uint32_t lo = min(a[r], a[r | step]), hi = max(a[r], a[r | step]);
+            a[r] = desc ? hi : lo;
+            a[r | step] = desc ? lo : hi;
+          }
+        }
+      }
+    }
+  }
+  __syncwarp();  // both lists have been read
+  float* v = sv + (second ? stride : 0);
+  uint16_t* id = si + (second ? stride : 0);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = l16 * R + r;
+    if (i < n) {
+      v[i] = HK::value(a[r]);
+      id[i] = static_cast<uint16_t>(HK::id(a[r]));
+    }
+  }
+  __syncwarp();
+}
+
+// Descending bitonic sort of 32 R keys in the lane-blocked layout (element lane * R + r in a[r]).  UNROLLED = false: as
+// loops, with only the stages inside a lane unrolled - kernels whose straight-line code exceeds the instruction cache spend
+// two thirds of their time fetching it (512 keys, top-128: 352 us with everything unrolled, 201 us with loops).
+template <int R, bool UNROLLED>
+__device__ __forceinline__ void sort_desc(uint32_t (&a)[R], int lane) {
+  if constexpr (UNROLLED) {
+    bitonic_desc_regs<R, uint32_t>(a, lane);
+  } else {
+    auto inside = [&](int from, bool desc_lane, bool by_reg, int size) {
+#pragma unroll
+      for (int step = R >> 1; step > 0; step >>= 1) {
+        if (step > from) continue;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if ((r & step) == 0) {
+            const bool desc = by_reg ? (r & size) == 0 : desc_lane;
+            const uint32_t lo = min(a[r], a[r | step]), hi = max(a[r], a[r | step]);
+            a[r] = desc ? hi : lo;
+            a[r | step] = desc ? lo : hi;
+          }
+        }
+      }
+    };
+#pragma unroll
+    for (int size = 2; size < R; size <<= 1) inside(size >> 1, true, true, size);
+    if (R > 1) inside(R >> 1, (lane & 1) == 0, false, 0);
+#pragma unroll 1
+    for (int ls2 = 2; ls2 <= 32; ls2 <<= 1) {  // blocks of ls2 lanes
+      const bool desc = ls2 == 32 || (lane & ls2) == 0;
+#pragma unroll 1
+      for (int ls = ls2 >> 1; ls > 0; ls >>= 1) {
+        const bool keep_max = ((lane & ls) == 0) == desc;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const uint32_t other = __shfl_xor_sync(kFull, a[r], ls);
+          a[r] = keep_max ? max(a[r], other) : min(a[r], other);
+        }
+      }
+      if (R > 1) inside(R >> 1, desc, false, 0);
+    }
+  }
+}
+
+// Sorts the n <= 32 R keys of `list` (shared memory) in place, or, with sv, into values and ids in rank order (they may lie
+// over the list).
+template <typename T, int R, bool UNROLLED>
+__device__ __noinline__ void sort_list(uint32_t* list, int n, float* sv, uint16_t* si, int lane) {
+  using HK = HalfKey<T>;
+  uint32_t a[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) a[r] = lane * R + r < n ? list[lane * R + r] : 0u;
+  sort_desc<R, UNROLLED>(a, lane);
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = lane * R + r;
+    if (i < n) {
+      if (sv != nullptr) {
+        sv[i] = HK::value(a[r]);
+        si[i] = static_cast<uint16_t>(HK::id(a[r]));
+      } else {
+        list[i] = a[r];
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// Sort of the 32 lanes, descending, of both 16-bit halves of v at once
+__device__ __forceinline__ uint32_t sort_lanes_packed(uint32_t v, int lane) {
+#pragma unroll
+  for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+    for (int step = size >> 1; step > 0; step >>= 1) {
+      const uint32_t other = __shfl_xor_sync(kFull, v, step);
+      const bool desc = size == 32 || (lane & size) == 0;
+      v = (((lane & step) == 0) == desc) ? __vmaxu2(v, other) : __vminu2(v, other);
+    }
+  return v;
+}
+
+template <typename T, int E, int CPL>
+__global__ void __launch_bounds__(128, E <= 8 ? 7 : 4)
+router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int k, RouterPrunedLayout L,
+                          T* __restrict__ scores, int64_t* __restrict__ indices, T* __restrict__ gates, int flags) {
+  using HK = HalfKey<T>;
+  constexpr int LOW = OrdLowBits<T>::value;
+  constexpr bool kKeysInRegs = E <= 8;     // both halves' values stay in registers up to the compaction
+  constexpr bool kUnrollCells = CPL <= 10;  // see sort_desc: small kernels are unrolled, large ones are loops
+  const int norm = flags & 1;
+  const bool from_logits = (flags & 2) != 0;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int nwarps = blockDim.x >> 5;
+  const int C = L.C, nkp = L.nkp, kp = L.kp;
+
+  // staircase table, built once per CTA: entry c -> (p << 16) | q with (p+1)(q+1) <= k; row p starts at rowstart[p]
+  uint32_t* pq = reinterpret_cast<uint32_t*>(smem);
+  int* rowstart = reinterpret_cast<int*>(smem) + L.Cp;
+  if (warp == 0) {
+    int running = 0;
+    for (int base = 0; base < k; base += 32) {
+      const int p = base + lane;
+      const int len = (p < k) ? k / (p + 1) : 0;
+      int incl = len;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int up = __shfl_up_sync(kFull, incl, d);
+        if (lane >= d) incl += up;
+      }
+      if (p < k) rowstart[p] = running + incl - len;
+      running += __shfl_sync(kFull, incl, 31);
+    }
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < C; c += blockDim.x) {  // entry c lies in the last row whose start is <= c
+    int lo = 0, hi = k - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (rowstart[mid] <= c) lo = mid; else hi = mid - 1;
+    }
+    pq[c] = (static_cast<uint32_t>(lo) << 16) | static_cast<uint32_t>(c - rowstart[lo]);
+  }
+  __syncthreads();
+  pdl_wait();  // the staircase table above depends on k alone; the logits come from the previous kernel
+
+  unsigned char* wbase = smem + L.cta_bytes + warp * L.warp_bytes;
+  float* sa = reinterpret_cast<float*>(wbase);  // values in rank order; the key lists lie here before they are sorted
+  float* sb = sa + nkp;
+  uint16_t* ia = reinterpret_cast<uint16_t*>(wbase + L.off_ids);
+  uint16_t* ib = ia + nkp;
+  uint64_t* win = reinterpret_cast<uint64_t*>(wbase + L.off_win);    // winners, 64-bit keys (rare) ...
+  uint32_t* win32 = reinterpret_cast<uint32_t*>(wbase + L.off_win);  // ... or 32-bit keys
+  uint32_t* cs = reinterpret_cast<uint32_t*>(wbase + L.off_cs);      // staircase sums
+  uint32_t* tl = reinterpret_cast<uint32_t*>(wbase + L.off_tl);      // flat ids of candidates equal to tau
+  int* tcnt = reinterpret_cast<int*>(tl + kTieCap);
+  const int qrank = (k + lane) / (lane + 1);  // ceil(k / (lane + 1)): the rank that pairs with rank lane + 1 of half 0
+  int idbits = 1;
+  while (idbits < 31 && (1 << idbits) < nk * nk) ++idbits;
+  const uint32_t idmask = (1u << idbits) - 1u;
+  const unsigned below = (1u << lane) - 1u;
+  auto flat_id = [&](int p, int q) { return static_cast<uint32_t>(ia[p]) * static_cast<uint32_t>(nk) + ib[q]; };
+  auto pair_ord = [&](int p, int q) { return f32_to_ord(round_to<T>(__fadd_rn(sa[p], sb[q])) + 0.0f); };
+
+  for (int64_t t = static_cast<int64_t>(blockIdx.x) * nwarps + warp; t < ntok;
+       t += static_cast<int64_t>(gridDim.x) * nwarps) {
+    if (t + static_cast<int64_t>(gridDim.x) * nwarps >= ntok) pdl_launch_dependents();  // last token of this warp
+    // 1. load both halves (lane-blocked: element lane * E + r in register r), from_logits: the per-half log-softmax
+    //    (flash_moe/modules/flash_moe.py:72) rounded to T like torch does; lane maxima
+    const T* a_row = from_logits ? logp + t * 2 * nk : logp + t * nk;
+    const T* b_row = from_logits ? a_row + nk : logp + (ntok + t) * nk;
+    uint32_t* la = reinterpret_cast<uint32_t*>(sa);
+    uint32_t* lb_list = reinterpret_cast<uint32_t*>(sb);
+    uint32_t key[kKeysInRegs ? 2 : 1][E];
+    uint32_t v = 0;      // this lane's maximum of both halves (16-bit order keys)
+    float poison = 0.f;  // NaN once a value is not finite
+    auto load_half = [&](int h, uint32_t (&kk)[E]) {
+      float lv[E];
+      load_blocked<T, E>(h == 0 ? a_row : b_row, nk, lane, lv);
+      if (from_logits) {
+        float m = -INFINITY;
+#pragma unroll
+        for (int r = 0; r < E; ++r) m = fmaxf(m, lv[r]);
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(kFull, m, d));
+        float sum = 0.f;
+#pragma unroll
+        for (int r = 0; r < E; ++r)
+          if (lane * E + r < nk) sum += expf(lv[r] - m);
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(kFull, sum, d);
+        const float lg = logf(sum);
+#pragma unroll
+        for (int r = 0; r < E; ++r) lv[r] = round_to<T>((lv[r] - m) - lg);
+      }
+      uint32_t best = 0;
+#pragma unroll
+      for (int r = 0; r < E; ++r) {
+        const bool in = lane * E + r < nk;
+        kk[r] = in ? HK::make(lv[r] + 0.0f, lane * E + r) : 0u;  // -0 -> +0
+        best = max(best, kk[r]);
+        if (in) poison = fmaf(lv[r], 0.f, poison);
+      }
+      v |= h == 0 ? best >> 16 : best & 0xFFFF0000u;
+    };
+    if constexpr (kKeysInRegs) {
+      load_half(0, key[0]);
+      load_half(1, key[1]);
+    } else {
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        load_half(h, key[0]);
+        store_blocked<E>(reinterpret_cast<float*>(h == 0 ? la : lb_list), lane, reinterpret_cast<const float (&)[E]>(key[0]));
+      }
+    }
+    // 2. lower bound on the k-th largest sum from the sorted lane maxima (0: absent), and the keys it leaves
+    uint32_t lb = 0;             // order key of the bound
+    uint32_t thr0 = 1, thr1 = 1;  // keys from here on are kept (0 pads the rows)
+    if (__all_sync(kFull, poison == 0.f)) {
+      v = sort_lanes_packed(v, lane);
+      const uint32_t other = __shfl_sync(kFull, v, qrank <= 32 ? qrank - 1 : 0);
+      const uint32_t ka = v << 16, kb = other & 0xFFFF0000u;
+      if (qrank <= 32 && ka != 0 && kb != 0)
+        lb = f32_to_ord(round_to<T>(__fadd_rn(HK::value(ka), HK::value(kb))) + 0.0f);
+      lb = __reduce_max_sync(kFull, lb);
+      const uint32_t top = __shfl_sync(kFull, v, 0);
+      const float ta = HK::value(top << 16), tb = HK::value(top), bound = ord_to_f32(lb);
+      // round(a + b) >= bound needs a + b >= bound less one step of T there; the threshold's key is rounded to T too
+      constexpr float kStep = LOW == 16 ? 0.0078125f : 0.0009765625f;
+      const float low = bound - (fabsf(bound) * kStep + 1e-7f);
+      const float xa = low - tb, xb = low - ta, blur = (fabsf(bound) + fabsf(ta) + fabsf(tb)) * 1e-6f + 1e-7f;
+      const float ya = xa - (fabsf(xa) * kStep + blur), yb = xb - (fabsf(xb) * kStep + blur);
+      if (lb != 0 && ya > -INFINITY && yb > -INFINITY) {
+        thr0 = max(HK::make(ya, 0) & 0xFFFF0000u, 1u);
+        thr1 = max(HK::make(yb, 0) & 0xFFFF0000u, 1u);
+      }
+    }
+    if (lane == 0) *tcnt = 0;
+    int na = 0, nb = 0;
+    if constexpr (kKeysInRegs) {
+      uint32_t cnt = 0;
+#pragma unroll
+      for (int r = 0; r < E; ++r) cnt += (key[0][r] >= thr0 ? 1u : 0u) + (key[1][r] >= thr1 ? 0x10000u : 0u);
+      const uint32_t mine = cnt;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t up = __shfl_up_sync(kFull, cnt, d);
+        if (lane >= d) cnt += up;
+      }
+      const uint32_t total = __shfl_sync(kFull, cnt, 31);
+      na = total & 0xFFFFu;
+      nb = total >> 16;
+      cnt -= mine;
+      uint32_t* da = la + (cnt & 0xFFFFu);
+      uint32_t* db = lb_list + (cnt >> 16);
+#pragma unroll
+      for (int r = 0; r < E; ++r) {
+        if (key[0][r] >= thr0) *da++ = key[0][r];
+        if (key[1][r] >= thr1) *db++ = key[1][r];
+      }
+      __syncwarp();
+      const int most = max(na, nb);
+      if (most <= 32) sort_both_halves<T, 2>(la, lb_list, na, nb, sa, ia, nkp, lane);
+      else if (E <= 2 || most <= 64) sort_both_halves<T, 4>(la, lb_list, na, nb, sa, ia, nkp, lane);
+      else if (E <= 4 || most <= 128) sort_both_halves<T, 8>(la, lb_list, na, nb, sa, ia, nkp, lane);
+      else {
+        sort_list<T, 8, false>(la, na, sa, ia, lane);
+        sort_list<T, 8, false>(lb_list, nb, sb, ib, lane);
+      }
+    } else {
+      __syncwarp();
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        uint32_t* list = h == 0 ? la : lb_list;
+        const uint32_t th = h == 0 ? thr0 : thr1;
+        int n = 0;
+#pragma unroll 2
+        for (int i = lane; i < nkp; i += 32) {  // in place: a key never moves up
+          const uint32_t kv = list[i];
+          const unsigned bal = __ballot_sync(kFull, kv >= th);
+          if (kv >= th) list[n + __popc(bal & below)] = kv;
+          n += __popc(bal);
+          __syncwarp();
+        }
+        float* sv = h == 0 ? sa : sb;
+        uint16_t* si = h == 0 ? ia : ib;
+        if (n <= 32) sort_list<T, 1, false>(list, n, sv, si, lane);
+        else if (n <= 64) sort_list<T, 2, false>(list, n, sv, si, lane);
+        else if (n <= 128) sort_list<T, 4, false>(list, n, sv, si, lane);
+        else if (n <= 256) sort_list<T, 8, false>(list, n, sv, si, lane);
+        else if (E <= 16 || n <= 512) sort_list<T, 16, false>(list, n, sv, si, lane);
+        else sort_list<T, E >= 32 ? 32 : 16, false>(list, n, sv, si, lane);
+        if (h == 0) na = n;
+        else nb = n;
+      }
+    }
+
+    // 3. staircase sums (in registers), threshold tau = k-th largest
+    uint32_t csr[CPL];
+    if constexpr (kUnrollCells) {
+#pragma unroll
+      for (int j = 0; j < CPL; ++j) {
+        const int c = 32 * j + lane;
+        const uint32_t e = c < C ? pq[c] : 0xFFFFFFFFu;
+        const int p = e >> 16, q = e & 0xFFFFu;
+        csr[j] = (p < na && q < nb) ? pair_ord(p, q) : 0u;  // 0 is below the key of every float, -inf included
+      }
+    } else {
+#pragma unroll 2
+      for (int c = lane; c < C; c += 32) {
+        const uint32_t e = pq[c];
+        const int p = e >> 16, q = e & 0xFFFFu;
+        cs[c] = (p < na && q < nb) ? pair_ord(p, q) : 0u;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < CPL; ++j) csr[j] = 32 * j + lane < C ? cs[32 * j + lane] : 0u;
+    }
+    const uint32_t cmax = pair_ord(0, 0);  // ranks (0, 0): the largest sum
+    uint32_t tau = cmax;
+    if (cmax != lb) {
+      // two bits a step: the three trial thresholds are counted in one packed reduction (at most 704 cells)
+      // (the last step may reach one bit below LOW: no value differs from its level there)
+      int bit = 31 - __clz(cmax ^ lb);
+      tau = bit >= 31 ? 0u : cmax & ~((2u << bit) - 1u);
+      for (; bit >= LOW; bit -= 2) {
+        const uint32_t t1 = tau | (1u << (bit - 1)), t2 = tau | (1u << bit), t3 = t1 | t2;
+        uint32_t n = 0;
+#pragma unroll
+        for (int j = 0; j < CPL; ++j)
+          n += (csr[j] >= t1 ? 1u : 0u) + (csr[j] >= t2 ? 1u << 10 : 0u) + (csr[j] >= t3 ? 1u << 20 : 0u);
+        n = __reduce_add_sync(kFull, n);
+        const uint32_t uk = static_cast<uint32_t>(k);
+        tau = (n >> 20) >= uk ? t3 : ((n >> 10) & 1023u) >= uk ? t2 : (n & 1023u) >= uk ? t1 : tau;
+      }
+      if ((tau >> 31) == 0) tau |= (1u << LOW) - 1u;
+    }
+    const uint32_t tlevel = tau >> LOW;
+    const bool fits = (cmax >> LOW) - tlevel < (1u << (32 - idbits)) - 1u;
+    auto put = [&](int pos, uint32_t ord, uint32_t flat) {
+      if (fits) win32[pos] = (((ord >> LOW) - tlevel + 1u) << idbits) | (idmask - flat);
+      else win[pos] = make_key(ord, flat);
+    };
+
+    // emit everything above tau; collect the staircase candidates equal to tau in the tie list
+    int filled = 0, nties = 0;
+    auto emit = [&](int base, uint32_t o) {
+      const unsigned bge = __ballot_sync(kFull, o >= tau);
+      if (bge == 0) return;
+      const unsigned bgt = __ballot_sync(kFull, o > tau);
+      if (o >= tau) {
+        const uint32_t e = pq[base + lane];
+        const uint32_t flat = flat_id(e >> 16, e & 0xFFFFu);
+        if (o > tau) {
+          const int pos = filled + __popc(bgt & below);
+          if (pos < k) put(pos, o, flat);
+        } else {
+          const int pos = nties + __popc((bge & ~bgt) & below);
+          if (pos < kTieCap) tl[pos] = flat;
+        }
+      }
+      filled += __popc(bgt);
+      nties += __popc(bge & ~bgt);
+    };
+    if constexpr (kUnrollCells) {
+#pragma unroll
+      for (int j = 0; j < CPL; ++j) emit(32 * j, csr[j]);
+    } else {
+#pragma unroll 1
+      for (int base = 0; base < C; base += 32) emit(base, base + lane < C ? cs[base + lane] : 0u);
+    }
+    int need = k - filled;
+
+    // 4. ties outside the staircase: runs that continue a row past its last cell, and runs from q = 0 in the rows below
+    //    (all sums there are at most tau and do not increase along a row)
+    for (int base = 0; base < na; base += 32) {
+      const int p = base + lane;
+      const int len = p < k ? (p + 1 < k ? rowstart[p + 1] : C) - rowstart[p] : 0;  // = k / (p + 1)
+      const bool hit = p < na && len < nb && pair_ord(p < na ? p : 0, len < nb ? len : 0) == tau;
+      const unsigned any = __ballot_sync(kFull, hit);
+      if (hit) {
+        for (int q = len; q < nb; ++q) {
+          if (pair_ord(p, q) != tau) break;
+          const int pos = nties + atomicAdd(tcnt, 1);
+          if (pos < kTieCap) tl[pos] = flat_id(p, q);
+        }
+      }
+      if (base >= k && any == 0u) break;  // rows are sorted: no later row can tie
+    }
+    __syncwarp();
+    nties += *tcnt;
+    __syncwarp();
+    if (nties <= 32) {
+      // the usual case, a handful of ties: one id per lane, its rank among them by a round of shuffles
+      const uint32_t id = lane < nties ? tl[lane] : 0xFFFFFFFFu;
+      int rank = 0;
+      for (int j = 0; j < nties; ++j) rank += (__shfl_sync(kFull, id, j) < id) ? 1 : 0;
+      if (lane < nties && rank < need) put(filled + rank, tau, id);
+      filled += min(nties, need);
+    } else if (nties <= kTieCap) {
+      uint32_t phi = 0xFFFFFFFFu;  // ids <= phi are taken
+      if (nties > need) {
+        // phi = the need-th smallest id = the largest v with fewer than `need` ids below v
+        uint32_t x = 0;
+        for (int bit = idbits - 1; bit >= 0; --bit) {
+          const uint32_t trial = x | (1u << bit);
+          int under = 0;
+          for (int i = lane; i < nties; i += 32) under += (tl[i] < trial) ? 1 : 0;
+          under = __reduce_add_sync(kFull, under);
+          if (under < need) x = trial;
+        }
+        phi = x;
+      }
+      for (int base = 0; base < nties; base += 32) {
+        const int i = base + lane;
+        const uint32_t id = (i < nties) ? tl[i] : 0xFFFFFFFFu;
+        const bool take = (i < nties) && (id <= phi);
+        const unsigned bal = __ballot_sync(kFull, take);
+        if (take) put(filled + __popc(bal & below), tau, id);
+        filled += __popc(bal);
+      }
+    } else {
+      // more ties than the list holds (e.g. constant inputs): rows in index order, inside a row the lowest column ids
+      int last = -1;
+      while (need > 0) {
+        uint32_t next = 0xFFFFFFFFu;  // (row id << 16) | rank of the next row
+        for (int p = lane; p < na; p += 32)
+          if (static_cast<int>(ia[p]) > last) next = min(next, (static_cast<uint32_t>(ia[p]) << 16) | static_cast<uint32_t>(p));
+        next = __reduce_min_sync(kFull, next);
+        if (next == 0xFFFFFFFFu) break;
+        last = static_cast<int>(next >> 16);
+        const int p = next & 0xFFFFu;
+        int run = 0;
+        for (int q = lane; q < nb; q += 32) run += pair_ord(p, q) == tau ? 1 : 0;
+        run = __reduce_add_sync(kFull, run);
+        if (run == 0) continue;
+        uint32_t phi = 0xFFFFu;  // column ids <= phi are taken
+        if (run > need) {
+          uint32_t x = 0;
+          for (int bit = 10; bit >= 0; --bit) {
+            const uint32_t trial = x | (1u << bit);
+            int under = 0;
+            for (int q = lane; q < nb; q += 32) under += (pair_ord(p, q) == tau && ib[q] < trial) ? 1 : 0;
+            under = __reduce_add_sync(kFull, under);
+            if (under < need) x = trial;
+          }
+          phi = x;
+        }
+        for (int base = 0; base < nb; base += 32) {
+          const int q = base + lane;
+          const bool take = q < nb && pair_ord(p, q < nb ? q : 0) == tau && ib[q < nb ? q : 0] <= phi;
+          const unsigned bal = __ballot_sync(kFull, take);
+          if (take) put(filled + __popc(bal & below), tau, flat_id(p, q));
+          filled += __popc(bal);
+          need -= __popc(bal);
+        }
+      }
+    }
+    __syncwarp();
+
+    // 5. order the winners and write out
+    if (fits) {
+      if (k <= 32) sort_list<T, 1, kUnrollCells>(win32, filled, nullptr, nullptr, lane);
+      else if (k <= 64) sort_list<T, 2, kUnrollCells>(win32, filled, nullptr, nullptr, lane);
+      else sort_list<T, 4, kUnrollCells>(win32, filled, nullptr, nullptr, lane);
+    } else {
+      for (int r = filled + lane; r < kp; r += 32) win[r] = 0;
+      __syncwarp();
+      bitonic_desc(win, nullptr, kp, lane);
+    }
+    float gsum = 0.f;
+    for (int r = lane; r < k; r += 32) {
+      uint64_t ky = 0;
+      if (!fits) {
+        ky = win[r];
+      } else if (r < filled) {
+        const uint32_t w = win32[r];
+        const uint32_t level = (w >> idbits) - 1u + tlevel;
+        // the low bits of a 16-bit value's order key: zeros for positive values, ones for negative ones
+        ky = make_key((level << LOW) | ((level >> (31 - LOW)) != 0 ? 0u : (1u << LOW) - 1u), idmask - (w & idmask));
+      }
+      const float s = key_val(ky);
+      scores[t * k + r] = from_f32<T>(s);
+      indices[t * k + r] = static_cast<int64_t>(key_id(ky));
+      if (gates != nullptr) {
+        const T g = from_f32<T>(expf(s));
+        gsum += to_f32<T>(g);
+        if (!norm) gates[t * k + r] = g;
+      }
+    }
+    if (gates != nullptr && norm) {
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) gsum += __shfl_xor_sync(kFull, gsum, d);
+      const float denom = round_to<T>(gsum);
+      __syncwarp();
+      for (int r = lane; r < k; r += 32) {  // this lane's own scores, written above
+        const float g = round_to<T>(expf(to_f32<T>(scores[t * k + r])));
+        gates[t * k + r] = from_f32<T>(g / denom);
+      }
+    }
+    __syncwarp();
+  }
+}
+
+RouterPrunedLayout make_pruned_layout(int nk, int k) {
+  RouterPrunedLayout L{};
+  L.nkp = next_pow2(nk) < 32 ? 32 : next_pow2(nk);
+  L.kp = next_pow2(k);
+  for (int p = 0; p < k; ++p) L.C += k / (p + 1);
+  L.Cp = (L.C + 3) / 4 * 4;
+  L.cta_bytes = static_cast<int>(align_up(static_cast<size_t>(L.Cp) * 4 + static_cast<size_t>(k) * 4, 16));
+  L.off_ids = 2 * L.nkp * 4;
+  L.off_win = L.off_ids + 2 * L.nkp * 2;
+  L.off_cs = L.off_win + (L.kp < 32 ? 32 : L.kp) * 8;
+  L.off_tl = L.off_cs + (L.C > 320 ? L.Cp * 4 : 0);  // up to 320 sums live in registers only
+  L.warp_bytes = static_cast<int>(align_up(L.off_tl + (kTieCap + 4) * 4, 16));
+  return L;
+}
+
+template <typename T, int E, int CPL>
+int launch_pruned_cpl(const void* logp, int64_t T_, int nk, int k, const RouterPrunedLayout& L, void* scores,
+                      int64_t* indices, void* gates, int norm, cudaStream_t stream) {
+  const int warps = 4;
   const int smem = L.cta_bytes + warps * L.warp_bytes;
-  auto kern = router_topk_reg_kernel<T, E, CPL>;
+  auto kern = router_topk_pruned_kernel<T, E, CPL>;
   FMOE_CUDA_TRY(allow_smem(kern, smem));
   int per_sm = 1;
   FMOE_CUDA_TRY(resident_ctas(kern, warps * 32, smem, &per_sm));
@@ -812,20 +1353,30 @@ int launch_reg_cpl(const void* logp, int64_t T_, int nk, int k, const RouterRegL
   return FMOE_OK;
 }
 
-// 16-bit dtypes with at least 128 keys per half (the shapes of real layers) keep the candidates in registers when
-// there are at most 320 of them (top-k up to 64: 22.5 vs 23.4 us at 4096 tokens x 128 keys, 539 vs 629 us at
-// 131072 x 256 keys, top-32); with 22 per lane (top-128) the shared-memory walk measured faster (348 vs 382 us)
+template <typename T, int E>
+int launch_pruned(const void* logp, int64_t T_, int nk, int k, void* scores, int64_t* indices, void* gates, int norm,
+                  cudaStream_t stream) {
+  const RouterPrunedLayout L = make_pruned_layout(nk, k);
+  if (L.C <= 32 * 4) return launch_pruned_cpl<T, E, 4>(logp, T_, nk, k, L, scores, indices, gates, norm, stream);
+  if (L.C <= 32 * 10) return launch_pruned_cpl<T, E, 10>(logp, T_, nk, k, L, scores, indices, gates, norm, stream);
+  return launch_pruned_cpl<T, E, 22>(logp, T_, nk, k, L, scores, indices, gates, norm, stream);
+}
+
 template <typename T, int E>
 int launch_reg(const void* logp, int64_t T_, int nk, int k, const RouterRegLayout& L, int warps, void* scores,
                int64_t* indices, void* gates, int norm, cudaStream_t stream) {
-  const char* force = std::getenv("FMOE_TOPK_CANDIDATES");  // measurement aid: "smem" forces the shared-memory walk
-  const bool in_regs = force == nullptr || force[0] != 's';
-  if constexpr (sizeof(T) == 2 && E >= 4) {
-    if (!in_regs) return launch_reg_cpl<T, E, 0>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
-    if (L.C <= 32 * 4) return launch_reg_cpl<T, E, 4>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
-    if (L.C <= 32 * 10) return launch_reg_cpl<T, E, 10>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
-  }
-  return launch_reg_cpl<T, E, 0>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
+  const int smem = L.cta_bytes + warps * L.warp_bytes;
+  auto kern = router_topk_reg_kernel<T, E>;
+  FMOE_CUDA_TRY(allow_smem(kern, smem));
+  int per_sm = 1;
+  FMOE_CUDA_TRY(resident_ctas(kern, warps * 32, smem, &per_sm));
+  if (per_sm < 1) per_sm = 1;
+  const int64_t want = (T_ + warps - 1) / warps;
+  const int64_t cap = static_cast<int64_t>(device_sm_count()) * per_sm;
+  const int grid = static_cast<int>(want < cap ? want : cap);
+  FMOE_CUDA_TRY(launch_pdl(2, kern, dim3(grid), dim3(warps * 32), smem, stream, 1, static_cast<const T*>(logp), T_, nk, k, L,
+                           static_cast<T*>(scores), indices, static_cast<T*>(gates), norm));
+  return FMOE_OK;
 }
 
 // register kernel when the halves fit 32 keys per lane and the per-warp scratch stays small
@@ -884,6 +1435,19 @@ int launch_smem(const void* logp, int64_t T_, int nk, int k, void* scores, int64
 template <typename T>
 int launch_typed(const void* logp, int64_t T_, int nk, int k, void* scores, int64_t* indices, void* gates, int norm,
                  cudaStream_t stream) {
+  if constexpr (sizeof(T) == 2) {
+    if (nk <= 1024 && k <= kPrunedMaxK) {
+      switch ((next_pow2(nk) < 32 ? 32 : next_pow2(nk)) / 32) {
+        case 1: return launch_pruned<T, 1>(logp, T_, nk, k, scores, indices, gates, norm, stream);
+        case 2: return launch_pruned<T, 2>(logp, T_, nk, k, scores, indices, gates, norm, stream);
+        case 4: return launch_pruned<T, 4>(logp, T_, nk, k, scores, indices, gates, norm, stream);
+        case 8: return launch_pruned<T, 8>(logp, T_, nk, k, scores, indices, gates, norm, stream);
+        case 16: return launch_pruned<T, 16>(logp, T_, nk, k, scores, indices, gates, norm, stream);
+        default: return launch_pruned<T, 32>(logp, T_, nk, k, scores, indices, gates, norm, stream);
+      }
+    }
+  }
+  // float32, and 16-bit rows of more than 128 winners
   if (nk <= 1024) {
     const RouterRegLayout L = make_reg_layout(nk, k);
     // few tokens per SM: small CTAs spread them over more SMs
@@ -891,9 +1455,15 @@ int launch_typed(const void* logp, int64_t T_, int nk, int k, void* scores, int6
     while (warps > 1 && L.cta_bytes + warps * L.warp_bytes > 96 * 1024) warps >>= 1;
     if (L.cta_bytes + warps * L.warp_bytes <= 200 * 1024) {
       switch (L.nkp / 32) {
-        case 1: return launch_reg<T, 1>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
-        case 2: return launch_reg<T, 2>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
-        case 4: return launch_reg<T, 4>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
+        case 1:
+          if constexpr (sizeof(T) == 4) return launch_reg<T, 1>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
+          break;
+        case 2:
+          if constexpr (sizeof(T) == 4) return launch_reg<T, 2>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
+          break;
+        case 4:
+          if constexpr (sizeof(T) == 4) return launch_reg<T, 4>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
+          break;
         case 8: return launch_reg<T, 8>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
         case 16: return launch_reg<T, 16>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
         case 32: return launch_reg<T, 32>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
