@@ -237,7 +237,7 @@ __global__ void router_topk_smem_kernel(const T* __restrict__ logp, int64_t ntok
 
 
 // ------------------------------------------------------------------------------------------
-// Register-resident variant for num_keys <= 1024: each half is sorted by a shuffle-based bitonic
+// Register-resident variant for num_keys <= 1024 (float32; 16-bit rows of which most is wanted): each half is sorted by a shuffle-based bitonic
 // network (E = padded num_keys / 32 keys per lane), sort keys are 32-bit for 16-bit dtypes
 // (16-bit order key | inverted index) and 64-bit for float32.  Shared memory only holds the
 // sorted halves (for the candidate gathers and binary searches), the index-order values, the
@@ -772,6 +772,12 @@ RouterRegLayout make_reg_layout(int nk, int k) {
 //      logits - is compacted in index order and sorted.
 //   3. Staircase sums, threshold, ties, winners as above; winners are 32-bit keys (level of the score above the threshold
 //      | inverted flat id) wherever the two fit.
+//
+// Bound by one token's chain of dependent instructions (about 24000 cycles at 128 keys, top-64, with seven warps per
+// scheduler) and, with more than 8 keys per lane, by instruction fetch.  us, both halves sorted whole -> this kernel:
+// 16384 x 512 keys top-128 319 -> 214; 8192 x 1024 top-64 349 -> 106; 131072 x 256 top-32 638 -> 396; 4096 x 128 top-64
+// 19.2 -> 20.3; one token 8.2 -> 7.5.  Measured and not kept: cell numbers first and keys in a second loop (214 -> 224),
+// one sort per list or both lists at once (the same), candidates walked in shared memory for top-64 too (396 -> 444).
 // ------------------------------------------------------------------------------------------
 struct RouterPrunedLayout {
   int cta_bytes, warp_bytes;
@@ -1436,9 +1442,11 @@ template <typename T>
 int launch_typed(const void* logp, int64_t T_, int nk, int k, void* scores, int64_t* indices, void* gates, int norm,
                  cudaStream_t stream) {
   if constexpr (sizeof(T) == 2) {
-    if (nk <= 1024 && k <= kPrunedMaxK) {
+    // Not where there is little to drop: one key per lane (20000 x 32 keys top-4: 27 us, 32 pruned), or more than half of a
+    // short row wanted (4096 x 128 top-128: 30 us, 33 pruned).
+    const bool prune = nk > 32 && (nk > 128 || 2 * k <= nk);
+    if (nk <= 1024 && k <= kPrunedMaxK && prune) {
       switch ((next_pow2(nk) < 32 ? 32 : next_pow2(nk)) / 32) {
-        case 1: return launch_pruned<T, 1>(logp, T_, nk, k, scores, indices, gates, norm, stream);
         case 2: return launch_pruned<T, 2>(logp, T_, nk, k, scores, indices, gates, norm, stream);
         case 4: return launch_pruned<T, 4>(logp, T_, nk, k, scores, indices, gates, norm, stream);
         case 8: return launch_pruned<T, 8>(logp, T_, nk, k, scores, indices, gates, norm, stream);
@@ -1447,7 +1455,7 @@ int launch_typed(const void* logp, int64_t T_, int nk, int k, void* scores, int6
       }
     }
   }
-  // float32, and 16-bit rows of more than 128 winners
+  // float32, and the 16-bit shapes the pruned kernel leaves
   if (nk <= 1024) {
     const RouterRegLayout L = make_reg_layout(nk, k);
     // few tokens per SM: small CTAs spread them over more SMs
@@ -1455,15 +1463,9 @@ int launch_typed(const void* logp, int64_t T_, int nk, int k, void* scores, int6
     while (warps > 1 && L.cta_bytes + warps * L.warp_bytes > 96 * 1024) warps >>= 1;
     if (L.cta_bytes + warps * L.warp_bytes <= 200 * 1024) {
       switch (L.nkp / 32) {
-        case 1:
-          if constexpr (sizeof(T) == 4) return launch_reg<T, 1>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
-          break;
-        case 2:
-          if constexpr (sizeof(T) == 4) return launch_reg<T, 2>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
-          break;
-        case 4:
-          if constexpr (sizeof(T) == 4) return launch_reg<T, 4>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
-          break;
+        case 1: return launch_reg<T, 1>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
+        case 2: return launch_reg<T, 2>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
+        case 4: return launch_reg<T, 4>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
         case 8: return launch_reg<T, 8>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
         case 16: return launch_reg<T, 16>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
         case 32: return launch_reg<T, 32>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);

@@ -149,3 +149,20 @@ def test_router_full_size_properties():
     sel = torch.arange(0, T, T // 64)
     want_s, want_i = O.router_topk(lp[:, sel], nk, k)
     assert torch.equal(s[sel].float(), want_s.float()) and torch.equal(i[sel], want_i)
+
+
+@pytest.mark.parametrize(
+    "T,nk,k",
+    [(33, 33, 16), (70, 64, 32), (70, 65, 33), (65, 128, 64), (41, 129, 128), (37, 256, 71), (37, 256, 34), (19, 513, 127),
+     (9, 1024, 128)],
+)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("scale", [0.05, 1.0, 12.0])
+def test_router_pruned_rows(T, nk, k, dtype, scale):
+    """Rows whose keys are dropped below a bound: nearly flat ones (everything stays, many ties), ordinary and peaked ones,
+    at the edges of the keys per lane and of the candidates per lane."""
+    lp = torch.log_softmax(randn((2, T, nk), T + nk + k, torch.float32) * scale, -1).to(dtype).contiguous()
+    want_s, want_i = O.router_topk(lp, nk, k)
+    got_s, got_i = run_router(lp, nk, k)
+    assert torch.equal(got_s.float(), want_s.float())
+    assert torch.equal(got_i, want_i)
