@@ -75,6 +75,9 @@ LAYER_ARGS = struct.Struct("@19Q2q7i2fQqQ")
 assert LAYER_ARGS.size == ctypes.sizeof(LayerArgs)
 
 
+# fmoe_train_args: 22 pointers and sizes up to stream, num_tokens, num_experts, six int32
+TRAIN_ARGS = struct.Struct("@22Q2q6i")
+
 _P = ctypes.c_void_p
 _I = ctypes.c_int
 _L = ctypes.c_int64
@@ -100,6 +103,11 @@ SIGNATURES = {
     "fmoe_expert_forward_saving_scores": (_I, [_P, _P, _P, _P, _P, _P, _P, _I, _I, _L, _I, _L, _I, _P, _Z, _P, _P]),
     "fmoe_expert_backward": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _L, _I, _L, _I, _P, _Z, _P, _P]),
     "fmoe_swiglu_backward": (_I, [_P, _P, _P, _P, _P, _P, _I, _L, _P]),
+    "fmoe_swiglu_backward_rows": (_I, [_P, _P, _P, _P, _P, _I, _L, _I, _P]),
+    "fmoe_train_forward_workspace_bytes": (_Z, [_L, _I, _I, _L, _I, _I]),
+    "fmoe_train_forward": (_I, [ctypes.c_char_p, ctypes.POINTER(_I)]),
+    "fmoe_train_backward_workspace_bytes": (_Z, [_L, _I, _L, _I, _I]),
+    "fmoe_train_backward": (_I, [ctypes.c_char_p]),
     "fmoe_gather_probe": (_I, [_P, _L, _P, _L, _I, _I, _I, _P, _P, _P]),
     "fmoe_rms_norm": (_I, [_P, _P, _P, _I, _L, _I, _F, _P]),
     "fmoe_selftest_wait_timeout": (_I, [ctypes.c_uint64, _P, _P, _P]),
@@ -188,6 +196,15 @@ def call(name: str, device: torch.device, *args) -> int:
         return fn(*args, torch._C._cuda_getCurrentRawStream(index))
     with torch.cuda.device(index):
         return fn(*args, torch._C._cuda_getCurrentRawStream(index))
+
+
+def call_struct(name: str, device: torch.device, *args) -> int:
+    """Run a library function that takes a packed argument block, with `device` current."""
+    fn = getattr(lib(), name)
+    if device_index(device) == torch._C._cuda_getDevice():
+        return fn(*args)
+    with torch.cuda.device(device):
+        return fn(*args)
 
 
 def layer_forward(device: torch.device, args: bytes) -> int:

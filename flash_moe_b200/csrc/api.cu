@@ -177,9 +177,7 @@ int mlp_up(const void* x, const void* gw, const void* uw, void* h, int dtype, in
     return launch_gemm_swiglu_narrow(x, gw, uw, h, dtype, T, I, H, false, status, stream, pre_gate, pre_up);
   if (tc && gemm_pair_supported(T, I, H))
     return launch_gemm_swiglu_pair(x, gw, uw, h, dtype, T, I, H, status, stream, pre_gate, pre_up);
-  if (pre_gate != nullptr || pre_up != nullptr) return FMOE_ERR_UNSUPPORTED;  // only the kernels above keep them
-  if (tc) return launch_gemm_swiglu(x, gw, uw, h, dtype, T, I, H, status, stream);
-  return launch_simt_gemm(x, H, gw, uw, nullptr, h, I, dtype, 1, T, I, H, stream);
+  return launch_simt_gemm(x, H, gw, uw, nullptr, h, I, dtype, 1, T, I, H, stream, nullptr, false, pre_gate, pre_up);
 }
 
 // residual (nullable): [T, H] in the module dtype, added with the float32 addend before the single rounding
@@ -191,7 +189,6 @@ int mlp_down(const void* h, const void* dw, const float* addend, void* out, int 
     return launch_gemm_add_narrow(h, dw, addend, out, dtype, T, H, I, true, status, stream, residual);
   if (tc && gemm_pair_supported(T, H, I))
     return launch_gemm_add_pair(h, dw, addend, out, dtype, T, H, I, status, stream, residual);
-  if (tc) return launch_gemm_add(h, dw, addend, out, dtype, T, H, I, status, stream, residual);
   return launch_simt_gemm(h, I, dw, nullptr, addend, out, H, dtype, 0, T, H, I, stream, residual);
 }
 
@@ -337,7 +334,14 @@ int fmoe_expert_backward(const void* dout, const void* x, const void* down, cons
 int fmoe_swiglu_backward(const void* dh, const void* a, const void* b, void* da, void* db, void* h, int dtype,
                          int64_t num_elements, fmoe_stream_t stream) {
   if (!valid_dtype(dtype)) return FMOE_ERR_BAD_ARG;
-  return launch_swiglu_backward(dh, a, b, da, db, h, dtype, num_elements, static_cast<cudaStream_t>(stream));
+  return launch_swiglu_backward(dh, a, b, da, db, h, dtype, num_elements, 0, static_cast<cudaStream_t>(stream));
+}
+
+int fmoe_swiglu_backward_rows(const void* dh, const void* a, const void* b, void* dab, void* h, int dtype, int64_t num_rows,
+                              int intermediate, fmoe_stream_t stream) {
+  if (!valid_dtype(dtype) || num_rows < 0 || intermediate <= 0) return FMOE_ERR_BAD_ARG;
+  return launch_swiglu_backward(dh, a, b, dab, static_cast<char*>(dab) + static_cast<size_t>(intermediate) * dtype_size(dtype),
+                                h, dtype, num_rows * intermediate, intermediate, static_cast<cudaStream_t>(stream));
 }
 
 int fmoe_gather_probe(const void* table, int64_t num_rows, const int32_t* row_ids, int64_t count, int row_bytes,
@@ -546,6 +550,81 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   FMOE_MARK(FMOE_STAGE_MLP_DOWN, 1, s);
 #undef FMOE_MARK
   return FMOE_OK;
+}
+
+namespace {
+struct TrainWs {
+  void *scores, *acc, *h, *expert;
+  size_t expert_bytes, total;
+};
+TrainWs carve_train(void* ws, int64_t T, int H, int I, int64_t N, int k, int dtype) {
+  Carver c(ws);
+  TrainWs w;
+  w.scores = c.take(static_cast<size_t>(T) * k * dtype_size(dtype));
+  w.acc = c.take(static_cast<size_t>(T) * H * 4);
+  w.h = c.take(static_cast<size_t>(T) * I * dtype_size(dtype));
+  w.expert_bytes = expert_workspace_bytes(T, H, N, k);
+  w.expert = c.take(w.expert_bytes);
+  w.total = c.off;
+  return w;
+}
+bool train_args_ok(const fmoe_train_args* a) {
+  return a != nullptr && valid_dtype(a->dtype) && a->num_tokens > 0 && a->num_experts > 0 && a->hidden > 0 &&
+         a->intermediate > 0 && a->num_keys > 0 && a->top_k > 0 && a->top_k <= a->num_keys &&
+         static_cast<int64_t>(a->num_keys) * a->num_keys <= a->num_experts && a->x && a->log_probs && a->down_embed &&
+         a->up_embed && a->indices && a->gates && a->expert_scores && a->workspace;
+}
+}  // namespace
+
+size_t fmoe_train_forward_workspace_bytes(int64_t num_tokens, int hidden, int intermediate, int64_t num_experts, int top_k,
+                                          int dtype) {
+  if (num_tokens < 0 || hidden <= 0 || intermediate <= 0 || num_experts <= 0 || top_k < 0) return 0;
+  return carve_train(nullptr, num_tokens, hidden, intermediate, num_experts, top_k, dtype).total;
+}
+
+int fmoe_train_forward(const fmoe_train_args* a, int* have_preacts) {
+  if (!train_args_ok(a) || have_preacts == nullptr || !a->gate_proj || !a->up_proj || !a->down_proj || !a->y)
+    return FMOE_ERR_BAD_ARG;
+  const int64_t T = a->num_tokens, N = a->num_experts;
+  const int H = a->hidden, I = a->intermediate, nk = a->num_keys, k = a->top_k, dtype = a->dtype;
+  const TrainWs w = carve_train(a->workspace, T, H, I, N, k, dtype);
+  if (a->workspace_bytes < w.total) return FMOE_ERR_WORKSPACE;
+  cudaStream_t s = static_cast<cudaStream_t>(a->stream);
+  int rc = launch_router_topk(a->log_probs, dtype, T, nk, k, w.scores, a->indices, a->gates, (a->norm_topk_prob ? 1 : 0) | 4, s);
+  if (rc != FMOE_OK) return rc;
+  rc = launch_expert_forward(a->x, a->down_embed, a->up_embed, a->indices, a->gates, w.acc, dtype, FMOE_DTYPE_F32, T, H, N, k,
+                             w.expert, w.expert_bytes, a->status, s, nullptr, kActSilu, a->expert_scores);
+  if (rc != FMOE_OK) return rc;
+  *have_preacts = a->pre_gate != nullptr && a->pre_up != nullptr ? 1 : 0;
+  rc = mlp_up(a->x, a->gate_proj, a->up_proj, w.h, dtype, T, H, I, a->status, s, a->pre_gate, a->pre_up);
+  if (rc == FMOE_ERR_UNSUPPORTED && *have_preacts) {
+    *have_preacts = 0;
+    rc = mlp_up(a->x, a->gate_proj, a->up_proj, w.h, dtype, T, H, I, a->status, s);
+  }
+  if (rc != FMOE_OK) return rc;
+  return mlp_down(w.h, a->down_proj, static_cast<const float*>(w.acc), a->y, dtype, T, H, I, a->status, s);
+}
+
+size_t fmoe_train_backward_workspace_bytes(int64_t num_tokens, int hidden, int64_t num_experts, int top_k, int dtype) {
+  if (num_tokens < 0 || hidden <= 0 || num_experts <= 0 || top_k < 0) return 0;
+  return align_up(static_cast<size_t>(num_tokens) * top_k * dtype_size(dtype), 256) +
+         expert_backward_workspace_bytes(num_tokens, hidden, num_experts, top_k);
+}
+
+int fmoe_train_backward(const fmoe_train_args* a) {
+  if (!train_args_ok(a) || !a->dy || !a->dx_experts || !a->ddown || !a->dup || !a->dlogits) return FMOE_ERR_BAD_ARG;
+  const int64_t T = a->num_tokens, N = a->num_experts;
+  const int H = a->hidden, nk = a->num_keys, k = a->top_k, dtype = a->dtype;
+  if (a->workspace_bytes < fmoe_train_backward_workspace_bytes(T, H, N, k, dtype)) return FMOE_ERR_WORKSPACE;
+  Carver c(a->workspace);
+  void* dgates = c.take(static_cast<size_t>(T) * k * dtype_size(dtype));
+  cudaStream_t s = static_cast<cudaStream_t>(a->stream);
+  int rc = launch_expert_backward(a->dy, a->x, a->down_embed, a->up_embed, a->indices, a->gates, a->dx_experts, a->ddown,
+                                  a->dup, dgates, dtype, T, H, N, k, static_cast<char*>(a->workspace) + c.off,
+                                  a->workspace_bytes - c.off, a->status, s, a->expert_scores);
+  if (rc != FMOE_OK) return rc;
+  return launch_router_chain_backward(dgates, a->gates, a->indices, a->log_probs, a->dlogits, dtype, T, nk, k,
+                                      a->norm_topk_prob ? 1 : 0, s);
 }
 
 }  // extern "C"

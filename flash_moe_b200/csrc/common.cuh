@@ -211,8 +211,6 @@ int launch_weighted_rows(const void* values, const void* weights, const int64_t*
 // and before the accumulate pass.
 
 // C[M,N] = A[M,K] * B[N,K]^T on tcgen05 with a fused epilogue (gemm_sm100.cu); bf16/fp16 only.
-int launch_gemm_swiglu(const void* x, const void* gate_w, const void* up_w, void* h, int dtype, int64_t M, int I, int K,
-                       int32_t* status, cudaStream_t stream);
 // residual (nullable): [M, N] in the module dtype, added to the float32 sum before the single rounding
 int launch_gemm_add(const void* a, const void* b, const float* addend, void* out, int dtype, int64_t M, int N, int K,
                     int32_t* status, cudaStream_t stream, const void* residual = nullptr);
@@ -249,7 +247,8 @@ int launch_gemm_add_narrow(const void* a, const void* b, const float* addend, vo
 // is one fmaf chain over ascending k (the router's logits, whose last bit decides between experts).
 int launch_simt_gemm(const void* a, int64_t lda, const void* b0, const void* b1, const float* addend, void* out,
                      int64_t ldo, int dtype, int swiglu, int64_t M, int N, int K, cudaStream_t stream,
-                     const void* residual = nullptr, bool ordered = false);
+                     const void* residual = nullptr, bool ordered = false, void* pre_gate = nullptr,
+                     void* pre_up = nullptr);
 
 // elementwise.cu
 int launch_log_softmax_halves(const void* logits, void* log_probs, int dtype, int64_t T, int nk, cudaStream_t stream);
@@ -260,8 +259,12 @@ int launch_expert_backward(const void* dout, const void* x, const void* down, co
                            const float* saved_scores = nullptr);
 int launch_router_topk_backward(const void* dscores, const int64_t* indices, int dtype, int64_t T, int nk, int k,
                                 void* dlog_probs, cudaStream_t stream);
+// dlogits [T, 2 nk] from the gradients of the gates: gates (exp, renormalised or not), top-k and log-softmax backwards
+int launch_router_chain_backward(const void* dgates, const void* gates, const int64_t* indices, const void* log_probs,
+                                 void* dlogits, int dtype, int64_t T, int nk, int k, int norm, cudaStream_t stream);
+// row > 0: da and db are the halves of rows of 2 * row elements (db = da + row)
 int launch_swiglu_backward(const void* dh, const void* a, const void* b, void* da, void* db, void* h, int dtype,
-                           int64_t n, cudaStream_t stream);
+                           int64_t n, int64_t row, cudaStream_t stream);
 int launch_gather_probe(const void* table, int64_t num_rows, const int32_t* row_ids, int64_t count, int row_bytes,
                         int ctas_per_sm, int mode, float* sink, int32_t* status, cudaStream_t stream);
 int launch_rms_norm(const void* x, const void* weight, void* out, int dtype, int64_t ntok, int H, float eps,

@@ -9,7 +9,6 @@
 //   warps 2..5         epilogue: tcgen05.ld the finished accumulator (one row per thread) while the
 //                      next tile's MMAs fill the other accumulator.
 // Fused epilogues:
-//   SWIGLU  B tile = 128 gate rows + 128 up rows of the same columns -> h = silu(g) * u   (bf16)
 //   ADD     out = acc (+ fp32 addend), one rounding                                        (bf16)
 //   ROUTER  one router half per N tile: logits rounded to the module dtype, then the per-half
 //           log-softmax of those rounded logits (flash_moe/modules/flash_moe.py:65-72)
@@ -28,15 +27,15 @@ constexpr int kThreads = 192;
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr int kSmemLimit = 227 * 1024;
 
-enum { EPI_ADD = 0, EPI_SWIGLU = 1, EPI_ROUTER = 2 };
+enum { EPI_ADD = 0, EPI_ROUTER = 2 };
 
 struct EpiParams {
-  void* out;            // ADD: out[M, ldo]; SWIGLU: h[M, ldo]; ROUTER: logits[M, ldo]
+  void* out;            // ADD: out[M, ldo]; ROUTER: logits[M, ldo]
   void* out2;           // ROUTER: log_probs[2, M, n_valid]
   const float* addend;  // ADD: optional fp32 [M, ldo]
   const void* residual; // ADD: optional [M, ldo] in the module dtype, added before the single rounding
   int64_t ldo;
-  int n_valid;      // ADD: N; SWIGLU: I; ROUTER: num_keys
+  int n_valid;      // ADD: N; ROUTER: num_keys
   int a_half_koff;  // ROUTER: K offset of half 1 inside a row of A
 };
 
@@ -55,8 +54,7 @@ using epi::UmmaFmt;
 
 template <int BLOCK_N, int EPI, typename T>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB0,
-                    const __grid_constant__ CUtensorMap tmB1, EpiParams ep, int M, int num_m_tiles, int num_n_tiles,
+gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB0, EpiParams ep, int M, int num_m_tiles, int num_n_tiles,
                     int num_k_blocks, int32_t* status) {
   using C = Cfg<BLOCK_N>;
   constexpr int STAGES = C::STAGES;
@@ -91,7 +89,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     ptx::mbar_fence_init();
     ptx::prefetch_tensormap(&tmA);
     ptx::prefetch_tensormap(&tmB0);
-    if (EPI == EPI_SWIGLU) ptx::prefetch_tensormap(&tmB1);
   }
   if (warp == 1) {
     ptx::tmem_alloc(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), C::TMEM_COLS);
@@ -117,10 +114,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           if (!ptx::mbar_wait_bounded(empty_bar(s), ph ^ 1u, abort_flag)) { ok = false; break; }
           ptx::mbar_arrive_expect_tx(full_bar(s), C::STAGE_BYTES);
           ptx::tma_load_2d(a_smem(s), &tmA, full_bar(s), a_k0 + kb * BLOCK_K, m_tile * BLOCK_M);
-          if (EPI == EPI_SWIGLU) {
-            ptx::tma_load_2d(b_smem(s), &tmB0, full_bar(s), kb * BLOCK_K, n_tile * (BLOCK_N / 2));
-            ptx::tma_load_2d(b_smem(s) + C::B_BYTES / 2, &tmB1, full_bar(s), kb * BLOCK_K, n_tile * (BLOCK_N / 2));
-          } else if (EPI == EPI_ROUTER) {
+          if (EPI == EPI_ROUTER) {
             ptx::tma_load_2d(b_smem(s), &tmB0, full_bar(s), kb * BLOCK_K, n_tile * ep.n_valid);
           } else {
             ptx::tma_load_2d(b_smem(s), &tmB0, full_bar(s), kb * BLOCK_K, n_tile * BLOCK_N);
@@ -183,10 +177,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int64_t row = static_cast<int64_t>(m_tile) * BLOCK_M + row_in_tile;
       const bool row_ok = row < M;
 
-      if constexpr (EPI == EPI_SWIGLU) {
-        T* orow = static_cast<T*>(ep.out) + row * ep.ldo;
-        epi::store_swiglu_row<T, BLOCK_N>(taddr, orow, nullptr, nullptr, n_tile * (BLOCK_N / 2), ep.n_valid, row_ok);
-      } else if constexpr (EPI == EPI_ADD) {
+      if constexpr (EPI == EPI_ADD) {
         T* orow = static_cast<T*>(ep.out) + row * ep.ldo;
         const float* arow = (ep.addend != nullptr && row_ok) ? ep.addend + row * ep.ldo : nullptr;
         const T* rrow = (ep.residual != nullptr && row_ok) ? static_cast<const T*>(ep.residual) + row * ep.ldo : nullptr;
@@ -280,7 +271,7 @@ int make_tmap(CUtensorMap* m, const void* basep, int dtype, uint64_t cols, uint6
 }
 
 template <int BLOCK_N, int EPI, typename T>
-int launch(const CUtensorMap& tA, const CUtensorMap& tB0, const CUtensorMap& tB1, const EpiParams& ep, int64_t M,
+int launch(const CUtensorMap& tA, const CUtensorMap& tB0, const EpiParams& ep, int64_t M,
            int num_n_tiles, int K, int32_t* status, cudaStream_t stream) {
   using C = Cfg<BLOCK_N>;
   auto kern = gemm_tcgen05_kernel<BLOCK_N, EPI, T>;
@@ -290,7 +281,7 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB0, const CUtensorMap& tB1
   const int64_t tiles = static_cast<int64_t>(num_m_tiles) * num_n_tiles;
   const int sms = device_sm_count();
   const int grid = static_cast<int>(tiles < sms ? tiles : sms);
-  kern<<<grid, kThreads, C::SMEM_BYTES, stream>>>(tA, tB0, tB1, ep, static_cast<int>(M), num_m_tiles, num_n_tiles,
+  kern<<<grid, kThreads, C::SMEM_BYTES, stream>>>(tA, tB0, ep, static_cast<int>(M), num_m_tiles, num_n_tiles,
                                                   num_k_blocks, status);
   FMOE_LAUNCH_CHECK();
   return FMOE_OK;
@@ -306,23 +297,6 @@ int check_gemm_args(const void* a, const void* b, const void* out, int dtype, in
 }
 
 }  // namespace
-
-int launch_gemm_swiglu(const void* x, const void* gate_w, const void* up_w, void* h, int dtype, int64_t M, int I, int K,
-                       int32_t* status, cudaStream_t stream) {
-  int rc = check_gemm_args(x, gate_w, h, dtype, M, K);
-  if (rc != FMOE_OK) return rc;
-  if (up_w == nullptr || I <= 0) return FMOE_ERR_BAD_ARG;
-  if (I % 8 != 0 || !aligned16(up_w)) return FMOE_ERR_ALIGNMENT;
-  CUtensorMap tA, tG, tU;
-  if ((rc = make_tmap(&tA, x, dtype, K, M, K, BLOCK_M)) != FMOE_OK) return rc;
-  if ((rc = make_tmap(&tG, gate_w, dtype, K, I, K, 128)) != FMOE_OK) return rc;
-  if ((rc = make_tmap(&tU, up_w, dtype, K, I, K, 128)) != FMOE_OK) return rc;
-  EpiParams ep{h, nullptr, nullptr, nullptr, I, I, 0};
-  const int n_tiles = (I + 127) / 128;
-  if (dtype == FMOE_DTYPE_BF16)
-    return launch<256, EPI_SWIGLU, __nv_bfloat16>(tA, tG, tU, ep, M, n_tiles, K, status, stream);
-  return launch<256, EPI_SWIGLU, __half>(tA, tG, tU, ep, M, n_tiles, K, status, stream);
-}
 
 int launch_gemm_add(const void* a, const void* b, const float* addend, void* out, int dtype, int64_t M, int N, int K,
                     int32_t* status, cudaStream_t stream, const void* residual) {
@@ -340,14 +314,14 @@ int launch_gemm_add(const void* a, const void* b, const float* addend, void* out
     if ((rc = make_tmap(&tB, b, dtype, K, N, K, 256)) != FMOE_OK) return rc;
     const int n_tiles = (N + 255) / 256;
     if (dtype == FMOE_DTYPE_BF16)
-      return launch<256, EPI_ADD, __nv_bfloat16>(tA, tB, tB, ep, M, n_tiles, K, status, stream);
-    return launch<256, EPI_ADD, __half>(tA, tB, tB, ep, M, n_tiles, K, status, stream);
+      return launch<256, EPI_ADD, __nv_bfloat16>(tA, tB, ep, M, n_tiles, K, status, stream);
+    return launch<256, EPI_ADD, __half>(tA, tB, ep, M, n_tiles, K, status, stream);
   }
   if ((rc = make_tmap(&tB, b, dtype, K, N, K, 128)) != FMOE_OK) return rc;
   const int n_tiles = (N + 127) / 128;
   if (dtype == FMOE_DTYPE_BF16)
-    return launch<128, EPI_ADD, __nv_bfloat16>(tA, tB, tB, ep, M, n_tiles, K, status, stream);
-  return launch<128, EPI_ADD, __half>(tA, tB, tB, ep, M, n_tiles, K, status, stream);
+    return launch<128, EPI_ADD, __nv_bfloat16>(tA, tB, ep, M, n_tiles, K, status, stream);
+  return launch<128, EPI_ADD, __half>(tA, tB, ep, M, n_tiles, K, status, stream);
 }
 
 bool gemm_router_fused_supported(int nk) { return nk >= 1 && nk <= 256; }
@@ -367,8 +341,8 @@ int launch_gemm_router(const void* xn, int64_t a_cols, int a_half_koff, const vo
 #define FMOE_ROUTER_CASE(BN)                                                                               \
   case BN:                                                                                                 \
     if (dtype == FMOE_DTYPE_BF16)                                                                          \
-      return launch<BN, EPI_ROUTER, __nv_bfloat16>(tA, tB, tB, ep, M, 2, K, status, stream);               \
-    return launch<BN, EPI_ROUTER, __half>(tA, tB, tB, ep, M, 2, K, status, stream);
+      return launch<BN, EPI_ROUTER, __nv_bfloat16>(tA, tB, ep, M, 2, K, status, stream);               \
+    return launch<BN, EPI_ROUTER, __half>(tA, tB, ep, M, 2, K, status, stream);
   switch (bn) {
     FMOE_ROUTER_CASE(32)
     FMOE_ROUTER_CASE(64)

@@ -467,8 +467,9 @@ int launch_narrow(const void* w0, const void* w1, const void* x, const NarrowEpi
 
 // 16-bit operands with 16-byte aligned rows (K % 8 == 0), where the estimate is below that of the pair tiles
 bool gemm_narrow_preferred(int64_t M, int N, int K, bool swiglu) {
-  if (M <= 0 || M > 8192 || N <= 0 || K <= 0 || K % 8 != 0) return false;
+  if (M <= 0 || M > (int64_t{1} << 23) || N <= 0 || K <= 0 || K % 8 != 0) return false;
   if (!gemm_pair_supported(M, N, K)) return true;
+  if (M > 8192) return false;
   return plan_narrow(M, N, K, swiglu ? 2 : 1).cost < pair_cost(M, N, K, swiglu ? 2 : 1);
 }
 

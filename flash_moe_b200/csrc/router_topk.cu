@@ -66,7 +66,9 @@ struct RouterSmemLayout {
 template <typename T>
 __global__ void router_topk_smem_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int k, RouterSmemLayout L,
                                    T* __restrict__ scores, int64_t* __restrict__ indices, T* __restrict__ gates,
-                                   int norm) {
+                                   int flags) {
+  const int norm = flags & 1;
+  const bool token_rows = (flags & 4) != 0;  // [T, 2, nk] instead of [2, T, nk]
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -114,8 +116,8 @@ __global__ void router_topk_smem_kernel(const T* __restrict__ logp, int64_t ntok
 
   for (int64_t t = static_cast<int64_t>(blockIdx.x) * nwarps + warp; t < ntok;
        t += static_cast<int64_t>(gridDim.x) * nwarps) {
-    const T* a_row = logp + t * nk;
-    const T* b_row = logp + (ntok + t) * nk;
+    const T* a_row = token_rows ? logp + t * 2 * nk : logp + t * nk;
+    const T* b_row = token_rows ? a_row + nk : logp + (ntok + t) * nk;
     // 1. load (canonicalising -0 to +0) and build sort keys
     for (int i = lane; i < nkp; i += 32) {
       if (i < nk) {
@@ -386,6 +388,7 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restric
                                                              int flags) {
   const int norm = flags & 1;
   const bool from_logits = (flags & 2) != 0;
+  const bool token_rows = (flags & 6) != 0;  // [T, 2, nk] instead of [2, T, nk]
   using HK = HalfKey<T>;
   using K = typename HK::type;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -443,8 +446,8 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restric
     if (t + static_cast<int64_t>(gridDim.x) * nwarps >= ntok) pdl_launch_dependents();  // last token of this warp
     // from_logits: the input is the raw router logits [T, 2*nk]; the per-half log-softmax
     // (flash_moe/modules/flash_moe.py:72) is applied here, rounded to T like torch does
-    const T* a_row = from_logits ? logp + t * 2 * nk : logp + t * nk;
-    const T* b_row = from_logits ? a_row + nk : logp + (ntok + t) * nk;
+    const T* a_row = token_rows ? logp + t * 2 * nk : logp + t * nk;
+    const T* b_row = token_rows ? a_row + nk : logp + (ntok + t) * nk;
     // 1. per half: load (lane-blocked: element lane * E + r in register r), optional log-softmax, keep the
     //    index-order copy, sort in registers, store the rank-order values and ids.  The two halves run through ONE copy
     //    of this code (the loop is not unrolled): the unrolled sorting network is most of the kernel's instructions -
@@ -932,6 +935,7 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
   constexpr bool kUnrollCells = CPL <= 10;  // see sort_desc: small kernels are unrolled, large ones are loops
   const int norm = flags & 1;
   const bool from_logits = (flags & 2) != 0;
+  const bool token_rows = (flags & 6) != 0;  // [T, 2, nk] instead of [2, T, nk]
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -991,8 +995,8 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
     if (t + static_cast<int64_t>(gridDim.x) * nwarps >= ntok) pdl_launch_dependents();  // last token of this warp
     // 1. load both halves (lane-blocked: element lane * E + r in register r), from_logits: the per-half log-softmax
     //    (flash_moe/modules/flash_moe.py:72) rounded to T like torch does; lane maxima
-    const T* a_row = from_logits ? logp + t * 2 * nk : logp + t * nk;
-    const T* b_row = from_logits ? a_row + nk : logp + (ntok + t) * nk;
+    const T* a_row = token_rows ? logp + t * 2 * nk : logp + t * nk;
+    const T* b_row = token_rows ? a_row + nk : logp + (ntok + t) * nk;
     uint32_t* la = reinterpret_cast<uint32_t*>(sa);
     uint32_t* lb_list = reinterpret_cast<uint32_t*>(sb);
     uint32_t key[kKeysInRegs ? 2 : 1][E];
@@ -1479,7 +1483,8 @@ int launch_typed(const void* logp, int64_t T_, int nk, int k, void* scores, int6
 
 }  // namespace
 
-// norm: bit 0 = renormalise the gates per token, bit 1 = `log_probs` holds raw logits [T, 2*nk]
+// norm: bit 0 = renormalise the gates per token, bit 1 = `log_probs` holds raw logits [T, 2*nk], bit 2 = it holds
+// log-probabilities [T, 2, nk]
 int launch_router_topk(const void* log_probs, int dtype, int64_t T, int nk, int k, void* scores, int64_t* indices,
                        void* gates, int norm, cudaStream_t stream) {
   if (T < 0 || nk <= 0 || k < 0 || k > nk) return FMOE_ERR_BAD_ARG;

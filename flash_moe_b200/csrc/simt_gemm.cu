@@ -38,7 +38,7 @@ template <int BM, int BN, int TM, int TN, int KG, int STAGES, bool SWIGLU>
 __global__ void __launch_bounds__(SgemmCfg<BM, BN, TM, TN, KG, STAGES, SWIGLU>::THREADS)
 sgemm_kernel(const float* __restrict__ A, int64_t lda, const float* __restrict__ B0, const float* __restrict__ B1,
              const float* __restrict__ addend, const float* __restrict__ residual, float* __restrict__ out, int64_t ldo,
-             int M, int N, int K) {
+             int M, int N, int K, float* __restrict__ pre_gate, float* __restrict__ pre_up) {
   using C = SgemmCfg<BM, BN, TM, TN, KG, STAGES, SWIGLU>;
   extern __shared__ float4 sg_smem[];
   float* sm = reinterpret_cast<float*>(sg_smem);
@@ -118,6 +118,10 @@ sgemm_kernel(const float* __restrict__ A, int64_t lda, const float* __restrict__
     if (m >= M || n >= N) return;
     const int64_t o = static_cast<int64_t>(m) * ldo + n;
     if (SWIGLU) {
+      if (pre_gate != nullptr) {
+        pre_gate[o] = v;
+        pre_up[o] = u;
+      }
       v = (v / (1.0f + expf(-v))) * u;
     } else {
       if (addend != nullptr) v += addend[o];
@@ -160,12 +164,12 @@ sgemm_kernel(const float* __restrict__ A, int64_t lda, const float* __restrict__
 
 template <int BM, int BN, int TM, int TN, int KG, int STAGES, bool SWIGLU>
 int run_sgemm(const float* a, int64_t lda, const float* b0, const float* b1, const float* addend, float* out, int64_t ldo,
-              int64_t M, int N, int K, cudaStream_t stream, const float* residual) {
+              int64_t M, int N, int K, cudaStream_t stream, const float* residual, float* pre_gate, float* pre_up) {
   using C = SgemmCfg<BM, BN, TM, TN, KG, STAGES, SWIGLU>;
   auto kern = sgemm_kernel<BM, BN, TM, TN, KG, STAGES, SWIGLU>;
   FMOE_CUDA_TRY(allow_smem(kern, C::SMEM));
   kern<<<dim3((N + BN - 1) / BN, static_cast<unsigned>((M + BM - 1) / BM)), C::THREADS, C::SMEM, stream>>>(
-      a, lda, b0, b1, addend, residual, out, ldo, static_cast<int>(M), N, K);
+      a, lda, b0, b1, addend, residual, out, ldo, static_cast<int>(M), N, K, pre_gate, pre_up);
   FMOE_LAUNCH_CHECK();
   return FMOE_OK;
 }
@@ -174,16 +178,20 @@ int run_sgemm(const float* a, int64_t lda, const float* b0, const float* b1, con
 // unsplit.
 template <bool SWIGLU>
 int pick_sgemm(const float* a, int64_t lda, const float* b0, const float* b1, const float* addend, float* out,
-               int64_t ldo, bool ordered, int64_t M, int N, int K, cudaStream_t stream, const float* residual) {
+               int64_t ldo, bool ordered, int64_t M, int N, int K, cudaStream_t stream, const float* residual,
+               float* pre_gate, float* pre_up) {
   const int64_t sms = device_sm_count();
   auto tiles = [&](int bm, int bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
   constexpr int WIDE = SWIGLU ? 64 : 128;  // both operands of the SwiGLU count as columns
   if (tiles(128, WIDE) >= sms)
-    return run_sgemm<128, WIDE, 8, WIDE / 16, 1, 4, SWIGLU>(a, lda, b0, b1, addend, out, ldo, M, N, K, stream, residual);
-  if (ordered) return run_sgemm<32, 32, 2, 4, 1, 6, SWIGLU>(a, lda, b0, b1, addend, out, ldo, M, N, K, stream, residual);
+    return run_sgemm<128, WIDE, 8, WIDE / 16, 1, 4, SWIGLU>(a, lda, b0, b1, addend, out, ldo, M, N, K, stream, residual, pre_gate,
+                                                      pre_up);
+  if (ordered) return run_sgemm<32, 32, 2, 4, 1, 6, SWIGLU>(a, lda, b0, b1, addend, out, ldo, M, N, K, stream, residual,
+                                                            pre_gate, pre_up);
   if (tiles(64, 64) >= sms)
-    return run_sgemm<64, 64, 4, SWIGLU ? 4 : 8, 2, 4, SWIGLU>(a, lda, b0, b1, addend, out, ldo, M, N, K, stream, residual);
-  return run_sgemm<32, 32, 4, 4, 4, 4, SWIGLU>(a, lda, b0, b1, addend, out, ldo, M, N, K, stream, residual);
+    return run_sgemm<64, 64, 4, SWIGLU ? 4 : 8, 2, 4, SWIGLU>(a, lda, b0, b1, addend, out, ldo, M, N, K, stream, residual,
+                                                              pre_gate, pre_up);
+  return run_sgemm<32, 32, 4, 4, 4, 4, SWIGLU>(a, lda, b0, b1, addend, out, ldo, M, N, K, stream, residual, pre_gate, pre_up);
 }
 
 // ---------------------------------------------------------------- any type, any alignment
@@ -276,7 +284,7 @@ int run(const void* a, int64_t lda, const void* b0, const void* b1, const float*
 
 int launch_simt_gemm(const void* a, int64_t lda, const void* b0, const void* b1, const float* addend, void* out,
                      int64_t ldo, int dtype, int swiglu, int64_t M, int N, int K, cudaStream_t stream,
-                     const void* residual, bool ordered) {
+                     const void* residual, bool ordered, void* pre_gate, void* pre_up) {
   if (a == nullptr || b0 == nullptr || out == nullptr || (swiglu && b1 == nullptr)) return FMOE_ERR_BAD_ARG;
   if (M <= 0 || N <= 0 || K <= 0 || M > 0x7FFFFFFFll - TM || (M + TM - 1) / TM > 65535) return FMOE_ERR_UNSUPPORTED;
   const bool rows16 = dtype == FMOE_DTYPE_F32 && K % 4 == 0 && lda % 4 == 0 && aligned16(a) && aligned16(b0) &&
@@ -285,9 +293,11 @@ int launch_simt_gemm(const void* a, int64_t lda, const void* b0, const void* b1,
     const float *af = static_cast<const float*>(a), *bf = static_cast<const float*>(b0), *cf = static_cast<const float*>(b1);
     const float* rf = static_cast<const float*>(residual);
     float* of = static_cast<float*>(out);
-    return swiglu ? pick_sgemm<true>(af, lda, bf, cf, nullptr, of, ldo, ordered, M, N, K, stream, nullptr)
-                  : pick_sgemm<false>(af, lda, bf, nullptr, addend, of, ldo, ordered, M, N, K, stream, rf);
+    return swiglu ? pick_sgemm<true>(af, lda, bf, cf, nullptr, of, ldo, ordered, M, N, K, stream, nullptr,
+                                     static_cast<float*>(pre_gate), static_cast<float*>(pre_up))
+                  : pick_sgemm<false>(af, lda, bf, nullptr, addend, of, ldo, ordered, M, N, K, stream, rf, nullptr, nullptr);
   }
+  if (pre_gate != nullptr || pre_up != nullptr) return FMOE_ERR_UNSUPPORTED;  // only the kernel above keeps them
   switch (dtype) {
     case FMOE_DTYPE_F32: return run<float>(a, lda, b0, b1, addend, out, ldo, swiglu, M, N, K, stream, residual);
     case FMOE_DTYPE_BF16: return run<__nv_bfloat16>(a, lda, b0, b1, addend, out, ldo, swiglu, M, N, K, stream, residual);

@@ -23,6 +23,10 @@ from .. import _lib
 _WEIGHT_MODULES = ("gate_proj", "up_proj", "down_proj", "router_gate", "down_embed", "up_embed")
 
 
+def _hooked(module: nn.Module) -> bool:
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
+
+
 class FlashMoEConfig:
     """Same six fields and defaults as the reference (flash_moe/modules/flash_moe.py:12-27)."""
 
@@ -140,6 +144,25 @@ class FlashMoE(nn.Module):
         return n
 
     def _forward_differentiable(self, hidden_states, return_routing=False):
+        """The layer with a graph recorded: the batch-norm as torch's module, everything behind it as one autograd node.  A
+        router_gate that is not a plain Linear (wrapped, hooked, with a bias) takes the chain of separate nodes."""
+        gate = self.router_gate
+        k = self.top_k
+        if type(gate) is not nn.Linear or gate.bias is not None or _hooked(gate) or k == 0 or hidden_states.numel() == 0 \
+                or self.hidden_size % (16 // hidden_states.element_size()) or self.intermediate_size % (16 // hidden_states.element_size()):
+            return self._forward_chain(hidden_states, return_routing)
+        from .training import LayerTrainingStep
+
+        bsz, seq_len, _ = hidden_states.shape
+        x = hidden_states.reshape(-1, self.hidden_size)
+        y, router_logits, indices, gates = LayerTrainingStep.apply(
+            x, self.router_norm(x), gate.weight, self.gate_proj.weight, self.up_proj.weight, self.down_proj.weight,
+            self.down_embed.weight, self.up_embed.weight, self.num_keys, k, self.norm_topk_prob)
+        if return_routing:
+            self.last_indices, self.last_gates = indices, gates
+        return y.view(bsz, seq_len, -1), router_logits.view(x.shape[0], 2, -1).transpose(0, 1)
+
+    def _forward_chain(self, hidden_states, return_routing=False):
         """The layer as a chain of autograd nodes (same order of operations as the reference module)."""
         from ..ops.flash_expert import flash_expert_func
         from ..ops.flash_mlp import flash_mlp_func

@@ -151,6 +151,9 @@ int fmoe_expert_backward(const void* dout, const void* x, const void* down, cons
                          size_t workspace_bytes, int32_t* status, fmoe_stream_t stream);
 int fmoe_swiglu_backward(const void* dh, const void* a, const void* b, void* da, void* db, void* h, int dtype,
                          int64_t num_elements, fmoe_stream_t stream);
+/* the same for a, b, h [rows, I] with both gradients in one buffer, dab [rows, 2 I] = [da | db] */
+int fmoe_swiglu_backward_rows(const void* dh, const void* a, const void* b, void* dab, void* h, int dtype, int64_t num_rows,
+                              int intermediate, fmoe_stream_t stream);
 
 /*
  * NOT PART OF THE LAYER - a measurement aid with no counterpart in the reference, exported only so that the
@@ -317,6 +320,55 @@ typedef struct fmoe_layer_args {
 size_t fmoe_layer_workspace_bytes(int64_t num_tokens, int hidden, int intermediate, int64_t num_experts, int num_keys,
                                   int top_k, int dtype);
 int fmoe_layer_forward(const fmoe_layer_args* args);
+
+/*
+ * Training step of the layer between its router logits and its output (flash_moe/modules/flash_moe.py:72-101), forward and
+ * backward in one call each.  The batch-norm, the router GEMM and the weight-gradient GEMMs of the shared MLP stay with the
+ * caller:
+ *   forward   log_probs [T, 2, nk] (log-softmax of the router logits) -> indices, gates; y = experts + shared MLP, one
+ *             rounding; keeps the expert scores and, where a kernel stores them, the MLP's two pre-activations
+ *             (*have_preacts = 1; else 0 and the caller recomputes them)
+ *   backward  dy -> dx_experts, ddown, dup (dense, zero rows for unselected experts) and dlogits [T, 2 nk], the gradient of
+ *             the router logits through gates (renormalised or not), top-k and log-softmax
+ */
+typedef struct fmoe_train_args {
+  const void* x;
+  const void* log_probs;
+  const void* gate_proj;
+  const void* up_proj;
+  const void* down_proj;
+  const void* down_embed;
+  const void* up_embed;
+  int64_t* indices;      /* [T, k]      written by the forward, read by the backward */
+  void* gates;           /* [T, k] */
+  float* expert_scores;  /* [T, k] */
+  void* pre_gate;        /* [T, I]      forward only */
+  void* pre_up;          /* [T, I] */
+  void* y;               /* [T, H] */
+  const void* dy;        /* [T, H]      backward only, like all below */
+  void* dx_experts;      /* [T, H] */
+  void* ddown;           /* [N, H] */
+  void* dup;             /* [N, H] */
+  void* dlogits;         /* [T, 2 nk] */
+  void* workspace;
+  size_t workspace_bytes;
+  int32_t* status; /* nullable */
+  fmoe_stream_t stream;
+  int64_t num_tokens;
+  int64_t num_experts;
+  int32_t hidden;
+  int32_t intermediate;
+  int32_t num_keys;
+  int32_t top_k;
+  int32_t dtype;
+  int32_t norm_topk_prob;
+} fmoe_train_args;
+
+size_t fmoe_train_forward_workspace_bytes(int64_t num_tokens, int hidden, int intermediate, int64_t num_experts, int top_k,
+                                          int dtype);
+int fmoe_train_forward(const fmoe_train_args* args, int* have_preacts);
+size_t fmoe_train_backward_workspace_bytes(int64_t num_tokens, int hidden, int64_t num_experts, int top_k, int dtype);
+int fmoe_train_backward(const fmoe_train_args* args);
 
 #ifdef __cplusplus
 }
