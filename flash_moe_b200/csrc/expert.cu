@@ -9,11 +9,10 @@
 //      store - no atomics, run-to-run deterministic.
 // Both have a form for few tokens that spreads one task over the warps of a CTA.  Ids outside [0, N) are skipped and
 // flagged.  16-bit tables of 1 GiB and more take the fused kernel of expert_fused.cu.
-#include <cub/device/device_radix_sort.cuh>
-
 #include <cstdlib>
 
 #include "common.cuh"
+#include "warp_sort.cuh"
 
 namespace fmoe {
 namespace {
@@ -797,44 +796,129 @@ int run_typed(const void* x, const void* down, const void* up, const int64_t* id
 //   dD[e] = sum_{pairs of e} ds * x[t]           dU[e] = sum_{pairs of e} silu(s) * g * dout[t]
 // s is recomputed (nothing but the forward's inputs is saved).  All sums are float32 in a fixed order with one
 // rounding on store: no atomics (the reference scatters with atomics), run-to-run deterministic.
-constexpr int kBwdChunk = 64;  // sorted pairs per warp task of the table-gradient pass
+// sorted pairs per warp task of the table-gradient pass: fewer when there are few pairs, so that every SM has warps at work
+// (500 tokens float32 x 512 columns, top-16: 41 us with 64, 8 with 16)
+int bwd_chunk(int64_t P) { return P >= (int64_t{1} << 18) ? 64 : P >= (int64_t{1} << 15) ? 32 : 16; }
 
-// The forward's counting sort orders the pairs of one expert by atomic arrival, which is fine for per-pair
-// results but would make the order of the gradient sums vary from run to run.  The backward therefore sorts
-// (expert id, pair id) with a stable radix sort (CUB, from the CUDA toolkit headers): pairs of one expert end up
-// in ascending pair id, skipped ids (key N) at the end.
-__global__ void expert_sort_keys_kernel(const int64_t* __restrict__ idx, int64_t P, int64_t N,
-                                        unsigned* __restrict__ keys, int* __restrict__ vals, int* __restrict__ counts,
-                                        int32_t* status) {
+// Pairs in the order of their experts, pairs of one expert in ascending pair id, so that the sums do not depend on timing:
+//   histogram   counts per expert and each pair's arrival rank (an atomic per group of equal ids in a warp);
+//   scan, scatter to offset + rank: segments per expert, in arrival order inside a segment;
+//   sort of each segment by pair id: segments of up to 256 pairs in a warp's registers, longer ones (listed by the first
+//   kernel, handled by the second) by setting their bits in a bitmap over the pair ids and reading it out in order.
+// Skipped ids take no part.  262144 pairs over 16384 experts: 25 us; a stable radix sort of (expert, pair) took 47.
+constexpr int kWarpSegment = 256;
+
+__global__ void expert_hist_kernel(const int64_t* __restrict__ idx, int64_t P, int64_t N, int* __restrict__ counts,
+                                   int* __restrict__ rank, int32_t* status) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  const int64_t warp_global = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   bool bad = false;
-  for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < P;
-       p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t e = idx[p];
+  for (int64_t base = warp_global * 32; base < P; base += warps_total * 32) {
+    const int64_t p = base + lane;
+    const int64_t e = p < P ? idx[p] : -1;
     const bool valid = e >= 0 && e < N;
-    bad |= !valid && e != -1;
-    keys[p] = valid ? static_cast<unsigned>(e) : static_cast<unsigned>(N);
-    vals[p] = static_cast<int>(p);
-    if (valid) atomicAdd(&counts[e], 1);  // integer counts: the result does not depend on the order
+    bad |= p < P && !valid && e != -1;  // -1 is the empty-slot value: skipped without a flag
+    const unsigned key = valid ? static_cast<unsigned>(e) : (0x80000000u | lane);
+    const unsigned peers = __match_any_sync(kFull, key);
+    const int leader = __ffs(peers) - 1;
+    int first = 0;
+    if (valid && lane == leader) first = atomicAdd(&counts[e], __popc(peers));
+    first = __shfl_sync(kFull, first, leader);
+    if (p < P) rank[p] = valid ? first + __popc(peers & ((1u << lane) - 1u)) : -1;
   }
   if (bad && status != nullptr) atomicOr(status, FMOE_STATUS_BAD_EXPERT_ID);
 }
 
-int key_bits(int64_t N) {
-  int b = 1;
-  while ((int64_t{1} << b) <= N) ++b;  // keys run from 0 to N inclusive
-  return b;
+__global__ void expert_scatter_kernel(const int64_t* __restrict__ idx, const int* __restrict__ rank,
+                                      const int* __restrict__ offsets, int64_t P, int* __restrict__ sorted_pair,
+                                      int* __restrict__ sorted_expert) {
+  for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < P;
+       p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int r = rank[p];
+    if (r < 0) continue;
+    const int e = static_cast<int>(idx[p]);
+    const int pos = offsets[e] + r;
+    sorted_pair[pos] = static_cast<int>(p);
+    sorted_expert[pos] = e;
+  }
 }
 
-size_t stable_sort_temp_bytes(int64_t P, int64_t N) {
-  size_t bytes = 0;
-  const cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, bytes, static_cast<const unsigned*>(nullptr),
-                                                        static_cast<unsigned*>(nullptr), static_cast<const int*>(nullptr),
-                                                        static_cast<int*>(nullptr), static_cast<int>(P), 0, key_bits(N));
-  if (e != cudaSuccess) {  // no device to ask (host-only size query): a bound that covers CUB's histograms
-    (void)cudaGetLastError();
-    bytes = static_cast<size_t>(P) * 8 + (size_t{4} << 20);
+template <int R>
+__device__ __forceinline__ void sort_segment(int* seg, int n, int lane) {
+  uint32_t a[R];  // descending keys of inverted ids: ascending ids; 0 pads
+#pragma unroll
+  for (int r = 0; r < R; ++r) a[r] = lane * R + r < n ? 0xFFFFFFFFu - static_cast<uint32_t>(seg[lane * R + r]) : 0u;
+  sort_desc<R, false>(a, lane);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (lane * R + r < n) seg[lane * R + r] = static_cast<int>(0xFFFFFFFFu - a[r]);
+}
+
+__global__ void __launch_bounds__(256) expert_segment_sort_kernel(const int* __restrict__ offsets, int64_t N,
+                                                                  int* __restrict__ sorted_pair, int* __restrict__ num_long,
+                                                                  int* __restrict__ long_experts) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t e = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; e < N; e += warps_total) {
+    const int b = offsets[e], n = offsets[e + 1] - b;
+    if (n < 2) continue;
+    if (n <= 32) sort_segment<1>(sorted_pair + b, n, lane);
+    else if (n <= 64) sort_segment<2>(sorted_pair + b, n, lane);
+    else if (n <= kWarpSegment) sort_segment<8>(sorted_pair + b, n, lane);
+    else if (lane == 0) long_experts[atomicAdd(num_long, 1)] = static_cast<int>(e);
   }
-  return bytes;
+}
+
+constexpr int kBitmapWords = 16384;  // pair ids per pass: 32 times as many
+__global__ void __launch_bounds__(512) expert_long_sort_kernel(const int* __restrict__ offsets, const int* __restrict__ num_long,
+                                                               const int* __restrict__ long_experts, int64_t P,
+                                                               int* __restrict__ sorted_pair, int* __restrict__ temp) {
+  extern __shared__ unsigned bitmap[];
+  __shared__ int warp_sum[16];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kPer = kBitmapWords / 512;
+  for (int l = blockIdx.x; l < *num_long; l += gridDim.x) {
+    const int e = long_experts[l];
+    const int b = offsets[e], en = offsets[e + 1];
+    int done = b;
+    for (int64_t r0 = 0; r0 < P; r0 += static_cast<int64_t>(kBitmapWords) * 32) {
+      for (int i = threadIdx.x; i < kBitmapWords; i += 512) bitmap[i] = 0;
+      __syncthreads();
+      for (int i = b + threadIdx.x; i < en; i += 512) {
+        const int64_t rel = sorted_pair[i] - r0;
+        if (rel >= 0 && rel < static_cast<int64_t>(kBitmapWords) * 32) atomicOr(&bitmap[rel >> 5], 1u << (rel & 31));
+      }
+      __syncthreads();
+      int mine = 0;
+      for (int i = 0; i < kPer; ++i) mine += __popc(bitmap[threadIdx.x * kPer + i]);
+      int incl = mine;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int up = __shfl_up_sync(kFull, incl, d);
+        if (lane >= d) incl += up;
+      }
+      if (lane == 31) warp_sum[warp] = incl;
+      __syncthreads();
+      int pos = done + incl - mine, all = 0;
+      for (int w = 0; w < 16; ++w) {
+        if (w < warp) pos += warp_sum[w];
+        all += warp_sum[w];
+      }
+      for (int i = 0; i < kPer; ++i) {
+        unsigned word = bitmap[threadIdx.x * kPer + i];
+        while (word != 0) {
+          const int bit = __ffs(word) - 1;
+          word &= word - 1;
+          temp[pos++] = static_cast<int>(r0 + (threadIdx.x * kPer + i) * 32 + bit);
+        }
+      }
+      done += all;
+      __syncthreads();
+    }
+    for (int i = b + threadIdx.x; i < en; i += 512) sorted_pair[i] = temp[i];
+    __syncthreads();
+  }
 }
 
 // in: s_in (raw <x, D>; may alias s_ds), q (raw <dout, U>), gates.  out: s_ds = ds, gs = silu(s) * g (over q), dgates.
@@ -860,28 +944,42 @@ __global__ void expert_bwd_pairs_kernel(const float* s_in, float* s_ds, float* _
   }
 }
 
-// One warp per (chunk of kBwdChunk sorted pairs, block of 32*VEC*NCH columns).  The warp walks its pairs in sorted
-// order with the running sums of the current expert's two gradient rows in registers.  A row whose pairs all lie
-// inside the chunk is stored directly; otherwise the partial sum goes to `partial` (slot 0: the expert began in an
-// earlier chunk, slot 1: it began here and continues) and expert_bwd_finish_kernel adds the pieces in chunk order.
-template <typename T, int NCH>
+// One warp per (chunk of sorted pairs, block of 32*VEC*NCH columns).  The warp walks its pairs in sorted
+// order with the running sums of the current expert's two gradient rows in registers.  An expert of up to kWholeExpert
+// pairs belongs whole to the chunk in which it begins and its rows are stored directly; a longer one is split at the chunk
+// boundaries, its partial sums go to `partial` (slot 0: the expert began in an earlier chunk, slot 1: it began here and
+// continues) and expert_bwd_finish_kernel adds the pieces in chunk order.  (With every expert split at the boundaries the
+// partial rows were 134 MB written and read at the benchmark shape.)
+// Bound by the gather of one x and one dout row per pair (1.07 GB at 4096 tokens x 1024 columns, top-64): 9.9 TB/s.
+constexpr int kWholeExpert = 256;
+// first sorted position of chunk c
+__device__ __forceinline__ int chunk_begin(int64_t c, int chunk_pairs, int total, const int* __restrict__ sorted_expert,
+                                           const int* __restrict__ offsets) {
+  if (c * chunk_pairs >= total) return total;
+  const int pos = static_cast<int>(c * chunk_pairs);
+  const int e = sorted_expert[pos];
+  const int b = offsets[e], en = offsets[e + 1];
+  return b == pos || en - b > kWholeExpert ? pos : en;
+}
+template <typename T, int NCH, int DEPTH>
 __global__ void __launch_bounds__(128) expert_bwd_tables_kernel(
     const T* __restrict__ x, const T* __restrict__ dout, const float* __restrict__ ds, const float* __restrict__ gs,
     const int* __restrict__ sorted_pair, const int* __restrict__ sorted_expert, const int* __restrict__ offsets,
     int64_t N, T* __restrict__ ddown, T* __restrict__ dup, float* __restrict__ partial_d, float* __restrict__ partial_u,
-    int H, int k, int colblocks) {
+    int H, int k, int colblocks, int chunk_pairs) {
   constexpr int VEC = Vec16<T>::N;
   const int lane = threadIdx.x & 31;
   const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   const int64_t warp_global = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int total = offsets[N];
-  const int64_t nchunks = (total + kBwdChunk - 1) / kBwdChunk;
+  const int64_t nchunks = (total + chunk_pairs - 1) / chunk_pairs;
   for (int64_t task = warp_global; task < nchunks * colblocks; task += warps_total) {
     const int64_t chunk = task / colblocks;
     const int cb = static_cast<int>(task - chunk * colblocks);
     const int col0 = cb * (32 * VEC * NCH);
-    const int pos0 = static_cast<int>(chunk * kBwdChunk);
-    const int pos1 = min(pos0 + kBwdChunk, total);
+    const int pos0 = chunk_begin(chunk, chunk_pairs, total, sorted_expert, offsets);
+    const int pos1 = chunk_begin(chunk + 1, chunk_pairs, total, sorted_expert, offsets);
+    if (pos0 >= pos1) continue;
     bool in[NCH];
 #pragma unroll
     for (int c = 0; c < NCH; ++c) in[c] = col0 + (c * 32 + lane) * VEC < H;
@@ -921,52 +1019,60 @@ __global__ void __launch_bounds__(128) expert_bwd_tables_kernel(
       }
     };
 
-    uint4 xn[NCH], on[NCH];
-    int p_next = sorted_pair[pos0];
-    {
-      const int64_t t = p_next / k;
-#pragma unroll
-      for (int c = 0; c < NCH; ++c) {
-        const int col = col0 + (c * 32 + lane) * VEC;
-        xn[c] = in[c] ? ldg16(x + t * H + col) : make_uint4(0, 0, 0, 0);
-        on[c] = in[c] ? ldg16(dout + t * H + col) : make_uint4(0, 0, 0, 0);
+    // 32 pairs at a time: each lane fetches one pair's token, expert and weights, a batch ahead of their use; the rows of
+    // DEPTH pairs are in flight together
+    int t_next = 0, e_next = 0;
+    float wd_next = 0.f, wu_next = 0.f;
+    auto fetch_pairs = [&](int base) {
+      if (base + lane < pos1) {
+        const int p = sorted_pair[base + lane];
+        e_next = sorted_expert[base + lane];
+        t_next = p / k;
+        wd_next = ds[p];
+        wu_next = gs[p];
       }
-    }
-    for (int pos = pos0; pos < pos1; ++pos) {
-      const int p = p_next;
-      const int e = sorted_expert[pos];
-      uint4 xq[NCH], oq[NCH];
+    };
+    fetch_pairs(pos0);
+    for (int base = pos0; base < pos1; base += 32) {
+      const int t_l = t_next, e_l = e_next;
+      const float wd_l = wd_next, wu_l = wu_next;
+      if (base + 32 < pos1) fetch_pairs(base + 32);
+      const int n = min(32, pos1 - base);
+      for (int s0 = 0; s0 < n; s0 += DEPTH) {
+        uint4 xq[DEPTH][NCH], oq[DEPTH][NCH];
 #pragma unroll
-      for (int c = 0; c < NCH; ++c) {
-        xq[c] = xn[c];
-        oq[c] = on[c];
-      }
-      if (pos + 1 < pos1) {  // issue the next pair's row gathers before this pair's math
-        p_next = sorted_pair[pos + 1];
-        const int64_t t = p_next / k;
+        for (int u = 0; u < DEPTH; ++u) {
+          const int64_t t = __shfl_sync(kFull, t_l, s0 + u);
+          const bool have = s0 + u < n;
 #pragma unroll
-        for (int c = 0; c < NCH; ++c) {
-          const int col = col0 + (c * 32 + lane) * VEC;
-          xn[c] = in[c] ? ldg16(x + t * H + col) : make_uint4(0, 0, 0, 0);
-          on[c] = in[c] ? ldg16(dout + t * H + col) : make_uint4(0, 0, 0, 0);
+          for (int c = 0; c < NCH; ++c) {
+            const int col = col0 + (c * 32 + lane) * VEC;
+            xq[u][c] = have && in[c] ? ldg16(x + t * H + col) : make_uint4(0, 0, 0, 0);
+            oq[u][c] = have && in[c] ? ldg16(dout + t * H + col) : make_uint4(0, 0, 0, 0);
+          }
         }
-      }
-      if (e != cur_e) {  // warp-uniform: cur_e ends inside this chunk
-        flush(cur_e, began_earlier, 0);
-        cur_e = e;
-        began_earlier = false;
-      }
-      const float wd = ds[p], wu = gs[p];
-      const uint64_t wd2 = pack_f32x2(wd, wd), wu2 = pack_f32x2(wu, wu);
 #pragma unroll
-      for (int c = 0; c < NCH; ++c) {
-        float xf[VEC], of[VEC];
-        unpack16<T>(xq[c], xf);
-        unpack16<T>(oq[c], of);
+        for (int u = 0; u < DEPTH; ++u) {
+          const int e = __shfl_sync(kFull, e_l, s0 + u);
+          const float wd = __shfl_sync(kFull, wd_l, s0 + u), wu = __shfl_sync(kFull, wu_l, s0 + u);
+          if (s0 + u >= n) break;
+          if (e != cur_e) {  // warp-uniform: cur_e ends inside this chunk
+            flush(cur_e, began_earlier, 0);
+            cur_e = e;
+            began_earlier = false;
+          }
+          const uint64_t wd2 = pack_f32x2(wd, wd), wu2 = pack_f32x2(wu, wu);
 #pragma unroll
-        for (int i = 0; i < VEC / 2; ++i) {
-          ffma2(ad[c][i], pack_f32x2(xf[2 * i], xf[2 * i + 1]), wd2);
-          ffma2(au[c][i], pack_f32x2(of[2 * i], of[2 * i + 1]), wu2);
+          for (int c = 0; c < NCH; ++c) {
+            float xf[VEC], of[VEC];
+            unpack16<T>(xq[u][c], xf);
+            unpack16<T>(oq[u][c], of);
+#pragma unroll
+            for (int i = 0; i < VEC / 2; ++i) {
+              ffma2(ad[c][i], pack_f32x2(xf[2 * i], xf[2 * i + 1]), wd2);
+              ffma2(au[c][i], pack_f32x2(of[2 * i], of[2 * i + 1]), wu2);
+            }
+          }
         }
       }
     }
@@ -975,28 +1081,24 @@ __global__ void __launch_bounds__(128) expert_bwd_tables_kernel(
   }
 }
 
-// One CTA per expert: rows of experts without pairs are zeroed, rows of experts whose pairs span several chunks are
-// the sum of their partial rows in chunk order; rows stored directly by the pass above are left alone.
+// One warp per expert: rows of experts without pairs are zeroed, rows of experts split over several chunks are the sum of
+// their partial rows in chunk order; rows stored by the pass above are left alone.
 template <typename T>
 __global__ void __launch_bounds__(256) expert_bwd_finish_kernel(const int* __restrict__ offsets, int64_t N,
                                                                 const float* __restrict__ partial_d,
                                                                 const float* __restrict__ partial_u,
-                                                                T* __restrict__ ddown, T* __restrict__ dup, int H) {
+                                                                T* __restrict__ ddown, T* __restrict__ dup, int H,
+                                                                int chunk_pairs) {
   constexpr int VEC = Vec16<T>::N;
-  for (int64_t e = blockIdx.x; e < N; e += gridDim.x) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t e = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; e < N; e += warps_total) {
     const int b = offsets[e], en = offsets[e + 1];
+    if (b != en && en - b <= kWholeExpert) continue;
     T* rd = ddown + e * H;
     T* ru = dup + e * H;
-    if (b == en) {
-      for (int col = threadIdx.x * VEC; col < H; col += blockDim.x * VEC) {
-        *reinterpret_cast<uint4*>(rd + col) = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(ru + col) = make_uint4(0, 0, 0, 0);
-      }
-      continue;
-    }
-    const int c0 = b / kBwdChunk, c1 = (en - 1) / kBwdChunk;
-    if (c0 == c1) continue;
-    for (int col = threadIdx.x * VEC; col < H; col += blockDim.x * VEC) {
+    const int c0 = b / chunk_pairs, c1 = b == en ? c0 - 1 : (en - 1) / chunk_pairs;  // no pairs: the empty sum
+    for (int col = lane * VEC; col < H; col += 32 * VEC) {
       float sd[VEC], su[VEC];
 #pragma unroll
       for (int i = 0; i < VEC; ++i) sd[i] = su[i] = 0.f;
@@ -1100,10 +1202,9 @@ int run_weighted_rows(const void* values, const void* weights, const int64_t* id
 struct ExpertBwdWs {
   ExpertWs fwd;  // sort arrays; fwd.gs holds s, then ds
   float* q;      // <dout, U>, then silu(s) * g
-  unsigned* keys_in;
-  int* vals_in;
-  void* sort_temp;
-  size_t sort_temp_bytes;
+  int* counts;        // [N + 1]: per expert, then the number of long segments
+  int* long_experts;  // experts of more than kWarpSegment pairs
+  int* temp;          // [P]
   float* partial_d;
   float* partial_u;
   size_t bytes;
@@ -1119,30 +1220,29 @@ ExpertBwdWs carve_bwd(void* ws, int64_t T, int H, int64_t N, int k) {
     return p;
   };
   const int64_t P = T * k;
-  const int64_t nchunks = (P + kBwdChunk - 1) / kBwdChunk;
+  const int64_t nchunks = (P + bwd_chunk(P) - 1) / bwd_chunk(P);
   w.q = static_cast<float*>(take(static_cast<size_t>(P) * 4));
-  w.keys_in = static_cast<unsigned*>(take(static_cast<size_t>(P) * 4));
-  w.vals_in = static_cast<int*>(take(static_cast<size_t>(P) * 4));
-  w.sort_temp_bytes = stable_sort_temp_bytes(P, N);
-  w.sort_temp = take(w.sort_temp_bytes);
+  w.counts = static_cast<int*>(take(static_cast<size_t>(N + 1) * 4));
+  w.long_experts = static_cast<int*>(take(static_cast<size_t>(P / kWarpSegment + 1) * 4));
+  w.temp = static_cast<int*>(take(static_cast<size_t>(P) * 4));
   w.partial_d = static_cast<float*>(take(static_cast<size_t>(nchunks) * 2 * H * 4));
   w.partial_u = static_cast<float*>(take(static_cast<size_t>(nchunks) * 2 * H * 4));
   w.bytes = off;
   return w;
 }
 
-template <typename T, int NCH>
+template <typename T, int NCH, int DEPTH>
 void launch_bwd_tables(const void* x, const void* dout, const ExpertBwdWs& w, int64_t N, void* ddown, void* dup, int H,
                        int k, int64_t P, cudaStream_t stream) {
   constexpr int VEC = Vec16<T>::N;
   const int colblocks = (H + 32 * VEC * NCH - 1) / (32 * VEC * NCH);
-  const int64_t tasks = ((P + kBwdChunk - 1) / kBwdChunk) * colblocks;
+  const int64_t tasks = ((P + bwd_chunk(P) - 1) / bwd_chunk(P)) * colblocks;
   const int64_t want = (tasks + 3) / 4;
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * 16;
   const int grid = static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
-  expert_bwd_tables_kernel<T, NCH><<<grid, 128, 0, stream>>>(
+  expert_bwd_tables_kernel<T, NCH, DEPTH><<<grid, 128, 0, stream>>>(
       static_cast<const T*>(x), static_cast<const T*>(dout), w.fwd.gs, w.q, w.fwd.sorted_pair, w.fwd.sorted_expert,
-      w.fwd.offsets, N, static_cast<T*>(ddown), static_cast<T*>(dup), w.partial_d, w.partial_u, H, k, colblocks);
+      w.fwd.offsets, N, static_cast<T*>(ddown), static_cast<T*>(dup), w.partial_d, w.partial_u, H, k, colblocks, bwd_chunk(P));
 }
 
 template <typename T>
@@ -1153,30 +1253,33 @@ int run_backward(const void* dout, const void* x, const void* down, const void* 
   const int64_t P = T_ * k;
   const int sms = device_sm_count();
   int rc;
-  {  // stable sort of the pairs by expert id + segment offsets
-    FMOE_CUDA_TRY(cudaMemsetAsync(w.fwd.counts, 0, static_cast<size_t>(N) * 4, stream));
+  {  // the pairs in the order of their experts + segment offsets
+    FMOE_CUDA_TRY(cudaMemsetAsync(w.counts, 0, static_cast<size_t>(N + 1) * 4, stream));
     const int64_t want = (P + 255) / 256;
     const int grid = static_cast<int>(want < sms * 8 ? want : sms * 8);
-    expert_sort_keys_kernel<<<grid, 256, 0, stream>>>(idx, P, N, w.keys_in, w.vals_in, w.fwd.counts, status);
+    expert_hist_kernel<<<grid, 256, 0, stream>>>(idx, P, N, w.counts, w.fwd.rank, status);
     FMOE_LAUNCH_CHECK();
     const int ntiles = static_cast<int>((N + kScanTile - 1) / kScanTile);
     if (ntiles > 16) {
-      scan_tile_sums_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.fwd.counts, N, w.fwd.tile_sums);
+      scan_tile_sums_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.counts, N, w.fwd.tile_sums);
       FMOE_LAUNCH_CHECK();
-      scan_apply_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.fwd.counts, N, w.fwd.tile_sums, w.fwd.offsets);
+      scan_apply_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.counts, N, w.fwd.tile_sums, w.fwd.offsets);
     } else {
-      scan_apply_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.fwd.counts, N, nullptr, w.fwd.offsets);
+      scan_apply_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.counts, N, nullptr, w.fwd.offsets);
     }
     FMOE_LAUNCH_CHECK();
-    size_t need = 0;
-    FMOE_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, need, w.keys_in,
-                                                  reinterpret_cast<unsigned*>(w.fwd.sorted_expert), w.vals_in,
-                                                  w.fwd.sorted_pair, static_cast<int>(P), 0, key_bits(N), stream));
-    if (need > w.sort_temp_bytes) return FMOE_ERR_WORKSPACE;
-    size_t have = w.sort_temp_bytes;
-    FMOE_CUDA_TRY(cub::DeviceRadixSort::SortPairs(w.sort_temp, have, w.keys_in,
-                                                  reinterpret_cast<unsigned*>(w.fwd.sorted_expert), w.vals_in,
-                                                  w.fwd.sorted_pair, static_cast<int>(P), 0, key_bits(N), stream));
+    expert_scatter_kernel<<<grid, 256, 0, stream>>>(idx, w.fwd.rank, w.fwd.offsets, P, w.fwd.sorted_pair, w.fwd.sorted_expert);
+    FMOE_LAUNCH_CHECK();
+    const int64_t seg_want = (N + 7) / 8;
+    const int seg_grid = static_cast<int>(seg_want < sms * 8 ? seg_want : sms * 8);
+    expert_segment_sort_kernel<<<seg_grid, 256, 0, stream>>>(w.fwd.offsets, N, w.fwd.sorted_pair, w.counts + N, w.long_experts);
+    FMOE_LAUNCH_CHECK();
+    if (P > kWarpSegment) {
+      FMOE_CUDA_TRY(allow_smem(expert_long_sort_kernel, kBitmapWords * 4));
+      expert_long_sort_kernel<<<sms, 512, kBitmapWords * 4, stream>>>(w.fwd.offsets, w.counts + N, w.long_experts, P,
+                                                                     w.fwd.sorted_pair, w.temp);
+      FMOE_LAUNCH_CHECK();
+    }
   }
   if (saved_scores == nullptr) {  // s = <x, D[e]> was not kept by the forward: recompute it
     rc = run_scores<T>(x, down, idx, nullptr, w.fwd.gs, T_, H, N, k, status, stream);
@@ -1194,15 +1297,20 @@ int run_backward(const void* dout, const void* x, const void* down, const void* 
   rc = run_accum<T>(down, idx, w.fwd.gs, dx, sizeof(T) == 4 ? 1 : 0, T_, H, N, k, stream);
   if (rc != FMOE_OK) return rc;
   const int need = (H + 32 * VEC - 1) / (32 * VEC);
-  if (need <= 1) launch_bwd_tables<T, 1>(x, dout, w, N, ddown, dup, H, k, P, stream);
-  else if (need <= 2) launch_bwd_tables<T, 2>(x, dout, w, N, ddown, dup, H, k, P, stream);
-  else launch_bwd_tables<T, 4>(x, dout, w, N, ddown, dup, H, k, P, stream);
+  // two 16-byte pieces of a row per lane and two pairs in flight measured best (4096 tokens x 1024 columns, top-64: 109 us;
+  // four pieces and the weights of one pair at a time 152, four pieces and two pairs 194, two and four 132, one and four
+  // 138); narrower column blocks where the tasks would not fill the SMs
+  const int64_t tasks = (P + bwd_chunk(P) - 1) / bwd_chunk(P) * ((need + 1) / 2);
+  if (need <= 1 || tasks < static_cast<int64_t>(sms) * 16)
+    launch_bwd_tables<T, 1, 4>(x, dout, w, N, ddown, dup, H, k, P, stream);
+  else
+    launch_bwd_tables<T, 2, 2>(x, dout, w, N, ddown, dup, H, k, P, stream);
   FMOE_LAUNCH_CHECK();
   {
-    const int64_t cap = static_cast<int64_t>(sms) * 16;
-    const int grid = static_cast<int>(N < cap ? N : cap);
+    const int64_t want = (N + 7) / 8, cap = static_cast<int64_t>(sms) * 8;
+    const int grid = static_cast<int>(want < cap ? want : cap);
     expert_bwd_finish_kernel<T><<<grid, 256, 0, stream>>>(w.fwd.offsets, N, w.partial_d, w.partial_u,
-                                                          static_cast<T*>(ddown), static_cast<T*>(dup), H);
+                                                          static_cast<T*>(ddown), static_cast<T*>(dup), H, bwd_chunk(P));
     FMOE_LAUNCH_CHECK();
   }
   return FMOE_OK;

@@ -259,3 +259,31 @@ def test_mlp_backward_with_kept_preactivations():
     want = O.mlp_backward(dy, x, wg, wu, wd)
     for leaf, w_ in zip(leaves, want):
         assert rel_err(leaf.grad, w_) <= 2e-2
+
+
+@pytest.mark.parametrize("T,H,N,k,dtype", [(3000, 64, 9, 8, torch.float32), (600, 1096, 40, 33, torch.bfloat16),
+                                           (70000, 64, 5, 8, torch.float16), (37, 520, 4000, 5, torch.bfloat16)])
+def test_expert_backward_segments(T, H, N, k, dtype):
+    """Segments sorted in a warp (up to 256 pairs) and through the bitmap (longer; more pair ids than one bitmap pass),
+    experts whole in a chunk and split over many, chunks of every size."""
+    from flash_moe_b200 import check_status
+    from flash_moe_b200.ops.flash_expert import _expert_backward
+
+    x, d, u, idx, gates, dout = expert_case(T, H, N, k, dtype, False, seed=T + N)
+    idx[0, 0] = -1
+    x, d, u, idx, gates, dout = (t.cuda() for t in (x, d, u, idx, gates, dout))
+    got = _expert_backward(dout, x, d, u, idx, gates)
+    again = _expert_backward(dout, x, d, u, idx, gates)
+    assert all(torch.equal(a, b) for a, b in zip(got, again))
+    ddown, dup = torch.zeros(N, H, device="cuda", dtype=torch.float64), torch.zeros(N, H, device="cuda", dtype=torch.float64)
+    for j in range(k):
+        e, ok = idx[:, j].clamp(min=0), (idx[:, j] >= 0).double()[:, None]
+        s = (x.double() * d[e].double()).sum(-1, keepdim=True)
+        q = (dout.double() * u[e].double()).sum(-1, keepdim=True)
+        g, sig = gates[:, j].double()[:, None], torch.sigmoid(s)
+        ddown.index_add_(0, e, ok * q * g * sig * (1 + s * (1 - sig)) * x.double())
+        dup.index_add_(0, e, ok * s * sig * g * dout.double())
+    tol = {torch.float32: 2e-5, torch.bfloat16: 4e-3, torch.float16: 1e-3}[dtype]
+    for a, b in ((got[1], ddown), (got[2], dup)):
+        assert (a.double() - b).norm() <= tol * b.norm()
+    check_status()
