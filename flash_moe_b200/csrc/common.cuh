@@ -172,6 +172,13 @@ template <> __device__ __forceinline__ uint4 pack16<__half>(const float (&f)[8])
 
 __device__ __forceinline__ uint4 ldg16(const void* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
 
+// 32 bytes (a 32-byte aligned address) in one load
+__device__ __forceinline__ void ldg32(const void* p, uint4& lo, uint4& hi) {
+  asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w), "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w)
+               : "l"(p));
+}
+
 // ---- order-preserving float <-> uint32 map (larger float <=> larger unsigned) ---------------
 __device__ __forceinline__ uint32_t f32_to_ord(float v) {
   const uint32_t b = __float_as_uint(v);
@@ -191,11 +198,6 @@ int launch_expert_forward(const void* x, const void* down, const void* up, const
                           size_t ws_bytes, int32_t* status, cudaStream_t stream, void* const* between_passes = nullptr,
                           int act = 0, float* raw_scores = nullptr);
 // raw_scores (nullable) [T, k] float32 receives <x[t], down[e]> before the activation, for the backward pass.
-// both steps in one kernel for 16-bit tables (expert_fused.cu): rows streamed through a shared-memory ring
-bool expert_fused_supported(int dtype, int64_t T, int H, int k);
-int launch_expert_fused(const void* x, const void* down, const void* up, const int64_t* idx, const void* gates,
-                        void* out, int dtype, int out_f32, int64_t T, int H, int64_t N, int k, int act,
-                        float* raw_scores, int32_t* status, cudaStream_t stream);
 // the same sum with both tables sharded by e % world over the GPUs of a node; *_shards are DEVICE arrays of `world`
 // row-0 pointers (peer pointers for the other GPUs); 16-bit dtypes only
 // hot_down / hot_up (nullable): hot_rows rows replicated on every GPU, addressed by the ids N .. N + hot_rows - 1

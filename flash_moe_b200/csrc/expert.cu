@@ -8,8 +8,9 @@
 //   3. accumulate: out[t] = sum_j gs[t,j] * U[e_tj] in fp32 (packed f32x2 FMAs), fixed slot order, one rounding on
 //      store - no atomics, run-to-run deterministic.
 // Both have a form for few tokens that spreads one task over the warps of a CTA.  Ids outside [0, N) are skipped and
-// flagged.  16-bit tables of 1 GiB and more take the fused kernel of expert_fused.cu.
-#include <cstdlib>
+// flagged.  (A single kernel that streamed the rows of both steps through shared memory was the faster one for tables of
+// 1 GiB and more until the scores pass read whole lines: 32768 tokens x 2048, 2^20 experts, Zipf 1.1 ids 562 us against 391
+// now, uniform ids 675 against 683.)
 
 #include "common.cuh"
 #include "warp_sort.cuh"
@@ -138,7 +139,7 @@ __device__ __forceinline__ const T* table_row(const T* table, const T* const* sh
 // waits for data waits for a gathered down row: batches of UNROLL 32-column blocks (2 * UNROLL x 16 B per lane) in
 // STAGES register buffers keep gathers in flight across batches to cover the L2 latency (measured at the
 // benchmark shape: 4 x 2 buffers 57.7 us, 8 x 1 61.9 us, 4 x 3 62.6 us, 2 x 2 57.8 us).
-template <typename T, int UNROLL, bool PEER = false, int STAGES = 1>
+template <typename T, int UNROLL, bool PEER = false, int STAGES = 1, int COLS = 8, bool LOAD32 = false>
 __global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* __restrict__ x, const T* __restrict__ down,
                                                                const int64_t* __restrict__ idx,
                                                                const T* __restrict__ gates, float* __restrict__ gs,
@@ -204,19 +205,43 @@ __global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* __restr
     const T* ra = table_row<T, PEER>(down, shards, world, oka ? ea : 0, H, sharded) + 8 * tq;
     const T* rb = table_row<T, PEER>(down, shards, world, okb ? eb : 0, H, sharded) + 8 * tq;
     float c[4] = {0.f, 0.f, 0.f, 0.f};
+    // COLS = 16: a lane takes 16 consecutive columns of a 64-column block, so that the four lanes of a row cover a whole
+    // 128-byte line; in one 32-byte load (LOAD32) an instruction then fetches whole lines of its 8 rows instead of halves:
+    // 51.6 -> 43.3 us at 4096 tokens x 1024 columns, top-64.  Two 16-byte loads give the same sums for tables that are only
+    // 16-byte aligned, or whose alignment the host does not know (PEER).
     auto load = [&](uint4 (&qa)[UNROLL], uint4 (&qb)[UNROLL], int c0) {
+      if constexpr (COLS == 16) {
 #pragma unroll
-      for (int u = 0; u < UNROLL; ++u) {
-        const int col = c0 + 32 * u;
-        const bool in = col + 8 * tq < H;
-        qa[u] = in ? ldg16(ra + col) : make_uint4(0, 0, 0, 0);
-        qb[u] = in ? ldg16(rb + col) : make_uint4(0, 0, 0, 0);
+        for (int u = 0; u < UNROLL; u += 2) {
+          const int col = c0 + 32 * u;
+          if (col + 16 * tq < H) {  // H % 16 == 0
+            if constexpr (LOAD32) {
+              ldg32(ra + col + 8 * tq, qa[u], qa[u + 1]);
+              ldg32(rb + col + 8 * tq, qb[u], qb[u + 1]);
+            } else {
+              qa[u] = ldg16(ra + col + 8 * tq);
+              qa[u + 1] = ldg16(ra + col + 8 * tq + 8);
+              qb[u] = ldg16(rb + col + 8 * tq);
+              qb[u + 1] = ldg16(rb + col + 8 * tq + 8);
+            }
+          } else {
+            qa[u] = qa[u + 1] = qb[u] = qb[u + 1] = make_uint4(0, 0, 0, 0);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) {
+          const int col = c0 + 32 * u;
+          const bool in = col + 8 * tq < H;
+          qa[u] = in ? ldg16(ra + col) : make_uint4(0, 0, 0, 0);
+          qb[u] = in ? ldg16(rb + col) : make_uint4(0, 0, 0, 0);
+        }
       }
     };
     auto consume = [&](const uint4 (&qa)[UNROLL], const uint4 (&qb)[UNROLL], int c0) {
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
-        const int piece = ((c0 + 32 * u) >> 3) + tq;
+        const int piece = COLS == 16 ? ((c0 + 32 * (u & ~1)) >> 3) + 2 * tq + (u & 1) : ((c0 + 32 * u) >> 3) + tq;
         const uint4 xq = piece < xs_stride ? xs[piece] : make_uint4(0, 0, 0, 0);
         Mma16816<T>::run(c, qa[u].x, qb[u].x, qa[u].y, qb[u].y, xq.x, xq.y);
         Mma16816<T>::run(c, qa[u].z, qb[u].z, qa[u].w, qb[u].w, xq.z, xq.w);
@@ -689,17 +714,6 @@ void launch_accum(const void* up, const int64_t* idx, const float* gs, void* out
                    H, N, k, colblocks, nullptr, 1, 0);  // launch errors surface through the caller's launch check
 }
 
-// debugging / measurement aid: FMOE_EXPERT_SCHEDULE=token|fused forces one schedule for 16-bit tables (read once per
-// process; `fused` only where that kernel applies); anything else leaves the default choice
-int forced_schedule() {
-  static const int forced = [] {
-    const char* v = std::getenv("FMOE_EXPERT_SCHEDULE");
-    if (v == nullptr) return 0;
-    return v[0] == 't' ? 1 : (v[0] == 'f' ? 3 : 0);
-  }();
-  return forced;
-}
-
 // per-pair dot products <rows[t], table[e]>: gates != nullptr stores silu(dot) * gate (forward), nullptr the
 // raw dot product
 template <typename T>
@@ -719,7 +733,9 @@ int run_scores(const void* rows, const void* table, const int64_t* idx, const vo
     const int grid = static_cast<int>(want < cap ? want : cap);
     const int xs_stride = ((H + 255) / 256) * 32;  // uint4 per warp, rows padded to 256 columns
     const int smem = 4 * 2 * xs_stride * 16;  // two x-row buffers per warp
-    auto kern = expert_scores_mma_kernel<T, 4, false, 2>;
+    const bool aligned32 = (reinterpret_cast<uintptr_t>(table) & 31u) == 0;
+    auto kern = H % 16 != 0 ? expert_scores_mma_kernel<T, 4, false, 2, 8>
+                            : aligned32 ? expert_scores_mma_kernel<T, 4, false, 2, 16, true> : expert_scores_mma_kernel<T, 4, false, 2, 16>;
     FMOE_CUDA_TRY(allow_smem(kern, smem));
     FMOE_CUDA_TRY(launch_pdl(4, kern, dim3(grid), dim3(128), smem, stream, 1, static_cast<const T*>(rows),
                              static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, T_, H, N, k, xs_stride,
@@ -761,7 +777,7 @@ int run_accum(const void* table, const int64_t* idx, const float* coef, void* ou
 template <typename T>
 int run_typed(const void* x, const void* down, const void* up, const int64_t* idx, const void* gates, void* out,
               int out_f32, int64_t T_, int H, int64_t N, int k, const ExpertWs& w, int32_t* status,
-              cudaStream_t stream, void* const* between_passes, int act, float* raw_scores, int dtype) {
+              cudaStream_t stream, void* const* between_passes, int act, float* raw_scores) {
   auto mark_between = [&]() -> int {
     if (between_passes != nullptr)
       for (int i = 0; i < 2; ++i)
@@ -769,17 +785,6 @@ int run_typed(const void* x, const void* down, const void* up, const int64_t* id
           FMOE_CUDA_TRY(cudaEventRecord(static_cast<cudaEvent_t>(between_passes[i]), stream));
     return FMOE_OK;
   };
-  // The fused kernel pays off once the tables are far larger than L2 (its deep ring of asynchronous copies covers
-  // the DRAM latency: 0.71 vs 0.93 ms at 2^20 experts x 2048); while they sit in L2 the two passes are faster
-  // (110 vs 162 us at 2^14 experts x 1024), so tables below 1 GiB each take the two-pass path.
-  const bool big_tables = static_cast<double>(N) * H * sizeof(T) >= 1073741824.0;
-  const bool want_fused = forced_schedule() == 3 || (forced_schedule() == 0 && big_tables);
-  if (sizeof(T) == 2 && want_fused && expert_fused_supported(dtype, T_, H, k)) {
-    // one kernel for both steps: the marks that separate the two passes fall in front of it
-    const int rc = mark_between();
-    if (rc != FMOE_OK) return rc;
-    return launch_expert_fused(x, down, up, idx, gates, out, dtype, out_f32, T_, H, N, k, act, raw_scores, status, stream);
-  }
   int rc = run_scores<T>(x, down, idx, gates, w.gs, T_, H, N, k, status, stream, act, raw_scores);
   if (rc != FMOE_OK) return rc;
   if ((rc = mark_between()) != FMOE_OK) return rc;
@@ -1145,7 +1150,7 @@ int run_typed_peer(const void* x, const void* const* down_shards, const void* co
       const int grid = static_cast<int>(want < cap ? want : cap);
       const int xs_stride = ((H + 255) / 256) * 32;
       const int smem = 4 * 2 * xs_stride * 16;  // two x-row buffers per warp
-      auto kern = expert_scores_mma_kernel<T, 4, true, 2>;
+      auto kern = H % 16 != 0 ? expert_scores_mma_kernel<T, 4, true, 2, 8> : expert_scores_mma_kernel<T, 4, true, 2, 16>;
       FMOE_CUDA_TRY(allow_smem(kern, smem));
       kern<<<grid, 128, smem, stream>>>(static_cast<const T*>(x), static_cast<const T*>(hot_down), idx,
                                         static_cast<const T*>(gates), w.gs, T_, H, N + hot_rows, k, xs_stride, status,
@@ -1348,13 +1353,13 @@ int launch_expert_forward(const void* x, const void* down, const void* up, const
   switch (dtype) {
     case FMOE_DTYPE_F32:
       return run_typed<float>(x, down, up, indices, gates, out, 1, T, H, N, k, w, status, stream, between_passes, act,
-                              raw_scores, dtype);
+                              raw_scores);
     case FMOE_DTYPE_BF16:
       return run_typed<__nv_bfloat16>(x, down, up, indices, gates, out, out_f32, T, H, N, k, w, status, stream,
-                                      between_passes, act, raw_scores, dtype);
+                                      between_passes, act, raw_scores);
     case FMOE_DTYPE_F16:
       return run_typed<__half>(x, down, up, indices, gates, out, out_f32, T, H, N, k, w, status, stream, between_passes,
-                               act, raw_scores, dtype);
+                               act, raw_scores);
     default:
       return FMOE_ERR_BAD_ARG;
   }

@@ -127,18 +127,14 @@ class FlashMoE(nn.Module):
     def kernels_per_forward(self) -> int:
         """Kernels of this library launched by one fused forward: router GEMM (16-bit modules: the batch-norm is applied
         inside it; float32: a separate normalisation pass), top-k (with the log-softmax inside for num_keys <= 1024),
-        experts (scores + accumulate, or one fused kernel once a 16-bit table reaches 1 GiB), MLP up GEMM, MLP down GEMM; training adds the batch statistics passes."""
+        experts (scores + accumulate), MLP up GEMM, MLP down GEMM; training adds the batch statistics passes."""
         sixteen = self.down_embed.weight.element_size() == 2
         n = 1 + 1 + 1 + 1  # router GEMM, top-k, MLP up, MLP down
         if not sixteen or self.hidden_size % 8 != 0 or self.hidden_size > 3072 or (2 * self.num_keys) % 8 != 0:
             n += 1  # stand-alone normalisation pass
         if self.num_keys > 1024 or not sixteen:
             n += 1  # separate log-softmax pass
-        if sixteen:
-            big = self.num_experts * self.hidden_size * 2 >= (1 << 30) and self.hidden_size <= 2048
-            n += 1 if big else 2
-        else:
-            n += 2
+        n += 2  # experts
         if self.training:
             n += 2  # batch statistics pass + finalize
         return n
