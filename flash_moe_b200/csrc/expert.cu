@@ -646,10 +646,11 @@ ExpertWs carve(void* ws, int64_t T, int64_t N, int k) {
   return w;
 }
 
-// Few tokens: the largest W in {8, 4} whose CTAs leave no warp without slots; 0 selects the one-warp-per-task kernels.
-// Those keep (SMs x 16) warps busy with several gathers in flight each, so splitting pays below half as many tasks.
-int split_warps(int64_t tasks, int pieces) {
-  if (tasks * 2 > static_cast<int64_t>(device_sm_count()) * 16) return 0;
+// Few tokens: warps per task, by the pieces it can be cut into; 0 selects the one-warp-per-task kernels.  `limit` is where
+// those take over (measured over 1 to 1000 tokens): the scores pass at 5 1/3 tasks per SM, the accumulate pass at 8 - or at
+// one, where a task has only 16 slots and two of its four warps would find none (500 tokens x 512, top-16: 9.6 -> 6.3 us).
+int split_warps(int64_t tasks, int pieces, int64_t limit) {
+  if (tasks > limit) return 0;
   return pieces >= 8 ? 8 : pieces >= 2 ? 4 : 0;
 }
 
@@ -666,7 +667,7 @@ bool try_scores_split(const void* rows, const void* table, const int64_t* idx, c
                       cudaError_t* rc) {
   const int groups = (k + 15) / 16;
   const int64_t tasks = T_ * groups;
-  const int split = split_warps(tasks, (H + 127) / 128);
+  const int split = split_warps(tasks, (H + 127) / 128, static_cast<int64_t>(device_sm_count()) * 16 / 3);
   if (split == 0) return false;
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * (64 / split);
   auto kern = split == 8 ? expert_scores_split_kernel<T, 8, PEER> : expert_scores_split_kernel<T, 4, PEER>;
@@ -680,7 +681,8 @@ template <typename T, bool PEER>
 bool try_accum_split(const void* table, const int64_t* idx, const float* coef, void* out, int out_f32, int64_t T_, int H,
                      int64_t N, int k, bool early, cudaStream_t stream, const PeerTable& pt, cudaError_t* rc) {
   constexpr int COLS = 32 * Vec16<T>::N;
-  const int split = split_warps(T_ * ((H + 2 * COLS - 1) / (2 * COLS)), (k + 7) / 8);
+  const int pieces = (k + 7) / 8;
+  const int split = split_warps(T_ * ((H + 2 * COLS - 1) / (2 * COLS)), pieces, static_cast<int64_t>(device_sm_count()) * (pieces >= 3 ? 8 : 1));
   if (split == 0) return false;
   const int colblocks = (H + COLS - 1) / COLS;
   const int64_t tasks = T_ * colblocks;
