@@ -206,8 +206,7 @@ __global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* __restr
     const T* rb = table_row<T, PEER>(down, shards, world, okb ? eb : 0, H, sharded) + 8 * tq;
     float c[4] = {0.f, 0.f, 0.f, 0.f};
     // COLS = 16: a lane takes 16 consecutive columns of a 64-column block, so that the four lanes of a row cover a whole
-    // 128-byte line; in one 32-byte load (LOAD32) an instruction then fetches whole lines of its 8 rows instead of halves:
-    // 51.6 -> 43.3 us at 4096 tokens x 1024 columns, top-64.  Two 16-byte loads give the same sums for tables that are only
+    // 128-byte line, in one 32-byte load (LOAD32) each.  Two 16-byte loads give the same sums for tables that are only
     // 16-byte aligned, or whose alignment the host does not know (PEER).
     auto load = [&](uint4 (&qa)[UNROLL], uint4 (&qb)[UNROLL], int c0) {
       if constexpr (COLS == 16) {
@@ -716,6 +715,16 @@ void launch_accum(const void* up, const int64_t* idx, const float* gs, void* out
                    H, N, k, colblocks, nullptr, 1, 0);  // launch errors surface through the caller's launch check
 }
 
+// Scores pass with one thread's share of a row in 16 columns at a time, for tables of more than 384 MiB: rows taken 64 bytes
+// at a time cost twice the time there (16384 tokens x 2048 columns, top-16, table of 512 MiB 283 -> 153 us, 4 GiB with Zipf
+// 1.1 ids 519 -> 185 at 32768 tokens), and make no difference at 256 MiB (253 and 246).  It also groups the columns of a
+// sum differently, so the smaller tables of a stack of layers, where the last bit of a score can decide a later layer's
+// selection, keep the order that they have; tables in L2 give 16% for that (51 and 43 us at 4096 x 1024, top-64).
+template <typename T>
+bool whole_lines(int64_t N, int H) {
+  return H % 16 == 0 && N * H * static_cast<int64_t>(sizeof(T)) > (384ll << 20);
+}
+
 // per-pair dot products <rows[t], table[e]>: gates != nullptr stores silu(dot) * gate (forward), nullptr the
 // raw dot product
 template <typename T>
@@ -736,8 +745,8 @@ int run_scores(const void* rows, const void* table, const int64_t* idx, const vo
     const int xs_stride = ((H + 255) / 256) * 32;  // uint4 per warp, rows padded to 256 columns
     const int smem = 4 * 2 * xs_stride * 16;  // two x-row buffers per warp
     const bool aligned32 = (reinterpret_cast<uintptr_t>(table) & 31u) == 0;
-    auto kern = H % 16 != 0 ? expert_scores_mma_kernel<T, 4, false, 2, 8>
-                            : aligned32 ? expert_scores_mma_kernel<T, 4, false, 2, 16, true> : expert_scores_mma_kernel<T, 4, false, 2, 16>;
+    auto kern = !whole_lines<T>(N, H) ? expert_scores_mma_kernel<T, 4, false, 2, 8>
+                : aligned32 ? expert_scores_mma_kernel<T, 4, false, 2, 16, true> : expert_scores_mma_kernel<T, 4, false, 2, 16>;
     FMOE_CUDA_TRY(allow_smem(kern, smem));
     FMOE_CUDA_TRY(launch_pdl(4, kern, dim3(grid), dim3(128), smem, stream, 1, static_cast<const T*>(rows),
                              static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, T_, H, N, k, xs_stride,
@@ -1152,7 +1161,7 @@ int run_typed_peer(const void* x, const void* const* down_shards, const void* co
       const int grid = static_cast<int>(want < cap ? want : cap);
       const int xs_stride = ((H + 255) / 256) * 32;
       const int smem = 4 * 2 * xs_stride * 16;  // two x-row buffers per warp
-      auto kern = H % 16 != 0 ? expert_scores_mma_kernel<T, 4, true, 2, 8> : expert_scores_mma_kernel<T, 4, true, 2, 16>;
+      auto kern = whole_lines<T>(N, H) ? expert_scores_mma_kernel<T, 4, true, 2, 16> : expert_scores_mma_kernel<T, 4, true, 2, 8>;
       FMOE_CUDA_TRY(allow_smem(kern, smem));
       kern<<<grid, 128, smem, stream>>>(static_cast<const T*>(x), static_cast<const T*>(hot_down), idx,
                                         static_cast<const T*>(gates), w.gs, T_, H, N + hot_rows, k, xs_stride, status,

@@ -39,3 +39,26 @@ def test_expert_passes_for_few_tokens(T, H, N, k, dtype):
     idx[0, 0] = N  # skipped and reported
     flash_expert_fp32(x, d, u, idx, gates)
     assert _lib.read_status() == _lib.STATUS_BAD_EXPERT_ID
+
+
+@pytest.mark.parametrize("H,offset", [(1040, 0), (1040, 8), (2048, 0), (1032, 0)])
+def test_scores_over_tables_beyond_the_tlb(H, offset):
+    """Tables of more than 384 MiB: whole-line loads, at both alignments and with a ragged last block of columns; 1032 has no
+    16-column pieces."""
+    from flash_moe_b200.ops.flash_expert import flash_expert_fp32
+
+    T, k, N = 801, 16, (400 << 20) // (2 * H)
+    gen = torch.Generator(device="cuda").manual_seed(H)
+
+    def normal(rows, std):
+        flat = torch.empty(rows * H + offset, device="cuda", dtype=torch.bfloat16).normal_(0, std, generator=gen)
+        return flat[offset:].view(rows, H)
+
+    x, d, u = normal(T, 0.5), normal(N, 0.1), normal(N, 1.0)
+    idx = torch.randint(0, N, (T, k), device="cuda", generator=gen)
+    gates = torch.rand(T, k, device="cuda", generator=gen).bfloat16()
+    want = torch.zeros(T, H, dtype=torch.float64, device="cuda")
+    for j in range(k):
+        s = (x.double() * d[idx[:, j]].double()).sum(-1)
+        want += (torch.nn.functional.silu(s) * gates[:, j].double())[:, None] * u[idx[:, j]].double()
+    assert (flash_expert_fp32(x, d, u, idx, gates).double() - want).norm() <= 5e-6 * want.norm()
