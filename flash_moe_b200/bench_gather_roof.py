@@ -18,8 +18,7 @@ from . import _lib
 
 def measure_gather_roof(device, row_bytes: int = 2048, rows: int = 16384, count: int = 262144, reps: int = 5):
     """Best gathered-row rate in GB/s over the probe's variants, and the per-variant results: register loads at a
-    few grid sizes, bulk copies and 16-byte cp.async copies into a shared-memory ring (the latter is how the fused expert
-    kernel fetches its rows)."""
+    few grid sizes, bulk copies and 16-byte cp.async copies into a shared-memory ring."""
     dev = torch.device(device)
     table = torch.ones(rows * row_bytes, dtype=torch.uint8, device=dev)
     ids = torch.randint(0, rows, (count,), device=dev, dtype=torch.int32, generator=torch.Generator(device=dev).manual_seed(1))

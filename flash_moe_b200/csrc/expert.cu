@@ -1137,7 +1137,7 @@ __global__ void __launch_bounds__(256) expert_bwd_finish_kernel(const int* __res
 }
 
 // Tables sharded over the GPUs of one node, rows of the other GPUs read through peer pointers: the two gather
-// kernels of the per-token schedule with the row address computed from (e % world, e / world).
+// kernels with the row address computed from (e % world, e / world).
 // hot_down / hot_up (nullable, hot_rows rows): tables replicated on every GPU, addressed by the ids N .. N + hot_rows - 1
 template <typename T>
 int run_typed_peer(const void* x, const void* const* down_shards, const void* const* up_shards, int world,

@@ -3,10 +3,9 @@
 // tables sit in L2.  Two ways of fetching a row:
 //   mode 0  16-byte loads into registers (4 rows x row_bytes / 512 loads per lane in flight, many CTAs per SM);
 //   mode 1  one bulk asynchronous copy per row into a shared-memory ring (one CTA per SM, a producer warp issuing
-//           groups of 16 rows on an mbarrier, a consumer warp handing the slots back), the way the fused expert
-//           kernel could fetch its rows;
+//           groups of 16 rows on an mbarrier, a consumer warp handing the slots back);
 //   mode 2  the same ring filled by four producer warps with 16-byte cp.async copies whose completion arrives on
-//           the group's mbarrier - the way the fused expert kernel does fetch them.
+//           the group's mbarrier.
 // Row ids outside [0, num_rows) read row 0 instead and raise FMOE_STATUS_BAD_ROW_INDEX.
 #include "common.cuh"
 #include "ptx_sm100.cuh"

@@ -12,9 +12,7 @@
 // Rules that follow from sharing one array:
 //   * shapes whose scratch need (fmoe_expert_workspace_bytes) exceeds 8 MiB are refused with
 //     FMOE_ERR_WORKSPACE - use fmoe_expert_forward with your own workspace for those;
-//   * the array keeps whatever the previous call left in it; the parts that must start at zero
-//     (the per-expert counters of the expert-centric schedule) are cleared on the stream by every
-//     call, nothing else is assumed about its contents;
+//   * the array keeps whatever the previous call left in it; nothing is assumed about its contents;
 //   * two calls that overlap on the GPU (different streams, no ordering between them) race on
 //     the array - serialise them on one stream or with events;
 //   * the first call on each device resolves the array's device address (cudaGetSymbolAddress) - with lazy module
