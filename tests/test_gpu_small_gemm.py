@@ -18,10 +18,12 @@ def mlp_case(T, H, I, dtype):
 
 @pytest.mark.parametrize(
     "T,H,I",
-    [(1, 4, 4), (33, 36, 68), (31, 1028, 132), (256, 256, 1024), (300, 192, 1500), (1030, 512, 2300)],
+    [(1, 4, 4), (33, 36, 68), (31, 1028, 132), (256, 256, 1024), (300, 192, 1500), (1030, 512, 2300), (100, 2052, 4100),
+     (16, 200, 1028), (700, 516, 1500)],
 )
 def test_mlp_float32_tiles(T, H, I):
-    """32 x 32 tiles with K split over thread groups, 64 x 64 and 128-row tiles, remainders in every dimension."""
+    """32 x 32 tiles with K split over thread groups and clusters of 2 and 4, 64 x 64 and 128-row tiles, remainders in every
+    dimension, a cluster with fewer k-steps than CTAs."""
     from flash_moe_b200.ops.flash_mlp import flash_mlp_add
 
     x, wg, wu, wd, h = mlp_case(T, H, I, torch.float32)
