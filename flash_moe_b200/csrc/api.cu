@@ -182,11 +182,12 @@ int mlp_up(const void* x, const void* gw, const void* uw, void* h, int dtype, in
 
 // residual (nullable): [T, H] in the module dtype, added with the float32 addend before the single rounding
 int mlp_down(const void* h, const void* dw, const float* addend, void* out, int dtype, int64_t T, int H, int I,
-             int32_t* status, cudaStream_t stream, const void* residual = nullptr) {
+             int32_t* status, cudaStream_t stream, const void* residual = nullptr, bool h_complete = false) {
   const bool tc = is16(dtype) && (H % 8 == 0) && (I % 8 == 0) && aligned16(dw) && aligned16(out) &&
                   (addend == nullptr || aligned16(addend)) && (residual == nullptr || aligned16(residual));
   if (tc && gemm_narrow_preferred(T, H, I, false))  // the up GEMM runs just before: its predecessor is always ours
-    return launch_gemm_add_narrow(h, dw, addend, out, dtype, T, H, I, true, status, stream, residual);
+    return launch_gemm_add_narrow(h, dw, addend, out, dtype, T, H, I, kEarlyWeights | (h_complete ? kEarlyTokens : 0), status,
+                                  stream, residual);
   if (tc && gemm_pair_supported(T, H, I))
     return launch_gemm_add_pair(h, dw, addend, out, dtype, T, H, I, status, stream, residual);
   return launch_simt_gemm(h, I, dw, nullptr, addend, out, H, dtype, 0, T, H, I, stream, residual);
@@ -545,7 +546,10 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   }
   // y = h Wd^T + experts, one rounding
   FMOE_MARK(FMOE_STAGE_MLP_DOWN, 0, s);
-  rc = mlp_down(w.h, a->down_proj, static_cast<const float*>(w.acc), a->y, dtype, T, H, I, a->status, s, a->residual);
+  // With the gate/up GEMM first, h is complete before the expert passes start (the top-k has waited for the router GEMM, that
+  // for the gate/up GEMM): the down GEMM runs beside them up to its epilogue, 1 token in a graph 29.4 -> 26.7 us, 64 tokens 54 -> 53.
+  rc = mlp_down(w.h, a->down_proj, static_cast<const float*>(w.acc), a->y, dtype, T, H, I, a->status, s, a->residual,
+                up_first && k > 0);
   if (rc != FMOE_OK) return fail(rc);
   FMOE_MARK(FMOE_STAGE_MLP_DOWN, 1, s);
 #undef FMOE_MARK

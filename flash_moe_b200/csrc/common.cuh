@@ -235,14 +235,16 @@ int launch_gemm_add_pair(const void* a, const void* b, const float* addend, void
                          int K, int32_t* status, cudaStream_t stream, const void* residual = nullptr);
 
 // the same two GEMMs for few tokens (gemm_sm100_narrow.cu): weight rows on the MMA's 128 rows, K split over a cluster.
-// early_weights: the kernel before this one in the stream is one of a forward's, so the weights cannot be written any
-// more and may be requested before it has finished.
+// early: kEarlyWeights - the kernel before this one in the stream is one of a forward's, so the weights cannot be written
+// any more and may be requested before it has finished; kEarlyTokens - the token rows are complete too, only the addend comes
+// from that kernel, and everything up to the epilogue runs beside it.
+enum { kEarlyWeights = 1, kEarlyTokens = 2 };
 bool gemm_narrow_preferred(int64_t M, int N, int K, bool swiglu);
 int launch_gemm_swiglu_narrow(const void* x, const void* gate_w, const void* up_w, void* h, int dtype, int64_t M, int I,
-                              int K, bool early_weights, int32_t* status, cudaStream_t stream, void* pre_gate = nullptr,
+                              int K, int early, int32_t* status, cudaStream_t stream, void* pre_gate = nullptr,
                               void* pre_up = nullptr);
 int launch_gemm_add_narrow(const void* a, const void* b, const float* addend, void* out, int dtype, int64_t M, int N,
-                           int K, bool early_weights, int32_t* status, cudaStream_t stream,
+                           int K, int early, int32_t* status, cudaStream_t stream,
                            const void* residual = nullptr);
 
 // fp32-FMA GEMM on CUDA cores (simt_gemm.cu): float32 modules and shapes TMA cannot address.  `ordered`: every output

@@ -542,6 +542,7 @@ __global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __r
   constexpr int SLOTS = 8;
   constexpr int COLS = 32 * VEC;
   __shared__ float part[W][COLS];
+  pdl_launch_dependents();  // all CTAs are resident once the last of them is here: the next kernel may start beside them
   if (!early) pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   bool waited = !early;
@@ -580,7 +581,6 @@ __global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __r
         for (int i = 0; i < VEC / 2; ++i) ffma2(acc[i], pack_f32x2(f[2 * i], f[2 * i + 1]), w2);
       }
     }
-    if (task + gridDim.x >= tasks) pdl_launch_dependents();
 #pragma unroll
     for (int i = 0; i < VEC / 2; ++i) {
       float lo, hi;

@@ -50,7 +50,7 @@ struct NarrowShape {
   int stages;
   int xchg_bytes;   // buffer of the partial sums (0 without a split)
   int acc_cols;     // TMEM columns per accumulator (power of two)
-  int early;        // the weights may be requested before the predecessor kernel has finished
+  int early;        // kEarlyWeights | kEarlyTokens
 };
 
 __device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, const uint32_t (&v)[4]) {
@@ -85,6 +85,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
   const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0);  // known to be warp-uniform
   const int lane = threadIdx.x & 31;
   const int S = gridDim.x;  // = cluster size
+  const bool late = (sh.early & kEarlyTokens) != 0;
   const int rank = blockIdx.x;
   const int r0 = blockIdx.y * BLOCK_R;
   const int t0 = blockIdx.z * sh.bn;
@@ -120,7 +121,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
       if (NB == 2) ptx::prefetch_tensormap(&tmW1);
     }
     const int first = nkb < sh.stages ? nkb : sh.stages;
-    if (sh.early) {
+    if (sh.early & kEarlyWeights) {
       for (int i = 0; i < first; ++i)
         if (ptx::elect_one()) {
           ptx::mbar_arrive_expect_tx(full_bar(i), stage_bytes);
@@ -128,11 +129,13 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
         }
     }
     __syncwarp();
-    pdl_wait();  // the tokens come from the kernel before this one
-    pdl_launch_dependents();
+    if (!late) {
+      pdl_wait();  // the tokens come from the kernel before this one
+      pdl_launch_dependents();
+    }
     for (int i = 0; i < first; ++i)
       if (ptx::elect_one()) {
-        if (!sh.early) {
+        if (!(sh.early & kEarlyWeights)) {
           ptx::mbar_arrive_expect_tx(full_bar(i), stage_bytes);
           load_weights(i, i);
         }
@@ -168,8 +171,10 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
     ptx::tc_fence_after();
     // a CTA's shared memory may be written by its peers once all have arrived here; the wait is in front of the exchange
     if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    pdl_wait();
-    pdl_launch_dependents();  // this CTA holds its tensor memory: once all do, the next kernel may set up
+    if (!late) {
+      pdl_wait();
+      pdl_launch_dependents();  // this CTA holds its tensor memory: once all do, the next kernel may set up
+    }
   }
   const uint32_t tmem_base = warp == 0 ? 0u : __shfl_sync(kFull, *tmem_slot, 0);
 
@@ -204,6 +209,10 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
   }
 
   // ---------------------------------------------------------------- epilogue
+  if (late) {  // the addend comes from the kernel before this one
+    pdl_wait();
+    pdl_launch_dependents();
+  }
   const bool epilogue_warp = warp >= 2;
   const int q = warp & 3;            // TMEM lane quarter this warp may read
   const int turn = (warp - 2) >> 2;  // which of the quarter's two warps
@@ -429,7 +438,7 @@ double pair_cost(int64_t M, int N, int K, int nb) {
 
 template <int BLOCK_R, int EPI, typename T>
 int launch_plan(const NarrowPlan& p, const void* w0, const void* w1, const void* x, const NarrowEpi& ep, int dtype, int64_t M,
-                int N, int K, bool early_weights, int32_t* status, cudaStream_t stream) {
+                int N, int K, int early, int32_t* status, cudaStream_t stream) {
   constexpr int NB = EPI == NARROW_SWIGLU ? 2 : 1;
   CUtensorMap tW0, tW1, tX;
   int rc;
@@ -446,7 +455,7 @@ int launch_plan(const NarrowPlan& p, const void* w0, const void* w1, const void*
   sh.stages = p.stages;
   sh.xchg_bytes = p.split > 1 ? NB * p.bn * BLOCK_R * 4 : 0;
   sh.acc_cols = next_pow2(p.bn);
-  sh.early = early_weights ? 1 : 0;
+  sh.early = early;
   const int smem = p.stages * (NB * BLOCK_R * BLOCK_K * 2 + p.bn * BLOCK_K * 2) + sh.xchg_bytes + kBarBytes + 1024;
   auto kern = gemm_narrow_kernel<BLOCK_R, EPI, T>;
   FMOE_CUDA_TRY(allow_smem(kern, kSmemLimit));
@@ -457,10 +466,10 @@ int launch_plan(const NarrowPlan& p, const void* w0, const void* w1, const void*
 
 template <int EPI, typename T>
 int launch_narrow(const void* w0, const void* w1, const void* x, const NarrowEpi& ep, int dtype, int64_t M, int N, int K,
-                  bool early_weights, int32_t* status, cudaStream_t stream) {
+                  int early, int32_t* status, cudaStream_t stream) {
   const NarrowPlan p = plan_narrow(M, N, K, EPI == NARROW_SWIGLU ? 2 : 1);
-  if (p.rows == 64) return launch_plan<64, EPI, T>(p, w0, w1, x, ep, dtype, M, N, K, early_weights, status, stream);
-  return launch_plan<128, EPI, T>(p, w0, w1, x, ep, dtype, M, N, K, early_weights, status, stream);
+  if (p.rows == 64) return launch_plan<64, EPI, T>(p, w0, w1, x, ep, dtype, M, N, K, early, status, stream);
+  return launch_plan<128, EPI, T>(p, w0, w1, x, ep, dtype, M, N, K, early, status, stream);
 }
 
 }  // namespace
@@ -474,21 +483,21 @@ bool gemm_narrow_preferred(int64_t M, int N, int K, bool swiglu) {
 }
 
 int launch_gemm_swiglu_narrow(const void* x, const void* gate_w, const void* up_w, void* h, int dtype, int64_t M, int I,
-                              int K, bool early_weights, int32_t* status, cudaStream_t stream, void* pre_gate,
+                              int K, int early, int32_t* status, cudaStream_t stream, void* pre_gate,
                               void* pre_up) {
   if ((pre_gate == nullptr) != (pre_up == nullptr)) return FMOE_ERR_BAD_ARG;
   const NarrowEpi ep{h, nullptr, nullptr, pre_gate, pre_up, I};
   if (dtype == FMOE_DTYPE_BF16)
-    return launch_narrow<NARROW_SWIGLU, __nv_bfloat16>(gate_w, up_w, x, ep, dtype, M, I, K, early_weights, status, stream);
-  return launch_narrow<NARROW_SWIGLU, __half>(gate_w, up_w, x, ep, dtype, M, I, K, early_weights, status, stream);
+    return launch_narrow<NARROW_SWIGLU, __nv_bfloat16>(gate_w, up_w, x, ep, dtype, M, I, K, early, status, stream);
+  return launch_narrow<NARROW_SWIGLU, __half>(gate_w, up_w, x, ep, dtype, M, I, K, early, status, stream);
 }
 
 int launch_gemm_add_narrow(const void* a, const void* b, const float* addend, void* out, int dtype, int64_t M, int N,
-                           int K, bool early_weights, int32_t* status, cudaStream_t stream, const void* residual) {
+                           int K, int early, int32_t* status, cudaStream_t stream, const void* residual) {
   const NarrowEpi ep{out, addend, residual, nullptr, nullptr, N};
   if (dtype == FMOE_DTYPE_BF16)
-    return launch_narrow<NARROW_ADD, __nv_bfloat16>(b, b, a, ep, dtype, M, N, K, early_weights, status, stream);
-  return launch_narrow<NARROW_ADD, __half>(b, b, a, ep, dtype, M, N, K, early_weights, status, stream);
+    return launch_narrow<NARROW_ADD, __nv_bfloat16>(b, b, a, ep, dtype, M, N, K, early, status, stream);
+  return launch_narrow<NARROW_ADD, __half>(b, b, a, ep, dtype, M, N, K, early, status, stream);
 }
 
 }  // namespace fmoe
