@@ -125,8 +125,7 @@ size_t router_front_ws(int64_t T, int H, int dtype) {
 // logp == nullptr: stop after the logits (the caller applies the log-softmax elsewhere)
 int router_front(const void* x, const void* w, void* rm, void* rv, int training, float momentum, float eps,
                  void* logits, void* logp, int dtype, int64_t T, int H, int nk, void* ws, size_t ws_bytes,
-                 int32_t* status, cudaStream_t stream, const float* bn_sums = nullptr, int64_t bn_count = 0,
-                 bool beside_predecessor = false) {
+                 int32_t* status, cudaStream_t stream, const float* bn_sums = nullptr, int64_t bn_count = 0) {
   if (!valid_dtype(dtype) || T < 0 || H <= 0 || nk <= 0) return FMOE_ERR_BAD_ARG;
   if (T == 0) return FMOE_OK;
   if (x == nullptr || w == nullptr || logits == nullptr) return FMOE_ERR_BAD_ARG;
@@ -147,7 +146,7 @@ int router_front(const void* x, const void* w, void* rm, void* rv, int training,
       return FMOE_ERR_BAD_ARG;
     }
     return launch_router_bn_gemm(x, w, mean, invstd, training ? nullptr : rm, training ? nullptr : rv, eps, logits, dtype,
-                                 T, 2 * nk, H, beside_predecessor && !training, status, stream);
+                                 T, 2 * nk, H, status, stream);
   }
   rc = launch_bn(x, xn, rm, rv, training, momentum, eps, dtype, T, H, bnws, bn_sums, bn_count, stream);
   if (rc != FMOE_OK) return rc;
@@ -171,10 +170,11 @@ bool mlp_up_is_narrow(const void* x, const void* gw, const void* uw, int dtype, 
 }
 
 int mlp_up(const void* x, const void* gw, const void* uw, void* h, int dtype, int64_t T, int H, int I, int32_t* status,
-           cudaStream_t stream, void* pre_gate = nullptr, void* pre_up = nullptr) {
+           cudaStream_t stream, void* pre_gate = nullptr, void* pre_up = nullptr, bool beside_predecessor = false) {
   const bool tc = is16(dtype) && (H % 8 == 0) && (I % 8 == 0) && aligned16(x) && aligned16(gw) && aligned16(uw);
   if (mlp_up_is_narrow(x, gw, uw, dtype, T, H, I))
-    return launch_gemm_swiglu_narrow(x, gw, uw, h, dtype, T, I, H, false, status, stream, pre_gate, pre_up);
+    return launch_gemm_swiglu_narrow(x, gw, uw, h, dtype, T, I, H, beside_predecessor ? kEarlyWeights | kEarlyTokens : 0, status,
+                                     stream, pre_gate, pre_up);
   if (tc && gemm_pair_supported(T, I, H))
     return launch_gemm_swiglu_pair(x, gw, uw, h, dtype, T, I, H, status, stream, pre_gate, pre_up);
   return launch_simt_gemm(x, H, gw, uw, nullptr, h, I, dtype, 1, T, I, H, stream, nullptr, false, pre_gate, pre_up);
@@ -452,22 +452,20 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   // kernel applies the per-half log-softmax itself (each warp already holds both halves of its
   // token in registers), which saves a [2, T, nk] round trip and a serial GEMM epilogue.
   const bool topk_from_logits = is16(dtype) && nk <= 1024;
-  // Few tokens: the gate/up GEMM goes first and the router GEMM runs beside it.  Both only read the caller's tensors, so
-  // the router GEMM need not wait for the other's end (with the few-token expert passes, 64 tokens in a graph: 81 -> 60 us).
-  // A caller that asks for stage events gets the stages one after the other.
-  const bool up_first = (s2 == nullptr || s2 == s) && !a->training && topk_from_logits && a->stage_events == nullptr &&
-                        mlp_up_is_narrow(a->x, a->gate_proj, a->up_proj, dtype, T, H, I);
-  if (up_first) {
-    rc = mlp_up(a->x, a->gate_proj, a->up_proj, w.h, dtype, T, H, I, a->status, s);
-    if (rc != FMOE_OK) return rc;
-  }
+  // Few tokens: the gate/up GEMM follows the router GEMM and needs nothing from it, so it runs beside it, and the top-k, which
+  // needs the logits only, beside the gate/up GEMM.  A caller that asks for stage events gets the stages one after the other.
+  const bool up_beside = (s2 == nullptr || s2 == s) && !a->training && topk_from_logits && a->stage_events == nullptr &&
+                         mlp_up_is_narrow(a->x, a->gate_proj, a->up_proj, dtype, T, H, I);
   FMOE_MARK(FMOE_STAGE_ROUTER_FRONT, 0, s);
   rc = router_front(a->x, a->router_gate, a->running_mean, a->running_var, a->training, a->bn_momentum, a->bn_eps,
                     a->router_logits, topk_from_logits ? nullptr : w.logp, dtype, T, H, nk, w.front, w.front_bytes,
-                    a->status, s, a->training ? a->bn_global_sums : nullptr, a->bn_global_count,
-                    up_first);
+                    a->status, s, a->training ? a->bn_global_sums : nullptr, a->bn_global_count);
   if (rc != FMOE_OK) return rc;
   FMOE_MARK(FMOE_STAGE_ROUTER_FRONT, 1, s);
+  if (up_beside) {
+    rc = mlp_up(a->x, a->gate_proj, a->up_proj, w.h, dtype, T, H, I, a->status, s, nullptr, nullptr, true);
+    if (rc != FMOE_OK) return rc;
+  }
 
   // shared MLP, first half: h = silu(x Wg^T) * (x Wu^T).  It is independent of routing; on the side
   // stream it is forked AFTER the router GEMM (both want a whole SM's shared memory and its tensor memory) so that
@@ -498,7 +496,7 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   rc = FMOE_ERR_UNSUPPORTED;
   if (topk_from_logits)
     rc = launch_router_topk(a->router_logits, dtype, T, nk, k, w.scores, indices, gates,
-                            (a->norm_topk_prob ? 1 : 0) | 2, s);
+                            (a->norm_topk_prob ? kTopkNorm : 0) | kTopkFromLogits | (up_beside ? kTopkLateWait : 0), s);
   if (rc == FMOE_ERR_UNSUPPORTED) {
     if (topk_from_logits) {  // shapes the register kernel does not cover: explicit log-softmax pass
       rc = launch_log_softmax_halves(a->router_logits, w.logp, dtype, T, nk, s);
@@ -514,7 +512,7 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   // the top-k held to one CTA per SM so that the GEMM fits beside it, the top-k itself takes 165 us, because one
   // token costs a warp about 20 us of dependent instructions and all 4096 tokens must be resident at once; and with
   // the GEMM's ring cut to four stages, so that four top-k CTAs fit beside it, the step takes 224 against 216 us.)
-  bool joined = up_first;
+  bool joined = up_beside;
   if (fj != nullptr) {
     if (cudaStreamWaitEvent(s, fj->join, 0) != cudaSuccess) return fail(-static_cast<int>(cudaErrorUnknown));
     fj = nullptr;
@@ -546,10 +544,9 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   }
   // y = h Wd^T + experts, one rounding
   FMOE_MARK(FMOE_STAGE_MLP_DOWN, 0, s);
-  // With the gate/up GEMM first, h is complete before the expert passes start (the top-k has waited for the router GEMM, that
-  // for the gate/up GEMM): the down GEMM runs beside them up to its epilogue, 1 token in a graph 29.4 -> 26.7 us, 64 tokens 54 -> 53.
+  // With the gate/up GEMM in front of the top-k, h is complete before the expert passes start: the down GEMM runs beside them up to its epilogue, 1 token in a graph 29.4 -> 26.7 us, 64 tokens 54 -> 53.
   rc = mlp_down(w.h, a->down_proj, static_cast<const float*>(w.acc), a->y, dtype, T, H, I, a->status, s, a->residual,
-                up_first && k > 0);
+                up_beside && k > 0);
   if (rc != FMOE_OK) return fail(rc);
   FMOE_MARK(FMOE_STAGE_MLP_DOWN, 1, s);
 #undef FMOE_MARK
@@ -594,7 +591,7 @@ int fmoe_train_forward(const fmoe_train_args* a, int* have_preacts) {
   const TrainWs w = carve_train(a->workspace, T, H, I, N, k, dtype);
   if (a->workspace_bytes < w.total) return FMOE_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
-  int rc = launch_router_topk(a->log_probs, dtype, T, nk, k, w.scores, a->indices, a->gates, (a->norm_topk_prob ? 1 : 0) | 4, s);
+  int rc = launch_router_topk(a->log_probs, dtype, T, nk, k, w.scores, a->indices, a->gates, (a->norm_topk_prob ? kTopkNorm : 0) | kTopkTokenRows, s);
   if (rc != FMOE_OK) return rc;
   rc = launch_expert_forward(a->x, a->down_embed, a->up_embed, a->indices, a->gates, w.acc, dtype, FMOE_DTYPE_F32, T, H, N, k,
                              w.expert, w.expert_bytes, a->status, s, nullptr, kActSilu, a->expert_scores);

@@ -68,8 +68,8 @@ template <typename T>
 __global__ void router_topk_smem_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int k, RouterSmemLayout L,
                                    T* __restrict__ scores, int64_t* __restrict__ indices, T* __restrict__ gates,
                                    int flags) {
-  const int norm = flags & 1;
-  const bool token_rows = (flags & 4) != 0;  // [T, 2, nk] instead of [2, T, nk]
+  const int norm = flags & kTopkNorm;
+  const bool token_rows = (flags & kTopkTokenRows) != 0;  // [T, 2, nk] instead of [2, T, nk]
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -274,6 +274,14 @@ template <> struct HalfKey<__half> : HalfKey16<__half> {};
 
 // One lane's E consecutive elements of a row (element lane * E + r -> v[r]); entries past nk read as -inf.  Whole
 // rows of 32 E elements at a 16-byte aligned address are fetched with one or a few vector loads.
+// Rows are read past the L1 cache: with kTopkLateWait a CTA starts beside an unrelated kernel.
+__device__ __forceinline__ float load_cg(const float* p) { return __ldcg(p); }
+template <typename T>
+__device__ __forceinline__ T load_cg(const T* p) {
+  const unsigned short raw = __ldcg(reinterpret_cast<const unsigned short*>(p));
+  return *reinterpret_cast<const T*>(&raw);
+}
+
 template <typename T, int E>
 __device__ __forceinline__ void load_blocked(const T* __restrict__ row, int nk, int lane, float (&v)[E]) {
   constexpr int BYTES = E * static_cast<int>(sizeof(T));
@@ -282,11 +290,11 @@ __device__ __forceinline__ void load_blocked(const T* __restrict__ row, int nk, 
     const T* src = row + lane * E;
     if constexpr (BYTES % 16 == 0) {
 #pragma unroll
-      for (int j = 0; j < BYTES / 16; ++j) reinterpret_cast<uint4*>(tmp)[j] = reinterpret_cast<const uint4*>(src)[j];
+      for (int j = 0; j < BYTES / 16; ++j) reinterpret_cast<uint4*>(tmp)[j] = __ldcg(reinterpret_cast<const uint4*>(src) + j);
     } else if constexpr (BYTES == 8) {
-      *reinterpret_cast<uint2*>(tmp) = *reinterpret_cast<const uint2*>(src);
+      *reinterpret_cast<uint2*>(tmp) = __ldcg(reinterpret_cast<const uint2*>(src));
     } else if constexpr (BYTES == 4) {
-      *reinterpret_cast<uint32_t*>(tmp) = *reinterpret_cast<const uint32_t*>(src);
+      *reinterpret_cast<uint32_t*>(tmp) = __ldcg(reinterpret_cast<const unsigned int*>(src));
     }
 #pragma unroll
     for (int r = 0; r < E; ++r) v[r] = to_f32<T>(tmp[r]);
@@ -294,7 +302,7 @@ __device__ __forceinline__ void load_blocked(const T* __restrict__ row, int nk, 
 #pragma unroll
     for (int r = 0; r < E; ++r) {
       const int i = lane * E + r;
-      v[r] = (i < nk) ? to_f32<T>(row[i]) : -INFINITY;
+      v[r] = (i < nk) ? to_f32<T>(load_cg(row + i)) : -INFINITY;
     }
   }
 }
@@ -346,9 +354,9 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restric
                                                              RouterRegLayout L, T* __restrict__ scores,
                                                              int64_t* __restrict__ indices, T* __restrict__ gates,
                                                              int flags) {
-  const int norm = flags & 1;
-  const bool from_logits = (flags & 2) != 0;
-  const bool token_rows = (flags & 6) != 0;  // [T, 2, nk] instead of [2, T, nk]
+  const int norm = flags & kTopkNorm;
+  const bool from_logits = (flags & kTopkFromLogits) != 0;
+  const bool token_rows = (flags & (kTopkFromLogits | kTopkTokenRows)) != 0;  // [T, 2, nk] instead of [2, T, nk]
   using HK = HalfKey<T>;
   using K = typename HK::type;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -384,7 +392,8 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restric
     pq[c] = (static_cast<uint32_t>(lo) << 16) | static_cast<uint32_t>(c - rowstart[lo]);
   }
   __syncthreads();
-  pdl_wait();  // the staircase table above depends on k alone; the logits come from the previous kernel
+  // the staircase table above depends on k alone; the logits come from the previous kernel (kTopkLateWait: the one before)
+  if (!(flags & kTopkLateWait)) pdl_wait();
 
   unsigned char* wbase = smem + L.cta_bytes + warp * L.warp_bytes;
   float* va = reinterpret_cast<float*>(wbase);  // index order
@@ -696,6 +705,7 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restric
     }
     __syncwarp();
   }
+  if (flags & kTopkLateWait) pdl_wait();
 }
 
 RouterRegLayout make_reg_layout(int nk, int k) {
@@ -850,9 +860,9 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
   constexpr int LOW = OrdLowBits<T>::value;
   constexpr bool kKeysInRegs = E <= 8;     // both halves' values stay in registers up to the compaction
   constexpr bool kUnrollCells = CPL <= 10;  // see sort_desc: small kernels are unrolled, large ones are loops
-  const int norm = flags & 1;
-  const bool from_logits = (flags & 2) != 0;
-  const bool token_rows = (flags & 6) != 0;  // [T, 2, nk] instead of [2, T, nk]
+  const int norm = flags & kTopkNorm;
+  const bool from_logits = (flags & kTopkFromLogits) != 0;
+  const bool token_rows = (flags & (kTopkFromLogits | kTopkTokenRows)) != 0;  // [T, 2, nk] instead of [2, T, nk]
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -887,7 +897,8 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
     pq[c] = (static_cast<uint32_t>(lo) << 16) | static_cast<uint32_t>(c - rowstart[lo]);
   }
   __syncthreads();
-  pdl_wait();  // the staircase table above depends on k alone; the logits come from the previous kernel
+  // the staircase table above depends on k alone; the logits come from the previous kernel (kTopkLateWait: the one before)
+  if (!(flags & kTopkLateWait)) pdl_wait();
 
   unsigned char* wbase = smem + L.cta_bytes + warp * L.warp_bytes;
   float* sa = reinterpret_cast<float*>(wbase);  // values in rank order; the key lists lie here before they are sorted
@@ -1245,6 +1256,7 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
     }
     __syncwarp();
   }
+  if (flags & kTopkLateWait) pdl_wait();
 }
 
 RouterPrunedLayout make_pruned_layout(int nk, int k) {
@@ -1394,14 +1406,12 @@ int launch_typed(const void* logp, int64_t T_, int nk, int k, void* scores, int6
       }
     }
   }
-  if (norm & 2) return FMOE_ERR_UNSUPPORTED;  // raw logits are only accepted by the register kernel
+  if (norm & kTopkFromLogits) return FMOE_ERR_UNSUPPORTED;  // raw logits are only accepted by the register kernel
   return launch_smem<T>(logp, T_, nk, k, scores, indices, gates, norm, stream);
 }
 
 }  // namespace
 
-// norm: bit 0 = renormalise the gates per token, bit 1 = `log_probs` holds raw logits [T, 2*nk], bit 2 = it holds
-// log-probabilities [T, 2, nk]
 int launch_router_topk(const void* log_probs, int dtype, int64_t T, int nk, int k, void* scores, int64_t* indices,
                        void* gates, int norm, cudaStream_t stream) {
   if (T < 0 || nk <= 0 || k < 0 || k > nk) return FMOE_ERR_BAD_ARG;
