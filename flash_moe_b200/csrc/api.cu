@@ -61,6 +61,16 @@ cudaError_t allow_smem_impl(const void* kern, int bytes) {
   return cudaSuccess;
 }
 
+cudaError_t prefer_smem_impl(const void* kern) {
+  thread_local KernelNotes notes;
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess || notes.find(kern, dev, 0, 0) != nullptr) return err;
+  err = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  if (err == cudaSuccess) notes.add({kern, dev, 0, 0, 1});
+  return err;
+}
+
 cudaError_t resident_ctas_impl(const void* kern, int threads, int smem, int* per_sm) {
   thread_local KernelNotes notes;
   int dev = 0;
@@ -169,6 +179,11 @@ bool mlp_up_is_narrow(const void* x, const void* gw, const void* uw, int dtype, 
          gemm_narrow_preferred(T, I, H, true);
 }
 
+bool mlp_up_on_tensor_cores(const void* x, const void* gw, const void* uw, int dtype, int64_t T, int H, int I) {
+  return mlp_up_is_narrow(x, gw, uw, dtype, T, H, I) ||
+         (is16(dtype) && (H % 8 == 0) && (I % 8 == 0) && aligned16(x) && aligned16(gw) && aligned16(uw) && gemm_pair_supported(T, I, H));
+}
+
 int mlp_up(const void* x, const void* gw, const void* uw, void* h, int dtype, int64_t T, int H, int I, int32_t* status,
            cudaStream_t stream, void* pre_gate = nullptr, void* pre_up = nullptr, bool beside_predecessor = false) {
   const bool tc = is16(dtype) && (H % 8 == 0) && (I % 8 == 0) && aligned16(x) && aligned16(gw) && aligned16(uw);
@@ -176,7 +191,7 @@ int mlp_up(const void* x, const void* gw, const void* uw, void* h, int dtype, in
     return launch_gemm_swiglu_narrow(x, gw, uw, h, dtype, T, I, H, beside_predecessor ? kEarlyWeights | kEarlyTokens : 0, status,
                                      stream, pre_gate, pre_up);
   if (tc && gemm_pair_supported(T, I, H))
-    return launch_gemm_swiglu_pair(x, gw, uw, h, dtype, T, I, H, status, stream, pre_gate, pre_up);
+    return launch_gemm_swiglu_pair(x, gw, uw, h, dtype, T, I, H, status, stream, pre_gate, pre_up, beside_predecessor);
   return launch_simt_gemm(x, H, gw, uw, nullptr, h, I, dtype, 1, T, I, H, stream, nullptr, false, pre_gate, pre_up);
 }
 
@@ -455,7 +470,7 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   // Few tokens: the gate/up GEMM follows the router GEMM and needs nothing from it, so it runs beside it, and the top-k, which
   // needs the logits only, beside the gate/up GEMM.  A caller that asks for stage events gets the stages one after the other.
   const bool up_beside = (s2 == nullptr || s2 == s) && !a->training && topk_from_logits && a->stage_events == nullptr &&
-                         mlp_up_is_narrow(a->x, a->gate_proj, a->up_proj, dtype, T, H, I);
+                         mlp_up_on_tensor_cores(a->x, a->gate_proj, a->up_proj, dtype, T, H, I);
   FMOE_MARK(FMOE_STAGE_ROUTER_FRONT, 0, s);
   rc = router_front(a->x, a->router_gate, a->running_mean, a->running_var, a->training, a->bn_momentum, a->bn_eps,
                     a->router_logits, topk_from_logits ? nullptr : w.logp, dtype, T, H, nk, w.front, w.front_bytes,

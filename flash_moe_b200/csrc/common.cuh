@@ -39,6 +39,10 @@ cudaError_t resident_ctas_impl(const void* kern, int threads, int smem, int* per
 template <typename K> inline cudaError_t allow_smem(K* kern, int bytes) {
   return allow_smem_impl(reinterpret_cast<const void*>(kern), bytes);
 }
+// The kernel's SMs are set up with as much shared memory as there is.  An SM changes that split only while it is idle, so
+// without it a kernel with little shared memory does not start beside one that fills an SM's.
+cudaError_t prefer_smem_impl(const void* kern);
+template <typename K> inline cudaError_t prefer_smem(K* kern) { return prefer_smem_impl(reinterpret_cast<const void*>(kern)); }
 template <typename K> inline cudaError_t resident_ctas(K* kern, int threads, int smem, int* per_sm) {
   return resident_ctas_impl(reinterpret_cast<const void*>(kern), threads, smem, per_sm);
 }
@@ -233,7 +237,7 @@ int launch_router_bn_gemm(const void* x, const void* w, const float* mean, const
 bool gemm_pair_supported(int64_t M, int N, int K);
 int launch_gemm_swiglu_pair(const void* x, const void* gate_w, const void* up_w, void* h, int dtype, int64_t M, int I,
                             int K, int32_t* status, cudaStream_t stream, void* pre_gate = nullptr,
-                            void* pre_up = nullptr);
+                            void* pre_up = nullptr, bool release_next = false);
 int launch_gemm_add_pair(const void* a, const void* b, const float* addend, void* out, int dtype, int64_t M, int N,
                          int K, int32_t* status, cudaStream_t stream, const void* residual = nullptr);
 

@@ -129,8 +129,10 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
         }
     }
     __syncwarp();
-    if (!late) pdl_wait();  // the tokens come from the kernel before this one
-    pdl_launch_dependents();
+    if (!late) {
+      pdl_wait();  // the tokens come from the kernel before this one
+      pdl_launch_dependents();
+    }
     for (int i = 0; i < first; ++i)
       if (ptx::elect_one()) {
         if (!(sh.early & kEarlyWeights)) {
@@ -169,9 +171,12 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
     ptx::tc_fence_after();
     // a CTA's shared memory may be written by its peers once all have arrived here; the wait is in front of the exchange
     if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    // late: only the epilogue waits; this CTA, and with it the next kernel, still ends after the kernel before this one
-    if (!late || warp >= 2) pdl_wait();
-    pdl_launch_dependents();  // this CTA holds its tensor memory: once all do, the next kernel may set up
+    // late: only the epilogue waits.  The first thread of a CTA that gets here lets the next kernel start, so with `late` that
+    // is one of those that have waited.
+    if (!late || warp >= 2) {
+      pdl_wait();
+      pdl_launch_dependents();  // this CTA holds its tensor memory: once all do, the next kernel may set up
+    }
   }
   const uint32_t tmem_base = warp == 0 ? 0u : __shfl_sync(kFull, *tmem_slot, 0);
 

@@ -37,7 +37,7 @@ constexpr int RING_BYTES = STAGES * STAGE_BYTES;
 constexpr int ADDEND_CHUNK_BYTES = BLOCK_M * 32 * 4;  // this CTA's 128 rows x 32 float32 columns of the addend
 constexpr int ADDEND_BUFS = 2;  // four (with a five-stage ring) measured the same: 35.4 vs 35.8 us
 constexpr int ADDEND_BYTES = ADDEND_BUFS * ADDEND_CHUNK_BYTES;  // chunks on their way while one is being added
-constexpr int SMEM_BYTES = RING_BYTES + ADDEND_BYTES + 256 + 1024;
+constexpr int smem_bytes(int addend_bytes) { return RING_BYTES + addend_bytes + 256 + 1024; }
 
 enum { PAIR_EPI_ADD = 0, PAIR_EPI_SWIGLU = 1 };
 
@@ -49,6 +49,7 @@ struct PairEpi {
   int n_valid;
   void* pre_gate;  // SWIGLU only, nullable: x Wg^T and x Wu^T rounded to T, kept for the backward pass
   void* pre_up;
+  int release_next;  // the next kernel may become resident at once and run beside this one
 };
 
 using epi::UmmaFmt;
@@ -76,7 +77,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   const uint32_t raw_u32 = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw_u32 + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - raw_u32);
-  const uint32_t bar_base = base + RING_BYTES + ADDEND_BYTES;
+  constexpr int kAddend = EPI == PAIR_EPI_ADD ? ADDEND_BYTES : 0;  // the rest is for CTAs of a kernel beside this one
+  const uint32_t bar_base = base + RING_BYTES + kAddend;
   auto a_smem = [&](int s) { return base + s * STAGE_BYTES; };
   auto b_smem = [&](int s) { return base + s * STAGE_BYTES + A_BYTES; };
   auto full_bar = [&](int s) { return bar_base + s * 8; };
@@ -84,8 +86,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   auto tfull_bar = [&](int a) { return bar_base + (2 * STAGES + a) * 8; };
   auto tempty_bar = [&](int a) { return bar_base + (2 * STAGES + 2 + a) * 8; };
   auto cfull_bar = [&](int b) { return bar_base + (2 * STAGES + 4 + b) * 8; };  // addend chunk b has landed
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + RING_BYTES + ADDEND_BYTES + (2 * STAGES + 4 + ADDEND_BUFS) * 8);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + RING_BYTES + ADDEND_BYTES + (2 * STAGES + 4 + ADDEND_BUFS) * 8 + 8);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + RING_BYTES + kAddend + (2 * STAGES + 4 + ADDEND_BUFS) * 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + RING_BYTES + kAddend + (2 * STAGES + 4 + ADDEND_BUFS) * 8 + 8);
 
   const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0);  // known to be warp-uniform
   const int lane = threadIdx.x & 31;
@@ -119,6 +121,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   ptx::tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(kFull, *tmem_slot, 0);
   pdl_wait();  // barriers, tensor memory and tensor maps are ready; the operands come from the kernel before this one
+  if (ep.release_next) pdl_launch_dependents();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -308,13 +311,15 @@ template <int EPI, typename T>
 int launch_pair(const CUtensorMap& tA, const CUtensorMap& tB0, const CUtensorMap& tB1, const PairEpi& ep, int64_t M,
                 int num_n_tiles, int K, int32_t* status, cudaStream_t stream) {
   auto kern = gemm_tcgen05_pair_kernel<EPI, T>;
-  FMOE_CUDA_TRY(allow_smem(kern, SMEM_BYTES));
+  const int smem = smem_bytes(EPI == PAIR_EPI_ADD ? ADDEND_BYTES : 0);
+  FMOE_CUDA_TRY(allow_smem(kern, smem));
+  if (ep.release_next) FMOE_CUDA_TRY(prefer_smem(kern));
   const int num_m_tiles = static_cast<int>((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M));
   const int num_k_blocks = (K + BLOCK_K - 1) / BLOCK_K;
   const int64_t tiles = static_cast<int64_t>(num_m_tiles) * num_n_tiles;
   const int max_pairs = device_sm_count() / 2;
   const int pairs = static_cast<int>(tiles < max_pairs ? tiles : max_pairs);
-  FMOE_CUDA_TRY(launch_pdl(16, kern, dim3(2 * pairs), dim3(kThreads), SMEM_BYTES, stream, 2, tA, tB0, tB1, ep,
+  FMOE_CUDA_TRY(launch_pdl(16, kern, dim3(2 * pairs), dim3(kThreads), smem, stream, 2, tA, tB0, tB1, ep,
                            static_cast<int>(M), num_m_tiles, num_n_tiles, num_k_blocks, status));
   return FMOE_OK;
 }
@@ -326,14 +331,15 @@ int launch_pair(const CUtensorMap& tA, const CUtensorMap& tB0, const CUtensorMap
 bool gemm_pair_supported(int64_t M, int N, int K) { return M >= 512 && N >= 256 && K >= 256; }
 
 int launch_gemm_swiglu_pair(const void* x, const void* gate_w, const void* up_w, void* h, int dtype, int64_t M, int I,
-                            int K, int32_t* status, cudaStream_t stream, void* pre_gate, void* pre_up) {
+                            int K, int32_t* status, cudaStream_t stream, void* pre_gate, void* pre_up,
+                            bool release_next) {
   CUtensorMap tA, tG, tU;
   int rc;
   if ((rc = make_map(&tA, x, dtype, K, M, BLOCK_M)) != FMOE_OK) return rc;
   if ((rc = make_map(&tG, gate_w, dtype, K, I, BLOCK_N / 2)) != FMOE_OK) return rc;
   if ((rc = make_map(&tU, up_w, dtype, K, I, BLOCK_N / 2)) != FMOE_OK) return rc;
   if ((pre_gate == nullptr) != (pre_up == nullptr)) return FMOE_ERR_BAD_ARG;
-  PairEpi ep{h, nullptr, nullptr, I, I, pre_gate, pre_up};
+  PairEpi ep{h, nullptr, nullptr, I, I, pre_gate, pre_up, release_next ? 1 : 0};
   const int n_tiles = (I + 127) / 128;
   if (dtype == FMOE_DTYPE_BF16)
     return launch_pair<PAIR_EPI_SWIGLU, __nv_bfloat16>(tA, tG, tU, ep, M, n_tiles, K, status, stream);
@@ -346,7 +352,7 @@ int launch_gemm_add_pair(const void* a, const void* b, const float* addend, void
   int rc;
   if ((rc = make_map(&tA, a, dtype, K, M, BLOCK_M)) != FMOE_OK) return rc;
   if ((rc = make_map(&tB, b, dtype, K, N, BLOCK_N / 2)) != FMOE_OK) return rc;
-  PairEpi ep{out, addend, residual, N, N, nullptr, nullptr};
+  PairEpi ep{out, addend, residual, N, N, nullptr, nullptr, 0};
   const int n_tiles = (N + 255) / 256;
   CUtensorMap tC = tB;  // third slot: the float32 addend's map (unused without an addend)
   if (addend != nullptr && (rc = epi::make_tensor_map_f32(&tC, addend, N, M, N, BLOCK_M)) != FMOE_OK) return rc;

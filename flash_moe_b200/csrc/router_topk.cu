@@ -705,7 +705,8 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restric
     }
     __syncwarp();
   }
-  if (flags & kTopkLateWait) pdl_wait();
+  // one waiting CTA keeps the grid from ending; more would keep later CTAs from starting
+  if ((flags & kTopkLateWait) && blockIdx.x == gridDim.x - 1) pdl_wait();
 }
 
 RouterRegLayout make_reg_layout(int nk, int k) {
@@ -1256,7 +1257,8 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
     }
     __syncwarp();
   }
-  if (flags & kTopkLateWait) pdl_wait();
+  // one waiting CTA keeps the grid from ending; more would keep later CTAs from starting
+  if ((flags & kTopkLateWait) && blockIdx.x == gridDim.x - 1) pdl_wait();
 }
 
 RouterPrunedLayout make_pruned_layout(int nk, int k) {
@@ -1281,6 +1283,7 @@ int launch_pruned_cpl(const void* logp, int64_t T_, int nk, int k, const RouterP
   const int smem = L.cta_bytes + warps * L.warp_bytes;
   auto kern = router_topk_pruned_kernel<T, E, CPL>;
   FMOE_CUDA_TRY(allow_smem(kern, smem));
+  if (norm & kTopkLateWait) FMOE_CUDA_TRY(prefer_smem(kern));
   int per_sm = 1;
   FMOE_CUDA_TRY(resident_ctas(kern, warps * 32, smem, &per_sm));
   if (per_sm < 1) per_sm = 1;
@@ -1307,6 +1310,7 @@ int launch_reg(const void* logp, int64_t T_, int nk, int k, const RouterRegLayou
   const int smem = L.cta_bytes + warps * L.warp_bytes;
   auto kern = router_topk_reg_kernel<T, E>;
   FMOE_CUDA_TRY(allow_smem(kern, smem));
+  if (norm & kTopkLateWait) FMOE_CUDA_TRY(prefer_smem(kern));
   int per_sm = 1;
   FMOE_CUDA_TRY(resident_ctas(kern, warps * 32, smem, &per_sm));
   if (per_sm < 1) per_sm = 1;

@@ -368,3 +368,28 @@ def test_pre_norm_stack_matches_torch_composition():
     check_status()
     assert torch.equal(got, cur) and torch.equal(replayed, got)
     assert torch.isfinite(got.float()).all()
+
+
+@pytest.mark.parametrize("T,H,I,N,k", [(1, 1024, 4096, 16384, 64), (64, 512, 1000, 4096, 16), (300, 256, 512, 1024, 8),
+                                       (777, 1000, 2728, 10000, 24), (2048, 512, 1024, 4096, 32)])
+@pytest.mark.parametrize("graph", [False, True])
+def test_kernels_beside_each_other_see_this_forwards_data(T, H, I, N, k, graph):
+    """Kernels of one forward run beside each other; with inputs that change from call to call and nothing between the calls,
+    each must read what its own forward wrote, not what the one before left."""
+    from flash_moe_b200 import FlashMoE, FlashMoEConfig, GraphedFlashMoE
+
+    torch.manual_seed(T)
+    with torch.device("cuda"):
+        layer = FlashMoE(FlashMoEConfig(H, I, "silu", N, k, True)).bfloat16().eval()
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    xs = [torch.randn(1, T, H, device="cuda", dtype=torch.bfloat16, generator=gen) for _ in range(5)]
+    run = GraphedFlashMoE(layer, xs[0]) if graph else layer
+    with torch.no_grad():
+        want = []
+        for x in xs:
+            want.append([t.clone() for t in layer(x)])
+            torch.cuda.synchronize()
+        for _ in range(3):
+            got = [[t.clone() for t in run(x)] for x in xs]
+            for (y, logits), (y0, logits0) in zip(got, want):
+                assert torch.equal(logits, logits0) and torch.equal(y, y0)
