@@ -195,8 +195,8 @@ __device__ __forceinline__ float ord_to_f32(uint32_t u) {
 // ---- internal launchers (one per .cu) -----------------------------------------------------
 // flags: kTopkNorm - renormalise the gates per token; kTopkFromLogits - `log_probs` holds raw logits [T, 2*nk];
 // kTopkTokenRows - it holds log-probabilities [T, 2, nk]; kTopkLateWait - the rows are complete already, the kernel before
-// this one in the stream need only have ended when this one ends.
-enum { kTopkNorm = 1, kTopkFromLogits = 2, kTopkTokenRows = 4, kTopkLateWait = 8 };
+// this one in the stream need only have ended when this one ends; kTopkReleaseNext - the next kernel may start at once.
+enum { kTopkNorm = 1, kTopkFromLogits = 2, kTopkTokenRows = 4, kTopkLateWait = 8, kTopkReleaseNext = 16 };
 int launch_router_topk(const void* log_probs, int dtype, int64_t T, int nk, int k, void* scores, int64_t* indices,
                        void* gates, int flags, cudaStream_t stream);
 
@@ -245,7 +245,9 @@ int launch_gemm_add_pair(const void* a, const void* b, const float* addend, void
 // early: kEarlyWeights - the kernel before this one in the stream is one of a forward's, so the weights cannot be written
 // any more and may be requested before it has finished; kEarlyTokens - the token rows are complete too (at most the addend
 // comes from that kernel), and everything up to the epilogue runs beside it; the next kernel starts when that one has ended.
-enum { kEarlyWeights = 1, kEarlyTokens = 2 };
+// kWaitAtEnd (with kEarlyTokens) - nothing at all comes from it, this kernel only ends after it.
+enum { kEarlyWeights = 1, kEarlyTokens = 2, kWaitAtEnd = 4 };
+int narrow_swiglu_ctas(int64_t M, int I, int K);
 bool gemm_narrow_preferred(int64_t M, int N, int K, bool swiglu);
 int launch_gemm_swiglu_narrow(const void* x, const void* gate_w, const void* up_w, void* h, int dtype, int64_t M, int I,
                               int K, int early, int32_t* status, cudaStream_t stream, void* pre_gate = nullptr,

@@ -173,7 +173,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
     if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     // late: only the epilogue waits.  The first thread of a CTA that gets here lets the next kernel start, so with `late` that
     // is one of those that have waited.
-    if (!late || warp >= 2) {
+    if (!late || (warp >= 2 && !(sh.early & kWaitAtEnd))) {
       pdl_wait();
       pdl_launch_dependents();  // this CTA holds its tensor memory: once all do, the next kernel may set up
     }
@@ -361,6 +361,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, tmem_cols);
   }
+  if (sh.early & kWaitAtEnd) pdl_wait();
   if (threadIdx.x == 0 && *abort_flag != 0 && status != nullptr) atomicOr(status, FMOE_STATUS_WAIT_TIMEOUT);
 }
 
@@ -471,6 +472,12 @@ int launch_narrow(const void* w0, const void* w1, const void* x, const NarrowEpi
 }
 
 }  // namespace
+
+// CTAs of the gate/up GEMM
+int narrow_swiglu_ctas(int64_t M, int I, int K) {
+  const NarrowPlan p = plan_narrow(M, I, K, 2);
+  return p.split * ((I + p.rows - 1) / p.rows) * p.tiles_t;
+}
 
 // 16-bit operands with 16-byte aligned rows (K % 8 == 0), where the estimate is below that of the pair tiles
 bool gemm_narrow_preferred(int64_t M, int N, int K, bool swiglu) {
