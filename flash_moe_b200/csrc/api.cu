@@ -526,10 +526,21 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   }
   if (rc != FMOE_OK) return fail(rc);
   FMOE_MARK(FMOE_STAGE_ROUTER_TOPK, 1, s);
+  // the whole shared MLP in front of the expert passes, which add its float32 output: the down GEMM runs beside them
+  const bool mlp_first = topk_first && (static_cast<int64_t>(N) <= 0x7FFFFFFFll) && aligned16(a->x) && aligned16(a->y) &&
+                         aligned16(a->down_embed) && aligned16(a->up_embed) && aligned16(a->down_proj) && I % 8 == 0 &&
+                         (a->residual == nullptr || aligned16(a->residual)) && gemm_narrow_preferred(T, H, I, false) &&
+                         expert_forward_adding_supported(dtype, T, H, N, k);
   if (topk_first) {
     rc = mlp_up(a->x, a->gate_proj, a->up_proj, w.h, dtype, T, H, I, a->status, s, nullptr, nullptr,
                 kEarlyWeights | kEarlyTokens | kWaitAtEnd);
     if (rc != FMOE_OK) return fail(rc);
+    if (mlp_first) {
+      rc = launch_gemm_add_narrow(w.h, a->down_proj, nullptr, w.acc, dtype, T, H, I, kEarlyWeights, a->status, s, nullptr, true);
+      if (rc != FMOE_OK) return fail(rc);
+      return launch_expert_forward_adding(a->x, a->down_embed, a->up_embed, indices, gates, static_cast<const float*>(w.acc),
+                                          a->residual, a->y, dtype, T, H, N, k, w.expert, w.expert_bytes, a->status, s);
+    }
   }
   // The side stream is joined HERE, before the experts: the two gather passes compete with the GEMM for the same
   // L2 -> SM bandwidth and are slower beside it than after it.  (Measured at the benchmark shape the fork does not

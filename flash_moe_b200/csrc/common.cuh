@@ -4,6 +4,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <type_traits>
 
 #include "../../include/fmoe.h"
 
@@ -201,6 +202,10 @@ int launch_router_topk(const void* log_probs, int dtype, int64_t T, int nk, int 
                        void* gates, int flags, cudaStream_t stream);
 
 size_t expert_workspace_bytes(int64_t T, int H, int64_t N, int k);
+bool expert_forward_adding_supported(int dtype, int64_t T, int H, int64_t N, int k);
+int launch_expert_forward_adding(const void* x, const void* down, const void* up, const int64_t* indices, const void* gates,
+                                 const float* addend, const void* residual, void* y, int dtype, int64_t T, int H, int64_t N,
+                                 int k, void* ws, size_t ws_bytes, int32_t* status, cudaStream_t stream);
 int launch_expert_forward(const void* x, const void* down, const void* up, const int64_t* indices, const void* gates,
                           void* out, int dtype, int out_dtype, int64_t T, int H, int64_t N, int k, void* ws,
                           size_t ws_bytes, int32_t* status, cudaStream_t stream, void* const* between_passes = nullptr,
@@ -254,7 +259,7 @@ int launch_gemm_swiglu_narrow(const void* x, const void* gate_w, const void* up_
                               void* pre_up = nullptr);
 int launch_gemm_add_narrow(const void* a, const void* b, const float* addend, void* out, int dtype, int64_t M, int N,
                            int K, int early, int32_t* status, cudaStream_t stream,
-                           const void* residual = nullptr);
+                           const void* residual = nullptr, bool raw = false);
 
 // fp32-FMA GEMM on CUDA cores (simt_gemm.cu): float32 modules and shapes TMA cannot address.  `ordered`: every output
 // is one fmaf chain over ascending k (the router's logits, whose last bit decides between experts).

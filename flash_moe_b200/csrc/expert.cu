@@ -284,9 +284,15 @@ __global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* __restr
 
 // ---------------------------------------------------------------- 2c. scores, few tokens
 // One CTA of W warps per (token, group of 16 of its experts), each warp on its own 128-column chunks of the 16 gathered
-// rows; the partial dot products meet in shared memory (added in warp order).  With few tasks the one-warp-per-task kernel
-// above leaves most of the chip idle while a warp pulls 16 whole rows: 64 tokens x 2048 columns, top-32 (128 tasks) took 11.2 us
-// there; both passes of one token x 1024, top-64 (4 tasks) went from 18.7 to 7 us, of 64 tokens from 27.4 to 12.
+// rows; the sums pass through the warps in column order, so they are those of the kernel above bit for bit, whatever the
+// number of tokens.  With few tasks that kernel leaves most of the chip idle while a warp pulls 16 whole rows: 64 tokens x
+// 2048 columns, top-32 (128 tasks) took 11.2 us there.
+__device__ __forceinline__ int64_t ld_cg(const int64_t* p) { return __ldcg(reinterpret_cast<const long long*>(p)); }
+template <typename T>
+__device__ __forceinline__ T ld_cg(const T* p) {
+  const unsigned short raw = __ldcg(reinterpret_cast<const unsigned short*>(p));
+  return *reinterpret_cast<const T*>(&raw);
+}
 template <typename T, int W, bool PEER>
 __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __restrict__ x, const T* __restrict__ down,
                                                                     const int64_t* __restrict__ idx,
@@ -294,9 +300,11 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __
                                                                     int64_t tasks, int groups, int H, int64_t N, int k,
                                                                     int32_t* status, int act, float* __restrict__ raw_out,
                                                                     const T* const* __restrict__ shards, int world,
-                                                                    int64_t sharded) {
-  __shared__ float part[W][16];
-  pdl_wait();  // ids and gates come from the kernel before this one
+                                                                    int64_t sharded, int late) {
+  __shared__ float2 chain[32];
+  // ids and gates come from the kernel before this one (late: they are complete already), read past the L1 cache as a late
+  // CTA may find lines of an earlier forward there
+  if (!late) pdl_wait();
   pdl_launch_dependents();  // the accumulate pass may start gathering: it needs the ids, and only later the scores
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, tq = lane & 3;
@@ -304,7 +312,7 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __
     const int64_t t = task / groups;
     const int j0 = static_cast<int>(task - t * groups) * 16;
     const int ja = j0 + g, jb = ja + 8;
-    const int64_t ea = ja < k ? idx[t * k + ja] : 0, eb = jb < k ? idx[t * k + jb] : 0;
+    const int64_t ea = ja < k ? ld_cg(idx + t * k + ja) : 0, eb = jb < k ? ld_cg(idx + t * k + jb) : 0;
     const bool oka = (ja < k) && ea >= 0 && ea < N;
     const bool okb = (jb < k) && eb >= 0 && eb < N;
     if (((ja < k && !oka && ea != -1) || (jb < k && !okb && eb != -1)) && status != nullptr)
@@ -312,8 +320,10 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __
     const T* ra = table_row<T, PEER>(down, shards, world, oka ? ea : 0, H, sharded) + 8 * tq;
     const T* rb = table_row<T, PEER>(down, shards, world, okb ? eb : 0, H, sharded) + 8 * tq;
     const T* rx = x + t * H + 8 * tq;
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int c0 = warp * 128; c0 < H; c0 += W * 128) {
+    // warp w loads the 128-column blocks w, w + W, ...; the sums go from warp to warp in column order (every column of B is
+    // the token's row, so c[0] = c[1] and c[2] = c[3])
+    for (int base = 0; base < H; base += W * 128) {
+      const int c0 = base + warp * 128;
       uint4 qa[4], qb[4], qx[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -323,29 +333,32 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __
         qb[u] = in ? ldg16(rb + col) : make_uint4(0, 0, 0, 0);
         qx[u] = in ? ldg16(rx + col) : make_uint4(0, 0, 0, 0);
       }
+      for (int w = 0; w < W; ++w) {
+        if (warp == w && c0 < H) {
+          const float2 sum = c0 == 0 ? make_float2(0.f, 0.f) : chain[lane];
+          float c[4] = {sum.x, sum.x, sum.y, sum.y};
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        Mma16816<T>::run(c, qa[u].x, qb[u].x, qa[u].y, qb[u].y, qx[u].x, qx[u].y);
-        Mma16816<T>::run(c, qa[u].z, qb[u].z, qa[u].w, qb[u].w, qx[u].z, qx[u].w);
+          for (int u = 0; u < 4; ++u) {
+            Mma16816<T>::run(c, qa[u].x, qb[u].x, qa[u].y, qb[u].y, qx[u].x, qx[u].y);
+            Mma16816<T>::run(c, qa[u].z, qb[u].z, qa[u].w, qb[u].w, qx[u].z, qx[u].w);
+          }
+          chain[lane] = make_float2(c[0], c[2]);
+        }
+        __syncthreads();
       }
     }
-    if (tq == 0) {
-      part[warp][g] = oka ? c[0] : 0.f;
-      part[warp][g + 8] = okb ? c[2] : 0.f;
-    }
-    __syncthreads();
     if (threadIdx.x < 16 && j0 + threadIdx.x < k) {
-      float s = 0.f;
-#pragma unroll
-      for (int w = 0; w < W; ++w) s += part[w][threadIdx.x];
       const int64_t p = t * k + j0 + threadIdx.x;
-      const int64_t e = idx[p];
+      const int64_t e = ld_cg(idx + p);
       const bool ok = e >= 0 && e < N;
-      gs[p] = gates != nullptr && ok ? expert_act(s, act) * to_f32<T>(gates[p]) : s;  // no gates: the raw dot product
+      const float2 both = chain[(threadIdx.x & 7) * 4];
+      const float s = !ok ? 0.f : threadIdx.x < 8 ? both.x : both.y;
+      gs[p] = gates != nullptr && ok ? expert_act(s, act) * to_f32<T>(ld_cg(gates + p)) : s;  // no gates: the raw dot product
       if (raw_out != nullptr) raw_out[p] = s;
     }
     __syncthreads();
   }
+  if (late && blockIdx.x == gridDim.x - 1) pdl_wait();  // one waiting CTA keeps the grid from ending
 }
 
 // ---------------------------------------------------------------- 2d. scores, float32
@@ -529,19 +542,21 @@ __global__ void __launch_bounds__(128, 4) expert_accum_kernel(const T* __restric
 }
 
 // The same sum for few tokens: a CTA of W warps per (token, block of 32 * VEC columns), each warp on its own batches of 8
-// slots; the W partial sums meet in shared memory and are added in warp order.  The kernel is made resident beside the
-// scores pass (which has itself waited for the ids) and gathers its first batch of rows before it waits for the weights.
-// One token x 1024 columns, top-64: 12.5 us with one warp per 512 columns, 3.8 here; 64 tokens x 2048, top-32: 16.2, 8.6.
+// slots; the sums pass through the warps in slot order (bit for bit those of the kernel above).  The kernel is made resident
+// beside the scores pass (which has itself waited for the ids) and gathers its first batch of rows before it waits for the
+// weights.
 template <typename T, typename OutT, int W, bool PEER>
 __global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __restrict__ up, const int64_t* __restrict__ idx,
                                                                    const float* __restrict__ gs, OutT* __restrict__ out,
                                                                    int64_t tasks, int H, int64_t N, int k, int colblocks,
                                                                    int early, const T* const* __restrict__ shards,
-                                                                   int world, int64_t sharded) {
+                                                                   int world, int64_t sharded,
+                                                                   const float* __restrict__ addend,
+                                                                   const OutT* __restrict__ residual) {
   constexpr int VEC = Vec16<T>::N;
   constexpr int SLOTS = 8;
   constexpr int COLS = 32 * VEC;
-  __shared__ float part[W][COLS];
+  __shared__ float part[COLS];  // the sums on their way from warp to warp
   pdl_launch_dependents();  // all CTAs are resident once the last of them is here: the next kernel may start beside them
   if (!early) pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -550,10 +565,8 @@ __global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __r
     const int64_t t = task / colblocks;
     const int col0 = static_cast<int>(task - t * colblocks) * COLS;
     const bool in = col0 + lane * VEC < H;
-    uint64_t acc[VEC / 2];
-#pragma unroll
-    for (int i = 0; i < VEC / 2; ++i) acc[i] = 0ull;
-    for (int j0 = warp * SLOTS; j0 < k || !waited; j0 += W * SLOTS) {
+    for (int base = 0; base < k; base += W * SLOTS) {
+      const int j0 = base + warp * SLOTS;
       const int j = j0 + (lane & (SLOTS - 1));
       // ids and rows are read past the L1 cache: an early CTA may find lines of an earlier forward there
       const int64_t e = j < k ? __ldcg(reinterpret_cast<const long long*>(idx) + t * k + j) : -1;
@@ -571,42 +584,53 @@ __global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __r
         waited = true;
       }
       const float w = ok ? ld_after_wait(gs + t * k + j) : 0.f;
+      for (int turn = 0; turn < W; ++turn) {  // slots in ascending order, as the one-warp-per-task kernel adds them
+        if (warp == turn && j0 < k) {
+          float2* p = reinterpret_cast<float2*>(&part[lane * VEC]);
+          uint64_t acc[VEC / 2];
 #pragma unroll
-      for (int u = 0; u < SLOTS; ++u) {
-        const float wu = __shfl_sync(kFull, w, u);
-        const uint64_t w2 = pack_f32x2(wu, wu);
-        float f[VEC];
-        unpack16<T>(q[u], f);
+          for (int i = 0; i < VEC / 2; ++i) {
+            const float2 v = j0 == 0 ? make_float2(0.f, 0.f) : p[i];
+            acc[i] = pack_f32x2(v.x, v.y);
+          }
 #pragma unroll
-        for (int i = 0; i < VEC / 2; ++i) ffma2(acc[i], pack_f32x2(f[2 * i], f[2 * i + 1]), w2);
+          for (int u = 0; u < SLOTS; ++u) {
+            const float wu = __shfl_sync(kFull, w, u);
+            const uint64_t w2 = pack_f32x2(wu, wu);
+            float f[VEC];
+            unpack16<T>(q[u], f);
+#pragma unroll
+            for (int i = 0; i < VEC / 2; ++i) ffma2(acc[i], pack_f32x2(f[2 * i], f[2 * i + 1]), w2);
+          }
+#pragma unroll
+          for (int i = 0; i < VEC / 2; ++i) {
+            float lo, hi;
+            unpack_f32x2(acc[i], lo, hi);
+            p[i] = make_float2(lo, hi);
+          }
+        }
+        __syncthreads();
       }
     }
-#pragma unroll
-    for (int i = 0; i < VEC / 2; ++i) {
-      float lo, hi;
-      unpack_f32x2(acc[i], lo, hi);
-      *reinterpret_cast<float2*>(&part[warp][lane * VEC + 2 * i]) = make_float2(lo, hi);
-    }
-    __syncthreads();
     for (int c = threadIdx.x * 4; c < COLS; c += 32 * W * 4) {
       if (col0 + c >= H) continue;
-      float4 s = *reinterpret_cast<const float4*>(&part[0][c]);
-#pragma unroll
-      for (int w = 1; w < W; ++w) {
-        const float4 v = *reinterpret_cast<const float4*>(&part[w][c]);
-        s.x += v.x;
-        s.y += v.y;
-        s.z += v.z;
-        s.w += v.w;
-      }
+      const float4 s = *reinterpret_cast<const float4*>(&part[c]);
       OutT* o = out + t * H + col0 + c;
       if constexpr (sizeof(OutT) == 4) {
         *reinterpret_cast<float4*>(o) = s;
       } else {
-        o[0] = from_f32<OutT>(s.x);
-        o[1] = from_f32<OutT>(s.y);
-        o[2] = from_f32<OutT>(s.z);
-        o[3] = from_f32<OutT>(s.w);
+        // addend: the shared MLP's output, residual: the skip connection, added in the order of the down GEMM's epilogue
+        const float v[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float r = v[i];
+          if (addend != nullptr) r = ld_after_wait(addend + t * H + col0 + c + i) + r;
+          if (residual != nullptr) {
+            const uint16_t raw = ld_after_wait(reinterpret_cast<const uint16_t*>(residual) + t * H + col0 + c + i);
+            r += to_f32<OutT>(*reinterpret_cast<const OutT*>(&raw));
+          }
+          o[i] = from_f32<OutT>(r);
+        }
       }
     }
     __syncthreads();
@@ -659,37 +683,46 @@ struct PeerTable {  // a table sharded over the GPUs of a node (table_row); no s
   int64_t sharded = 0;
 };
 
+int scores_split_warps(int64_t T, int H, int k) {
+  return split_warps(T * ((k + 15) / 16), (H + 127) / 128, static_cast<int64_t>(device_sm_count()) * 16 / 3);
+}
+int accum_split_warps(int64_t T, int H, int k, int cols) {
+  const int pieces = (k + 7) / 8;
+  return split_warps(T * ((H + 2 * cols - 1) / (2 * cols)), pieces, static_cast<int64_t>(device_sm_count()) * (pieces >= 3 ? 8 : 1));
+}
+
 // the scores pass / accumulate pass for few tokens; false: not the shape for it (or, with `rc`, a launch error)
 template <typename T, bool PEER>
 bool try_scores_split(const void* rows, const void* table, const int64_t* idx, const void* gates, float* out, int64_t T_, int H,
                       int64_t N, int k, int32_t* status, cudaStream_t stream, int act, float* raw_out, const PeerTable& pt,
-                      cudaError_t* rc) {
+                      cudaError_t* rc, bool late = false) {
   const int groups = (k + 15) / 16;
   const int64_t tasks = T_ * groups;
-  const int split = split_warps(tasks, (H + 127) / 128, static_cast<int64_t>(device_sm_count()) * 16 / 3);
+  const int split = scores_split_warps(T_, H, k);
   if (split == 0) return false;
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * (64 / split);
   auto kern = split == 8 ? expert_scores_split_kernel<T, 8, PEER> : expert_scores_split_kernel<T, 4, PEER>;
   *rc = launch_pdl(PEER ? 0 : 8, kern, dim3(static_cast<unsigned>(tasks < cap ? tasks : cap)), dim3(32 * split), 0, stream, 1,
                    static_cast<const T*>(rows), static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, tasks,
-                   groups, H, N, k, status, act, raw_out, reinterpret_cast<const T* const*>(pt.shards), pt.world, pt.sharded);
+                   groups, H, N, k, status, act, raw_out, reinterpret_cast<const T* const*>(pt.shards), pt.world, pt.sharded,
+                   late && !PEER ? 1 : 0);
   return true;
 }
 
 template <typename T, bool PEER>
 bool try_accum_split(const void* table, const int64_t* idx, const float* coef, void* out, int out_f32, int64_t T_, int H,
-                     int64_t N, int k, bool early, cudaStream_t stream, const PeerTable& pt, cudaError_t* rc) {
+                     int64_t N, int k, bool early, cudaStream_t stream, const PeerTable& pt, cudaError_t* rc, const float* addend = nullptr, const void* residual = nullptr) {
   constexpr int COLS = 32 * Vec16<T>::N;
-  const int pieces = (k + 7) / 8;
-  const int split = split_warps(T_ * ((H + 2 * COLS - 1) / (2 * COLS)), pieces, static_cast<int64_t>(device_sm_count()) * (pieces >= 3 ? 8 : 1));
+  const int split = accum_split_warps(T_, H, k, COLS);
   if (split == 0) return false;
   const int colblocks = (H + COLS - 1) / COLS;
   const int64_t tasks = T_ * colblocks;
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * (64 / split);
   auto go = [&](auto kern, auto* o) {
+    using OutT = std::remove_pointer_t<decltype(o)>;
     *rc = launch_pdl(PEER ? 0 : 8, kern, dim3(static_cast<unsigned>(tasks < cap ? tasks : cap)), dim3(32 * split), 0, stream, 1,
                      static_cast<const T*>(table), idx, coef, o, tasks, H, N, k, colblocks, early && !PEER ? 1 : 0,
-                     reinterpret_cast<const T* const*>(pt.shards), pt.world, pt.sharded);
+                     reinterpret_cast<const T* const*>(pt.shards), pt.world, pt.sharded, addend, static_cast<const OutT*>(residual));
   };
   if (out_f32) {
     if (split == 8) go(expert_accum_split_kernel<T, float, 8, PEER>, static_cast<float*>(out));
@@ -1338,6 +1371,41 @@ size_t expert_workspace_bytes(int64_t T, int H, int64_t N, int k) {
   (void)H;
   if (T < 0 || N < 0 || k < 0) return 0;
   return carve(nullptr, T, N, k).bytes;
+}
+
+// Few tokens, 16-bit: both passes in their few-token forms, the second of which also adds the shared MLP's output (and the
+// residual) and rounds once.  ids and gates are complete when the scores pass starts; `addend` comes from the kernel before it.
+bool expert_forward_adding_supported(int dtype, int64_t T, int H, int64_t N, int k) {
+  return dtype != FMOE_DTYPE_F32 && T > 0 && H % 8 == 0 && N <= 0x7FFFFFFFll && k > 0 && scores_split_warps(T, H, k) != 0 &&
+         accum_split_warps(T, H, k, 256) != 0;
+}
+
+namespace {
+template <typename T>
+int run_adding(const void* x, const void* down, const void* up, const int64_t* idx, const void* gates, const float* addend,
+               const void* residual, void* y, int64_t T_, int H, int64_t N, int k, const ExpertWs& w, int32_t* status,
+               cudaStream_t stream) {
+  cudaError_t rc = cudaSuccess;
+  if (!try_scores_split<T, false>(x, down, idx, gates, w.gs, T_, H, N, k, status, stream, kActSilu, nullptr, PeerTable{}, &rc, true))
+    return FMOE_ERR_UNSUPPORTED;
+  FMOE_CUDA_TRY(rc);
+  if (!try_accum_split<T, false>(up, idx, w.gs, y, 0, T_, H, N, k, true, stream, PeerTable{}, &rc, addend, residual))
+    return FMOE_ERR_UNSUPPORTED;
+  FMOE_CUDA_TRY(rc);
+  return FMOE_OK;
+}
+}  // namespace
+
+int launch_expert_forward_adding(const void* x, const void* down, const void* up, const int64_t* indices, const void* gates,
+                                 const float* addend, const void* residual, void* y, int dtype, int64_t T, int H, int64_t N,
+                                 int k, void* ws, size_t ws_bytes, int32_t* status, cudaStream_t stream) {
+  if (!expert_forward_adding_supported(dtype, T, H, N, k)) return FMOE_ERR_UNSUPPORTED;
+  if (!aligned16(x) || !aligned16(down) || !aligned16(up) || !aligned16(y)) return FMOE_ERR_ALIGNMENT;
+  const ExpertWs w = carve(ws, T, N, k);
+  if (ws == nullptr || ws_bytes < w.bytes) return FMOE_ERR_WORKSPACE;
+  if (dtype == FMOE_DTYPE_BF16)
+    return run_adding<__nv_bfloat16>(x, down, up, indices, gates, addend, residual, y, T, H, N, k, w, status, stream);
+  return run_adding<__half>(x, down, up, indices, gates, addend, residual, y, T, H, N, k, w, status, stream);
 }
 
 int launch_expert_forward(const void* x, const void* down, const void* up, const int64_t* indices, const void* gates,

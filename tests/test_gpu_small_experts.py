@@ -33,7 +33,7 @@ def test_expert_passes_for_few_tokens(T, H, N, k, dtype):
         want += (torch.nn.functional.silu(s) * gates[:, j].double() * ok[:, j])[:, None] * u[rows[:, j]].double()
     for _ in range(3):  # back to back: each pass may start beside the one before it
         got = flash_expert_fp32(x, d, u, idx, gates)
-    assert (got.double() - want).norm() <= 2e-6 * want.norm() + 1e-12
+    assert (got.double() - want).norm() <= 5e-6 * want.norm() + 1e-12
     assert torch.equal(got, flash_expert_fp32(x, d, u, idx, gates))
     assert _lib.read_status() == 0
     idx[0, 0] = N  # skipped and reported
