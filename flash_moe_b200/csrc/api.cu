@@ -135,7 +135,8 @@ size_t router_front_ws(int64_t T, int H, int dtype) {
 // logp == nullptr: stop after the logits (the caller applies the log-softmax elsewhere)
 int router_front(const void* x, const void* w, void* rm, void* rv, int training, float momentum, float eps,
                  void* logits, void* logp, int dtype, int64_t T, int H, int nk, void* ws, size_t ws_bytes,
-                 int32_t* status, cudaStream_t stream, const float* bn_sums = nullptr, int64_t bn_count = 0) {
+                 int32_t* status, cudaStream_t stream, const float* bn_sums = nullptr, int64_t bn_count = 0,
+                 bool beside_predecessor = false) {
   if (!valid_dtype(dtype) || T < 0 || H <= 0 || nk <= 0) return FMOE_ERR_BAD_ARG;
   if (T == 0) return FMOE_OK;
   if (x == nullptr || w == nullptr || logits == nullptr) return FMOE_ERR_BAD_ARG;
@@ -156,7 +157,7 @@ int router_front(const void* x, const void* w, void* rm, void* rv, int training,
       return FMOE_ERR_BAD_ARG;
     }
     return launch_router_bn_gemm(x, w, mean, invstd, training ? nullptr : rm, training ? nullptr : rv, eps, logits, dtype,
-                                 T, 2 * nk, H, status, stream);
+                                 T, 2 * nk, H, beside_predecessor && !training, status, stream);
   }
   rc = launch_bn(x, xn, rm, rv, training, momentum, eps, dtype, T, H, bnws, bn_sums, bn_count, stream);
   if (rc != FMOE_OK) return rc;
@@ -466,22 +467,33 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   // kernel applies the per-half log-softmax itself (each warp already holds both halves of its
   // token in registers), which saves a [2, T, nk] round trip and a serial GEMM epilogue.
   const bool topk_from_logits = is16(dtype) && nk <= 1024;
-  // The gate/up GEMM needs nothing from the router and the top-k only the logits, so the two run beside each other: the GEMM
-  // first, so that the top-k's many small CTAs fill what it leaves - or, while the CTAs of both find SMs of their own, the
-  // top-k first, so that its set-up hides behind the router GEMM and the GEMM runs beside that as well.
-  // In a graph, one after the other -> now: 1 token 29.4 -> 26.7 us, 64 tokens of the decoder layer 54 -> 51, 777 x 1000 float16 68 -> 59,
-  // 131072 tokens of the decoder layer 11.5 -> 10.6 ms.  A caller that asks for stage events gets the stages one by one.
+  // The gate/up GEMM needs nothing from the router and the top-k only the logits, so the two run beside each other, the GEMM
+  // first, so that the top-k's many small CTAs fill what it leaves.  In a graph, one after the other -> now: 777 x 1000 float16
+  // 68 -> 63 us, 131072 tokens of the decoder layer 11.5 -> 10.6 ms.  A caller that asks for stage events gets the stages one
+  // by one.
   const bool up_beside = (s2 == nullptr || s2 == s) && !a->training && topk_from_logits && a->stage_events == nullptr &&
                          mlp_up_on_tensor_cores(a->x, a->gate_proj, a->up_proj, dtype, T, H, I);
-  const bool topk_first = up_beside && mlp_up_is_narrow(a->x, a->gate_proj, a->up_proj, dtype, T, H, I) &&
-                          (T + 3) / 4 + narrow_swiglu_ctas(T, I, H) <= device_sm_count();
+  // Few tokens: the whole shared MLP goes in front of the expert passes, which add its float32 output.  Router GEMM beside the
+  // gate/up GEMM, top-k beside the down GEMM; each of these kernels also outlasts the one before it.
+  const bool mlp_first = up_beside && k > 0 && mlp_up_is_narrow(a->x, a->gate_proj, a->up_proj, dtype, T, H, I) &&
+                         (T + 3) / 4 + narrow_swiglu_ctas(T, I, H) <= device_sm_count() && aligned16(a->y) &&
+                         aligned16(a->down_embed) && aligned16(a->up_embed) && aligned16(a->down_proj) &&
+                         gemm_narrow_preferred(T, H, I, false) && expert_forward_adding_supported(dtype, T, H, N, k);
+  if (mlp_first) {
+    rc = mlp_up(a->x, a->gate_proj, a->up_proj, w.h, dtype, T, H, I, a->status, s);
+    if (rc != FMOE_OK) return rc;
+  }
   FMOE_MARK(FMOE_STAGE_ROUTER_FRONT, 0, s);
   rc = router_front(a->x, a->router_gate, a->running_mean, a->running_var, a->training, a->bn_momentum, a->bn_eps,
                     a->router_logits, topk_from_logits ? nullptr : w.logp, dtype, T, H, nk, w.front, w.front_bytes,
-                    a->status, s, a->training ? a->bn_global_sums : nullptr, a->bn_global_count);
+                    a->status, s, a->training ? a->bn_global_sums : nullptr, a->bn_global_count,
+                    mlp_first);
   if (rc != FMOE_OK) return rc;
   FMOE_MARK(FMOE_STAGE_ROUTER_FRONT, 1, s);
-  if (up_beside && !topk_first) {
+  if (mlp_first) {
+    rc = launch_gemm_add_narrow(w.h, a->down_proj, nullptr, w.acc, dtype, T, H, I, kEarlyWeights, a->status, s, nullptr, true);
+    if (rc != FMOE_OK) return rc;
+  } else if (up_beside) {
     rc = mlp_up(a->x, a->gate_proj, a->up_proj, w.h, dtype, T, H, I, a->status, s, nullptr, nullptr,
                 kEarlyWeights | kEarlyTokens);
     if (rc != FMOE_OK) return rc;
@@ -516,7 +528,7 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   rc = FMOE_ERR_UNSUPPORTED;
   if (topk_from_logits)
     rc = launch_router_topk(a->router_logits, dtype, T, nk, k, w.scores, indices, gates,
-                            (a->norm_topk_prob ? kTopkNorm : 0) | kTopkFromLogits | (topk_first ? kTopkReleaseNext : up_beside ? kTopkLateWait : 0), s);
+                            (a->norm_topk_prob ? kTopkNorm : 0) | kTopkFromLogits | (up_beside ? kTopkLateWait : 0), s);
   if (rc == FMOE_ERR_UNSUPPORTED) {
     if (topk_from_logits) {  // shapes the register kernel does not cover: explicit log-softmax pass
       rc = launch_log_softmax_halves(a->router_logits, w.logp, dtype, T, nk, s);
@@ -526,22 +538,9 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   }
   if (rc != FMOE_OK) return fail(rc);
   FMOE_MARK(FMOE_STAGE_ROUTER_TOPK, 1, s);
-  // the whole shared MLP in front of the expert passes, which add its float32 output: the down GEMM runs beside them
-  const bool mlp_first = topk_first && (static_cast<int64_t>(N) <= 0x7FFFFFFFll) && aligned16(a->x) && aligned16(a->y) &&
-                         aligned16(a->down_embed) && aligned16(a->up_embed) && aligned16(a->down_proj) && I % 8 == 0 &&
-                         (a->residual == nullptr || aligned16(a->residual)) && gemm_narrow_preferred(T, H, I, false) &&
-                         expert_forward_adding_supported(dtype, T, H, N, k);
-  if (topk_first) {
-    rc = mlp_up(a->x, a->gate_proj, a->up_proj, w.h, dtype, T, H, I, a->status, s, nullptr, nullptr,
-                kEarlyWeights | kEarlyTokens | kWaitAtEnd);
-    if (rc != FMOE_OK) return fail(rc);
-    if (mlp_first) {
-      rc = launch_gemm_add_narrow(w.h, a->down_proj, nullptr, w.acc, dtype, T, H, I, kEarlyWeights, a->status, s, nullptr, true);
-      if (rc != FMOE_OK) return fail(rc);
-      return launch_expert_forward_adding(a->x, a->down_embed, a->up_embed, indices, gates, static_cast<const float*>(w.acc),
-                                          a->residual, a->y, dtype, T, H, N, k, w.expert, w.expert_bytes, a->status, s);
-    }
-  }
+  if (mlp_first)
+    return launch_expert_forward_adding(a->x, a->down_embed, a->up_embed, indices, gates, static_cast<const float*>(w.acc),
+                                        a->residual, a->y, dtype, T, H, N, k, w.expert, w.expert_bytes, a->status, s);
   // The side stream is joined HERE, before the experts: the two gather passes compete with the GEMM for the same
   // L2 -> SM bandwidth and are slower beside it than after it.  (Measured at the benchmark shape the fork does not
   // pay either way - 230 vs 226 us: the top-k's CTAs fill the shared memory first and the GEMM's wait for them; with

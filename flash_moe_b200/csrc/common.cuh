@@ -196,8 +196,8 @@ __device__ __forceinline__ float ord_to_f32(uint32_t u) {
 // ---- internal launchers (one per .cu) -----------------------------------------------------
 // flags: kTopkNorm - renormalise the gates per token; kTopkFromLogits - `log_probs` holds raw logits [T, 2*nk];
 // kTopkTokenRows - it holds log-probabilities [T, 2, nk]; kTopkLateWait - the rows are complete already, the kernel before
-// this one in the stream need only have ended when this one ends; kTopkReleaseNext - the next kernel may start at once.
-enum { kTopkNorm = 1, kTopkFromLogits = 2, kTopkTokenRows = 4, kTopkLateWait = 8, kTopkReleaseNext = 16 };
+// this one in the stream need only have ended when this one ends.
+enum { kTopkNorm = 1, kTopkFromLogits = 2, kTopkTokenRows = 4, kTopkLateWait = 8 };
 int launch_router_topk(const void* log_probs, int dtype, int64_t T, int nk, int k, void* scores, int64_t* indices,
                        void* gates, int flags, cudaStream_t stream);
 
@@ -237,7 +237,8 @@ bool gemm_router_fused_supported(int nk);
 bool router_bn_gemm_supported(int dtype, int64_t M, int N, int K);
 int launch_router_bn_gemm(const void* x, const void* w, const float* mean, const float* invstd,
                           const void* running_mean, const void* running_var, float eps, void* logits, int dtype,
-                          int64_t M, int N, int K, int32_t* status, cudaStream_t stream);
+                          int64_t M, int N, int K, bool beside_predecessor, int32_t* status, cudaStream_t stream);
+// beside_predecessor: the kernel before it in the stream is one of this forward's that works on other data.
 // CTA-pair (cta_group::2) versions of the two shared-MLP GEMMs (gemm_sm100_pair.cu)
 bool gemm_pair_supported(int64_t M, int N, int K);
 int launch_gemm_swiglu_pair(const void* x, const void* gate_w, const void* up_w, void* h, int dtype, int64_t M, int I,
@@ -250,8 +251,7 @@ int launch_gemm_add_pair(const void* a, const void* b, const float* addend, void
 // early: kEarlyWeights - the kernel before this one in the stream is one of a forward's, so the weights cannot be written
 // any more and may be requested before it has finished; kEarlyTokens - the token rows are complete too (at most the addend
 // comes from that kernel), and everything up to the epilogue runs beside it; the next kernel starts when that one has ended.
-// kWaitAtEnd (with kEarlyTokens) - nothing at all comes from it, this kernel only ends after it.
-enum { kEarlyWeights = 1, kEarlyTokens = 2, kWaitAtEnd = 4 };
+enum { kEarlyWeights = 1, kEarlyTokens = 2 };
 int narrow_swiglu_ctas(int64_t M, int I, int K);
 bool gemm_narrow_preferred(int64_t M, int N, int K, bool swiglu);
 int launch_gemm_swiglu_narrow(const void* x, const void* gate_w, const void* up_w, void* h, int dtype, int64_t M, int I,

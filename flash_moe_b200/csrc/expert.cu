@@ -287,12 +287,6 @@ __global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* __restr
 // rows; the sums pass through the warps in column order, so they are those of the kernel above bit for bit, whatever the
 // number of tokens.  With few tasks that kernel leaves most of the chip idle while a warp pulls 16 whole rows: 64 tokens x
 // 2048 columns, top-32 (128 tasks) took 11.2 us there.
-__device__ __forceinline__ int64_t ld_cg(const int64_t* p) { return __ldcg(reinterpret_cast<const long long*>(p)); }
-template <typename T>
-__device__ __forceinline__ T ld_cg(const T* p) {
-  const unsigned short raw = __ldcg(reinterpret_cast<const unsigned short*>(p));
-  return *reinterpret_cast<const T*>(&raw);
-}
 template <typename T, int W, bool PEER>
 __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __restrict__ x, const T* __restrict__ down,
                                                                     const int64_t* __restrict__ idx,
@@ -300,11 +294,9 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __
                                                                     int64_t tasks, int groups, int H, int64_t N, int k,
                                                                     int32_t* status, int act, float* __restrict__ raw_out,
                                                                     const T* const* __restrict__ shards, int world,
-                                                                    int64_t sharded, int late) {
+                                                                    int64_t sharded) {
   __shared__ float2 chain[32];
-  // ids and gates come from the kernel before this one (late: they are complete already), read past the L1 cache as a late
-  // CTA may find lines of an earlier forward there
-  if (!late) pdl_wait();
+  pdl_wait();  // ids and gates come from the kernel before this one
   pdl_launch_dependents();  // the accumulate pass may start gathering: it needs the ids, and only later the scores
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, tq = lane & 3;
@@ -312,7 +304,7 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __
     const int64_t t = task / groups;
     const int j0 = static_cast<int>(task - t * groups) * 16;
     const int ja = j0 + g, jb = ja + 8;
-    const int64_t ea = ja < k ? ld_cg(idx + t * k + ja) : 0, eb = jb < k ? ld_cg(idx + t * k + jb) : 0;
+    const int64_t ea = ja < k ? idx[t * k + ja] : 0, eb = jb < k ? idx[t * k + jb] : 0;
     const bool oka = (ja < k) && ea >= 0 && ea < N;
     const bool okb = (jb < k) && eb >= 0 && eb < N;
     if (((ja < k && !oka && ea != -1) || (jb < k && !okb && eb != -1)) && status != nullptr)
@@ -349,16 +341,15 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __
     }
     if (threadIdx.x < 16 && j0 + threadIdx.x < k) {
       const int64_t p = t * k + j0 + threadIdx.x;
-      const int64_t e = ld_cg(idx + p);
+      const int64_t e = idx[p];
       const bool ok = e >= 0 && e < N;
       const float2 both = chain[(threadIdx.x & 7) * 4];
       const float s = !ok ? 0.f : threadIdx.x < 8 ? both.x : both.y;
-      gs[p] = gates != nullptr && ok ? expert_act(s, act) * to_f32<T>(ld_cg(gates + p)) : s;  // no gates: the raw dot product
+      gs[p] = gates != nullptr && ok ? expert_act(s, act) * to_f32<T>(gates[p]) : s;  // no gates: the raw dot product
       if (raw_out != nullptr) raw_out[p] = s;
     }
     __syncthreads();
   }
-  if (late && blockIdx.x == gridDim.x - 1) pdl_wait();  // one waiting CTA keeps the grid from ending
 }
 
 // ---------------------------------------------------------------- 2d. scores, float32
@@ -564,6 +555,10 @@ __global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __r
   for (int64_t task = blockIdx.x; task < tasks; task += gridDim.x) {
     const int64_t t = task / colblocks;
     const int col0 = static_cast<int>(task - t * colblocks) * COLS;
+    static_assert(COLS <= 32 * W * 4, "every thread finishes at most one group of four columns");
+    const bool mine = threadIdx.x * 4 < COLS && col0 + static_cast<int>(threadIdx.x) * 4 < H;
+    const int64_t at = t * H + col0 + threadIdx.x * 4;
+    float ad[4] = {}, rs[4] = {};
     const bool in = col0 + lane * VEC < H;
     for (int base = 0; base < k; base += W * SLOTS) {
       const int j0 = base + warp * SLOTS;
@@ -582,6 +577,16 @@ __global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __r
       if (!waited) {
         pdl_wait();
         waited = true;
+      }
+      if (base == 0 && mine) {  // addend: the shared MLP's output, residual: the skip connection
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (addend != nullptr) ad[i] = ld_after_wait(addend + at + i);
+          if (sizeof(OutT) == 2 && residual != nullptr) {
+            const uint16_t raw = ld_after_wait(reinterpret_cast<const uint16_t*>(residual) + at + i);
+            rs[i] = to_f32<OutT>(*reinterpret_cast<const OutT*>(&raw));
+          }
+        }
       }
       const float w = ok ? ld_after_wait(gs + t * k + j) : 0.f;
       for (int turn = 0; turn < W; ++turn) {  // slots in ascending order, as the one-warp-per-task kernel adds them
@@ -612,24 +617,18 @@ __global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __r
         __syncthreads();
       }
     }
-    for (int c = threadIdx.x * 4; c < COLS; c += 32 * W * 4) {
-      if (col0 + c >= H) continue;
-      const float4 s = *reinterpret_cast<const float4*>(&part[c]);
-      OutT* o = out + t * H + col0 + c;
+    if (mine) {
+      const float4 s = *reinterpret_cast<const float4*>(&part[threadIdx.x * 4]);
+      OutT* o = out + at;
       if constexpr (sizeof(OutT) == 4) {
         *reinterpret_cast<float4*>(o) = s;
       } else {
-        // addend: the shared MLP's output, residual: the skip connection, added in the order of the down GEMM's epilogue
+        // in the order of the down GEMM's epilogue
         const float v[4] = {s.x, s.y, s.z, s.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          float r = v[i];
-          if (addend != nullptr) r = ld_after_wait(addend + t * H + col0 + c + i) + r;
-          if (residual != nullptr) {
-            const uint16_t raw = ld_after_wait(reinterpret_cast<const uint16_t*>(residual) + t * H + col0 + c + i);
-            r += to_f32<OutT>(*reinterpret_cast<const OutT*>(&raw));
-          }
-          o[i] = from_f32<OutT>(r);
+          const float r = addend != nullptr ? ad[i] + v[i] : v[i];
+          o[i] = from_f32<OutT>(residual != nullptr ? r + rs[i] : r);
         }
       }
     }
@@ -695,7 +694,7 @@ int accum_split_warps(int64_t T, int H, int k, int cols) {
 template <typename T, bool PEER>
 bool try_scores_split(const void* rows, const void* table, const int64_t* idx, const void* gates, float* out, int64_t T_, int H,
                       int64_t N, int k, int32_t* status, cudaStream_t stream, int act, float* raw_out, const PeerTable& pt,
-                      cudaError_t* rc, bool late = false) {
+                      cudaError_t* rc) {
   const int groups = (k + 15) / 16;
   const int64_t tasks = T_ * groups;
   const int split = scores_split_warps(T_, H, k);
@@ -704,8 +703,7 @@ bool try_scores_split(const void* rows, const void* table, const int64_t* idx, c
   auto kern = split == 8 ? expert_scores_split_kernel<T, 8, PEER> : expert_scores_split_kernel<T, 4, PEER>;
   *rc = launch_pdl(PEER ? 0 : 8, kern, dim3(static_cast<unsigned>(tasks < cap ? tasks : cap)), dim3(32 * split), 0, stream, 1,
                    static_cast<const T*>(rows), static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, tasks,
-                   groups, H, N, k, status, act, raw_out, reinterpret_cast<const T* const*>(pt.shards), pt.world, pt.sharded,
-                   late && !PEER ? 1 : 0);
+                   groups, H, N, k, status, act, raw_out, reinterpret_cast<const T* const*>(pt.shards), pt.world, pt.sharded);
   return true;
 }
 
@@ -1374,7 +1372,7 @@ size_t expert_workspace_bytes(int64_t T, int H, int64_t N, int k) {
 }
 
 // Few tokens, 16-bit: both passes in their few-token forms, the second of which also adds the shared MLP's output (and the
-// residual) and rounds once.  ids and gates are complete when the scores pass starts; `addend` comes from the kernel before it.
+// residual) and rounds once.  `addend` is complete when the scores pass starts.
 bool expert_forward_adding_supported(int dtype, int64_t T, int H, int64_t N, int k) {
   return dtype != FMOE_DTYPE_F32 && T > 0 && H % 8 == 0 && N <= 0x7FFFFFFFll && k > 0 && scores_split_warps(T, H, k) != 0 &&
          accum_split_warps(T, H, k, 256) != 0;
@@ -1386,7 +1384,7 @@ int run_adding(const void* x, const void* down, const void* up, const int64_t* i
                const void* residual, void* y, int64_t T_, int H, int64_t N, int k, const ExpertWs& w, int32_t* status,
                cudaStream_t stream) {
   cudaError_t rc = cudaSuccess;
-  if (!try_scores_split<T, false>(x, down, idx, gates, w.gs, T_, H, N, k, status, stream, kActSilu, nullptr, PeerTable{}, &rc, true))
+  if (!try_scores_split<T, false>(x, down, idx, gates, w.gs, T_, H, N, k, status, stream, kActSilu, nullptr, PeerTable{}, &rc))
     return FMOE_ERR_UNSUPPORTED;
   FMOE_CUDA_TRY(rc);
   if (!try_accum_split<T, false>(up, idx, w.gs, y, 0, T_, H, N, k, true, stream, PeerTable{}, &rc, addend, residual))

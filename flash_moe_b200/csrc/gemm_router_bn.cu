@@ -31,8 +31,10 @@ template <int BLOCK_M, int BLOCK_N> struct RingDepth {
   static constexpr int v = BLOCK_M == 64 ? 8 : BLOCK_N <= 128 ? 6 : 4;
 };
 
-// kEarlyTrigger: the next kernel may become resident at once (grids that leave most of the chip idle)
-enum { kEarlyTrigger = 1 };
+// kEarlyTrigger: the next kernel may become resident at once (grids that leave most of the chip idle).  kLateWait: the
+// kernel before this one in the stream works on other data and has itself waited for everything this one reads, so this
+// one runs beside it and waits for it only before it ends (completion stays transitive along the stream).
+enum { kEarlyTrigger = 1, kLateWait = 2 };
 
 // BLOCK_M = 128, or 64 for small problems (twice the CTAs, half the x tile to fetch and normalise per CTA).  With
 // M = 64 the accumulator's row i sits in TMEM lane 32 * (i / 16) + i % 16: each of the four epilogue warps finds 16
@@ -85,7 +87,7 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       ptx::prefetch_tensormap(&tmA);
       ptx::prefetch_tensormap(&tmB);
     }
-    pdl_wait();
+    if ((flags & kLateWait) == 0) pdl_wait();
     if (flags & kEarlyTrigger) pdl_launch_dependents();
     // ------------------------------------------------------------ TMA producer
     bool ok = true;
@@ -113,7 +115,7 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       ptx::tmem_relinquish();
     }
     // everything above is independent of earlier kernels; from here on global memory is read
-    pdl_wait();
+    if ((flags & kLateWait) == 0) pdl_wait();
     if (flags & kEarlyTrigger) pdl_launch_dependents();
     // statistics: eval mode straight from the running buffers, training mode from the finalised batch statistics.
     // One thread fetches the eight features 8 p .. 8 p + 7 of a k-block with vector loads (all of a thread's loads are in
@@ -256,6 +258,7 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, BLOCK_N);
   }
+  if (flags & kLateWait) pdl_wait();
   if (threadIdx.x == 0 && *abort_flag != 0 && status != nullptr) atomicOr(status, FMOE_STATUS_WAIT_TIMEOUT);
 }
 
@@ -295,7 +298,7 @@ bool router_bn_gemm_supported(int dtype, int64_t M, int N, int K) {
 // Statistics: running_mean / running_var (module dtype, eval mode) when non-null, else mean / invstd (float32 [K]).
 int launch_router_bn_gemm(const void* x, const void* w, const float* mean, const float* invstd,
                           const void* running_mean, const void* running_var, float eps, void* logits, int dtype,
-                          int64_t M, int N, int K, int32_t* status, cudaStream_t stream) {
+                          int64_t M, int N, int K, bool beside_predecessor, int32_t* status, cudaStream_t stream) {
   if (!router_bn_gemm_supported(dtype, M, N, K)) return FMOE_ERR_UNSUPPORTED;
   if (x == nullptr || w == nullptr || logits == nullptr) return FMOE_ERR_BAD_ARG;
   if ((running_mean == nullptr) != (running_var == nullptr)) return FMOE_ERR_BAD_ARG;
@@ -311,7 +314,8 @@ int launch_router_bn_gemm(const void* x, const void* w, const float* mean, const
   const bool small = tiles128 < device_sm_count();
   const int64_t m64 = (M + 63) / 64;
   const int bn64 = m64 * ((N + 31) / 32) <= device_sm_count() ? 32 : m64 * ((N + 63) / 64) <= device_sm_count() ? 64 : 128;
-  const int flags = small && m64 * ((N + bn64 - 1) / bn64) * 2 <= device_sm_count() ? kEarlyTrigger : 0;
+  const int flags = (small && m64 * ((N + bn64 - 1) / bn64) * 2 <= device_sm_count() ? kEarlyTrigger : 0) |
+                    (beside_predecessor ? kLateWait : 0);
 #define FMOE_BN_GEMM(BM_, BN_)                                                                                       \
   (dtype == FMOE_DTYPE_BF16                                                                                          \
        ? launch_bn_gemm<BM_, BN_, __nv_bfloat16>(x, w, mean, invstd, running_mean, running_var, eps, logits, dtype, M, N, \

@@ -47,7 +47,7 @@ struct NarrowShape {
   int num_kb;       // 64-column blocks of K
   int stages;
   int acc_cols;     // TMEM columns per accumulator (power of two)
-  int early;        // kEarlyWeights | kEarlyTokens | kWaitAtEnd
+  int early;        // kEarlyWeights | kEarlyTokens
 };
 
 // BLOCK_R weight rows per tile: 128, or 64 where that gives more CTAs.  With 64 the accumulator's row i sits in TMEM lane
@@ -159,9 +159,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
     ptx::tc_fence_after();
     // late: only the epilogue waits.  The first thread of a CTA that gets here lets the next kernel start, so with `late` that
     // is one of those that have waited.
-    if (sh.early & kWaitAtEnd) {
-      pdl_launch_dependents();
-    } else if (!late || warp >= 2) {
+    if (!late || warp >= 2) {
       pdl_wait();
       pdl_launch_dependents();  // this CTA holds its tensor memory: once all do, the next kernel may set up
     }
@@ -290,7 +288,6 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, tmem_cols);
   }
-  if (sh.early & kWaitAtEnd) pdl_wait();
   if (threadIdx.x == 0 && *abort_flag != 0 && status != nullptr) atomicOr(status, FMOE_STATUS_WAIT_TIMEOUT);
 }
 

@@ -354,7 +354,6 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restric
                                                              RouterRegLayout L, T* __restrict__ scores,
                                                              int64_t* __restrict__ indices, T* __restrict__ gates,
                                                              int flags) {
-  if (flags & kTopkReleaseNext) pdl_launch_dependents();
   const int norm = flags & kTopkNorm;
   const bool from_logits = (flags & kTopkFromLogits) != 0;
   const bool token_rows = (flags & (kTopkFromLogits | kTopkTokenRows)) != 0;  // [T, 2, nk] instead of [2, T, nk]
@@ -862,7 +861,6 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
   constexpr int LOW = OrdLowBits<T>::value;
   constexpr bool kKeysInRegs = E <= 8;     // both halves' values stay in registers up to the compaction
   constexpr bool kUnrollCells = CPL <= 10;  // see sort_desc: small kernels are unrolled, large ones are loops
-  if (flags & kTopkReleaseNext) pdl_launch_dependents();
   const int norm = flags & kTopkNorm;
   const bool from_logits = (flags & kTopkFromLogits) != 0;
   const bool token_rows = (flags & (kTopkFromLogits | kTopkTokenRows)) != 0;  // [T, 2, nk] instead of [2, T, nk]
