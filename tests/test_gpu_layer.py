@@ -393,3 +393,24 @@ def test_kernels_beside_each_other_see_this_forwards_data(T, H, I, N, k, graph):
             got = [[t.clone() for t in run(x)] for x in xs]
             for (y, logits), (y0, logits0) in zip(got, want):
                 assert torch.equal(logits, logits0) and torch.equal(y, y0)
+
+
+@pytest.mark.parametrize("T,H,I,N,k", [(1, 1024, 4096, 16384, 64), (37, 1000, 2728, 10000, 24), (64, 2048, 1000, 4096, 33),
+                                       (148, 512, 1024, 4096, 16), (149, 512, 1024, 4096, 16), (600, 256, 512, 1024, 8)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_stages_beside_each_other_equal_stages_one_by_one(T, H, I, N, k, dtype):
+    """With and without the skip connection, where the accumulate pass adds the shared MLP and where the down GEMM adds the
+    experts: the same bits as the stages in order (which a stage timer enforces)."""
+    from flash_moe_b200 import FlashMoE, FlashMoEConfig
+    from flash_moe_b200.modules.flash_moe import StageTimer
+
+    torch.manual_seed(k)
+    with torch.device("cuda"):
+        layer = FlashMoE(FlashMoEConfig(H, I, "silu", N, k, False)).to(dtype).eval()
+        x, skip = torch.randn(1, T, H, dtype=dtype), torch.randn(1, T, H, dtype=dtype)
+    with torch.no_grad():
+        for residual in (None, skip):
+            want = layer(x, residual=residual, stage_timer=StageTimer())
+            for _ in range(3):
+                got = layer(x, residual=residual)
+            assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
