@@ -164,8 +164,7 @@ int fmoe_swiglu_backward_rows(const void* dh, const void* a, const void* b, void
  *           2048 or 4096);
  *   mode 1: one bulk asynchronous copy per row into a shared-memory ring, one CTA per SM (row_bytes a multiple of
  *           16 up to 6144; ctas_per_sm ignored);
- *   mode 2: the same ring filled with 16-byte cp.async copies by four producer warps - the way the fused expert
- *           kernel fetches its rows (row_bytes = 512, 1024 or 2048).
+ *   mode 2: the same ring filled with 16-byte cp.async copies by four producer warps (row_bytes = 512, 1024 or 2048).
  * count * row_bytes / duration is the rate at which this GPU can bring gathered rows to its SMs.  `sink` (nullable)
  * is one float that is never written in practice.
  */
