@@ -342,6 +342,7 @@ __device__ __forceinline__ void store_blocked(uint16_t* base, int lane, const ui
 }
 
 constexpr int kTieCap = 256;  // entries of the per-warp list of candidates that tie with tau
+constexpr int kPrunedTieCap = 80;  // smaller, so that three CTAs of 128 keys fit beside a gate/up GEMM CTA (32 KB left)
 
 struct RouterRegLayout {
   int cta_bytes, warp_bytes;
@@ -870,9 +871,9 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
   const int nwarps = blockDim.x >> 5;
   const int C = L.C, nkp = L.nkp, kp = L.kp;
 
-  // staircase table, built once per CTA: entry c -> (p << 16) | q with (p+1)(q+1) <= k; row p starts at rowstart[p]
-  uint32_t* pq = reinterpret_cast<uint32_t*>(smem);
-  int* rowstart = reinterpret_cast<int*>(smem) + L.Cp;
+  // staircase table, built once per CTA: entry c -> (p << 8) | q (top_k <= 128) with (p+1)(q+1) <= k; row p starts at rowstart[p]
+  uint16_t* pq16 = reinterpret_cast<uint16_t*>(smem);
+  int* rowstart = reinterpret_cast<int*>(smem + 2 * L.Cp);
   if (warp == 0) {
     int running = 0;
     for (int base = 0; base < k; base += 32) {
@@ -895,8 +896,12 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
       const int mid = (lo + hi + 1) >> 1;
       if (rowstart[mid] <= c) lo = mid; else hi = mid - 1;
     }
-    pq[c] = (static_cast<uint32_t>(lo) << 16) | static_cast<uint32_t>(c - rowstart[lo]);
+    pq16[c] = static_cast<uint16_t>((lo << 8) | (c - rowstart[lo]));
   }
+  auto pq = [&](int c) {  // (p << 16) | q
+    const uint32_t e = pq16[c];
+    return ((e & 0xFF00u) << 8) | (e & 0xFFu);
+  };
   __syncthreads();
   // the staircase table above depends on k alone; the logits come from the previous kernel (kTopkLateWait: the one before)
   if (!(flags & kTopkLateWait)) pdl_wait();
@@ -910,7 +915,7 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
   uint32_t* win32 = reinterpret_cast<uint32_t*>(wbase + L.off_win);  // ... or 32-bit keys
   uint32_t* cs = reinterpret_cast<uint32_t*>(wbase + L.off_cs);      // staircase sums
   uint32_t* tl = reinterpret_cast<uint32_t*>(wbase + L.off_tl);      // flat ids of candidates equal to tau
-  int* tcnt = reinterpret_cast<int*>(tl + kTieCap);
+  int* tcnt = reinterpret_cast<int*>(tl + kPrunedTieCap);
   const int qrank = (k + lane) / (lane + 1);  // ceil(k / (lane + 1)): the rank that pairs with rank lane + 1 of half 0
   int idbits = 1;
   while (idbits < 31 && (1 << idbits) < nk * nk) ++idbits;
@@ -1058,14 +1063,14 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
 #pragma unroll
       for (int j = 0; j < CPL; ++j) {
         const int c = 32 * j + lane;
-        const uint32_t e = c < C ? pq[c] : 0xFFFFFFFFu;
+        const uint32_t e = c < C ? pq(c) : 0xFFFFFFFFu;
         const int p = e >> 16, q = e & 0xFFFFu;
         csr[j] = (p < na && q < nb) ? pair_ord(p, q) : 0u;  // 0 is below the key of every float, -inf included
       }
     } else {
 #pragma unroll 2
       for (int c = lane; c < C; c += 32) {
-        const uint32_t e = pq[c];
+        const uint32_t e = pq(c);
         const int p = e >> 16, q = e & 0xFFFFu;
         cs[c] = (p < na && q < nb) ? pair_ord(p, q) : 0u;
       }
@@ -1106,14 +1111,14 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
       if (bge == 0) return;
       const unsigned bgt = __ballot_sync(kFull, o > tau);
       if (o >= tau) {
-        const uint32_t e = pq[base + lane];
+        const uint32_t e = pq(base + lane);
         const uint32_t flat = flat_id(e >> 16, e & 0xFFFFu);
         if (o > tau) {
           const int pos = filled + __popc(bgt & below);
           if (pos < k) put(pos, o, flat);
         } else {
           const int pos = nties + __popc((bge & ~bgt) & below);
-          if (pos < kTieCap) tl[pos] = flat;
+          if (pos < kPrunedTieCap) tl[pos] = flat;
         }
       }
       filled += __popc(bgt);
@@ -1139,7 +1144,7 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
         for (int q = len; q < nb; ++q) {
           if (pair_ord(p, q) != tau) break;
           const int pos = nties + atomicAdd(tcnt, 1);
-          if (pos < kTieCap) tl[pos] = flat_id(p, q);
+          if (pos < kPrunedTieCap) tl[pos] = flat_id(p, q);
         }
       }
       if (base >= k && any == 0u) break;  // rows are sorted: no later row can tie
@@ -1154,7 +1159,7 @@ router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int 
       for (int j = 0; j < nties; ++j) rank += (__shfl_sync(kFull, id, j) < id) ? 1 : 0;
       if (lane < nties && rank < need) put(filled + rank, tau, id);
       filled += min(nties, need);
-    } else if (nties <= kTieCap) {
+    } else if (nties <= kPrunedTieCap) {
       uint32_t phi = 0xFFFFFFFFu;  // ids <= phi are taken
       if (nties > need) {
         // phi = the need-th smallest id = the largest v with fewer than `need` ids below v
@@ -1267,12 +1272,12 @@ RouterPrunedLayout make_pruned_layout(int nk, int k) {
   L.kp = next_pow2(k);
   for (int p = 0; p < k; ++p) L.C += k / (p + 1);
   L.Cp = (L.C + 3) / 4 * 4;
-  L.cta_bytes = static_cast<int>(align_up(static_cast<size_t>(L.Cp) * 4 + static_cast<size_t>(k) * 4, 16));
+  L.cta_bytes = static_cast<int>(align_up(static_cast<size_t>(L.Cp) * 2 + static_cast<size_t>(k) * 4, 16));
   L.off_ids = 2 * L.nkp * 4;
   L.off_win = L.off_ids + 2 * L.nkp * 2;
   L.off_cs = L.off_win + (L.kp < 32 ? 32 : L.kp) * 8;
   L.off_tl = L.off_cs + (L.C > 320 ? L.Cp * 4 : 0);  // up to 320 sums live in registers only
-  L.warp_bytes = static_cast<int>(align_up(L.off_tl + (kTieCap + 4) * 4, 16));
+  L.warp_bytes = static_cast<int>(align_up(L.off_tl + (kPrunedTieCap + 4) * 4, 16));
   return L;
 }
 
