@@ -52,10 +52,11 @@ template <typename K> inline cudaError_t resident_ctas(K* kern, int threads, int
 // The six kernels of a layer forward run back to back on one stream.  Launched with programmatic stream
 // serialisation, a kernel's CTAs may become resident, and run their set-up (barrier init, tensor-map prefetch, tensor
 // memory allocation, index tables), while the previous kernel is still draining; pdl_wait() then blocks until the
-// previous kernel has finished and its writes are visible.  Rules every kernel launched through launch_pdl keeps:
-// all threads call pdl_launch_dependents() first and pdl_wait() before their first access to global memory that is
-// not a launch-time constant (weights are read by kernels only, so even those accesses sit behind the wait).  Because
-// each kernel waits for its predecessor before it finishes, completion is transitive along the stream.
+// previous kernel has finished and its writes are visible.  Rules every kernel launched through launch_pdl keeps: pdl_wait()
+// stands before the first access to memory that the previous kernel writes; a kernel told that its operands are older may
+// run on and wait later, but some thread of it waits before the kernel ends, so completion is transitive along the stream.
+// The FIRST thread of a CTA to call pdl_launch_dependents() releases the next kernel (once every CTA has such a thread): where
+// that kernel relies on this one's wait, only threads that have waited may call it.
 // FMOE_PDL=<bit mask of kernel classes> in the environment chooses which kernels get the attribute (0: none; the
 // device-side instructions are no-ops without it).
 // measured: the scores pass (4) is slower when it is made resident early - at the benchmark shape 215 vs 213 us per
