@@ -284,10 +284,10 @@ __global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* __restr
 
 // ---------------------------------------------------------------- 2c. scores, few tokens
 // One CTA of W warps per (token, group of 16 of its experts), each warp on its own 128-column chunks of the 16 gathered
-// rows; the sums pass through the warps in column order, so they are those of the kernel above bit for bit, whatever the
-// number of tokens.  With few tasks that kernel leaves most of the chip idle while a warp pulls 16 whole rows: 64 tokens x
-// 2048 columns, top-32 (128 tasks) took 11.2 us there.
-template <typename T, int W, bool PEER>
+// rows; the sums pass through the warps in column order, so they are those of the kernel above with the same COLS bit for
+// bit, whatever the number of tokens.  With few tasks that kernel leaves most of the chip idle while a warp pulls 16 whole
+// rows: 64 tokens x 2048 columns, top-32 (128 tasks) took 11.2 us there.
+template <typename T, int W, bool PEER, int COLS>
 __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __restrict__ x, const T* __restrict__ down,
                                                                     const int64_t* __restrict__ idx,
                                                                     const T* __restrict__ gates, float* __restrict__ gs,
@@ -309,9 +309,9 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __
     const bool okb = (jb < k) && eb >= 0 && eb < N;
     if (((ja < k && !oka && ea != -1) || (jb < k && !okb && eb != -1)) && status != nullptr)
       atomicOr(status, FMOE_STATUS_BAD_EXPERT_ID);  // -1: empty slot, no flag
-    const T* ra = table_row<T, PEER>(down, shards, world, oka ? ea : 0, H, sharded) + 8 * tq;
-    const T* rb = table_row<T, PEER>(down, shards, world, okb ? eb : 0, H, sharded) + 8 * tq;
-    const T* rx = x + t * H + 8 * tq;
+    const T* ra = table_row<T, PEER>(down, shards, world, oka ? ea : 0, H, sharded) + COLS * tq;
+    const T* rb = table_row<T, PEER>(down, shards, world, okb ? eb : 0, H, sharded) + COLS * tq;
+    const T* rx = x + t * H + COLS * tq;
     // warp w loads the 128-column blocks w, w + W, ...; the sums go from warp to warp in column order (every column of B is
     // the token's row, so c[0] = c[1] and c[2] = c[3])
     for (int base = 0; base < H; base += W * 128) {
@@ -319,8 +319,9 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __
       uint4 qa[4], qb[4], qx[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int col = c0 + 32 * u;
-        const bool in = col + 8 * tq < H;
+        // COLS = 16: lane tq has the columns 16 tq .. 16 tq + 15 of a 64-column block, the first eight of them in step u = 0, 2
+        const int col = COLS == 16 ? c0 + 64 * (u >> 1) + 8 * (u & 1) : c0 + 32 * u;
+        const bool in = col + COLS * tq < H;
         qa[u] = in ? ldg16(ra + col) : make_uint4(0, 0, 0, 0);
         qb[u] = in ? ldg16(rb + col) : make_uint4(0, 0, 0, 0);
         qx[u] = in ? ldg16(rx + col) : make_uint4(0, 0, 0, 0);
@@ -690,17 +691,30 @@ int accum_split_warps(int64_t T, int H, int k, int cols) {
   return split_warps(T * ((H + 2 * cols - 1) / (2 * cols)), pieces, static_cast<int64_t>(device_sm_count()) * (pieces >= 3 ? 8 : 1));
 }
 
+// Scores pass with one thread's share of a row in 16 columns at a time, for tables of more than 384 MiB: rows taken 64 bytes
+// at a time cost twice the time there (16384 tokens x 2048 columns, top-16, table of 512 MiB 283 -> 153 us, 4 GiB with Zipf
+// 1.1 ids 519 -> 185 at 32768 tokens), and make no difference at 256 MiB (253 and 246).  It also groups the columns of a
+// sum differently, so the smaller tables of a stack of layers, where the last bit of a score can decide a later layer's
+// selection, keep the order that they have; tables in L2 give 16% for that (51 and 43 us at 4096 x 1024, top-64).  The rule
+// looks at the table alone and holds for every scores kernel: a token has the same bits alone and in a batch.
+template <typename T>
+bool whole_lines(int64_t N, int H) {
+  return H % 16 == 0 && N * H * static_cast<int64_t>(sizeof(T)) > (384ll << 20);
+}
+
 // the scores pass / accumulate pass for few tokens; false: not the shape for it (or, with `rc`, a launch error)
 template <typename T, bool PEER>
 bool try_scores_split(const void* rows, const void* table, const int64_t* idx, const void* gates, float* out, int64_t T_, int H,
                       int64_t N, int k, int32_t* status, cudaStream_t stream, int act, float* raw_out, const PeerTable& pt,
                       cudaError_t* rc) {
+  const bool lines = whole_lines<T>(PEER ? pt.sharded : N, H);
   const int groups = (k + 15) / 16;
   const int64_t tasks = T_ * groups;
   const int split = scores_split_warps(T_, H, k);
   if (split == 0) return false;
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * (64 / split);
-  auto kern = split == 8 ? expert_scores_split_kernel<T, 8, PEER> : expert_scores_split_kernel<T, 4, PEER>;
+  auto kern = split == 8 ? (lines ? expert_scores_split_kernel<T, 8, PEER, 16> : expert_scores_split_kernel<T, 8, PEER, 8>)
+                         : (lines ? expert_scores_split_kernel<T, 4, PEER, 16> : expert_scores_split_kernel<T, 4, PEER, 8>);
   *rc = launch_pdl(PEER ? 0 : 8, kern, dim3(static_cast<unsigned>(tasks < cap ? tasks : cap)), dim3(32 * split), 0, stream, 1,
                    static_cast<const T*>(rows), static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, tasks,
                    groups, H, N, k, status, act, raw_out, reinterpret_cast<const T* const*>(pt.shards), pt.world, pt.sharded);
@@ -744,16 +758,6 @@ void launch_accum(const void* up, const int64_t* idx, const float* gs, void* out
   auto kern = expert_accum_kernel<T, OutT, NCH>;
   (void)launch_pdl(8, kern, dim3(grid), dim3(128), 0, stream, 1, static_cast<const T*>(up), idx, gs, static_cast<OutT*>(out), T_,
                    H, N, k, colblocks, nullptr, 1, 0);  // launch errors surface through the caller's launch check
-}
-
-// Scores pass with one thread's share of a row in 16 columns at a time, for tables of more than 384 MiB: rows taken 64 bytes
-// at a time cost twice the time there (16384 tokens x 2048 columns, top-16, table of 512 MiB 283 -> 153 us, 4 GiB with Zipf
-// 1.1 ids 519 -> 185 at 32768 tokens), and make no difference at 256 MiB (253 and 246).  It also groups the columns of a
-// sum differently, so the smaller tables of a stack of layers, where the last bit of a score can decide a later layer's
-// selection, keep the order that they have; tables in L2 give 16% for that (51 and 43 us at 4096 x 1024, top-64).
-template <typename T>
-bool whole_lines(int64_t N, int H) {
-  return H % 16 == 0 && N * H * static_cast<int64_t>(sizeof(T)) > (384ll << 20);
 }
 
 // per-pair dot products <rows[t], table[e]>: gates != nullptr stores silu(dot) * gate (forward), nullptr the

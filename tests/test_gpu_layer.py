@@ -414,3 +414,21 @@ def test_stages_beside_each_other_equal_stages_one_by_one(T, H, I, N, k, dtype):
             for _ in range(3):
                 got = layer(x, residual=residual)
             assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("H,I,N,k,dtype", [(1024, 4096, 16384, 64, torch.bfloat16), (1000, 2728, 10000, 24, torch.float16)])
+def test_a_token_has_the_same_bits_in_any_batch(H, I, N, k, dtype):
+    """Tiles, kernels and their order depend on the number of tokens; the sums of one token do not."""
+    from flash_moe_b200 import FlashMoE, FlashMoEConfig
+
+    torch.manual_seed(k)
+    with torch.device("cuda"):
+        layer = FlashMoE(FlashMoEConfig(H, I, "silu", N, k, True)).to(dtype).eval()
+        x, skip = torch.randn(1, 9000, H, dtype=dtype), torch.randn(1, 9000, H, dtype=dtype)
+    with torch.no_grad():
+        want, logits = layer(x, residual=skip)
+        for first, count in ((0, 1), (8999, 1), (100, 16), (7, 64), (300, 149), (1000, 600), (17, 777), (4000, 4096)):
+            rows = slice(first, first + count)
+            y, lg = layer(x[:, rows], residual=skip[:, rows])
+            assert torch.equal(lg, logits[:, rows]), count
+            assert torch.equal(y, want[:, rows]), count

@@ -62,3 +62,22 @@ def test_scores_over_tables_beyond_the_tlb(H, offset):
         s = (x.double() * d[idx[:, j]].double()).sum(-1)
         want += (torch.nn.functional.silu(s) * gates[:, j].double())[:, None] * u[idx[:, j]].double()
     assert (flash_expert_fp32(x, d, u, idx, gates).double() - want).norm() <= 5e-6 * want.norm()
+
+
+@pytest.mark.parametrize("H,N", [(1040, 3000), (1040, (400 << 20) // 2080), (1032, (400 << 20) // 2064)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_a_token_alone_has_the_bits_it_has_in_a_batch(H, N, dtype):
+    """The order of a sum depends on the table alone, not on the number of tokens: few-token kernels (1 and 40 tokens) against
+    the one-warp-per-task kernels (801 tokens), for tables below and above 384 MiB (whole-line loads, where H allows them)."""
+    from flash_moe_b200.ops.flash_expert import _expert_forward
+
+    T, k = 801, 16
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    x, d, u = (torch.empty(rows, H, device="cuda", dtype=dtype).normal_(0, std, generator=gen)
+               for rows, std in ((T, 0.5), (N, 0.1), (N, 1.0)))
+    idx = torch.randint(0, N, (T, k), device="cuda", generator=gen)
+    gates = torch.rand(T, k, device="cuda", generator=gen).to(dtype)
+    out, scores = _expert_forward(x, d, u, idx, gates, torch.float32, save_scores=True)
+    for rows in (slice(5, 6), slice(800, 801), slice(100, 140)):
+        few, few_scores = _expert_forward(x[rows], d, u, idx[rows], gates[rows], torch.float32, save_scores=True)
+        assert torch.equal(few_scores, scores[rows]) and torch.equal(few, out[rows])
