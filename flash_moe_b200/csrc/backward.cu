@@ -169,16 +169,23 @@ int launch_router_topk_backward(const void* dscores, const int64_t* indices, int
 int launch_router_chain_backward(const void* dgates, const void* gates, const int64_t* indices, const void* log_probs,
                                  void* dlogits, int dtype, int64_t T, int nk, int k, int norm, cudaStream_t stream) {
   if (T <= 0) return FMOE_OK;
-  if (nk > 6144) return FMOE_ERR_UNSUPPORTED;  // the float32 sums of a CTA's four tokens sit in shared memory
-  const int smem = 4 * 2 * nk * 4;
-  const int64_t want = (T + 3) / 4;
+  // The float32 sums of a CTA's tokens, one per warp, sit in shared memory: four tokens up to 6144 keys, fewer above.  One
+  // fits up to 28672 keys, far beyond the 8192 or so that the forward's top-k takes.
+  constexpr int kMaxSmem = 224 * 1024;
+  int warps = 4;
+  while (warps > 1 && static_cast<int64_t>(warps) * 8 * nk > (192 << 10)) warps >>= 1;
+  if (static_cast<int64_t>(warps) * 8 * nk > kMaxSmem) return FMOE_ERR_UNSUPPORTED;
+  const int smem = warps * 8 * nk;
+  const int64_t want = (T + warps - 1) / warps;
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * 16;
   const int grid = static_cast<int>(want < cap ? want : cap);
   auto go = [&](auto kern, auto* tag) -> int {
     using P = decltype(tag);
     FMOE_CUDA_TRY(allow_smem(kern, smem));
-    kern<<<grid, 128, smem, stream>>>(static_cast<P>(dgates), static_cast<P>(gates), indices, static_cast<P>(log_probs),
-                                      static_cast<std::remove_const_t<std::remove_pointer_t<P>>*>(dlogits), T, nk, k, norm);
+    kern<<<grid, warps * 32, smem, stream>>>(static_cast<P>(dgates), static_cast<P>(gates), indices,
+                                             static_cast<P>(log_probs),
+                                             static_cast<std::remove_const_t<std::remove_pointer_t<P>>*>(dlogits), T, nk, k,
+                                             norm);
     FMOE_LAUNCH_CHECK();
     return FMOE_OK;
   };

@@ -287,3 +287,45 @@ def test_expert_backward_segments(T, H, N, k, dtype):
     for a, b in ((got[1], ddown), (got[2], dup)):
         assert (a.double() - b).norm() <= tol * b.norm()
     check_status()
+
+
+@pytest.mark.parametrize("nk", [6145, 8192])
+def test_training_step_with_the_widest_routers(nk):
+    """Router halves up to the widest that the top-k takes (their sums do not fit four tokens to a CTA): float32 gradients
+    against the same layer in float64 on the experts that it selected."""
+    from flash_moe_b200 import FlashMoE, FlashMoEConfig, check_status
+
+    T, H, I, k = 6, 8, 16, 4
+    torch.manual_seed(nk)
+    with torch.device("cuda"):
+        layer = FlashMoE(FlashMoEConfig(H, I, "silu", nk * nk, k, True)).eval()
+        x, dy = torch.randn(1, T, H), torch.randn(1, T, H)
+    x.requires_grad_()
+    y, _ = layer(x, return_routing=True)
+    y.backward(dy)
+    check_status()
+    idx = layer.last_indices
+    leaf = {n: getattr(layer, n).weight.detach().double().requires_grad_()
+            for n in ("router_gate", "gate_proj", "up_proj", "down_proj")}
+    leaf.update({n: getattr(layer, n).weight.detach()[idx].double().requires_grad_() for n in ("down_embed", "up_embed")})
+    xr = x.detach()[0].double().requires_grad_()
+    logits = (xr / (1.0 + layer.router_norm.eps) ** 0.5) @ leaf["router_gate"].t()
+    lp = torch.log_softmax(logits.view(T, 2, nk), -1)
+    gates = torch.exp(lp[:, 0].gather(1, idx // nk) + lp[:, 1].gather(1, idx % nk))
+    gates = gates / gates.sum(-1, keepdim=True)
+    s = (xr[:, None] * leaf["down_embed"]).sum(-1)
+    experts = ((torch.nn.functional.silu(s) * gates)[..., None] * leaf["up_embed"]).sum(1)
+    h = torch.nn.functional.silu(xr @ leaf["gate_proj"].t()) * (xr @ leaf["up_proj"].t())
+    want = experts + h @ leaf["down_proj"].t()
+    want.backward(dy[0].double())
+    assert rel_err(y[0], want.detach().cpu()) < 1e-5
+    assert rel_err(x.grad[0], xr.grad.cpu()) < 2e-5
+    for n, w in leaf.items():
+        got = getattr(layer, n).weight.grad
+        if n.endswith("embed"):  # a row's gradient is the sum over its slots; rows that no slot selects get zeros
+            rows, at = idx.unique(return_inverse=True)
+            ref = torch.zeros(len(rows), H, dtype=torch.float64, device="cuda").index_add_(0, at.flatten(), w.grad.flatten(0, 1))
+            assert rel_err(got[rows], ref.cpu()) < 2e-5, n
+            assert int(got.count_nonzero()) <= rows.numel() * H
+        else:
+            assert rel_err(got, w.grad.cpu()) < 2e-5, n
