@@ -66,8 +66,11 @@ constexpr int kPdlDefaultMask = 27;
 bool pdl_enabled(int kernel_class);  // api.cu; classes: 1 router GEMM, 2 top-k, 4 scores, 8 accumulate, 16 MLP GEMMs
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Loads of what the predecessor writes, for kernels that do work of their own before pdl_wait(): the compiler may move an
-// ordinary load through a const __restrict__ pointer (or __ldg) in front of the wait, it does not reorder these.
+// What the kernel before this one may write is read behind pdl_wait() through pointers without __restrict__, by ordinary or
+// volatile loads: a load through a const __restrict__ parameter counts as one of memory that does not change while the kernel
+// runs (as ld.global.nc and __ldg say outright), so the compiler may move it in front of the wait.  Only weights and tables,
+// which no kernel of this library writes, keep __restrict__ and __ldg.
+// The next two are such loads for kernels that do work of their own before they wait.
 __device__ __forceinline__ float ld_after_wait(const float* p) {
   float v;
   asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
@@ -176,6 +179,7 @@ template <> __device__ __forceinline__ uint4 pack16<__half>(const float (&f)[8])
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+__device__ __forceinline__ uint4 ld16(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 __device__ __forceinline__ uint4 ldg16(const void* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
 
 // 32 bytes (a 32-byte aligned address) in one load

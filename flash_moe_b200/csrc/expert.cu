@@ -140,9 +140,8 @@ __device__ __forceinline__ const T* table_row(const T* table, const T* const* sh
 // STAGES register buffers keep gathers in flight across batches to cover the L2 latency (measured at the
 // benchmark shape: 4 x 2 buffers 57.7 us, 8 x 1 61.9 us, 4 x 3 62.6 us, 2 x 2 57.8 us).
 template <typename T, int UNROLL, bool PEER = false, int STAGES = 1, int COLS = 8, bool LOAD32 = false>
-__global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* __restrict__ x, const T* __restrict__ down,
-                                                               const int64_t* __restrict__ idx,
-                                                               const T* __restrict__ gates, float* __restrict__ gs,
+__global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* x, const T* __restrict__ down,
+                                                               const int64_t* idx, const T* gates, float* __restrict__ gs,
                                                                int64_t ntok, int H, int64_t N, int k, int xs_stride,
                                                                int32_t* status, int act,
                                                                const T* const* __restrict__ shards = nullptr,
@@ -288,9 +287,8 @@ __global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* __restr
 // bit, whatever the number of tokens.  With few tasks that kernel leaves most of the chip idle while a warp pulls 16 whole
 // rows: 64 tokens x 2048 columns, top-32 (128 tasks) took 11.2 us there.
 template <typename T, int W, bool PEER, int COLS>
-__global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __restrict__ x, const T* __restrict__ down,
-                                                                    const int64_t* __restrict__ idx,
-                                                                    const T* __restrict__ gates, float* __restrict__ gs,
+__global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* x, const T* __restrict__ down,
+                                                                    const int64_t* idx, const T* gates, float* __restrict__ gs,
                                                                     int64_t tasks, int groups, int H, int64_t N, int k,
                                                                     int32_t* status, int act, float* __restrict__ raw_out,
                                                                     const T* const* __restrict__ shards, int world,
@@ -324,7 +322,7 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __
         const bool in = col + COLS * tq < H;
         qa[u] = in ? ldg16(ra + col) : make_uint4(0, 0, 0, 0);
         qb[u] = in ? ldg16(rb + col) : make_uint4(0, 0, 0, 0);
-        qx[u] = in ? ldg16(rx + col) : make_uint4(0, 0, 0, 0);
+        qx[u] = in ? ld16(rx + col) : make_uint4(0, 0, 0, 0);
       }
       for (int w = 0; w < W; ++w) {
         if (warp == w && c0 < H) {
@@ -357,9 +355,8 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* __
 // One warp per (token, 4 of its experts): 16-byte pieces of the four gathered rows and of the token's row, fp32 FMAs, one
 // shuffle reduction.  No sort in front of it (histogram, scan, scatter and a pass over the sorted pairs took 5 launches and
 // 22 us at 256 tokens x 256 columns, top-8; this takes one and 9).
-__global__ void __launch_bounds__(128) expert_scores_f32_kernel(const float* __restrict__ x, const float* __restrict__ down,
-                                                               const int64_t* __restrict__ idx,
-                                                               const float* __restrict__ gates, float* __restrict__ gs,
+__global__ void __launch_bounds__(128) expert_scores_f32_kernel(const float* x, const float* __restrict__ down,
+                                                               const int64_t* idx, const float* gates, float* __restrict__ gs,
                                                                int64_t ntok, int H, int64_t N, int k, int32_t* status,
                                                                int act, float* __restrict__ raw_out) {
   constexpr int G = 4;
@@ -387,7 +384,7 @@ __global__ void __launch_bounds__(128) expert_scores_f32_kernel(const float* __r
     const int hv = H >> 2;
 #pragma unroll 2
     for (int c = lane; c < hv; c += 32) {
-      const float4 v = __ldg(rx + c);
+      const float4 v = rx[c];
 #pragma unroll
       for (int i = 0; i < G; ++i) {
         const float4 d = __ldg(row[i] + c);
@@ -432,8 +429,8 @@ __device__ __forceinline__ void ffma2(uint64_t& acc, uint64_t a, uint64_t b) {
 }
 
 template <typename T, typename OutT, int NCH, bool PEER = false>
-__global__ void __launch_bounds__(128, 4) expert_accum_kernel(const T* __restrict__ up, const int64_t* __restrict__ idx,
-                                                          const float* __restrict__ gs, OutT* __restrict__ out,
+__global__ void __launch_bounds__(128, 4) expert_accum_kernel(const T* __restrict__ up, const int64_t* idx,
+                                                          const float* gs, OutT* __restrict__ out,
                                                           int64_t ntok, int H, int64_t N, int k, int colblocks,
                                                           const T* const* __restrict__ shards = nullptr,
                                                           int world = 1, int64_t sharded = 0) {
@@ -538,13 +535,12 @@ __global__ void __launch_bounds__(128, 4) expert_accum_kernel(const T* __restric
 // beside the scores pass (which has itself waited for the ids) and gathers its first batch of rows before it waits for the
 // weights.
 template <typename T, typename OutT, int W, bool PEER>
-__global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __restrict__ up, const int64_t* __restrict__ idx,
-                                                                   const float* __restrict__ gs, OutT* __restrict__ out,
+__global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __restrict__ up, const int64_t* idx,
+                                                                   const float* gs, OutT* __restrict__ out,
                                                                    int64_t tasks, int H, int64_t N, int k, int colblocks,
                                                                    int early, const T* const* __restrict__ shards,
                                                                    int world, int64_t sharded,
-                                                                   const float* __restrict__ addend,
-                                                                   const OutT* __restrict__ residual) {
+                                                                   const float* addend, const OutT* residual) {
   constexpr int VEC = Vec16<T>::N;
   constexpr int SLOTS = 8;
   constexpr int COLS = 32 * VEC;

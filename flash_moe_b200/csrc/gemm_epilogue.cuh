@@ -28,11 +28,11 @@ __device__ __forceinline__ bool store_add_row(uint32_t taddr, T* orow, const flo
     const int col0 = col_base + c * 32;
 #pragma unroll
     for (int v = 0; v < 8; ++v)
-      a[v] = (arow != nullptr && col0 + v * 4 < n_valid) ? __ldg(reinterpret_cast<const float4*>(arow + col0 + v * 4))
+      a[v] = (arow != nullptr && col0 + v * 4 < n_valid) ? *reinterpret_cast<const float4*>(arow + col0 + v * 4)
                                                          : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int v = 0; v < 4; ++v)
-      r[v] = (rrow != nullptr && col0 + v * 8 < n_valid) ? ldg16(rrow + col0 + v * 8) : make_uint4(0, 0, 0, 0);
+      r[v] = (rrow != nullptr && col0 + v * 8 < n_valid) ? ld16(rrow + col0 + v * 8) : make_uint4(0, 0, 0, 0);
   };
   fetch(0, ad[0], rs[0]);
   if (NCHUNK > 1) fetch(1, ad[1], rs[1]);

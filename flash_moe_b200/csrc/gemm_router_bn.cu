@@ -42,8 +42,7 @@ enum { kEarlyTrigger = 1, kLateWait = 2 };
 template <int BLOCK_M, int BLOCK_N, typename T>
 __global__ void __launch_bounds__(kThreads, 1)
 router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                      const float* __restrict__ mean, const float* __restrict__ invstd,
-                      const T* __restrict__ running_mean, const T* __restrict__ running_var, float eps, T* __restrict__ out,
+                      const float* mean, const float* invstd, const T* running_mean, const T* running_var, float eps, T* __restrict__ out,
                       int M, int N, int K, int num_m_tiles, int num_k_blocks, int flags, int32_t* status) {
   constexpr int A_BYTES = BLOCK_M * BLOCK_K * 2;
   constexpr int B_BYTES = BLOCK_N * BLOCK_K * 2;
@@ -131,8 +130,8 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (vec_stats && c0 + 8 <= K) {
         if (running_mean != nullptr) {
           float v[8];
-          unpack16<T>(ldg16(running_mean + c0), m);
-          unpack16<T>(ldg16(running_var + c0), v);
+          unpack16<T>(ld16(running_mean + c0), m);
+          unpack16<T>(ld16(running_var + c0), v);
   #pragma unroll
           for (int i = 0; i < 8; ++i) sd[i] = 1.0f / sqrtf(v[i] + eps);
         } else {

@@ -264,7 +264,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             const int col0 = n_tile * BLOCK_N + c * 32;
 #pragma unroll
             for (int v = 0; v < 4; ++v)
-              rcur[v] = (rrow != nullptr && col0 + v * 8 < ep.n_valid) ? ldg16(rrow + col0 + v * 8) : make_uint4(0, 0, 0, 0);
+              rcur[v] = (rrow != nullptr && col0 + v * 8 < ep.n_valid) ? ld16(rrow + col0 + v * 8) : make_uint4(0, 0, 0, 0);
             if (cok)
               epi::store_add_chunk_smem<T>(taddr + c * 32, orow, gen + RING_BYTES + b * ADDEND_CHUNK_BYTES, row_in_tile, rcur,
                                            rrow != nullptr, col0, ep.n_valid, row_ok);

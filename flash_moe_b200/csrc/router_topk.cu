@@ -283,7 +283,7 @@ __device__ __forceinline__ T load_cg(const T* p) {
 }
 
 template <typename T, int E>
-__device__ __forceinline__ void load_blocked(const T* __restrict__ row, int nk, int lane, float (&v)[E]) {
+__device__ __forceinline__ void load_blocked(const T* row, int nk, int lane, float (&v)[E]) {
   constexpr int BYTES = E * static_cast<int>(sizeof(T));
   if (BYTES >= 4 && nk == 32 * E && (reinterpret_cast<uintptr_t>(row) & 15u) == 0) {
     __align__(16) T tmp[E];
@@ -351,7 +351,7 @@ struct RouterRegLayout {
 };
 
 template <typename T, int E>
-__global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int k,
+__global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* logp, int64_t ntok, int nk, int k,
                                                              RouterRegLayout L, T* __restrict__ scores,
                                                              int64_t* __restrict__ indices, T* __restrict__ gates,
                                                              int flags) {
@@ -856,7 +856,7 @@ __device__ __forceinline__ uint32_t sort_lanes_packed(uint32_t v, int lane) {
 
 template <typename T, int E, int CPL>
 __global__ void __launch_bounds__(128, E <= 8 ? 7 : 4)
-router_topk_pruned_kernel(const T* __restrict__ logp, int64_t ntok, int nk, int k, RouterPrunedLayout L,
+router_topk_pruned_kernel(const T* logp, int64_t ntok, int nk, int k, RouterPrunedLayout L,
                           T* __restrict__ scores, int64_t* __restrict__ indices, T* __restrict__ gates, int flags) {
   using HK = HalfKey<T>;
   constexpr int LOW = OrdLowBits<T>::value;

@@ -47,8 +47,8 @@ struct SgemmCfg {
 
 template <int BM, int BN, int TM, int TN, int KG, int STAGES, bool SWIGLU, int KSL, int S, int CTAS>
 __global__ void __launch_bounds__(SgemmCfg<BM, BN, TM, TN, KG, STAGES, SWIGLU, KSL, S, CTAS>::THREADS, CTAS)
-sgemm_kernel(const float* __restrict__ A, int64_t lda, const float* __restrict__ B0, const float* __restrict__ B1,
-             const float* __restrict__ addend, const float* __restrict__ residual, float* __restrict__ out, int64_t ldo,
+sgemm_kernel(const float* A, int64_t lda, const float* __restrict__ B0, const float* __restrict__ B1,
+             const float* addend, const float* residual, float* __restrict__ out, int64_t ldo,
              int M, int N, int K, float* __restrict__ pre_gate, float* __restrict__ pre_up) {
   using C = SgemmCfg<BM, BN, TM, TN, KG, STAGES, SWIGLU, KSL, S, CTAS>;
   extern __shared__ float4 sg_smem[];
