@@ -213,7 +213,7 @@ struct LayerWs {
   size_t front_bytes, expert_bytes, total;
 };
 
-LayerWs carve_layer(void* ws, int64_t T, int H, int I, int64_t N, int nk, int k, int dtype) {
+LayerWs carve_layer(void* ws, int64_t T, int H, int I, int nk, int k, int dtype) {
   Carver c(ws);
   LayerWs w;
   const size_t es = dtype_size(dtype);
@@ -225,7 +225,7 @@ LayerWs carve_layer(void* ws, int64_t T, int H, int I, int64_t N, int nk, int k,
   w.gates = c.take(static_cast<size_t>(T) * k * es);
   w.acc = c.take(static_cast<size_t>(T) * H * 4);
   w.h = c.take(static_cast<size_t>(T) * I * es);
-  w.expert_bytes = expert_workspace_bytes(T, H, N, k);
+  w.expert_bytes = expert_forward_bytes(T, k);
   w.expert = c.take(w.expert_bytes);
   w.total = c.off;
   return w;
@@ -430,7 +430,7 @@ int fmoe_mlp_forward_saving_preacts(const void* x, const void* gate_w, const voi
 size_t fmoe_layer_workspace_bytes(int64_t num_tokens, int hidden, int intermediate, int64_t num_experts, int num_keys,
                                   int top_k, int dtype) {
   if (num_tokens < 0 || hidden <= 0 || intermediate <= 0 || num_experts <= 0 || num_keys <= 0 || top_k < 0) return 0;
-  return carve_layer(nullptr, num_tokens, hidden, intermediate, num_experts, num_keys, top_k, dtype).total;
+  return carve_layer(nullptr, num_tokens, hidden, intermediate, num_keys, top_k, dtype).total;
 }
 
 int fmoe_layer_forward(const fmoe_layer_args* a) {
@@ -444,7 +444,7 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   if (!a->x || !a->gate_proj || !a->up_proj || !a->down_proj || !a->router_gate || !a->down_embed || !a->up_embed ||
       !a->y || !a->router_logits)
     return FMOE_ERR_BAD_ARG;
-  const LayerWs w = carve_layer(a->workspace, T, H, I, N, nk, k, dtype);
+  const LayerWs w = carve_layer(a->workspace, T, H, I, nk, k, dtype);
   if (a->workspace == nullptr || a->workspace_bytes < w.total) return FMOE_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
   cudaStream_t s2 = static_cast<cudaStream_t>(a->aux_stream);
@@ -593,13 +593,13 @@ struct TrainWs {
   void *scores, *acc, *h, *expert;
   size_t expert_bytes, total;
 };
-TrainWs carve_train(void* ws, int64_t T, int H, int I, int64_t N, int k, int dtype) {
+TrainWs carve_train(void* ws, int64_t T, int H, int I, int k, int dtype) {
   Carver c(ws);
   TrainWs w;
   w.scores = c.take(static_cast<size_t>(T) * k * dtype_size(dtype));
   w.acc = c.take(static_cast<size_t>(T) * H * 4);
   w.h = c.take(static_cast<size_t>(T) * I * dtype_size(dtype));
-  w.expert_bytes = expert_workspace_bytes(T, H, N, k);
+  w.expert_bytes = expert_forward_bytes(T, k);
   w.expert = c.take(w.expert_bytes);
   w.total = c.off;
   return w;
@@ -615,7 +615,7 @@ bool train_args_ok(const fmoe_train_args* a) {
 size_t fmoe_train_forward_workspace_bytes(int64_t num_tokens, int hidden, int intermediate, int64_t num_experts, int top_k,
                                           int dtype) {
   if (num_tokens < 0 || hidden <= 0 || intermediate <= 0 || num_experts <= 0 || top_k < 0) return 0;
-  return carve_train(nullptr, num_tokens, hidden, intermediate, num_experts, top_k, dtype).total;
+  return carve_train(nullptr, num_tokens, hidden, intermediate, top_k, dtype).total;
 }
 
 int fmoe_train_forward(const fmoe_train_args* a, int* have_preacts) {
@@ -623,7 +623,7 @@ int fmoe_train_forward(const fmoe_train_args* a, int* have_preacts) {
     return FMOE_ERR_BAD_ARG;
   const int64_t T = a->num_tokens, N = a->num_experts;
   const int H = a->hidden, I = a->intermediate, nk = a->num_keys, k = a->top_k, dtype = a->dtype;
-  const TrainWs w = carve_train(a->workspace, T, H, I, N, k, dtype);
+  const TrainWs w = carve_train(a->workspace, T, H, I, k, dtype);
   if (a->workspace_bytes < w.total) return FMOE_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
   int rc = launch_router_topk(a->log_probs, dtype, T, nk, k, w.scores, a->indices, a->gates, (a->norm_topk_prob ? kTopkNorm : 0) | kTopkTokenRows, s);

@@ -206,7 +206,8 @@ enum { kTopkNorm = 1, kTopkFromLogits = 2, kTopkTokenRows = 4, kTopkLateWait = 8
 int launch_router_topk(const void* log_probs, int dtype, int64_t T, int nk, int k, void* scores, int64_t* indices,
                        void* gates, int flags, cudaStream_t stream);
 
-size_t expert_workspace_bytes(int64_t T, int H, int64_t N, int k);
+size_t expert_workspace_bytes(int64_t T, int H, int64_t N, int k);  // what the public query answers
+size_t expert_forward_bytes(int64_t T, int k);                       // what the forward uses of it
 bool expert_forward_adding_supported(int dtype, int64_t T, int H, int64_t N, int k);
 int launch_expert_forward_adding(const void* x, const void* down, const void* up, const int64_t* indices, const void* gates,
                                  const float* addend, const void* residual, void* y, int dtype, int64_t T, int H, int64_t N,

@@ -633,35 +633,27 @@ __global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __r
   }
 }
 
+struct Carver {
+  char* base;
+  size_t off = 0;
+  template <typename E> E* take(size_t count) {
+    E* p = base ? reinterpret_cast<E*>(base + off) : nullptr;
+    off += align_up(count * sizeof(E), 256);
+    return p;
+  }
+};
+
+// forward: the weights of the pairs, between the two passes
 struct ExpertWs {
-  int* counts;
-  int* offsets;
-  int* tile_sums;
-  int* rank;
-  int* sorted_pair;
-  int* sorted_expert;
   float* gs;
   size_t bytes;
 };
 
-ExpertWs carve(void* ws, int64_t T, int64_t N, int k) {
-  const int64_t P = T * k;
-  const int64_t ntiles = (N + kScanTile - 1) / kScanTile;
-  size_t off = 0;
-  auto take = [&](size_t bytes) {
-    void* p = ws ? static_cast<char*>(ws) + off : nullptr;
-    off += align_up(bytes, 256);
-    return p;
-  };
+ExpertWs carve(void* ws, int64_t T, int k) {
+  Carver c{static_cast<char*>(ws)};
   ExpertWs w;
-  w.counts = static_cast<int*>(take(static_cast<size_t>(N) * 4));
-  w.offsets = static_cast<int*>(take(static_cast<size_t>(N + 1) * 4));
-  w.tile_sums = static_cast<int*>(take(static_cast<size_t>(ntiles) * 4));
-  w.rank = static_cast<int*>(take(static_cast<size_t>(P) * 4));
-  w.sorted_pair = static_cast<int*>(take(static_cast<size_t>(P) * 4));
-  w.sorted_expert = static_cast<int*>(take(static_cast<size_t>(P) * 4));
-  w.gs = static_cast<float*>(take(static_cast<size_t>(P) * 4));
-  w.bytes = off;
+  w.gs = c.take<float>(static_cast<size_t>(T) * k);
+  w.bytes = c.off;
   return w;
 }
 
@@ -1247,9 +1239,14 @@ int run_weighted_rows(const void* values, const void* weights, const int64_t* id
 }
 
 struct ExpertBwdWs {
-  ExpertWs fwd;  // sort arrays; fwd.gs holds s, then ds
-  float* q;      // <dout, U>, then silu(s) * g
+  float* ds;          // s, then ds
+  float* q;           // <dout, U>, then silu(s) * g
   int* counts;        // [N + 1]: per expert, then the number of long segments
+  int* offsets;       // [N + 1]
+  int* tile_sums;
+  int* rank;
+  int* sorted_pair;
+  int* sorted_expert;
   int* long_experts;  // experts of more than kWarpSegment pairs
   int* temp;          // [P]
   float* partial_d;
@@ -1258,23 +1255,23 @@ struct ExpertBwdWs {
 };
 
 ExpertBwdWs carve_bwd(void* ws, int64_t T, int H, int64_t N, int k) {
+  Carver c{static_cast<char*>(ws)};
   ExpertBwdWs w;
-  w.fwd = carve(ws, T, N, k);
-  size_t off = w.fwd.bytes;
-  auto take = [&](size_t bytes) {
-    void* p = ws ? static_cast<char*>(ws) + off : nullptr;
-    off += align_up(bytes, 256);
-    return p;
-  };
   const int64_t P = T * k;
   const int64_t nchunks = (P + bwd_chunk(P) - 1) / bwd_chunk(P);
-  w.q = static_cast<float*>(take(static_cast<size_t>(P) * 4));
-  w.counts = static_cast<int*>(take(static_cast<size_t>(N + 1) * 4));
-  w.long_experts = static_cast<int*>(take(static_cast<size_t>(P / kWarpSegment + 1) * 4));
-  w.temp = static_cast<int*>(take(static_cast<size_t>(P) * 4));
-  w.partial_d = static_cast<float*>(take(static_cast<size_t>(nchunks) * 2 * H * 4));
-  w.partial_u = static_cast<float*>(take(static_cast<size_t>(nchunks) * 2 * H * 4));
-  w.bytes = off;
+  w.ds = c.take<float>(P);
+  w.q = c.take<float>(P);
+  w.counts = c.take<int>(N + 1);
+  w.offsets = c.take<int>(N + 1);
+  w.tile_sums = c.take<int>((N + kScanTile - 1) / kScanTile);
+  w.rank = c.take<int>(P);
+  w.sorted_pair = c.take<int>(P);
+  w.sorted_expert = c.take<int>(P);
+  w.long_experts = c.take<int>(P / kWarpSegment + 1);
+  w.temp = c.take<int>(P);
+  w.partial_d = c.take<float>(static_cast<size_t>(nchunks) * 2 * H);
+  w.partial_u = c.take<float>(static_cast<size_t>(nchunks) * 2 * H);
+  w.bytes = c.off;
   return w;
 }
 
@@ -1288,8 +1285,8 @@ void launch_bwd_tables(const void* x, const void* dout, const ExpertBwdWs& w, in
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * 16;
   const int grid = static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
   expert_bwd_tables_kernel<T, NCH, DEPTH><<<grid, 128, 0, stream>>>(
-      static_cast<const T*>(x), static_cast<const T*>(dout), w.fwd.gs, w.q, w.fwd.sorted_pair, w.fwd.sorted_expert,
-      w.fwd.offsets, N, static_cast<T*>(ddown), static_cast<T*>(dup), w.partial_d, w.partial_u, H, k, colblocks, bwd_chunk(P));
+      static_cast<const T*>(x), static_cast<const T*>(dout), w.ds, w.q, w.sorted_pair, w.sorted_expert,
+      w.offsets, N, static_cast<T*>(ddown), static_cast<T*>(dup), w.partial_d, w.partial_u, H, k, colblocks, bwd_chunk(P));
 }
 
 template <typename T>
@@ -1304,32 +1301,32 @@ int run_backward(const void* dout, const void* x, const void* down, const void* 
     FMOE_CUDA_TRY(cudaMemsetAsync(w.counts, 0, static_cast<size_t>(N + 1) * 4, stream));
     const int64_t want = (P + 255) / 256;
     const int grid = static_cast<int>(want < sms * 8 ? want : sms * 8);
-    expert_hist_kernel<<<grid, 256, 0, stream>>>(idx, P, N, w.counts, w.fwd.rank, status);
+    expert_hist_kernel<<<grid, 256, 0, stream>>>(idx, P, N, w.counts, w.rank, status);
     FMOE_LAUNCH_CHECK();
     const int ntiles = static_cast<int>((N + kScanTile - 1) / kScanTile);
     if (ntiles > 16) {
-      scan_tile_sums_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.counts, N, w.fwd.tile_sums);
+      scan_tile_sums_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.counts, N, w.tile_sums);
       FMOE_LAUNCH_CHECK();
-      scan_apply_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.counts, N, w.fwd.tile_sums, w.fwd.offsets);
+      scan_apply_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.counts, N, w.tile_sums, w.offsets);
     } else {
-      scan_apply_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.counts, N, nullptr, w.fwd.offsets);
+      scan_apply_kernel<<<ntiles, kScanThreads, 0, stream>>>(w.counts, N, nullptr, w.offsets);
     }
     FMOE_LAUNCH_CHECK();
-    expert_scatter_kernel<<<grid, 256, 0, stream>>>(idx, w.fwd.rank, w.fwd.offsets, P, w.fwd.sorted_pair, w.fwd.sorted_expert);
+    expert_scatter_kernel<<<grid, 256, 0, stream>>>(idx, w.rank, w.offsets, P, w.sorted_pair, w.sorted_expert);
     FMOE_LAUNCH_CHECK();
     const int64_t seg_want = (N + 7) / 8;
     const int seg_grid = static_cast<int>(seg_want < sms * 8 ? seg_want : sms * 8);
-    expert_segment_sort_kernel<<<seg_grid, 256, 0, stream>>>(w.fwd.offsets, N, w.fwd.sorted_pair, w.counts + N, w.long_experts);
+    expert_segment_sort_kernel<<<seg_grid, 256, 0, stream>>>(w.offsets, N, w.sorted_pair, w.counts + N, w.long_experts);
     FMOE_LAUNCH_CHECK();
     if (P > kWarpSegment) {
       FMOE_CUDA_TRY(allow_smem(expert_long_sort_kernel, kBitmapWords * 4));
-      expert_long_sort_kernel<<<sms, 512, kBitmapWords * 4, stream>>>(w.fwd.offsets, w.counts + N, w.long_experts, P,
-                                                                     w.fwd.sorted_pair, w.temp);
+      expert_long_sort_kernel<<<sms, 512, kBitmapWords * 4, stream>>>(w.offsets, w.counts + N, w.long_experts, P,
+                                                                     w.sorted_pair, w.temp);
       FMOE_LAUNCH_CHECK();
     }
   }
   if (saved_scores == nullptr) {  // s = <x, D[e]> was not kept by the forward: recompute it
-    rc = run_scores<T>(x, down, idx, nullptr, w.fwd.gs, T_, H, N, k, status, stream);
+    rc = run_scores<T>(x, down, idx, nullptr, w.ds, T_, H, N, k, status, stream);
     if (rc != FMOE_OK) return rc;
   }
   rc = run_scores<T>(dout, up, idx, nullptr, w.q, T_, H, N, k, status, stream);
@@ -1337,11 +1334,11 @@ int run_backward(const void* dout, const void* x, const void* down, const void* 
   {
     const int64_t want = (P + 255) / 256;
     const int grid = static_cast<int>(want < sms * 8 ? want : sms * 8);
-    expert_bwd_pairs_kernel<T><<<grid, 256, 0, stream>>>(saved_scores != nullptr ? saved_scores : w.fwd.gs, w.fwd.gs, w.q,
+    expert_bwd_pairs_kernel<T><<<grid, 256, 0, stream>>>(saved_scores != nullptr ? saved_scores : w.ds, w.ds, w.q,
                                                         static_cast<const T*>(gates), idx, N, static_cast<T*>(dgates), P);
     FMOE_LAUNCH_CHECK();
   }
-  rc = run_accum<T>(down, idx, w.fwd.gs, dx, sizeof(T) == 4 ? 1 : 0, T_, H, N, k, stream);
+  rc = run_accum<T>(down, idx, w.ds, dx, sizeof(T) == 4 ? 1 : 0, T_, H, N, k, stream);
   if (rc != FMOE_OK) return rc;
   const int need = (H + 32 * VEC - 1) / (32 * VEC);
   // two 16-byte pieces of a row per lane and two pairs in flight measured best (4096 tokens x 1024 columns, top-64: 109 us;
@@ -1356,7 +1353,7 @@ int run_backward(const void* dout, const void* x, const void* down, const void* 
   {
     const int64_t want = (N + 7) / 8, cap = static_cast<int64_t>(sms) * 8;
     const int grid = static_cast<int>(want < cap ? want : cap);
-    expert_bwd_finish_kernel<T><<<grid, 256, 0, stream>>>(w.fwd.offsets, N, w.partial_d, w.partial_u,
+    expert_bwd_finish_kernel<T><<<grid, 256, 0, stream>>>(w.offsets, N, w.partial_d, w.partial_u,
                                                           static_cast<T*>(ddown), static_cast<T*>(dup), H, bwd_chunk(P));
     FMOE_LAUNCH_CHECK();
   }
@@ -1365,10 +1362,20 @@ int run_backward(const void* dout, const void* x, const void* down, const void* 
 
 }  // namespace
 
+size_t expert_forward_bytes(int64_t T, int k) { return carve(nullptr, T, k).bytes; }
+
+// What the entry points of the op ask their callers for.  The forward needs expert_forward_bytes(); the rest, room for an
+// order of the pairs by expert, is kept: callers hold buffers of this size, and the limit of fmoe_expert_forward_static is
+// stated in it.
 size_t expert_workspace_bytes(int64_t T, int H, int64_t N, int k) {
   (void)H;
   if (T < 0 || N < 0 || k < 0) return 0;
-  return carve(nullptr, T, N, k).bytes;
+  Carver c{nullptr};
+  c.take<int>(N);
+  c.take<int>(N + 1);
+  c.take<int>((N + kScanTile - 1) / kScanTile);
+  for (int i = 0; i < 4; ++i) c.take<int>(T * k);
+  return c.off;
 }
 
 // Few tokens, 16-bit: both passes in their few-token forms, the second of which also adds the shared MLP's output (and the
@@ -1399,7 +1406,7 @@ int launch_expert_forward_adding(const void* x, const void* down, const void* up
                                  int k, void* ws, size_t ws_bytes, int32_t* status, cudaStream_t stream) {
   if (!expert_forward_adding_supported(dtype, T, H, N, k)) return FMOE_ERR_UNSUPPORTED;
   if (!aligned16(x) || !aligned16(down) || !aligned16(up) || !aligned16(y)) return FMOE_ERR_ALIGNMENT;
-  const ExpertWs w = carve(ws, T, N, k);
+  const ExpertWs w = carve(ws, T, k);
   if (ws == nullptr || ws_bytes < w.bytes) return FMOE_ERR_WORKSPACE;
   if (dtype == FMOE_DTYPE_BF16)
     return run_adding<__nv_bfloat16>(x, down, up, indices, gates, addend, residual, y, T, H, N, k, w, status, stream);
@@ -1424,7 +1431,7 @@ int launch_expert_forward(const void* x, const void* down, const void* up, const
     FMOE_CUDA_TRY(cudaMemsetAsync(out, 0, static_cast<size_t>(T) * H * dtype_size(out_dtype), stream));
     return FMOE_OK;
   }
-  const ExpertWs w = carve(ws, T, N, k);
+  const ExpertWs w = carve(ws, T, k);
   if (ws == nullptr || ws_bytes < w.bytes) return FMOE_ERR_WORKSPACE;
   const int out_f32 = (out_dtype == FMOE_DTYPE_F32) ? 1 : 0;
   switch (dtype) {
@@ -1528,7 +1535,7 @@ int launch_expert_forward_peer(const void* x, const void* const* down_shards, co
     FMOE_CUDA_TRY(cudaMemsetAsync(out, 0, static_cast<size_t>(T) * H * dtype_size(out_dtype), stream));
     return FMOE_OK;
   }
-  const ExpertWs w = carve(ws, T, N, k);
+  const ExpertWs w = carve(ws, T, k);
   if (ws == nullptr || ws_bytes < w.bytes) return FMOE_ERR_WORKSPACE;
   const int out_f32 = (out_dtype == FMOE_DTYPE_F32) ? 1 : 0;
   if (dtype == FMOE_DTYPE_BF16)

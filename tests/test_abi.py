@@ -87,3 +87,16 @@ def test_product_does_not_import_oracle():
             if f.endswith((".py", ".cu", ".cuh", ".h")):
                 text = open(os.path.join(dirpath, f)).read()
                 assert "oracle" not in text, f"{f} mentions the oracle"
+
+
+def test_scratch_of_a_forward_does_not_grow_with_the_number_of_experts(built_lib):
+    """The expert passes keep one float32 per (token, expert) pair between them, nothing per expert."""
+    from flash_moe_b200 import _lib
+
+    L = _lib.lib()
+    T, H, I, k = 64, 2048, 5632, 16
+    layer = [L.fmoe_layer_workspace_bytes(T, H, I, N, 256, k, 1) for N in (1 << 16, 1 << 20)]
+    train = [L.fmoe_train_forward_workspace_bytes(T, H, I, N, k, 1) for N in (1 << 16, 1 << 20)]
+    assert layer[0] == layer[1] and train[0] == train[1]
+    # scores in the module dtype, float32 sums, the MLP intermediate, the pairs' weights; each rounded up to 256 bytes
+    assert train[0] == T * k * 2 + T * H * 4 + T * I * 2 + T * k * 4
