@@ -92,8 +92,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const int* __r
 }
 
 // ---------------------------------------------------------------- 2b. scores per token on mma.sync
-// Token-centric scores for 16-bit dtypes when the tables are small enough to stay in L2: no
-// sort.  One warp per token; groups of 16 of its experts form the A operand (their down rows,
+// Token-centric scores for 16-bit dtypes, no sort.  Groups of 16 of a token's experts form the A operand (their down rows,
 // gathered with 128-bit loads), the token's x row is every column of B, so each accumulator
 // column holds <x, D[e]> for the 16 rows (fp32 accumulate).  The k index inside a 32-column
 // block is permuted identically for A and B so that every thread's 16-byte load feeds two MMAs.
@@ -137,9 +136,9 @@ __device__ __forceinline__ const T* table_row(const T* table, const T* const* sh
 // slice of shared memory (read back as B fragments right before each MMA; fetched with cp.async one task ahead,
 // together with the next task's expert ids), so every register that
 // waits for data waits for a gathered down row: batches of UNROLL 32-column blocks (2 * UNROLL x 16 B per lane) in
-// STAGES register buffers keep gathers in flight across batches to cover the L2 latency (measured at the
+// two register buffers keep gathers in flight across batches to cover the L2 latency (measured at the
 // benchmark shape: 4 x 2 buffers 57.7 us, 8 x 1 61.9 us, 4 x 3 62.6 us, 2 x 2 57.8 us).
-template <typename T, int UNROLL, bool PEER = false, int STAGES = 1, int COLS = 8, bool LOAD32 = false>
+template <typename T, int UNROLL, bool PEER, int COLS, bool LOAD32 = false>
 __global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* x, const T* __restrict__ down,
                                                                const int64_t* idx, const T* gates, float* __restrict__ gs,
                                                                int64_t ntok, int H, int64_t N, int k, int xs_stride,
@@ -245,24 +244,16 @@ __global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* x, cons
         Mma16816<T>::run(c, qa[u].z, qb[u].z, qa[u].w, qb[u].w, xq.z, xq.w);
       }
     };
-    if constexpr (STAGES == 2) {
-      // two register buffers: the next batch of gathers is issued before the current one is consumed, so the
-      // loads in flight never drain between batches (same column order, hence the same sums)
-      constexpr int STEP = 32 * UNROLL;
-      uint4 a0[UNROLL], b0[UNROLL], a1[UNROLL], b1[UNROLL];
-      load(a0, b0, 0);
-      for (int c0 = 0; c0 < H; c0 += 2 * STEP) {
-        if (c0 + STEP < H) load(a1, b1, c0 + STEP);
-        consume(a0, b0, c0);
-        if (c0 + 2 * STEP < H) load(a0, b0, c0 + 2 * STEP);
-        if (c0 + STEP < H) consume(a1, b1, c0 + STEP);
-      }
-    } else {
-      for (int c0 = 0; c0 < H; c0 += 32 * UNROLL) {
-        uint4 qa[UNROLL], qb[UNROLL];
-        load(qa, qb, c0);
-        consume(qa, qb, c0);
-      }
+    // two register buffers: the next batch of gathers is issued before the current one is consumed, so the loads in flight
+    // never drain between batches (same column order, hence the same sums)
+    constexpr int STEP = 32 * UNROLL;
+    uint4 a0[UNROLL], b0[UNROLL], a1[UNROLL], b1[UNROLL];
+    load(a0, b0, 0);
+    for (int c0 = 0; c0 < H; c0 += 2 * STEP) {
+      if (c0 + STEP < H) load(a1, b1, c0 + STEP);
+      consume(a0, b0, c0);
+      if (c0 + 2 * STEP < H) load(a0, b0, c0 + 2 * STEP);
+      if (c0 + STEP < H) consume(a1, b1, c0 + STEP);
     }
     if (tq == 0) {
       if (gates != nullptr) {
@@ -435,7 +426,7 @@ __global__ void __launch_bounds__(128, 4) expert_accum_kernel(const T* __restric
                                                           const T* const* __restrict__ shards = nullptr,
                                                           int world = 1, int64_t sharded = 0) {
   constexpr int VEC = Vec16<T>::N;
-  constexpr int SLOTS = NCH >= 4 ? 4 : 8;
+  constexpr int SLOTS = 8;
   pdl_wait();  // the weights gs come from the scores pass
   const int lane = threadIdx.x & 31;
   const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
@@ -768,8 +759,8 @@ int run_scores(const void* rows, const void* table, const int64_t* idx, const vo
     const int xs_stride = ((H + 255) / 256) * 32;  // uint4 per warp, rows padded to 256 columns
     const int smem = 4 * 2 * xs_stride * 16;  // two x-row buffers per warp
     const bool aligned32 = (reinterpret_cast<uintptr_t>(table) & 31u) == 0;
-    auto kern = !whole_lines<T>(N, H) ? expert_scores_mma_kernel<T, 4, false, 2, 8>
-                : aligned32 ? expert_scores_mma_kernel<T, 4, false, 2, 16, true> : expert_scores_mma_kernel<T, 4, false, 2, 16>;
+    auto kern = !whole_lines<T>(N, H) ? expert_scores_mma_kernel<T, 4, false, 8>
+                : aligned32 ? expert_scores_mma_kernel<T, 4, false, 16, true> : expert_scores_mma_kernel<T, 4, false, 16>;
     FMOE_CUDA_TRY(allow_smem(kern, smem));
     FMOE_CUDA_TRY(launch_pdl(4, kern, dim3(grid), dim3(128), smem, stream, 1, static_cast<const T*>(rows),
                              static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, T_, H, N, k, xs_stride,
@@ -1184,7 +1175,7 @@ int run_typed_peer(const void* x, const void* const* down_shards, const void* co
       const int grid = static_cast<int>(want < cap ? want : cap);
       const int xs_stride = ((H + 255) / 256) * 32;
       const int smem = 4 * 2 * xs_stride * 16;  // two x-row buffers per warp
-      auto kern = whole_lines<T>(N, H) ? expert_scores_mma_kernel<T, 4, true, 2, 16> : expert_scores_mma_kernel<T, 4, true, 2, 8>;
+      auto kern = whole_lines<T>(N, H) ? expert_scores_mma_kernel<T, 4, true, 16> : expert_scores_mma_kernel<T, 4, true, 8>;
       FMOE_CUDA_TRY(allow_smem(kern, smem));
       kern<<<grid, 128, smem, stream>>>(static_cast<const T*>(x), static_cast<const T*>(hot_down), idx,
                                         static_cast<const T*>(gates), w.gs, T_, H, N + hot_rows, k, xs_stride, status,
