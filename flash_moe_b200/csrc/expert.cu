@@ -301,6 +301,11 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* x,
     const T* ra = table_row<T, PEER>(down, shards, world, oka ? ea : 0, H, sharded) + COLS * tq;
     const T* rb = table_row<T, PEER>(down, shards, world, okb ? eb : 0, H, sharded) + COLS * tq;
     const T* rx = x + t * H + COLS * tq;
+    // the thread that finishes a slot fetches its id and gate now, beside the rows
+    const int64_t p = t * k + j0 + threadIdx.x;
+    const bool mine = threadIdx.x < 16 && j0 + static_cast<int>(threadIdx.x) < k;
+    const int64_t e = mine ? idx[p] : -1;
+    const float gate = mine && gates != nullptr ? to_f32<T>(gates[p]) : 0.f;
     // warp w loads the 128-column blocks w, w + W, ...; the sums go from warp to warp in column order (every column of B is
     // the token's row, so c[0] = c[1] and c[2] = c[3])
     for (int base = 0; base < H; base += W * 128) {
@@ -329,13 +334,11 @@ __global__ void __launch_bounds__(32 * W) expert_scores_split_kernel(const T* x,
         __syncthreads();
       }
     }
-    if (threadIdx.x < 16 && j0 + threadIdx.x < k) {
-      const int64_t p = t * k + j0 + threadIdx.x;
-      const int64_t e = idx[p];
+    if (mine) {
       const bool ok = e >= 0 && e < N;
       const float2 both = chain[(threadIdx.x & 7) * 4];
       const float s = !ok ? 0.f : threadIdx.x < 8 ? both.x : both.y;
-      gs[p] = gates != nullptr && ok ? expert_act(s, act) * to_f32<T>(gates[p]) : s;  // no gates: the raw dot product
+      gs[p] = gates != nullptr && ok ? expert_act(s, act) * gate : s;  // no gates: the raw dot product
       if (raw_out != nullptr) raw_out[p] = s;
     }
     __syncthreads();
