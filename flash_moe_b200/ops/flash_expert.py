@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from .utils import contiguous
+from .utils import contiguous, plain_call
 
 
 def _expert_forward(hidden_states, down_weights, up_weights, indices, routing_weights, out_dtype=None, save_scores=False):
@@ -84,7 +84,7 @@ class FlashExpertFunc(torch.autograd.Function):
 
 def flash_expert_func(hidden_states, down_weights, up_weights, indices, routing_weights):
     """experts_states[T,H] = sum_j silu(<x, down[idx_j]>) * routing_weights_j * up[idx_j], in hidden_states.dtype."""
-    if not torch.is_grad_enabled():  # an autograd node costs several microseconds of host time
+    if plain_call():
         return _expert_forward(hidden_states, down_weights, up_weights, indices, routing_weights)
     return FlashExpertFunc.apply(hidden_states, down_weights, up_weights, indices, routing_weights)
 

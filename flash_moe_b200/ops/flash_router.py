@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from .utils import contiguous
+from .utils import contiguous, plain_call
 
 
 def _router_forward(router_logits: torch.Tensor, num_expert_keys: int, num_experts_per_tok: int, want_gates=False,
@@ -66,7 +66,7 @@ class FlashRouterFunc(torch.autograd.Function):
 
 def flash_router_func(router_logits, num_expert_keys, num_experts_per_tok):
     """(scores[T,k] in the input dtype, indices[T,k] int64) for log-probs ``router_logits[2,T,nk]``."""
-    if not torch.is_grad_enabled():  # an autograd node costs several microseconds of host time
+    if plain_call():
         return _router_forward(router_logits, num_expert_keys, num_experts_per_tok)
     return FlashRouterFunc.apply(router_logits, num_expert_keys, num_experts_per_tok)
 

@@ -3,8 +3,16 @@
 from __future__ import annotations
 
 import torch
+from torch.autograd import forward_ad
 
 
 def contiguous(t):
     """The reference makes every tensor argument contiguous before a kernel sees it (ops/utils.py:35-45)."""
     return t.contiguous() if isinstance(t, torch.Tensor) else t
+
+
+def plain_call() -> bool:
+    """True where an op may run without its autograd node, which costs several microseconds of host time: no gradient is
+    recorded, no forward-mode level is open (the node is what refuses tangents, which would be dropped silently) and
+    torch.jit is not tracing (the node is what a trace records)."""
+    return not torch.is_grad_enabled() and forward_ad._current_level < 0 and torch._C._get_tracing_state() is None
