@@ -23,8 +23,11 @@ from .. import _lib
 _WEIGHT_MODULES = ("gate_proj", "up_proj", "down_proj", "router_gate", "down_embed", "up_embed")
 
 
-def _hooked(module: nn.Module) -> bool:
-    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
+def _plain_linear(module: nn.Module) -> bool:
+    """True where calling the module is nothing but a product with its weight: no subclass, bias, replaced forward or hook."""
+    return not (type(module) is not nn.Linear or module.bias is not None or "forward" in module.__dict__
+                or module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
+                or nn.modules.module._has_any_global_hook())
 
 
 class FlashMoEConfig:
@@ -141,10 +144,11 @@ class FlashMoE(nn.Module):
 
     def _forward_differentiable(self, hidden_states, return_routing=False):
         """The layer with a graph recorded: the batch-norm as torch's module, everything behind it as one autograd node.  A
-        router_gate that is not a plain Linear (wrapped, hooked, with a bias) takes the chain of separate nodes."""
+        router_gate whose call is more than a product with its weight (wrapped, hooked, with a bias) takes the chain of separate
+        nodes, which calls it."""
         gate = self.router_gate
         k = self.top_k
-        if type(gate) is not nn.Linear or gate.bias is not None or _hooked(gate) or k == 0 or hidden_states.numel() == 0 \
+        if not _plain_linear(gate) or k == 0 or hidden_states.numel() == 0 \
                 or self.hidden_size % (16 // hidden_states.element_size()) or self.intermediate_size % (16 // hidden_states.element_size()):
             return self._forward_chain(hidden_states, return_routing)
         from .training import LayerTrainingStep

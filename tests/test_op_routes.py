@@ -47,3 +47,55 @@ def test_a_trace_records_the_op(op):
     with torch.no_grad():
         traced = torch.jit.trace(op, (torch.ones(2, 3),), check_trace=False)
         assert torch.equal(traced(torch.full((2, 3), 3.0)), torch.full((2, 3), 6.0))
+
+
+def wrap_forward(layer):
+    inner = layer.router_gate.forward
+    layer.router_gate.forward = lambda x: inner(x)
+
+
+def hook(layer):
+    layer.router_gate.register_forward_hook(lambda *a: None)
+
+
+@pytest.fixture
+def taken(monkeypatch):
+    """(layer, call): which of the two differentiable forms of the layer a call takes."""
+    from flash_moe_b200 import FlashMoE, FlashMoEConfig
+    from flash_moe_b200.modules import training
+
+    layer = FlashMoE(FlashMoEConfig(16, 16, "silu", 16, 2))
+    route = []
+
+    def node(x, *a):
+        route.append("node")
+        return x, x.new_zeros(x.shape[0], 8), None, None
+
+    monkeypatch.setattr(training.LayerTrainingStep, "apply", node)
+    monkeypatch.setattr(layer, "_forward_chain", lambda *a: route.append("chain"))
+
+    def call():
+        layer._forward_differentiable(torch.ones(1, 4, 16))
+        return route.pop()
+
+    return layer, call
+
+
+def test_a_plain_layer_trains_in_one_node(taken):
+    assert taken[1]() == "node"
+
+
+@pytest.mark.parametrize("change", [wrap_forward, hook])
+def test_a_router_gate_that_does_more_is_called(taken, change):
+    layer, call = taken
+    change(layer)
+    assert call() == "chain"
+
+
+def test_global_hooks_see_the_router_gate(taken):
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    try:
+        assert taken[1]() == "chain"
+    finally:
+        handle.remove()
+    assert taken[1]() == "node"
