@@ -145,10 +145,10 @@ class FlashMoE(nn.Module):
     def _forward_differentiable(self, hidden_states, return_routing=False):
         """The layer with a graph recorded: the batch-norm as torch's module, everything behind it as one autograd node.  A
         router_gate whose call is more than a product with its weight (wrapped, hooked, with a bias) takes the chain of separate
-        nodes, which calls it."""
+        nodes, which calls it; so does a call under autocast, which gives the log-probabilities another type than the layer's."""
         gate = self.router_gate
         k = self.top_k
-        if not _plain_linear(gate) or k == 0 or hidden_states.numel() == 0 \
+        if not _plain_linear(gate) or k == 0 or hidden_states.numel() == 0 or torch.is_autocast_enabled("cuda") \
                 or self.hidden_size % (16 // hidden_states.element_size()) or self.intermediate_size % (16 // hidden_states.element_size()):
             return self._forward_chain(hidden_states, return_routing)
         from .training import LayerTrainingStep

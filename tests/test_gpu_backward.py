@@ -329,3 +329,21 @@ def test_training_step_with_the_widest_routers(nk):
             assert int(got.count_nonzero()) <= rows.numel() * H
         else:
             assert rel_err(got, w.grad.cpu()) < 2e-5, n
+
+
+def test_autocast_selects_on_float32_log_probabilities():
+    """Under autocast the log-softmax returns float32, whatever the layer's type, and the selection is made on that."""
+    from flash_moe_b200 import FlashMoE, FlashMoEConfig
+
+    torch.manual_seed(2)
+    with torch.device("cuda"):
+        layer = FlashMoE(FlashMoEConfig(256, 512, "silu", 4096, 16, False)).to(torch.bfloat16).eval()
+        x = torch.randn(2, 200, 256).to(torch.bfloat16)
+    with torch.autocast("cuda", torch.bfloat16):
+        y, logits = layer(x, return_routing=True)
+        lp = torch.log_softmax(logits.detach(), -1)
+    assert lp.dtype == torch.float32
+    scores, idx = O.router_topk(lp.cpu(), 64, 16)
+    assert torch.equal(layer.last_indices.cpu(), idx)
+    y.float().sum().backward()
+    assert torch.isfinite(layer.router_gate.weight.grad.float()).all()
