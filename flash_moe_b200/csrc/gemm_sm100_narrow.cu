@@ -16,6 +16,8 @@
 // 1024, intermediate 4096 (25 MB of weights, both GEMMs inside a forward, us): 33 -> 17; 64 tokens, 2048 x 5632 (69 MB): 48 ->
 // 29; 777 tokens, 1000 x 2728: 43 -> 40 (128-row token tiles in one or two CTAs per row of tiles before).  The set-up runs
 // ahead of the predecessor's end: barriers and the first ring of weight tiles need nothing from it.
+#include <algorithm>
+
 #include "gemm_epilogue.cuh"
 
 namespace fmoe {
@@ -365,12 +367,30 @@ int launch_plan(const NarrowPlan& p, const void* w0, const void* w1, const void*
   return FMOE_OK;
 }
 
+// Token tiles are the grid's second dimension (at most 65535 of them): more tokens than this go in several launches.  Each
+// stands to the one in front of it as that one to its predecessor, so `early` holds for all of them.
+constexpr int64_t kMaxTokens = int64_t{1} << 23;
+
 template <int EPI, typename T>
 int launch_narrow(const void* w0, const void* w1, const void* x, const NarrowEpi& ep, int dtype, int64_t M, int N, int K,
                   int early, int32_t* status, cudaStream_t stream) {
-  const NarrowPlan p = plan_narrow(M, N, K, EPI == NARROW_SWIGLU ? 2 : 1);
-  if (p.rows == 64) return launch_plan<64, EPI, T>(p, w0, w1, x, ep, dtype, M, N, K, early, status, stream);
-  return launch_plan<128, EPI, T>(p, w0, w1, x, ep, dtype, M, N, K, early, status, stream);
+  auto from = [](auto* p, int64_t row, int64_t row_bytes) {
+    using P = decltype(p);
+    using Byte = std::conditional_t<std::is_const_v<std::remove_pointer_t<P>>, const char, char>;
+    return p == nullptr ? p : reinterpret_cast<P>(reinterpret_cast<Byte*>(p) + row * row_bytes);
+  };
+  for (int64_t m0 = 0; m0 < M; m0 += kMaxTokens) {
+    const int64_t rows = std::min(M - m0, kMaxTokens);
+    const int64_t pitch = static_cast<int64_t>(N) * sizeof(T);
+    const NarrowEpi part{from(ep.out, m0, EPI == NARROW_RAW ? N * int64_t{4} : pitch), from(ep.addend, m0, N * int64_t{4}),
+                         from(ep.residual, m0, pitch), from(ep.pre_gate, m0, pitch), from(ep.pre_up, m0, pitch), ep.n_valid};
+    const void* xp = from(x, m0, static_cast<int64_t>(K) * sizeof(T));
+    const NarrowPlan p = plan_narrow(rows, N, K, EPI == NARROW_SWIGLU ? 2 : 1);
+    const int rc = p.rows == 64 ? launch_plan<64, EPI, T>(p, w0, w1, xp, part, dtype, rows, N, K, early, status, stream)
+                                : launch_plan<128, EPI, T>(p, w0, w1, xp, part, dtype, rows, N, K, early, status, stream);
+    if (rc != FMOE_OK) return rc;
+  }
+  return FMOE_OK;
 }
 
 }  // namespace
@@ -383,7 +403,7 @@ int narrow_swiglu_ctas(int64_t M, int I, int K) {
 
 // 16-bit operands with 16-byte aligned rows (K % 8 == 0), where the estimate is below that of the pair tiles
 bool gemm_narrow_preferred(int64_t M, int N, int K, bool swiglu) {
-  if (M <= 0 || M > (int64_t{1} << 23) || N <= 0 || K <= 0 || K % 8 != 0) return false;
+  if (M <= 0 || N <= 0 || K <= 0 || K % 8 != 0) return false;
   if (!gemm_pair_supported(M, N, K)) return true;
   if (M > 8192) return false;
   return plan_narrow(M, N, K, swiglu ? 2 : 1).cost < pair_cost(M, N, K, swiglu ? 2 : 1);

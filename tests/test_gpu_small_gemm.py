@@ -61,3 +61,22 @@ def test_mlp_few_tokens(T, H, I, dtype):
         if kept is not None:
             assert (kept.float() - ref).norm() <= ulp * ref.norm()
     check_status()
+
+
+@pytest.mark.parametrize("T,H,I,dtype", [((1 << 23) + 300, 8, 8, torch.bfloat16)])
+def test_mlp_with_more_tokens_than_one_grid_takes(T, H, I, dtype):
+    """More token tiles than the grid's second dimension holds: rows around the seam, at both ends and in between."""
+    from flash_moe_b200 import check_status
+    from flash_moe_b200.ops.flash_mlp import flash_mlp_func
+
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    x, wg, wu, wd = (torch.empty(shape, device="cuda", dtype=dtype).normal_(0, std, generator=gen)
+                     for shape, std in (((T, H), 0.5), ((I, H), H**-0.5), ((I, H), H**-0.5), ((H, I), I**-0.5)))
+    with torch.no_grad():
+        got = flash_mlp_func(x, wg, wu, wd)
+    check_status()
+    for rows in (slice(0, 400), slice(T // 2, T // 2 + 400), slice(T - 700, T)):
+        xs = x[rows].double()
+        h = torch.nn.functional.silu(xs @ wg.double().t()) * (xs @ wu.double().t())
+        want = (h if dtype == torch.float32 else h.to(dtype).double()) @ wd.double().t()
+        assert (got[rows].double() - want).norm() <= (2e-6 if dtype == torch.float32 else 2.0**-8) * want.norm()
