@@ -240,6 +240,7 @@ int pick_sgemm(const float* a, int64_t lda, const float* b0, const float* b1, co
     return FMOE_SGEMM(32, 32, 2, 4, 1, 6, SWIGLU, 1, 1, 1);
   }
   auto cost = [&](int bm, int bn, int kstep, int split, double rate) {
+    if ((M + bm - 1) / bm > 65535) return 1e30;  // rows of tiles are the grid's second dimension
     const int64_t ctas = (tiles(bm, bn) * split + sms - 1) / sms;
     const int64_t steps = (K + kstep - 1) / kstep;
     const double macs = static_cast<double>(ctas) * bm * bn * NB * ((steps + split - 1) / split * kstep);

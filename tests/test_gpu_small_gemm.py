@@ -63,7 +63,7 @@ def test_mlp_few_tokens(T, H, I, dtype):
     check_status()
 
 
-@pytest.mark.parametrize("T,H,I,dtype", [((1 << 23) + 300, 8, 8, torch.bfloat16)])
+@pytest.mark.parametrize("T,H,I,dtype", [((1 << 23) + 300, 8, 8, torch.bfloat16), (2_100_001, 64, 8, torch.float32)])
 def test_mlp_with_more_tokens_than_one_grid_takes(T, H, I, dtype):
     """More token tiles than the grid's second dimension holds: rows around the seam, at both ends and in between."""
     from flash_moe_b200 import check_status
