@@ -240,7 +240,7 @@ __global__ void router_topk_smem_kernel(const T* __restrict__ logp, int64_t ntok
 
 
 // ------------------------------------------------------------------------------------------
-// Register-resident variant for num_keys <= 1024 (float32; 16-bit rows of which most is wanted): each half is sorted by a shuffle-based bitonic
+// Register-resident variant for num_keys <= 1024 (float32; 16-bit rows where it is the faster one, see launch_typed): each half is sorted by a shuffle-based bitonic
 // network (E = padded num_keys / 32 keys per lane), sort keys are 32-bit for 16-bit dtypes
 // (16-bit order key | inverted index) and 64-bit for float32.  Shared memory only holds the
 // sorted halves (for the candidate gathers and binary searches), the index-order values, the
@@ -350,7 +350,9 @@ struct RouterRegLayout {
   int nkp, kp, kq, C, Cp;
 };
 
-template <typename T, int E>
+// CPL > 0: the staircase candidates (at most 32 * CPL of them) stay in registers, CPL per lane, through the threshold
+// search and the emit step, whose loops then have compile-time bounds and no shared-memory round trips between rounds.
+template <typename T, int E, int CPL = 0>
 __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* logp, int64_t ntok, int nk, int k,
                                                              RouterRegLayout L, T* __restrict__ scores,
                                                              int64_t* __restrict__ indices, T* __restrict__ gates,
@@ -473,11 +475,26 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* logp, int
 
     // 2. staircase candidate scores; track the smallest to narrow the threshold search
     uint32_t cmin = 0xFFFFFFFFu;
-    for (int c = lane; c < C; c += 32) {
-      const uint32_t e = pq[c];
-      const uint32_t o = f32_to_ord(round_to<T>(__fadd_rn(sa[e >> 16], sb[e & 0xFFFFu])) + 0.0f);
-      cs[c] = o;
-      cmin = min(cmin, o);
+    uint32_t csr[CPL > 0 ? CPL : 1], pqr[CPL > 0 ? CPL : 1];
+    auto pair_ord = [&](uint32_t e) { return f32_to_ord(round_to<T>(__fadd_rn(sa[e >> 16], sb[e & 0xFFFFu])) + 0.0f); };
+    if constexpr (CPL > 0) {
+#pragma unroll
+      for (int j = 0; j < CPL; ++j) {
+        const int c = 32 * j + lane;
+        const bool in = c < C;
+        pqr[j] = in ? pq[c] : 0u;
+        const uint32_t o = pair_ord(pqr[j]);
+        csr[j] = in ? o : 0u;  // 0 is below the key of every float, -inf included
+        if (in) {
+          cs[c] = o;  // the tie search below looks up single cells
+          cmin = min(cmin, o);
+        }
+      }
+    } else {
+      for (int c = lane; c < C; c += 32) {
+        cs[c] = pair_ord(pq[c]);
+        cmin = min(cmin, cs[c]);
+      }
     }
     cmin = __reduce_min_sync(kFull, cmin);
     __syncwarp();
@@ -491,7 +508,12 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* logp, int
       for (int bit = top; bit >= LOW; --bit) {
         const uint32_t trial = tau | (1u << bit);
         int n_ge = 0;
-        for (int c = lane; c < C; c += 32) n_ge += (cs[c] >= trial) ? 1 : 0;
+        if constexpr (CPL > 0) {
+#pragma unroll
+          for (int j = 0; j < CPL; ++j) n_ge += (csr[j] >= trial) ? 1 : 0;
+        } else {
+          for (int c = lane; c < C; c += 32) n_ge += (cs[c] >= trial) ? 1 : 0;
+        }
         n_ge = __reduce_add_sync(kFull, n_ge);
         if (n_ge >= k) tau = trial;
       }
@@ -500,15 +522,13 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* logp, int
 
     // emit everything above tau; collect the staircase candidates equal to tau in the tie list
     int filled = 0, nties = 0;
-    for (int base = 0; base < C; base += 32) {
-      const int c = base + lane;
-      const uint32_t v = (c < C) ? cs[c] : 0u;
-      const bool g = (c < C) && (v > tau);
-      const bool eq = (c < C) && (v == tau);
+    auto emit = [&](bool in, uint32_t v, auto cell) {
+      const bool g = in && v > tau;
+      const bool eq = in && v == tau;
       const unsigned bal = __ballot_sync(kFull, g);
       const unsigned beq = __ballot_sync(kFull, eq);
       if (g || eq) {
-        const uint32_t e = pq[c];
+        const uint32_t e = cell();
         const uint32_t flat = static_cast<uint32_t>(ia[e >> 16]) * static_cast<uint32_t>(nk) + ib[e & 0xFFFFu];
         if (g) {
           const int pos = filled + __popc(bal & ((1u << lane) - 1u));
@@ -520,6 +540,16 @@ __global__ void __launch_bounds__(256) router_topk_reg_kernel(const T* logp, int
       }
       filled += __popc(bal);
       nties += __popc(beq);
+    };
+    if constexpr (CPL > 0) {
+#pragma unroll
+      for (int j = 0; j < CPL; ++j)
+        if (32 * j < C) emit(32 * j + lane < C, csr[j], [&] { return pqr[j]; });
+    } else {
+      for (int base = 0; base < C; base += 32) {
+        const int c = base + lane;
+        emit(c < C, (c < C) ? cs[c] : 0u, [&] { return pq[c]; });
+      }
     }
     int need = k - filled;
 
@@ -750,8 +780,8 @@ RouterRegLayout make_reg_layout(int nk, int k) {
 //
 // Bound by one token's chain of dependent instructions (about 24000 cycles at 128 keys, top-64, with seven warps per
 // scheduler) and, with more than 8 keys per lane, by instruction fetch.  us, both halves sorted whole -> this kernel:
-// 16384 x 512 keys top-128 319 -> 214; 8192 x 1024 top-64 349 -> 106; 131072 x 256 top-32 638 -> 396; 4096 x 128 top-64
-// 19.2 -> 20.3; one token 8.2 -> 7.5.  Measured and not kept: cell numbers first and keys in a second loop (214 -> 224),
+// 16384 x 512 keys top-128 319 -> 214; 8192 x 1024 top-64 349 -> 106; 131072 x 256 top-32 558 -> 358; 4096 x 128 top-64 the
+// same (17.5); one token 7.8 -> 7.2.  Measured and not kept: cell numbers first and keys in a second loop (214 -> 224),
 // one sort per list or both lists at once (the same), candidates walked in shared memory for top-64 too (396 -> 444).
 // ------------------------------------------------------------------------------------------
 struct RouterPrunedLayout {
@@ -1309,11 +1339,11 @@ int launch_pruned(const void* logp, int64_t T_, int nk, int k, void* scores, int
   return launch_pruned_cpl<T, E, 22>(logp, T_, nk, k, L, scores, indices, gates, norm, stream);
 }
 
-template <typename T, int E>
+template <typename T, int E, int CPL = 0>
 int launch_reg(const void* logp, int64_t T_, int nk, int k, const RouterRegLayout& L, int warps, void* scores,
                int64_t* indices, void* gates, int norm, cudaStream_t stream) {
   const int smem = L.cta_bytes + warps * L.warp_bytes;
-  auto kern = router_topk_reg_kernel<T, E>;
+  auto kern = router_topk_reg_kernel<T, E, CPL>;
   FMOE_CUDA_TRY(allow_smem(kern, smem));
   if (norm & kTopkLateWait) FMOE_CUDA_TRY(prefer_smem(kern));
   int per_sm = 1;
@@ -1385,8 +1415,16 @@ int launch_typed(const void* logp, int64_t T_, int nk, int k, void* scores, int6
                  cudaStream_t stream) {
   if constexpr (sizeof(T) == 2) {
     // Not where there is little to drop: one key per lane (20000 x 32 keys top-4: 27 us, 32 pruned), or more than half of a
-    // short row wanted (4096 x 128 top-128: 30 us, 33 pruned).
-    const bool prune = nk > 32 && (nk > 128 || 2 * k <= nk);
+    // short row wanted (4096 x 128 top-128: 30 us, 33 pruned; 16384 x 100 top-70 69, 73).
+    // Of rows of 65 to 128 keys with the candidates in registers (k of 35 to 71), the whole sort takes fewer instructions in
+    // all and the pruned one a shorter chain per token, so the first is faster once the tokens are more than one wave of the
+    // pruned one (28 warps per SM): whole and pruned, 16384 x 128 top-64 52.9 and 63.9 us, top-40 52.5 and 57.5; 4700 x 128
+    // top-64 17.8 and 22.3; 4096 17.5 and 17.6, top-40 17.4 and 16.2; 64 tokens 8.1 and 7.8.  Beside a GEMM the pruned one's
+    // smaller shared memory counts whatever the number of tokens (layer of 4096 tokens, 128 keys, top-64: 209.8 and 205.2).
+    const int cells = make_pruned_layout(nk, k).C;
+    const bool many = nk > 64 && nk <= 128 && cells > 128 && cells <= 320 && !(norm & kTopkLateWait) &&
+                      T_ > static_cast<int64_t>(device_sm_count()) * 28;
+    const bool prune = nk > 32 && (nk > 128 || 2 * k <= nk) && !many;
     if (nk <= 1024 && k <= kPrunedMaxK && prune) {
       switch ((next_pow2(nk) < 32 ? 32 : next_pow2(nk)) / 32) {
         case 2: return launch_pruned<T, 2>(logp, T_, nk, k, scores, indices, gates, norm, stream);
@@ -1407,7 +1445,11 @@ int launch_typed(const void* logp, int64_t T_, int nk, int k, void* scores, int6
       switch (L.nkp / 32) {
         case 1: return launch_reg<T, 1>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
         case 2: return launch_reg<T, 2>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
-        case 4: return launch_reg<T, 4>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
+        case 4:
+          if constexpr (sizeof(T) == 2)  // 16384 x 100 keys top-70: 72.6 us with the candidates in shared memory, 68.8 in registers
+            if (L.C > 128 && L.C <= 320)
+              return launch_reg<T, 4, 10>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
+          return launch_reg<T, 4>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
         case 8: return launch_reg<T, 8>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
         case 16: return launch_reg<T, 16>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);
         case 32: return launch_reg<T, 32>(logp, T_, nk, k, L, warps, scores, indices, gates, norm, stream);

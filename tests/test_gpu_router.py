@@ -166,3 +166,23 @@ def test_router_pruned_rows(T, nk, k, dtype, scale):
     got_s, got_i = run_router(lp, nk, k)
     assert torch.equal(got_s.float(), want_s.float())
     assert torch.equal(got_i, want_i)
+
+
+@pytest.mark.parametrize("nk,k", [(65, 36), (72, 60), (100, 50), (100, 71), (128, 40), (128, 64), (128, 72)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_router_in_more_than_one_wave(nk, k, dtype):
+    """The kernel may change with the number of tokens, the result of a token does not: 65 to 128 keys, both sides of the
+    number of candidates that stay in registers, ordinary rows and rows full of ties, more tokens than are resident at once
+    against the same tokens in small batches and, for some of them, against the oracle."""
+    T = 6001
+    lp = torch.log_softmax(randn((2, T, nk), nk * k, torch.float32), -1)
+    lp[:, ::3] = torch.round(lp[:, ::3] * 2) / 2
+    lp[0, 9, 3] = float("-inf")
+    lp[1, 12] = float("-inf")
+    lp = lp.to(dtype).contiguous()
+    got_s, got_i = run_router(lp, nk, k)
+    for t0 in (0, 1000, T - 500):
+        s, i = run_router(lp[:, t0:t0 + 500], nk, k)
+        assert torch.equal(s.float(), got_s[t0:t0 + 500].float()) and torch.equal(i, got_i[t0:t0 + 500])
+    want_s, want_i = O.router_topk(lp[:, :200].contiguous(), nk, k)
+    assert torch.equal(got_s[:200].float(), want_s.float()) and torch.equal(got_i[:200], want_i)
