@@ -81,9 +81,9 @@ def run_expert_backward(x, d, u, idx, gates, dout):
     "T,H,N,k,dtype,zipf",
     [
         (5, 8, 7, 1, torch.float32, False),
-        (64, 72, 50, 3, torch.float32, False),      # sorted schedule, ragged column block
+        (64, 72, 50, 3, torch.float32, False),      # ragged column block
         (300, 256, 64, 8, torch.float32, True),     # hot experts: rows assembled from several chunk partials
-        (128, 64, 4096, 4, torch.bfloat16, False),  # token-centric schedule, most experts untouched
+        (128, 64, 4096, 4, torch.bfloat16, False),  # most experts untouched
         (512, 1280, 96, 16, torch.bfloat16, True),  # two column blocks, hot experts
         (200, 128, 33, 6, torch.float16, True),
         (2048, 1024, 16384, 16, torch.bfloat16, False),
@@ -185,7 +185,7 @@ def test_layer_backward_bf16_runs_and_no_grad_path_is_unchanged():
 
 
 def test_training_step_replays_from_a_cuda_graph():
-    """Forward + backward of the layer captured as one CUDA graph (every launch of the library, the stable sort
+    """Forward + backward of the layer captured as one CUDA graph (every launch of the library, the ordering of the pairs
     included, is capturable): replayed gradients are bit-equal to the eager step's."""
     from flash_moe_b200 import FlashMoE, FlashMoEConfig, check_status
 

@@ -88,7 +88,7 @@ def test_expert_out_of_range_ids_are_skipped_and_flagged():
     want = O.expert_forward(x, d, u, bad.clamp(0, N - 1), g2)
     assert O.rel_rms_error(got.cpu(), want) < 1e-4
     assert read_status() == 0
-    # -1 alone is the empty-slot value: skipped without raising the flag, in both dtypes' schedules
+    # -1 alone is the empty-slot value: skipped without raising the flag, in both dtypes' kernels
     for dtype in (torch.bfloat16, torch.float32):
         x, d, u, idx, gates = expert_inputs(T, H, N, k, dtype, seed=2)
         empty = idx.clone()

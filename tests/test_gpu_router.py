@@ -51,8 +51,8 @@ def test_router_topk_matches_reference_kernel_fixture(golden_dir, name):
 @pytest.mark.parametrize("T,nk,k", [(16, 64, 32), (8, 128, 64), (8, 256, 32), (6, 512, 16)])
 def test_router_heavy_ties_and_infinities(T, nk, k):
     """Log-probabilities on a grid of 0.5: hundreds of candidates tie with the threshold (short tie lists ranked by
-    shuffles, long ones by the bitwise search, overflowing ones by the per-row search), at shapes that keep the
-    candidates in shared memory (64 keys) and in registers (128 and more keys)."""
+    shuffles, long ones by the bitwise search, overflowing ones by the per-row search), float32 through the kernel that sorts
+    whole rows and 16-bit through the one that drops keys."""
     lp = torch.round(randn((2, T, nk), 3) * 2) / 2 - 3.0
     lp[0, 0, :] = -1.0  # a whole half tied
     lp[1, 1, :] = float("-inf")  # every sum is -inf for this token

@@ -41,8 +41,8 @@ def test_mlp_float32_tiles(T, H, I):
 )
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_mlp_few_tokens(T, H, I, dtype):
-    """Weight-row tiles of 64 and 128 rows, 1 to 256 token columns, K unsplit and split over 2, 4 and 8 CTAs; with the
-    addend, and the pre-activations kept for the backward."""
+    """Weight-row tiles of 64 and 128 rows, 16 to 256 token columns, remainders in every dimension; with the addend, and the
+    pre-activations kept for the backward."""
     from flash_moe_b200 import check_status
     from flash_moe_b200.ops.flash_mlp import _mlp_forward, flash_mlp_add
 

@@ -44,8 +44,7 @@ def _call(fn_name, tensors, T, H, N, k, dtype, with_workspace):
     return rc, out
 
 
-# the first shape takes the gather-per-token schedule, the second (float32) the expert-centric
-# sort whose counters live in the scratch and must be re-zeroed by every call
+# one shape for each scores kernel: 16-bit and float32
 @pytest.mark.parametrize("T,H,N,k,dtype", [(256, 512, 2048, 16, torch.bfloat16), (192, 256, 4096, 8, torch.float32)])
 def test_static_scratch_entry_point_matches_workspace_entry_point(T, H, N, k, dtype):
     from flash_moe_b200 import _lib
