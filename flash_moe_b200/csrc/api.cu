@@ -468,13 +468,16 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   // token in registers), which saves a [2, T, nk] round trip and a serial GEMM epilogue.
   const bool topk_from_logits = is16(dtype) && nk <= 1024;
   // The gate/up GEMM needs nothing from the router and the top-k only the logits, so the two run beside each other, the GEMM
-  // first, so that the top-k's many small CTAs fill what it leaves.  In a graph, one after the other -> now: 777 x 1000 float16
-  // 68 -> 63 us, 131072 tokens of the decoder layer 11.5 -> 10.6 ms.  A caller that asks for stage events gets the stages one
-  // by one.
+  // first, so that the top-k's many small CTAs fill what it leaves.  One after the other -> now: 777 x 1000 float16 73.0 ->
+  // 65.5 us, the default layer at 4096 tokens 205.4 -> 203.6, four decoder blocks of 16384 tokens 6297 -> 6179; at 131072
+  // tokens no difference beyond the 1 % that runs of one side differ by.  A caller that asks for stage events gets the stages
+  // one by one.
   const bool up_beside = (s2 == nullptr || s2 == s) && !a->training && topk_from_logits && a->stage_events == nullptr &&
                          mlp_up_on_tensor_cores(a->x, a->gate_proj, a->up_proj, dtype, T, H, I);
   // Few tokens: the whole shared MLP goes in front of the expert passes, which add its float32 output.  Router GEMM beside the
-  // gate/up GEMM, top-k beside the down GEMM; each of these kernels also outlasts the one before it.
+  // gate/up GEMM, top-k beside the down GEMM; each of these kernels also outlasts the one before it.  Against the order for
+  // more tokens: 1 token of the default layer 34.5 -> 30.0 us, 64 tokens of the decoder layer from a graph 63.0 -> 51.0.  As
+  // long as the gate/up GEMM leaves SMs for the top-k's CTAs; beyond, the down GEMM would run without anything beside it.
   const bool mlp_first = up_beside && k > 0 && mlp_up_is_narrow(a->x, a->gate_proj, a->up_proj, dtype, T, H, I) &&
                          (T + 3) / 4 + narrow_swiglu_ctas(T, I, H) <= device_sm_count() && aligned16(a->y) &&
                          aligned16(a->down_embed) && aligned16(a->up_embed) && aligned16(a->down_proj) &&
@@ -542,11 +545,9 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
     return launch_expert_forward_adding(a->x, a->down_embed, a->up_embed, indices, gates, static_cast<const float*>(w.acc),
                                         a->residual, a->y, dtype, T, H, N, k, w.expert, w.expert_bytes, a->status, s);
   // The side stream is joined HERE, before the experts: the two gather passes compete with the GEMM for the same
-  // L2 -> SM bandwidth and are slower beside it than after it.  (Measured at the benchmark shape the fork does not
-  // pay either way - 230 vs 226 us: the top-k's CTAs fill the shared memory first and the GEMM's wait for them; with
-  // the top-k held to one CTA per SM so that the GEMM fits beside it, the top-k itself takes 165 us, because one
-  // token costs a warp about 20 us of dependent instructions and all 4096 tokens must be resident at once; and with
-  // the GEMM's ring cut to four stages, so that four top-k CTAs fit beside it, the step takes 224 against 216 us.)
+  // L2 -> SM bandwidth and are slower beside it than after it.  (At the benchmark shape the fork does not pay, 230 against
+  // 226 us when it was measured: the top-k's CTAs take the shared memory first and the GEMM's wait for them.  On one stream
+  // the GEMM goes first, above.)
   bool joined = up_beside;
   if (fj != nullptr) {
     if (cudaStreamWaitEvent(s, fj->join, 0) != cudaSuccess) return fail(-static_cast<int>(cudaErrorUnknown));
@@ -579,7 +580,8 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
   }
   // y = h Wd^T + experts, one rounding
   FMOE_MARK(FMOE_STAGE_MLP_DOWN, 0, s);
-  // With the gate/up GEMM in front of the top-k, h is complete before the expert passes start: the down GEMM runs beside them up to its epilogue, 1 token in a graph 29.4 -> 26.7 us, 64 tokens 54 -> 53.
+  // With the gate/up GEMM in front of the top-k, h is complete before the expert passes start: a narrow down GEMM runs beside
+  // them up to its epilogue.
   rc = mlp_down(w.h, a->down_proj, static_cast<const float*>(w.acc), a->y, dtype, T, H, I, a->status, s, a->residual,
                 up_beside && k > 0);
   if (rc != FMOE_OK) return fail(rc);

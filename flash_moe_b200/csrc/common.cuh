@@ -253,7 +253,7 @@ int launch_gemm_swiglu_pair(const void* x, const void* gate_w, const void* up_w,
 int launch_gemm_add_pair(const void* a, const void* b, const float* addend, void* out, int dtype, int64_t M, int N,
                          int K, int32_t* status, cudaStream_t stream, const void* residual = nullptr);
 
-// the same two GEMMs for few tokens (gemm_sm100_narrow.cu): weight rows on the MMA's 128 rows, K split over a cluster.
+// the same two GEMMs for few tokens (gemm_sm100_narrow.cu): weight rows on the MMA's 64 or 128 rows, K unsplit.
 // early: kEarlyWeights - the kernel before this one in the stream is one of a forward's, so the weights cannot be written
 // any more and may be requested before it has finished; kEarlyTokens - the token rows are complete too (at most the addend
 // comes from that kernel), and everything up to the epilogue runs beside it; the next kernel starts when that one has ended.

@@ -195,9 +195,9 @@ class FlashMoE(nn.Module):
         """(y[B,S,H], router_logits[2, B*S, num_keys]) like the reference.
 
         With autograd off (``torch.no_grad()`` / inference mode, or nothing that requires grad) one fused library
-        call runs the whole layer.  When a graph is being recorded the layer is composed of the three
-        differentiable ops with torch's batch-norm, linear and log-softmax around them, exactly like the
-        reference's forward (flash_moe/modules/flash_moe.py:55-105), so ``backward()`` works.
+        call runs the whole layer.  When a graph is being recorded, torch's batch-norm is followed by one autograd node
+        for everything behind it (training.py) or, where that does not apply, by the three differentiable ops with
+        torch's linear and log-softmax around them like the reference's forward (flash_moe/modules/flash_moe.py:55-105).
 
         ``bn_sync_group``: a torch.distributed process group over which the tokens are sharded.  In
         training mode the router batch-norm then uses the statistics of the whole (global) batch: the
