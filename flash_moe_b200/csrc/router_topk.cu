@@ -1421,9 +1421,11 @@ int launch_typed(const void* logp, int64_t T_, int nk, int k, void* scores, int6
     // pruned one (28 warps per SM): whole and pruned, 16384 x 128 top-64 52.9 and 63.9 us, top-40 52.5 and 57.5; 4700 x 128
     // top-64 17.8 and 22.3; 4096 17.5 and 17.6, top-40 17.4 and 16.2; 64 tokens 8.1 and 7.8.  Beside a GEMM the pruned one's
     // smaller shared memory counts whatever the number of tokens (layer of 4096 tokens, 128 keys, top-64: 209.8 and 205.2).
-    const int cells = make_pruned_layout(nk, k).C;
-    const bool many = nk > 64 && nk <= 128 && cells > 128 && cells <= 320 && !(norm & kTopkLateWait) &&
-                      T_ > static_cast<int64_t>(device_sm_count()) * 28;
+    bool many = nk > 64 && nk <= 128 && !(norm & kTopkLateWait) && T_ > static_cast<int64_t>(device_sm_count()) * 28;
+    if (many) {
+      const int cells = make_pruned_layout(nk, k).C;
+      many = cells > 128 && cells <= 320;
+    }
     const bool prune = nk > 32 && (nk > 128 || 2 * k <= nk) && !many;
     if (nk <= 1024 && k <= kPrunedMaxK && prune) {
       switch ((next_pow2(nk) < 32 ? 32 : next_pow2(nk)) / 32) {

@@ -11,8 +11,11 @@ def contiguous(t):
     return t.contiguous() if isinstance(t, torch.Tensor) else t
 
 
+_grad_enabled, _tracing = torch.is_grad_enabled, torch._C._is_tracing
+
+
 def plain_call() -> bool:
     """True where an op may run without its autograd node, which costs several microseconds of host time: no gradient is
     recorded, no forward-mode level is open (the node is what refuses tangents, which would be dropped silently) and
     torch.jit is not tracing (the node is what a trace records)."""
-    return not torch.is_grad_enabled() and forward_ad._current_level < 0 and torch._C._get_tracing_state() is None
+    return not _grad_enabled() and forward_ad._current_level < 0 and not _tracing()
