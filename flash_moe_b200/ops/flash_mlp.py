@@ -29,7 +29,7 @@ def _mlp_forward(x, gate_weight, up_weight, down_weight, addend=None, save_preac
     ws_bytes = L.fmoe_mlp_workspace_bytes(T, H, I, code)
     ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dev)
     if save_preacts and addend is None and T > 0:
-        # the fused gate/up GEMM can also store the two pre-activations (its CTA-pair form only)
+        # the fused gate/up GEMMs can also store the two pre-activations; the general one refuses
         a = torch.empty((T, I), device=dev, dtype=x2.dtype)
         b = torch.empty((T, I), device=dev, dtype=x2.dtype)
         rc = _lib.call("fmoe_mlp_forward_saving_preacts", dev, x2.data_ptr(), wg.data_ptr(), wu.data_ptr(), wd.data_ptr(),

@@ -248,8 +248,8 @@ int fmoe_mlp_forward(const void* x, const void* gate_w, const void* up_w, const 
 /*
  * fmoe_mlp_forward that also keeps the two pre-activations pre_gate = x Wg^T and pre_up = x Wu^T ([T, I] of `dtype`),
  * the tensors the reference's TritonSwiGLUFunc saves for its backward (flash_moe/ops/triton/flash_mlp.py:150-156).
- * They are written by the epilogue of the fused gate/up GEMM, which only its CTA-pair form supports: 16-bit dtypes,
- * T >= 512, I >= 256, H >= 256 - other shapes return FMOE_ERR_UNSUPPORTED (callers then recompute in the backward).
+ * They are written by the epilogue of the fused gate/up GEMM: 16-bit dtypes with H and I multiples of 8, float32 with H a
+ * multiple of 4, operands 16-byte aligned - other calls return FMOE_ERR_UNSUPPORTED (callers then recompute in the backward).
  */
 int fmoe_mlp_forward_saving_preacts(const void* x, const void* gate_w, const void* up_w, const void* down_w,
                                     void* out, void* pre_gate, void* pre_up, int dtype, int64_t num_tokens, int hidden,
