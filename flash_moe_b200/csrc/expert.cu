@@ -422,6 +422,34 @@ __device__ __forceinline__ void ffma2(uint64_t& acc, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
+// The columns from col0 of one token, slot by slot and without the absent ones: the rare case of the kernel below, apart so
+// that its registers and loads do not weigh on that one's loop.  Same sums in the same order.
+template <typename T, typename OutT, int NCH, bool PEER>
+__device__ __noinline__ void accum_present_slots(const T* up, const int64_t* idx, const float* gs, OutT* out, int64_t t, int col0,
+                                                 int H, int64_t N, int k, const T* const* shards, int world, int64_t sharded) {
+  constexpr int VEC = Vec16<T>::N;
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int c = 0; c < NCH; ++c) {
+    const int col = col0 + (c * 32 + lane) * VEC;
+    if (col >= H) continue;
+    float acc[VEC] = {};
+#pragma unroll 1
+    for (int j = 0; j < k; ++j) {
+      const int64_t e = idx[t * k + j];
+      if (e < 0 || e >= N) continue;
+      const float w = gs[t * k + j];
+      float f[VEC];
+      unpack16<T>(ldg16(table_row<T, PEER>(up, shards, world, e, H, sharded) + col), f);
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) acc[i] = fmaf(f[i], w, acc[i]);
+    }
+    OutT* o = out + t * H + col;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) o[i] = from_f32<OutT>(acc[i]);
+  }
+}
+
 template <typename T, typename OutT, int NCH, bool PEER = false>
 __global__ void __launch_bounds__(128, 4) expert_accum_kernel(const T* __restrict__ up, const int64_t* idx,
                                                           const float* gs, OutT* __restrict__ out,
@@ -437,10 +465,10 @@ __global__ void __launch_bounds__(128, 4) expert_accum_kernel(const T* __restric
   const int64_t tasks = ntok * colblocks;
   // each lane fetches one slot's (expert id, weight) - one batch of 32 slots AHEAD of the batch being gathered,
   // also across tasks, so that the gathers of a batch never wait for their own ids; invalid or absent slots get
-  // weight 0
+  // weight -0, which adds nothing and marks them
   auto fetch_slot = [&](int64_t t_, int j0_, int& e_, float& w_) {
     e_ = 0;
-    w_ = 0.f;
+    w_ = -0.f;
     const int j = j0_ + lane;
     if (j < k) {
       const int64_t e = idx[t_ * k + j];
@@ -467,12 +495,14 @@ __global__ void __launch_bounds__(128, 4) expert_accum_kernel(const T* __restric
 #pragma unroll
       for (int i = 0; i < VEC / 2; ++i) acc[c][i] = 0ull;
 
+    bool some_absent = false;
     for (int j0 = 0; j0 < k; j0 += 32) {
       const int e_l = e_next;
       const float w_l = w_next;
       if (j0 + 32 < k) fetch_slot(t, j0 + 32, e_next, w_next);
       else if (task + warps_total < tasks) fetch_slot((task + warps_total) / colblocks, 0, e_next, w_next);
       const int nslots = min(32, k - j0);
+      some_absent |= __any_sync(kFull, lane < (nslots + SLOTS - 1) / SLOTS * SLOTS && __float_as_uint(w_l) == 0x80000000u);
       auto load = [&](uint4 (&q)[SLOTS][NCH], uint64_t (&ww)[SLOTS], int s) {
 #pragma unroll
         for (int u = 0; u < SLOTS; ++u) {
@@ -501,6 +531,22 @@ __global__ void __launch_bounds__(128, 4) expert_accum_kernel(const T* __restric
         uint64_t ww[SLOTS];
         load(q, ww, s);
         consume(q, ww);
+      }
+    }
+    // Absent slots above read row 0 with weight 0, and that product is not 0 where the row is not finite: a sum that is not
+    // finite is then formed again from the present slots alone.  (Leaving the loads out above makes the sums wait for all of them:
+    // both passes of 32768 tokens x 2048, top-16, 392 -> 450 us.)
+    if (some_absent) {
+      uint64_t check = 0ull;
+#pragma unroll
+      for (int c = 0; c < NCH; ++c)
+#pragma unroll
+        for (int i = 0; i < VEC / 2; ++i) ffma2(check, acc[c][i], 0ull);
+      float lo, hi;
+      unpack_f32x2(check, lo, hi);
+      if (__any_sync(kFull, !(lo + hi == 0.f))) {
+        accum_present_slots<T, OutT, NCH, PEER>(up, idx, gs, out, t, col0, H, N, k, shards, world, sharded);
+        continue;
       }
     }
     OutT* orow = out + t * H + col0;
@@ -557,13 +603,13 @@ __global__ void __launch_bounds__(32 * W) expert_accum_split_kernel(const T* __r
       // ids and rows are read past the L1 cache: an early CTA may find lines of an earlier forward there
       const int64_t e = j < k ? __ldcg(reinterpret_cast<const long long*>(idx) + t * k + j) : -1;
       const bool ok = e >= 0 && e < N;
-      const int row = ok ? static_cast<int>(e) : 0;
+      const int row = ok ? static_cast<int>(e) : -1;  // -1: nothing is read
       uint4 q[SLOTS];
 #pragma unroll
       for (int u = 0; u < SLOTS; ++u) {
         const int r = __shfl_sync(kFull, row, u);
-        q[u] = in ? __ldcg(reinterpret_cast<const uint4*>(table_row<T, PEER>(up, shards, world, r, H, sharded) + col0 + lane * VEC))
-                  : make_uint4(0, 0, 0, 0);
+        q[u] = in && r >= 0 ? __ldcg(reinterpret_cast<const uint4*>(table_row<T, PEER>(up, shards, world, r, H, sharded) + col0 + lane * VEC))
+                            : make_uint4(0, 0, 0, 0);
       }
       if (!waited) {
         pdl_wait();

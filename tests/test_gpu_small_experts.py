@@ -81,3 +81,28 @@ def test_a_token_alone_has_the_bits_it_has_in_a_batch(H, N, dtype):
     for rows in (slice(5, 6), slice(800, 801), slice(100, 140)):
         few, few_scores = _expert_forward(x[rows], d, u, idx[rows], gates[rows], torch.float32, save_scores=True)
         assert torch.equal(few_scores, scores[rows]) and torch.equal(few, out[rows])
+
+
+@pytest.mark.parametrize("T,k", [(5, 3), (64, 20), (1200, 20), (1200, 33)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_a_row_that_nobody_selects_has_no_effect(T, k, dtype):
+    """Slots beyond top-k, empty slots and out-of-range ids read no row: infinities and NaN in the first rows of the tables
+    reach only the tokens that select them."""
+    from flash_moe_b200 import _lib
+    from flash_moe_b200.ops.flash_expert import _expert_backward, flash_expert_fp32
+
+    N, H = 300, 264
+    x, d, u, dout = (randn(shape, s, dtype).cuda() for shape, s in (((T, H), 1), ((N, H), 2), ((N, H), 3), ((T, H), 4)))
+    gen = torch.Generator().manual_seed(k)
+    idx = torch.randint(2, N, (T, k), generator=gen)
+    idx[1, 0], idx[2, -1], idx[3, 0] = -1, N, 0
+    idx = idx.cuda()
+    gates = torch.rand(T, k, generator=gen).to(dtype).cuda()
+    want, grads = flash_expert_fp32(x, d, u, idx, gates), _expert_backward(dout, x, d, u, idx, gates)
+    for t in (d, u):
+        t[0], t[1] = float("inf"), float("nan")
+    got, bad = flash_expert_fp32(x, d, u, idx, gates), _expert_backward(dout, x, d, u, idx, gates)
+    others = torch.arange(T, device="cuda") != 3
+    assert torch.equal(got[others], want[others]) and torch.equal(bad[0][others], grads[0][others])
+    assert not torch.isfinite(got[3]).any()
+    _lib.read_status()
