@@ -132,43 +132,57 @@ __device__ __forceinline__ const T* table_row(const T* table, const T* const* sh
   }
 }
 
-// One warp per (token, group of 16 of its experts).  The token's x row is parked in the warp's
-// slice of shared memory (read back as B fragments right before each MMA; fetched with cp.async one task ahead,
-// together with the next task's expert ids), so every register that
-// waits for data waits for a gathered down row: batches of UNROLL 32-column blocks (2 * UNROLL x 16 B per lane) in
-// two register buffers keep gathers in flight across batches to cover the L2 latency (measured at the
-// benchmark shape: 4 x 2 buffers 57.7 us, 8 x 1 61.9 us, 4 x 3 62.6 us, 2 x 2 57.8 us).
-template <typename T, int UNROLL, bool PEER, int COLS, bool LOAD32 = false>
-__global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* x, const T* __restrict__ down,
-                                                               const int64_t* idx, const T* gates, float* __restrict__ gs,
-                                                               int64_t ntok, int H, int64_t N, int k, int xs_stride,
-                                                               int32_t* status, int act,
-                                                               const T* const* __restrict__ shards = nullptr,
-                                                               int world = 1, float* __restrict__ raw_out = nullptr,
-                                                               int64_t sharded = 0) {
+// One warp per (token, group of 16 of its experts).  The token's x row is parked in the warp's slice of shared memory (read back
+// as B fragments right before each MMA; fetched with cp.async one task ahead, together with the next task's expert ids), so
+// every register that waits for data waits for a gathered down row: batches of 128 columns (8 x 16 B per lane) in two register
+// buffers keep gathers in flight across batches to cover the L2 latency.
+//
+// Tables beyond what L2 keeps are walked in slabs of columns, every task of a slab before the next slab; the sums so far wait
+// in gs, where the thread that stored them takes them up again (same order of columns, same bits).  Gathers from a slab that
+// fits L2 run at up to 18 TB/s, from 256 MiB at 9.7 (loads alone): 131072 tokens x 2048, 2^16 experts, top-32 1945 -> 1560 us.
+//
+// Bound by the L1's data path: a load takes 64 bytes of each of eight rows, eight of its cycles for 512 bytes, and the x
+// fragments as much again for each fourth load.  Measured and not kept at 4096 x 1024, top-64 (52 us): whole lines per load and
+// an exchange between lanes (56), whole lines and sums handed from lane to lane between the halves of a line (twice the MMAs:
+// 56; rows as B: 71), rows as B and the token as A (twice the MMAs for no register moves: 53.7), 32 rows per fragment (54).
+template <typename T, bool PEER, int COLS, bool LOAD32 = false>
+__global__ void __launch_bounds__(128, 4) expert_scores_mma_kernel(const T* x, const T* __restrict__ down, const int64_t* idx,
+                                                                  const T* gates, float* gs, int64_t ntok, int H, int64_t N,
+                                                                  int k, int slab, int32_t* status, int act,
+                                                                  const T* const* __restrict__ shards, int world,
+                                                                  float* __restrict__ raw_out, int64_t sharded) {
   extern __shared__ uint4 xs_all[];
   pdl_wait();  // ids and gates come from the kernel before this one
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, tq = lane & 3;
-  // two x-row buffers per warp (xs_stride uint4 each, >= ceil(H/256)*32): while one task is computed, the next
-  // task's ids and x row are already on their way (cp.async), so a task does not start with an exposed round trip
+  const int xs_stride = (slab + 255) / 256 * 32;  // 16-byte pieces of an x row buffer, two per warp
   uint4* xs_buf = xs_all + (threadIdx.x >> 5) * 2 * xs_stride;
   const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   const int64_t warp_global = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  // the next task's first batch is requested before this task's last one is consumed (52.5 -> 51.5 us at 4096 tokens x 1024,
+  // top-64); with the wider loads or several tables that takes more registers than it gives
+  constexpr bool kCross = COLS == 8 && !PEER;
+  constexpr int UNROLL = 4, STEP = 32 * UNROLL;
   const int groups = (k + 15) >> 4;
   const int64_t tasks = ntok * groups;
-  const int hv = H >> 3;  // 16-byte pieces per row
+  if (warp_global >= tasks) return;
+  const bool lone = warp_global + warps_total >= tasks;  // one task: its partial sums stay in registers
+  // the slot whose sum this lane finishes
+  const int own = g + 8 * tq;  // tq < 2
   bool bad = false;
-  auto fetch_ids = [&](int64_t task_, int64_t& ea_, int64_t& eb_) {
-    const int64_t t_ = task_ / groups;
-    const int ja_ = static_cast<int>(task_ - t_ * groups) * 16 + g, jb_ = ja_ + 8;
-    ea_ = ja_ < k ? idx[t_ * k + ja_] : 0;
-    eb_ = jb_ < k ? idx[t_ * k + jb_] : 0;
+  int64_t e[2];
+  auto fetch_ids = [&](int64_t t_, int G_) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int j_ = G_ * 16 + g + 8 * i;
+      e[i] = j_ < k ? idx[t_ * k + j_] : -1;
+    }
   };
-  auto fetch_x = [&](int64_t t_, uint4* dst) {
-    const T* xr = x + t_ * H;
+  auto fetch_x = [&](int64_t t_, int col_, uint4* dst) {
+    const T* xr = x + t_ * H + col_;
+    const int pieces = min(slab, H - col_) >> 3;
     for (int c = lane; c < xs_stride; c += 32) {
-      if (c < hv) {
+      if (c < pieces) {
         asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst + c))),
                      "l"(reinterpret_cast<uint64_t>(xr + c * 8))
                      : "memory");
@@ -177,95 +191,131 @@ __global__ void __launch_bounds__(128) expert_scores_mma_kernel(const T* x, cons
       }
     }
   };
-  int cur = 0;
-  int64_t ea_next = 0, eb_next = 0;
-  if (warp_global < tasks) {
-    fetch_ids(warp_global, ea_next, eb_next);
-    fetch_x(warp_global / groups, xs_buf);
-  }
-  for (int64_t task = warp_global; task < tasks; task += warps_total) {
-    if (task + warps_total >= tasks) pdl_launch_dependents();  // last task of this warp: the next kernel may set up
-    const int64_t t = task / groups;
-    const int G = static_cast<int>(task - t * groups);
-    const int ja = G * 16 + g, jb = ja + 8;
-    const int64_t ea = ea_next, eb = eb_next;
-    const uint4* xs = xs_buf + cur * xs_stride;
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncwarp();  // this task's x row has landed; the other buffer is free (its task is finished)
-    if (task + warps_total < tasks) {
-      fetch_ids(task + warps_total, ea_next, eb_next);
-      fetch_x((task + warps_total) / groups, xs_buf + (cur ^ 1) * xs_stride);
-    }
-    cur ^= 1;
-    const bool oka = (ja < k) && ea >= 0 && ea < N;
-    const bool okb = (jb < k) && eb >= 0 && eb < N;
-    if ((ja < k && !oka && ea != -1) || (jb < k && !okb && eb != -1)) bad = true;  // -1: empty slot, no flag
-    const T* ra = table_row<T, PEER>(down, shards, world, oka ? ea : 0, H, sharded) + 8 * tq;
-    const T* rb = table_row<T, PEER>(down, shards, world, okb ? eb : 0, H, sharded) + 8 * tq;
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
-    // COLS = 16: a lane takes 16 consecutive columns of a 64-column block, so that the four lanes of a row cover a whole
-    // 128-byte line, in one 32-byte load (LOAD32) each.  Two 16-byte loads give the same sums for tables that are only
-    // 16-byte aligned, or whose alignment the host does not know (PEER).
-    auto load = [&](uint4 (&qa)[UNROLL], uint4 (&qb)[UNROLL], int c0) {
-      if constexpr (COLS == 16) {
+  const T* row[2];
+  auto rows_of = [&](int col_) {
 #pragma unroll
-        for (int u = 0; u < UNROLL; u += 2) {
-          const int col = c0 + 32 * u;
-          if (col + 16 * tq < H) {  // H % 16 == 0
+    for (int i = 0; i < 2; ++i)
+      row[i] = table_row<T, PEER>(down, shards, world, e[i] >= 0 && e[i] < N ? e[i] : 0, H, sharded) + col_ + COLS * tq;
+  };
+  struct Batch {
+    uint4 q[2][UNROLL];
+  };
+  // COLS = 8: lane tq has columns 8 tq .. 8 tq + 7 of each 32-column block u.  COLS = 16: columns 16 tq .. 16 tq + 15 of each
+  // 64-column block, so that the four lanes of a row cover a whole 128-byte line, in one 32-byte load (LOAD32) or, for tables
+  // that are only 16-byte aligned or whose alignment the host does not know (PEER), in two.
+  auto load = [&](Batch& b, int c0, int cols) {
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      if constexpr (COLS == 8) {
+        const bool in = c0 + 32 * u + 8 * tq < cols;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) b.q[i][u] = in ? ldg16(row[i] + c0 + 32 * u) : zero;
+      } else if ((u & 1) == 0) {
+        if (c0 + 32 * u + 16 * tq < cols) {  // H % 16 == 0
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
             if constexpr (LOAD32) {
-              ldg32(ra + col + 8 * tq, qa[u], qa[u + 1]);
-              ldg32(rb + col + 8 * tq, qb[u], qb[u + 1]);
+              ldg32(row[i] + c0 + 32 * u, b.q[i][u], b.q[i][u + 1]);
             } else {
-              qa[u] = ldg16(ra + col + 8 * tq);
-              qa[u + 1] = ldg16(ra + col + 8 * tq + 8);
-              qb[u] = ldg16(rb + col + 8 * tq);
-              qb[u + 1] = ldg16(rb + col + 8 * tq + 8);
+              b.q[i][u] = ldg16(row[i] + c0 + 32 * u);
+              b.q[i][u + 1] = ldg16(row[i] + c0 + 32 * u + 8);
             }
-          } else {
-            qa[u] = qa[u + 1] = qb[u] = qb[u + 1] = make_uint4(0, 0, 0, 0);
           }
-        }
-      } else {
-#pragma unroll
-        for (int u = 0; u < UNROLL; ++u) {
-          const int col = c0 + 32 * u;
-          const bool in = col + 8 * tq < H;
-          qa[u] = in ? ldg16(ra + col) : make_uint4(0, 0, 0, 0);
-          qb[u] = in ? ldg16(rb + col) : make_uint4(0, 0, 0, 0);
+        } else {
+          b.q[0][u] = b.q[0][u + 1] = b.q[1][u] = b.q[1][u + 1] = zero;
         }
       }
-    };
-    auto consume = [&](const uint4 (&qa)[UNROLL], const uint4 (&qb)[UNROLL], int c0) {
-#pragma unroll
-      for (int u = 0; u < UNROLL; ++u) {
-        const int piece = COLS == 16 ? ((c0 + 32 * (u & ~1)) >> 3) + 2 * tq + (u & 1) : ((c0 + 32 * u) >> 3) + tq;
-        const uint4 xq = piece < xs_stride ? xs[piece] : make_uint4(0, 0, 0, 0);
-        Mma16816<T>::run(c, qa[u].x, qb[u].x, qa[u].y, qb[u].y, xq.x, xq.y);
-        Mma16816<T>::run(c, qa[u].z, qb[u].z, qa[u].w, qb[u].w, xq.z, xq.w);
-      }
-    };
-    // two register buffers: the next batch of gathers is issued before the current one is consumed, so the loads in flight
-    // never drain between batches (same column order, hence the same sums)
-    constexpr int STEP = 32 * UNROLL;
-    uint4 a0[UNROLL], b0[UNROLL], a1[UNROLL], b1[UNROLL];
-    load(a0, b0, 0);
-    for (int c0 = 0; c0 < H; c0 += 2 * STEP) {
-      if (c0 + STEP < H) load(a1, b1, c0 + STEP);
-      consume(a0, b0, c0);
-      if (c0 + 2 * STEP < H) load(a0, b0, c0 + 2 * STEP);
-      if (c0 + STEP < H) consume(a1, b1, c0 + STEP);
     }
-    if (tq == 0) {
-      if (gates != nullptr) {
-        if (ja < k) gs[t * k + ja] = oka ? expert_act(c[0], act) * to_f32<T>(gates[t * k + ja]) : 0.f;
-        if (jb < k) gs[t * k + jb] = okb ? expert_act(c[2], act) * to_f32<T>(gates[t * k + jb]) : 0.f;
-        if (raw_out != nullptr) {  // pre-activation scores kept for the backward pass
-          if (ja < k) raw_out[t * k + ja] = oka ? c[0] : 0.f;
-          if (jb < k) raw_out[t * k + jb] = okb ? c[2] : 0.f;
+  };
+  float c[4] = {};
+  int cur = 0;
+  auto consume = [&](const Batch& b, int c0) {
+    const uint4* xs = xs_buf + cur * xs_stride + (c0 >> 3);
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      const uint4 xq = xs[COLS == 16 ? 4 * (u & ~1) + 2 * tq + (u & 1) : 4 * u + tq];
+      const uint4 &qa = b.q[0][u], &qb = b.q[1][u];
+      Mma16816<T>::run(c, qa.x, qb.x, qa.y, qb.y, xq.x, xq.y);
+      Mma16816<T>::run(c, qa.z, qb.z, qa.w, qb.w, xq.z, xq.w);
+    }
+  };
+
+  // (token, group) of tasks, stepped without divisions
+  const int64_t dt = warps_total / groups, t_first = warp_global / groups;
+  const int dG = static_cast<int>(warps_total - dt * groups), G_first = static_cast<int>(warp_global - t_first * groups);
+  int64_t t_next = t_first;
+  int G_next = G_first;
+  Batch b0, b1;
+  fetch_ids(t_first, G_first);
+  float part_next = 0.f;
+  fetch_x(t_first, 0, xs_buf);
+  rows_of(0);
+  load(b0, 0, min(slab, H));
+  for (int col = 0; col < H; col += slab) {
+    const int cols = min(slab, H - col);
+    const bool last_slab = col + slab >= H;
+    for (int64_t task = warp_global; task < tasks; task += warps_total) {
+      const bool last_task = task + warps_total >= tasks;
+      const bool more = !(last_slab && last_task);
+      if (!more) pdl_launch_dependents();  // the next kernel may set up
+      const int next_col = last_task ? col + slab : col;
+      const int64_t t = t_next;
+      const int j = G_next * 16;
+      if (last_task) {
+        t_next = t_first;
+        G_next = G_first;
+      } else {
+        t_next += dt;
+        if ((G_next += dG) >= groups) {
+          G_next -= groups;
+          ++t_next;
         }
-      } else {  // raw dot products (backward pass)
-        if (ja < k) gs[t * k + ja] = oka ? c[0] : 0.f;
-        if (jb < k) gs[t * k + jb] = okb ? c[2] : 0.f;
+      }
+      bool present = false;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const bool ok = e[i] >= 0 && e[i] < N;
+        bad |= !ok && e[i] != -1;  // -1: empty slot, no flag
+        if (tq == i) present = ok;
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();  // this task's x row has landed; the other buffer is free (its task is finished)
+      c[0] = c[2] = part_next;  // of this lane's sums that of its own slot counts
+      if (more) {
+        fetch_ids(t_next, G_next);
+        fetch_x(t_next, next_col, xs_buf + (cur ^ 1) * xs_stride);
+        part_next = 0.f;
+        if (next_col > 0 && !lone && tq < 2 && G_next * 16 + own < k) part_next = gs[t_next * k + G_next * 16 + own];
+      }
+      for (int c0 = 0; c0 < cols; c0 += 2 * STEP) {
+        const bool two = c0 + STEP < cols;
+        if (two) load(b1, c0 + STEP, cols);
+        consume(b0, c0);
+        if (c0 + 2 * STEP < cols) {
+          load(b0, c0 + 2 * STEP, cols);
+        } else if (kCross && more) {
+          rows_of(next_col);
+          load(b0, 0, min(slab, H - next_col));
+        }
+        if (two) consume(b1, c0 + STEP);
+      }
+      if (!kCross && more) {
+        rows_of(next_col);
+        load(b0, 0, min(slab, H - next_col));
+      }
+      cur ^= 1;
+      if (tq < 2 && j + own < k) {
+        const int64_t p = t * k + j + own;
+        const float v = tq == 0 ? c[0] : c[2];
+        if (!last_slab) {
+          if (lone) part_next = v;
+          else gs[p] = v;
+        } else {
+          const float s = present ? v : 0.f;
+          gs[p] = gates != nullptr && present ? expert_act(v, act) * to_f32<T>(gates[p]) : s;
+          if (raw_out != nullptr) raw_out[p] = s;
+        }
       }
     }
   }
@@ -410,6 +460,10 @@ __global__ void __launch_bounds__(128) expert_scores_f32_kernel(const float* x, 
 // per lane, packed f32x2 FMAs (two accumulators per instruction).  The launch bound keeps the kernel at 120
 // registers so that four CTAs (not three) fit an SM: a third more gathers in flight, 52 -> 48 us at the benchmark
 // shape (a fifth CTA would need spills and is slower: 120 vs 105 us for both passes).
+// The column blocks are the outer loop: all tokens gather from the same 512 columns of the table before the next ones, which
+// stay in L2 where the whole table does not (131072 tokens x 2048, 65536 experts top-32: 1960 -> 1400 us with the CTAs in
+// step).  Bound by the gathers in flight: loads alone reach 11 TB/s with as many as four such CTAs hold, 17 with eight.  Half of
+// the batches through shared memory by cp.async put more of them in flight and took longer all the same (48 -> 50 us).
 __device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -480,12 +534,25 @@ __global__ void __launch_bounds__(128, 4) expert_accum_kernel(const T* __restric
   };
   int e_next = 0;
   float w_next = 0.f;
-  if (warp_global < tasks) fetch_slot(warp_global / colblocks, 0, e_next, w_next);
+  int64_t t_next = warp_global;
+  int col_next = 0;
+  auto wrap = [&]() {
+    while (t_next >= ntok) {
+      t_next -= ntok;
+      col_next += 32 * VEC * NCH;
+    }
+  };
+  auto step = [&]() {
+    t_next += warps_total;
+    wrap();
+  };
+  wrap();
+  if (warp_global < tasks) fetch_slot(t_next, 0, e_next, w_next);
   for (int64_t task = warp_global; task < tasks; task += warps_total) {
     if (task + warps_total >= tasks) pdl_launch_dependents();  // last task of this warp: the next kernel may set up
-    const int64_t t = task / colblocks;
-    const int cb = static_cast<int>(task - t * colblocks);
-    const int col0 = cb * (32 * VEC * NCH);
+    const int64_t t = t_next;
+    const int col0 = col_next;
+    step();
     bool in[NCH];
 #pragma unroll
     for (int c = 0; c < NCH; ++c) in[c] = col0 + (c * 32 + lane) * VEC < H;
@@ -500,7 +567,7 @@ __global__ void __launch_bounds__(128, 4) expert_accum_kernel(const T* __restric
       const int e_l = e_next;
       const float w_l = w_next;
       if (j0 + 32 < k) fetch_slot(t, j0 + 32, e_next, w_next);
-      else if (task + warps_total < tasks) fetch_slot((task + warps_total) / colblocks, 0, e_next, w_next);
+      else if (task + warps_total < tasks) fetch_slot(t_next, 0, e_next, w_next);
       const int nslots = min(32, k - j0);
       some_absent |= __any_sync(kFull, lane < (nslots + SLOTS - 1) / SLOTS * SLOTS && __float_as_uint(w_l) == 0x80000000u);
       auto load = [&](uint4 (&q)[SLOTS][NCH], uint64_t (&ww)[SLOTS], int s) {
@@ -730,6 +797,23 @@ bool whole_lines(int64_t N, int H) {
   return H % 16 == 0 && N * H * static_cast<int64_t>(sizeof(T)) > (384ll << 20);
 }
 
+// Tables that do not stay in L2 (126 MB) are gathered from in slabs of 512 columns, both passes with exactly the CTAs that are
+// resident at once, so that all of them are at the same slab: 16384 tokens, both passes, 65536 experts x 2048 top-32 513 -> 396
+// us, 131072 x 2048 top-16 327 -> 267.  Up to 128 MiB slabs give nothing to the scores pass and cost it a round trip per task
+// (65536 x 1024: 112.3 and 112.7 us; 4096 tokens, 16384 x 1024 top-64: 51.8 and 55.1).  Of 2^20 experts no slab stays, the
+// scores pass only walks a row in two steps (32768 tokens x 2048 top-16: Zipf 1.1 ids 216 us in slabs of 512, 193 of 1024,
+// 187 whole; uniform ids 354, 350, 366).
+template <typename T>
+bool beyond_l2(int64_t N, int H) {
+  return N * H * static_cast<int64_t>(sizeof(T)) > (144ll << 20);
+}
+template <typename T>
+int slab_columns(int64_t N, int H) {
+  if (!beyond_l2<T>(N, H)) return H;
+  const int slab = N * 512 * static_cast<int64_t>(sizeof(T)) <= (256ll << 20) ? 512 : 1024;
+  return slab < H ? slab : H;
+}
+
 // the scores pass / accumulate pass for few tokens; false: not the shape for it (or, with `rc`, a launch error)
 template <typename T, bool PEER>
 bool try_scores_split(const void* rows, const void* table, const int64_t* idx, const void* gates, float* out, int64_t T_, int H,
@@ -781,7 +865,7 @@ void launch_accum(const void* up, const int64_t* idx, const float* gs, void* out
   const int colblocks = (H + 32 * VEC * NCH - 1) / (32 * VEC * NCH);
   const int64_t tasks = T_ * colblocks;
   const int64_t want = (tasks + 3) / 4;
-  const int64_t cap = static_cast<int64_t>(device_sm_count()) * 16;
+  const int64_t cap = static_cast<int64_t>(device_sm_count()) * (beyond_l2<T>(N, H) ? 4 : 16);
   const int grid = static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
   auto kern = expert_accum_kernel<T, OutT, NCH>;
   (void)launch_pdl(8, kern, dim3(grid), dim3(128), 0, stream, 1, static_cast<const T*>(up), idx, gs, static_cast<OutT*>(out), T_,
@@ -805,14 +889,14 @@ int run_scores(const void* rows, const void* table, const int64_t* idx, const vo
     // the next one's ids and x row already in flight, and the work ends evenly (53.7 vs 55.7 us with 16 per SM)
     const int64_t cap = static_cast<int64_t>(sms) * 4;
     const int grid = static_cast<int>(want < cap ? want : cap);
-    const int xs_stride = ((H + 255) / 256) * 32;  // uint4 per warp, rows padded to 256 columns
-    const int smem = 4 * 2 * xs_stride * 16;  // two x-row buffers per warp
+    const int slab = slab_columns<T>(N, H);
+    const int smem = 4 * 2 * ((slab + 255) / 256 * 32) * 16;  // two x-row buffers per warp
     const bool aligned32 = (reinterpret_cast<uintptr_t>(table) & 31u) == 0;
-    auto kern = !whole_lines<T>(N, H) ? expert_scores_mma_kernel<T, 4, false, 8>
-                : aligned32 ? expert_scores_mma_kernel<T, 4, false, 16, true> : expert_scores_mma_kernel<T, 4, false, 16>;
+    auto kern = !whole_lines<T>(N, H) ? expert_scores_mma_kernel<T, false, 8>
+                : aligned32 ? expert_scores_mma_kernel<T, false, 16, true> : expert_scores_mma_kernel<T, false, 16>;
     FMOE_CUDA_TRY(allow_smem(kern, smem));
     FMOE_CUDA_TRY(launch_pdl(4, kern, dim3(grid), dim3(128), smem, stream, 1, static_cast<const T*>(rows),
-                             static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, T_, H, N, k, xs_stride,
+                             static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, T_, H, N, k, slab,
                              status, act, nullptr, 1, raw_out, 0));
   } else {
     const int64_t want = (T_ * ((k + 3) / 4) + 3) / 4;
@@ -1222,12 +1306,11 @@ int run_typed_peer(const void* x, const void* const* down_shards, const void* co
       const int64_t want = (T_ * ((k + 15) / 16) + 3) / 4;
       const int64_t cap = static_cast<int64_t>(sms) * 16;
       const int grid = static_cast<int>(want < cap ? want : cap);
-      const int xs_stride = ((H + 255) / 256) * 32;
-      const int smem = 4 * 2 * xs_stride * 16;  // two x-row buffers per warp
-      auto kern = whole_lines<T>(N, H) ? expert_scores_mma_kernel<T, 4, true, 16> : expert_scores_mma_kernel<T, 4, true, 8>;
+      const int smem = 4 * 2 * ((H + 255) / 256 * 32) * 16;  // two x-row buffers per warp
+      auto kern = whole_lines<T>(N, H) ? expert_scores_mma_kernel<T, true, 16> : expert_scores_mma_kernel<T, true, 8>;
       FMOE_CUDA_TRY(allow_smem(kern, smem));
       kern<<<grid, 128, smem, stream>>>(static_cast<const T*>(x), static_cast<const T*>(hot_down), idx,
-                                        static_cast<const T*>(gates), w.gs, T_, H, N + hot_rows, k, xs_stride, status,
+                                        static_cast<const T*>(gates), w.gs, T_, H, N + hot_rows, k, H, status,
                                         kActSilu, reinterpret_cast<const T* const*>(down_shards), world, nullptr, N);
       FMOE_LAUNCH_CHECK();
     }

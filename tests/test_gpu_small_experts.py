@@ -83,6 +83,32 @@ def test_a_token_alone_has_the_bits_it_has_in_a_batch(H, N, dtype):
         assert torch.equal(few_scores, scores[rows]) and torch.equal(few, out[rows])
 
 
+@pytest.mark.parametrize("H,T,k", [(520, 430, 17), (1000, 1500, 17), (1024, 1500, 32), (1544, 801, 16)])
+def test_columns_in_slabs(H, T, k):
+    """Tables of more than 144 MiB are walked in slabs of 512 columns, the sums so far kept in registers (warps with one task)
+    or in memory: last slabs of 8, 488, 512 and 8 columns give the bits of the few-token kernels, which have no slabs, and the
+    float64 sums up to float32 rounding; empty slots stay empty."""
+    from flash_moe_b200.ops.flash_expert import _expert_forward
+
+    N = (150 << 20) // (2 * H)
+    gen = torch.Generator(device="cuda").manual_seed(H)
+    x, d, u = (torch.empty(rows, H, device="cuda", dtype=torch.bfloat16).normal_(0, std, generator=gen)
+               for rows, std in ((T, 0.5), (N, 0.1), (N, 1.0)))
+    idx = torch.randint(0, N, (T, k), device="cuda", generator=gen)
+    idx[::7, k // 2] = -1
+    gates = torch.rand(T, k, device="cuda", generator=gen).bfloat16()
+    out, scores = _expert_forward(x, d, u, idx, gates, torch.float32, save_scores=True)
+    for rows in (slice(0, 20), slice(T - 20, T)):
+        few, few_scores = _expert_forward(x[rows], d, u, idx[rows], gates[rows], torch.float32, save_scores=True)
+        assert torch.equal(few_scores, scores[rows]) and torch.equal(few, out[rows])
+    want = torch.zeros(T, H, dtype=torch.float64, device="cuda")
+    for j in range(k):
+        e = idx[:, j].clamp(min=0)
+        s = (x.double() * d[e].double()).sum(-1)
+        want += (torch.nn.functional.silu(s) * gates[:, j].double() * (idx[:, j] >= 0))[:, None] * u[e].double()
+    assert (out.double() - want).norm() <= 5e-6 * want.norm()
+
+
 @pytest.mark.parametrize("T,k", [(5, 3), (64, 20), (1200, 20), (1200, 33)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_row_that_nobody_selects_has_no_effect(T, k, dtype):
