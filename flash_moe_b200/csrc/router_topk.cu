@@ -269,7 +269,17 @@ template <typename T16> struct HalfKey16 {
   }
   static __device__ __forceinline__ uint32_t id(uint32_t k) { return 0xFFFFu - (k & 0xFFFFu); }
 };
-template <> struct HalfKey<__nv_bfloat16> : HalfKey16<__nv_bfloat16> {};
+template <> struct HalfKey<__nv_bfloat16> {  // the upper half of the float is the value: no conversions
+  using type = uint32_t;
+  static __device__ __forceinline__ uint32_t make(float v, uint32_t i) {
+    const uint32_t x = __float_as_uint(v);
+    return ((x ^ (static_cast<uint32_t>(static_cast<int32_t>(x) >> 31) | 0x80000000u)) & 0xFFFF0000u) | (0xFFFFu - i);
+  }
+  static __device__ __forceinline__ float value(uint32_t k) {
+    return __uint_as_float((k ^ (static_cast<int32_t>(k) < 0 ? 0x80000000u : 0xFFFFFFFFu)) & 0xFFFF0000u);
+  }
+  static __device__ __forceinline__ uint32_t id(uint32_t k) { return 0xFFFFu - (k & 0xFFFFu); }
+};
 template <> struct HalfKey<__half> : HalfKey16<__half> {};
 
 // One lane's E consecutive elements of a row (element lane * E + r -> v[r]); entries past nk read as -inf.  Whole
@@ -342,7 +352,6 @@ __device__ __forceinline__ void store_blocked(uint16_t* base, int lane, const ui
 }
 
 constexpr int kTieCap = 256;  // entries of the per-warp list of candidates that tie with tau
-constexpr int kPrunedTieCap = 80;  // smaller, so that three CTAs of 128 keys fit beside a gate/up GEMM CTA (32 KB left)
 
 struct RouterRegLayout {
   int cta_bytes, warp_bytes;
@@ -767,89 +776,40 @@ RouterRegLayout make_reg_layout(int nk, int k) {
 }
 
 // ------------------------------------------------------------------------------------------
-// 16-bit inputs, num_keys <= 1024, top_k <= 128: the same steps on the few keys that can matter.
+// 16-bit inputs, num_keys <= 1024, top_k <= 128: only the sums that can be among the k largest are ever formed.
 //
 //   1. The 32 lane maxima of each half, sorted (both halves in one packed 16-bit network), give a lower bound on the k-th
-//      largest sum: p maxima of the first half and ceil(k / p) of the second make at least k sums of at least
-//      A_p + B_ceil(k/p); the best p counts.
+//      largest sum: first the best rectangle (p maxima of one half and ceil(k / p) of the other make at least k sums of at
+//      least A_p + B_ceil(k/p)), then, by bisection, the largest value that k of the 32 x 32 sums reach.
 //   2. A key whose sum with the other half's maximum stays below the bound is dropped (a superset is kept where rounding
-//      or a non-finite value blurs the test).  What is left - 41 of 128 keys at top-64, 101 of 512 at top-128 for normal
-//      logits - is compacted in index order and sorted.
-//   3. Staircase sums, threshold, ties, winners as above; winners are 32-bit keys (level of the score above the threshold
-//      | inverted flat id) wherever the two fit.
+//      or a non-finite value blurs the test).  What is left - 25 of 128 keys at top-64, 56 of 512 at top-128 for normal
+//      logits; 41 and 105 with the rectangle alone - is compacted and sorted.
+//   3. Each row of the first half counts its sums at or above the bound by a binary search (they do not increase along a
+//      row).  Where there are at most 2 k in all - raising the bound by bisection if there are more - they are the only
+//      candidates: numbered through a running maximum over marks at the rows' first numbers, formed, and sorted as 32-bit keys
+//      (level of the score above the bound | inverted flat id), which puts ties in the order of their ids as well.
+//   4. Otherwise (long runs of equal sums, non-finite values, a range of levels that does not fit the keys) the level of the
+//      k-th sum is found exactly, the sums above it are taken, and the ties with the lowest flat ids fill the rest.
 //
-// Bound by one token's chain of dependent instructions (about 24000 cycles at 128 keys, top-64, with seven warps per
-// scheduler) and, with more than 8 keys per lane, by instruction fetch.  us, both halves sorted whole -> this kernel:
-// 16384 x 512 keys top-128 319 -> 214; 8192 x 1024 top-64 349 -> 106; 131072 x 256 top-32 558 -> 358; 4096 x 128 top-64 the
-// same (17.5); one token 7.8 -> 7.2.  Measured and not kept: cell numbers first and keys in a second loop (214 -> 224),
-// one sort per list or both lists at once (the same), candidates walked in shared memory for top-64 too (396 -> 444).
+// Bound by one token's chain of dependent instructions and by instruction issue (with all keys kept, a threshold search over the
+// staircase (p + 1)(q + 1) <= k and a separate treatment of ties a token of 512 keys, top-128 took 7100 instructions).  us, that
+// form -> this one: 16384 x 512 keys top-128 217 -> 104, 131072 x 256 top-32 359 -> 262, 16384 x 128 top-64 53.5 -> 39.2,
+// 4096 x 128 top-64 18.7 -> 12.6, 8192 x 1024 top-64 102 -> 78, one token 7.5 -> 6.0; logits 100 times smaller, whose sums tie in
+// long runs, 2000 x 512 top-128 606 -> 60.  Slower only where half the probability is in one key and k is large (2000 x 512
+// top-128, logits 6 x |x|: 44 -> 68).  Measured and not kept: both halves sorted (16384 x 512 top-128 152, 122 with the second
+// alone), four CTAs per SM for 512 keys instead of six (122, 107), rows counted 32 at a time (108, 104 with 64).
 // ------------------------------------------------------------------------------------------
 struct RouterPrunedLayout {
-  int cta_bytes, warp_bytes;
-  int off_ids, off_win, off_cs, off_tl;
-  int nkp, kp, C, Cp;
+  int warp_bytes;
+  int off_ids, off_win, off_runs;
+  int nkp;
 };
 
-constexpr int kPrunedMaxK = 128;  // at most 22 staircase cells per lane stay in registers
+constexpr int kPrunedMaxK = 128;  // at most 256 candidates, eight per lane
 
-// Sorts two key lists (la: na keys, lb: nb keys, in shared memory) descending, 16 lanes and 16 R slots each, and writes
-// values and ids in rank order (first half at 0, second at `stride`); the lists may lie under the values.
-template <typename T, int R>
-__device__ __noinline__ void sort_both_halves(const uint32_t* la, const uint32_t* lb, int na, int nb, float* sv, uint16_t* si,
-                                              int stride, int lane) {
-  using HK = HalfKey<T>;
-  const int l16 = lane & 15;
-  const bool second = lane >= 16;
-  const uint32_t* src = second ? lb : la;
-  const int n = second ? nb : na;
-  uint32_t a[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) a[r] = l16 * R + r < n ? src[l16 * R + r] : 0u;
-  constexpr int N = 16 * R;
-#pragma unroll
-  for (int size = 2; size <= N; size <<= 1) {
-#pragma unroll
-    for (int step = size >> 1; step > 0; step >>= 1) {
-      if (step >= R) {
-        const int ls = step / R;
-        const bool desc = (size == N) || (((l16 * R) & size) == 0);
-        const bool keep_max = ((l16 & ls) == 0) == desc;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const uint32_t other = __shfl_xor_sync(kFull, a[r], ls);
-          a[r] = keep_max ? max(a[r], other) : min(a[r], other);
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if ((r & step) == 0) {
-            const bool desc = (size == N) || (size < R ? ((r & size) == 0) : (((l16 * R) & size) == 0));
-            const uint32_t lo = min(a[r], a[r | step]), hi = max(a[r], a[r | step]);
-            a[r] = desc ? hi : lo;
-            a[r | step] = desc ? lo : hi;
-          }
-        }
-      }
-    }
-  }
-  __syncwarp();  // both lists have been read
-  float* v = sv + (second ? stride : 0);
-  uint16_t* id = si + (second ? stride : 0);
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int i = l16 * R + r;
-    if (i < n) {
-      v[i] = HK::value(a[r]);
-      id[i] = static_cast<uint16_t>(HK::id(a[r]));
-    }
-  }
-  __syncwarp();
-}
-
-// Sorts the n <= 32 R keys of `list` (shared memory) in place, or, with sv, into values and ids in rank order (they may lie
-// over the list).
+// Sorts the n <= 32 R keys of `list` (shared memory) into values and ids in rank order (the values may lie over the list).
 template <typename T, int R, bool UNROLLED>
-__device__ __noinline__ void sort_list(uint32_t* list, int n, float* sv, uint16_t* si, int lane) {
+__device__ __noinline__ void sort_list(const uint32_t* list, int n, float* sv, uint16_t* si, int lane) {
   using HK = HalfKey<T>;
   uint32_t a[R];
 #pragma unroll
@@ -860,12 +820,8 @@ __device__ __noinline__ void sort_list(uint32_t* list, int n, float* sv, uint16_
   for (int r = 0; r < R; ++r) {
     const int i = lane * R + r;
     if (i < n) {
-      if (sv != nullptr) {
-        sv[i] = HK::value(a[r]);
-        si[i] = static_cast<uint16_t>(HK::id(a[r]));
-      } else {
-        list[i] = a[r];
-      }
+      sv[i] = HK::value(a[r]);
+      si[i] = static_cast<uint16_t>(HK::id(a[r]));
     }
   }
   __syncwarp();
@@ -884,14 +840,163 @@ __device__ __forceinline__ uint32_t sort_lanes_packed(uint32_t v, int lane) {
   return v;
 }
 
-template <typename T, int E, int CPL>
-__global__ void __launch_bounds__(128, E <= 8 ? 7 : 4)
+// Order level of a sum in the type of the input: larger sum <=> larger level, -0 as +0
+template <typename T>
+__device__ __forceinline__ uint32_t sum_level(float s) {
+  return HalfKey<T>::make(round_to<T>(s) + 0.0f, 0) >> 16;
+}
+
+// Step 4 of the kernel below, for the rare rows: exactly k winners as 64-bit keys (level, inverted flat id), in order.  At least k
+// sums reach level lo, fewer level hi.  rows: the keys kept of the first half (na, in the order of their ids); sb, ib: the second
+// half sorted (nb); runs: scratch, na entries.
+template <typename T>
+__device__ __noinline__ void select_exactly(uint32_t* rows, const float* sb, const uint16_t* ib, int na, int nb, int nk, int k,
+                                            uint32_t lo, uint32_t hi, uint32_t* runs, uint64_t* win, int lane) {
+  using HK = HalfKey<T>;
+  auto level = [&](int p, int q) { return sum_level<T>(__fadd_rn(HK::value(rows[p]), sb[q])); };
+  const int first = 1 << (31 - __clz(nb));
+  auto reach = [&](int p, uint32_t x) {  // sums of row p at or above level x
+    int n = 0;
+    for (int w = first; w > 0; w >>= 1)
+      if (n + w <= nb && level(p, n + w - 1) >= x) n += w;
+    return n;
+  };
+  int kept = 0;  // rows that reach lo at all (a row never moves up)
+  for (int base = 0; base < na; base += 32) {
+    const int p = base + lane;
+    const uint32_t row = p < na ? rows[p] : 0u;
+    const bool keep = p < na && (lo == 0 || level(p, 0) >= lo);
+    const unsigned bal = __ballot_sync(kFull, keep);
+    if (keep) rows[kept + __popc(bal & ((1u << lane) - 1u))] = row;
+    kept += __popc(bal);
+    __syncwarp();
+  }
+  na = kept;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    int n = 0;
+    for (int p = lane; p < na; p += 32) n += reach(p, mid);
+    if (static_cast<int>(__reduce_add_sync(kFull, n)) >= k) lo = mid;
+    else hi = mid;
+  }
+  // everything above; the runs of ties: (first column rank << 16) | columns
+  auto row_id = [&](int p) { return HK::id(rows[p]); };
+  auto flat_id = [&](int p, int q) { return row_id(p) * static_cast<uint32_t>(nk) + ib[q]; };
+  int filled = 0;
+  for (int base = 0; base < na; base += 32) {
+    const int p = base + lane;
+    int n = 0;
+    if (p < na) {
+      n = reach(p, hi);
+      runs[p] = (static_cast<uint32_t>(n) << 16) | static_cast<uint32_t>(max(reach(p, lo) - n, 0));
+    }
+    int incl = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int up = __shfl_up_sync(kFull, incl, d);
+      if (lane >= d) incl += up;
+    }
+    for (int q = 0; q < n && filled + incl - n + q < k; ++q) win[filled + incl - n + q] = make_key(level(p, q), flat_id(p, q));
+    filled += __shfl_sync(kFull, incl, 31);
+  }
+  __syncwarp();
+  // ties with the lowest flat ids: the rows whose id is below `row` whole (the largest id for which they do not suffice), then
+  // the lowest column ids of that row
+  const int need = k - filled;
+  uint32_t row = 0;
+  int whole = 0;  // ties in the rows below `row`
+  for (int bit = 31 - __clz(nk); bit >= 0; --bit) {
+    const uint32_t trial = row | (1u << bit);
+    int n = 0;
+    for (int p = lane; p < na; p += 32) n += row_id(p) < trial ? static_cast<int>(runs[p] & 0xFFFFu) : 0;
+    n = __reduce_add_sync(kFull, n);
+    if (n < need) {
+      row = trial;
+      whole = n;
+    }
+  }
+  int at = filled;
+  for (int base = 0; base < na; base += 32) {
+    const int p = base + lane;
+    const bool take = p < na && row_id(p) < row;
+    const uint32_t run = take ? runs[p] : 0u;
+    const int n = run & 0xFFFFu;
+    int incl = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int up = __shfl_up_sync(kFull, incl, d);
+      if (lane >= d) incl += up;
+    }
+    for (int q = 0; q < n && at + incl - n + q < k; ++q) win[at + incl - n + q] = make_key(lo, flat_id(p, (run >> 16) + q));
+    at += __shfl_sync(kFull, incl, 31);
+    const unsigned here = __ballot_sync(kFull, p < na && row_id(p) == row);
+    if (here != 0) {
+      const int split = base + __ffs(here) - 1, from = runs[split] >> 16, cols = runs[split] & 0xFFFFu, rest = need - whole;
+      uint32_t phi = 0;  // the largest id with fewer than `rest` column ids of the run below it: those and phi are taken
+      for (int bit = 31 - __clz(nk); bit >= 0; --bit) {
+        const uint32_t trial = phi | (1u << bit);
+        int under = 0;
+        for (int q = lane; q < cols; q += 32) under += ib[from + q] < trial ? 1 : 0;
+        if (static_cast<int>(__reduce_add_sync(kFull, under)) < rest) phi = trial;
+      }
+      int done = filled + whole;
+      for (int c = 0; c < cols; c += 32) {
+        const bool in = c + lane < cols && ib[from + min(c + lane, cols - 1)] <= phi;
+        const unsigned bal = __ballot_sync(kFull, in);
+        const int pos = done + __popc(bal & ((1u << lane) - 1u));
+        if (in && pos < k) win[pos] = make_key(lo, flat_id(split, from + c + lane));
+        done += __popc(bal);
+      }
+    }
+  }
+  filled = min(k, filled + whole + max(need - whole, 0));
+  int kp = 1;
+  while (kp < k) kp <<= 1;
+  __syncwarp();
+  for (int r = filled + lane; r < kp; r += 32) win[r] = 0;
+  __syncwarp();
+  bitonic_desc(win, nullptr, kp, lane);
+}
+
+// The numbered candidates as 64-bit keys (level, inverted flat id), sorted over the rows and values that they come from
+// (32 R keys are at most the 2 nkp entries of those); the first k to `win`.  For levels too far apart for 32-bit keys.
+template <typename T, int R>
+__device__ __noinline__ void sort_wide(const uint32_t* rows, const float* sb, const uint16_t* ib, const uint32_t* marks, int found,
+                                       int nk, int k, uint64_t* keys, uint64_t* win, int lane) {
+  using HK = HalfKey<T>;
+  uint64_t cand[R];
+  uint32_t carry = 0;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = 32 * r + lane;
+    uint32_t m = marks[i];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) m = max(m, __shfl_up_sync(kFull, m, d));
+    m = max(m, carry);
+    carry = __shfl_sync(kFull, m, 31);
+    cand[r] = 0;
+    if (i < found) {
+      const int p = m >> 16, q = i - static_cast<int>(m & 0xFFFFu);
+      cand[r] = make_key(sum_level<T>(__fadd_rn(HK::value(rows[p]), sb[q])), HK::id(rows[p]) * static_cast<uint32_t>(nk) + ib[q]);
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < R; ++r) keys[32 * r + lane] = cand[r];
+  __syncwarp();
+  bitonic_desc(keys, nullptr, 32 * R, lane);
+  for (int r = lane; r < k; r += 32) win[r] = keys[r];
+  __syncwarp();
+}
+
+// E: keys per lane and half; R: candidates per lane, 32 R >= 2 k
+template <typename T, int E, int R>
+__global__ void __launch_bounds__(128, E <= 8 ? 7 : E <= 16 ? 6 : 4)
 router_topk_pruned_kernel(const T* logp, int64_t ntok, int nk, int k, RouterPrunedLayout L,
                           T* __restrict__ scores, int64_t* __restrict__ indices, T* __restrict__ gates, int flags) {
   using HK = HalfKey<T>;
-  constexpr int LOW = OrdLowBits<T>::value;
-  constexpr bool kKeysInRegs = E <= 8;     // both halves' values stay in registers up to the compaction
-  constexpr bool kUnrollCells = CPL <= 10;  // see sort_desc: small kernels are unrolled, large ones are loops
+  constexpr bool kKeysInRegs = E <= 16;  // both halves' keys stay in registers up to the compaction
+  constexpr int kCap = 32 * R;
   const int norm = flags & kTopkNorm;
   const bool from_logits = (flags & kTopkFromLogits) != 0;
   const bool token_rows = (flags & (kTopkFromLogits | kTopkTokenRows)) != 0;  // [T, 2, nk] instead of [2, T, nk]
@@ -899,60 +1004,20 @@ router_topk_pruned_kernel(const T* logp, int64_t ntok, int nk, int k, RouterPrun
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
-  const int C = L.C, nkp = L.nkp, kp = L.kp;
+  const int nkp = L.nkp;
+  if (!(flags & kTopkLateWait)) pdl_wait();  // the logits come from the previous kernel (kTopkLateWait: the one before)
 
-  // staircase table, built once per CTA: entry c -> (p << 8) | q (top_k <= 128) with (p+1)(q+1) <= k; row p starts at rowstart[p]
-  uint16_t* pq16 = reinterpret_cast<uint16_t*>(smem);
-  int* rowstart = reinterpret_cast<int*>(smem + 2 * L.Cp);
-  if (warp == 0) {
-    int running = 0;
-    for (int base = 0; base < k; base += 32) {
-      const int p = base + lane;
-      const int len = (p < k) ? k / (p + 1) : 0;
-      int incl = len;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int up = __shfl_up_sync(kFull, incl, d);
-        if (lane >= d) incl += up;
-      }
-      if (p < k) rowstart[p] = running + incl - len;
-      running += __shfl_sync(kFull, incl, 31);
-    }
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {  // entry c lies in the last row whose start is <= c
-    int lo = 0, hi = k - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (rowstart[mid] <= c) lo = mid; else hi = mid - 1;
-    }
-    pq16[c] = static_cast<uint16_t>((lo << 8) | (c - rowstart[lo]));
-  }
-  auto pq = [&](int c) {  // (p << 16) | q
-    const uint32_t e = pq16[c];
-    return ((e & 0xFF00u) << 8) | (e & 0xFFu);
-  };
-  __syncthreads();
-  // the staircase table above depends on k alone; the logits come from the previous kernel (kTopkLateWait: the one before)
-  if (!(flags & kTopkLateWait)) pdl_wait();
-
-  unsigned char* wbase = smem + L.cta_bytes + warp * L.warp_bytes;
-  float* sa = reinterpret_cast<float*>(wbase);  // values in rank order; the key lists lie here before they are sorted
-  float* sb = sa + nkp;
-  uint16_t* ia = reinterpret_cast<uint16_t*>(wbase + L.off_ids);
-  uint16_t* ib = ia + nkp;
-  uint64_t* win = reinterpret_cast<uint64_t*>(wbase + L.off_win);    // winners, 64-bit keys (rare) ...
-  uint32_t* win32 = reinterpret_cast<uint32_t*>(wbase + L.off_win);  // ... or 32-bit keys
-  uint32_t* cs = reinterpret_cast<uint32_t*>(wbase + L.off_cs);      // staircase sums
-  uint32_t* tl = reinterpret_cast<uint32_t*>(wbase + L.off_tl);      // flat ids of candidates equal to tau
-  int* tcnt = reinterpret_cast<int*>(tl + kPrunedTieCap);
+  unsigned char* wbase = smem + warp * L.warp_bytes;
+  uint32_t* rows = reinterpret_cast<uint32_t*>(wbase);  // keys kept of the first half, in the order of their ids
+  uint32_t* cols = rows + nkp;                           // of the second half ...
+  float* sb = reinterpret_cast<float*>(cols);            // ... then its values in rank order
+  uint16_t* ib = reinterpret_cast<uint16_t*>(wbase + L.off_ids);
+  uint32_t* win32 = reinterpret_cast<uint32_t*>(wbase + L.off_win);  // marks, then the winners' 32-bit keys ...
+  uint64_t* win = reinterpret_cast<uint64_t*>(wbase + L.off_win);    // ... or their 64-bit keys (rare)
   const int qrank = (k + lane) / (lane + 1);  // ceil(k / (lane + 1)): the rank that pairs with rank lane + 1 of half 0
   int idbits = 1;
   while (idbits < 31 && (1 << idbits) < nk * nk) ++idbits;
   const uint32_t idmask = (1u << idbits) - 1u;
-  const unsigned below = (1u << lane) - 1u;
-  auto flat_id = [&](int p, int q) { return static_cast<uint32_t>(ia[p]) * static_cast<uint32_t>(nk) + ib[q]; };
-  auto pair_ord = [&](int p, int q) { return f32_to_ord(round_to<T>(__fadd_rn(sa[p], sb[q])) + 0.0f); };
 
   for (int64_t t = static_cast<int64_t>(blockIdx.x) * nwarps + warp; t < ntok;
        t += static_cast<int64_t>(gridDim.x) * nwarps) {
@@ -961,8 +1026,6 @@ router_topk_pruned_kernel(const T* logp, int64_t ntok, int nk, int k, RouterPrun
     //    (flash_moe/modules/flash_moe.py:72) rounded to T like torch does; lane maxima
     const T* a_row = token_rows ? logp + t * 2 * nk : logp + t * nk;
     const T* b_row = token_rows ? a_row + nk : logp + (ntok + t) * nk;
-    uint32_t* la = reinterpret_cast<uint32_t*>(sa);
-    uint32_t* lb_list = reinterpret_cast<uint32_t*>(sb);
     uint32_t key[kKeysInRegs ? 2 : 1][E];
     uint32_t v = 0;      // this lane's maximum of both halves (16-bit order keys)
     float poison = 0.f;  // NaN once a value is not finite
@@ -1002,32 +1065,63 @@ router_topk_pruned_kernel(const T* logp, int64_t ntok, int nk, int k, RouterPrun
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
         load_half(h, key[0]);
-        store_blocked<E>(reinterpret_cast<float*>(h == 0 ? la : lb_list), lane, reinterpret_cast<const float (&)[E]>(key[0]));
+        store_blocked<E>(reinterpret_cast<float*>(h == 0 ? rows : cols), lane, reinterpret_cast<const float (&)[E]>(key[0]));
       }
     }
     // 2. lower bound on the k-th largest sum from the sorted lane maxima (0: absent), and the keys it leaves
-    uint32_t lb = 0;             // order key of the bound
+    uint32_t level = 0;          // order level of the bound: at least k sums reach it
+    uint32_t cmax = 0;           // level of the largest sum
     uint32_t thr0 = 1, thr1 = 1;  // keys from here on are kept (0 pads the rows)
-    if (__all_sync(kFull, poison == 0.f)) {
+    bool ordinary = __all_sync(kFull, poison == 0.f);  // no NaN, no +inf (-inf is but the lowest value)
+    if (!ordinary) {
+      constexpr uint32_t kMinusInf = OrdLowBits<T>::value == 16 ? 0x007Fu : 0x03FFu;
+      bool ok = true;
+#pragma unroll(kKeysInRegs ? E : 1)
+      for (int r = 0; r < E; ++r) {
+        const uint32_t a = kKeysInRegs ? key[0][r] : rows[lane * E + r];
+        const uint32_t b = kKeysInRegs ? key[kKeysInRegs ? 1 : 0][r] : cols[lane * E + r];
+        ok = ok && (a == 0 || (a >> 16) - kMinusInf < 0xFFFFu - 2 * kMinusInf);  // the level of +inf is 0xFFFF - kMinusInf
+        ok = ok && (b == 0 || (b >> 16) - kMinusInf < 0xFFFFu - 2 * kMinusInf);
+      }
+      ordinary = __all_sync(kFull, ok);
+    }
+    if (ordinary) {
       v = sort_lanes_packed(v, lane);
       const uint32_t other = __shfl_sync(kFull, v, qrank <= 32 ? qrank - 1 : 0);
       const uint32_t ka = v << 16, kb = other & 0xFFFF0000u;
-      if (qrank <= 32 && ka != 0 && kb != 0)
-        lb = f32_to_ord(round_to<T>(__fadd_rn(HK::value(ka), HK::value(kb))) + 0.0f);
-      lb = __reduce_max_sync(kFull, lb);
+      uint32_t rect = 0;
+      if (qrank <= 32 && ka != 0 && kb != 0) rect = f32_to_ord(__fadd_rn(HK::value(ka), HK::value(kb)));
+      rect = __reduce_max_sync(kFull, rect);
       const uint32_t top = __shfl_sync(kFull, v, 0);
-      const float ta = HK::value(top << 16), tb = HK::value(top), bound = ord_to_f32(lb);
-      // round(a + b) >= bound needs a + b >= bound less one step of T there; the threshold's key is rounded to T too
-      constexpr float kStep = LOW == 16 ? 0.0078125f : 0.0009765625f;
-      const float low = bound - (fabsf(bound) * kStep + 1e-7f);
-      const float xa = low - tb, xb = low - ta, blur = (fabsf(bound) + fabsf(ta) + fabsf(tb)) * 1e-6f + 1e-7f;
-      const float ya = xa - (fabsf(xa) * kStep + blur), yb = xb - (fabsf(xb) * kStep + blur);
-      if (lb != 0 && ya > -INFINITY && yb > -INFINITY) {
-        thr0 = max(HK::make(ya, 0) & 0xFFFF0000u, 1u);
-        thr1 = max(HK::make(yb, 0) & 0xFFFF0000u, 1u);
+      const float ta = HK::value(top << 16), tb = HK::value(top);
+      cmax = sum_level<T>(__fadd_rn(ta, tb));
+      if (rect != 0) {
+        const float a = ka != 0 ? HK::value(ka) : -INFINITY;
+        const float b = (v & 0xFFFF0000u) != 0 ? HK::value(v & 0xFFFF0000u) : -INFINITY;
+        float lo = ord_to_f32(rect), hi = __fadd_rn(ta, tb);
+#pragma unroll 1
+        for (int step = 0; step < 5; ++step) {
+          const float mid = 0.5f * lo + 0.5f * hi;
+          int n = 0;  // sums of this lane's maximum of the first half that reach mid (at most 31 are counted)
+#pragma unroll
+          for (int w = 16; w > 0; w >>= 1)
+            if (__fadd_rn(a, __shfl_sync(kFull, b, n + w - 1)) >= mid) n += w;
+          if (static_cast<int>(__reduce_add_sync(kFull, n)) >= k) lo = mid;
+          else hi = mid;
+        }
+        level = sum_level<T>(lo);
+        const float bound = HK::value(level << 16);
+        // round(a + b) >= bound needs a + b >= bound less one step of T there; the threshold's key is rounded to T too
+        constexpr float kStep = OrdLowBits<T>::value == 16 ? 0.0078125f : 0.0009765625f;
+        const float low = bound - (fabsf(bound) * kStep + 1e-7f);
+        const float xa = low - tb, xb = low - ta, blur = (fabsf(bound) + fabsf(ta) + fabsf(tb)) * 1e-6f + 1e-7f;
+        const float ya = xa - (fabsf(xa) * kStep + blur), yb = xb - (fabsf(xb) * kStep + blur);
+        if (ya > -INFINITY && yb > -INFINITY) {
+          thr0 = max(HK::make(round_to<T>(ya), 0) & 0xFFFF0000u, 1u);
+          thr1 = max(HK::make(round_to<T>(yb), 0) & 0xFFFF0000u, 1u);
+        }
       }
     }
-    if (lane == 0) *tcnt = 0;
     int na = 0, nb = 0;
     if constexpr (kKeysInRegs) {
       uint32_t cnt = 0;
@@ -1043,27 +1137,20 @@ router_topk_pruned_kernel(const T* logp, int64_t ntok, int nk, int k, RouterPrun
       na = total & 0xFFFFu;
       nb = total >> 16;
       cnt -= mine;
-      uint32_t* da = la + (cnt & 0xFFFFu);
-      uint32_t* db = lb_list + (cnt >> 16);
+      uint32_t* da = rows + (cnt & 0xFFFFu);
+      uint32_t* db = cols + (cnt >> 16);
 #pragma unroll
       for (int r = 0; r < E; ++r) {
         if (key[0][r] >= thr0) *da++ = key[0][r];
         if (key[1][r] >= thr1) *db++ = key[1][r];
       }
       __syncwarp();
-      const int most = max(na, nb);
-      if (most <= 32) sort_both_halves<T, 2>(la, lb_list, na, nb, sa, ia, nkp, lane);
-      else if (E <= 2 || most <= 64) sort_both_halves<T, 4>(la, lb_list, na, nb, sa, ia, nkp, lane);
-      else if (E <= 4 || most <= 128) sort_both_halves<T, 8>(la, lb_list, na, nb, sa, ia, nkp, lane);
-      else {
-        sort_list<T, 8, false>(la, na, sa, ia, lane);
-        sort_list<T, 8, false>(lb_list, nb, sb, ib, lane);
-      }
     } else {
+      const unsigned below = (1u << lane) - 1u;
       __syncwarp();
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
-        uint32_t* list = h == 0 ? la : lb_list;
+        uint32_t* list = h == 0 ? rows : cols;
         const uint32_t th = h == 0 ? thr0 : thr1;
         int n = 0;
 #pragma unroll 2
@@ -1074,206 +1161,132 @@ router_topk_pruned_kernel(const T* logp, int64_t ntok, int nk, int k, RouterPrun
           n += __popc(bal);
           __syncwarp();
         }
-        float* sv = h == 0 ? sa : sb;
-        uint16_t* si = h == 0 ? ia : ib;
-        if (n <= 32) sort_list<T, 1, false>(list, n, sv, si, lane);
-        else if (n <= 64) sort_list<T, 2, false>(list, n, sv, si, lane);
-        else if (n <= 128) sort_list<T, 4, false>(list, n, sv, si, lane);
-        else if (n <= 256) sort_list<T, 8, false>(list, n, sv, si, lane);
-        else if (E <= 16 || n <= 512) sort_list<T, 16, false>(list, n, sv, si, lane);
-        else sort_list<T, E >= 32 ? 32 : 16, false>(list, n, sv, si, lane);
         if (h == 0) na = n;
         else nb = n;
       }
     }
+    if (nb <= 32) sort_list<T, 1, true>(cols, nb, sb, ib, lane);
+    else if (E <= 2 || nb <= 64) sort_list<T, 2, true>(cols, nb, sb, ib, lane);
+    else if (E <= 4 || nb <= 128) sort_list<T, 4, false>(cols, nb, sb, ib, lane);
+    else if (E <= 8 || nb <= 256) sort_list<T, 8, false>(cols, nb, sb, ib, lane);
+    else if (E <= 16 || nb <= 512) sort_list<T, 16, false>(cols, nb, sb, ib, lane);
+    else sort_list<T, E >= 32 ? 32 : 16, false>(cols, nb, sb, ib, lane);
 
-    // 3. staircase sums (in registers), threshold tau = k-th largest
-    uint32_t csr[CPL];
-    if constexpr (kUnrollCells) {
-#pragma unroll
-      for (int j = 0; j < CPL; ++j) {
-        const int c = 32 * j + lane;
-        const uint32_t e = c < C ? pq(c) : 0xFFFFFFFFu;
-        const int p = e >> 16, q = e & 0xFFFFu;
-        csr[j] = (p < na && q < nb) ? pair_ord(p, q) : 0u;  // 0 is below the key of every float, -inf included
-      }
-    } else {
-#pragma unroll 2
-      for (int c = lane; c < C; c += 32) {
-        const uint32_t e = pq(c);
-        const int p = e >> 16, q = e & 0xFFFFu;
-        cs[c] = (p < na && q < nb) ? pair_ord(p, q) : 0u;
-      }
-      __syncwarp();
-#pragma unroll
-      for (int j = 0; j < CPL; ++j) csr[j] = 32 * j + lane < C ? cs[32 * j + lane] : 0u;
-    }
-    const uint32_t cmax = pair_ord(0, 0);  // ranks (0, 0): the largest sum
-    uint32_t tau = cmax;
-    if (cmax != lb) {
-      // two bits a step: the three trial thresholds are counted in one packed reduction (at most 704 cells)
-      // (the last step may reach one bit below LOW: no value differs from its level there)
-      int bit = 31 - __clz(cmax ^ lb);
-      tau = bit >= 31 ? 0u : cmax & ~((2u << bit) - 1u);
-      for (; bit >= LOW; bit -= 2) {
-        const uint32_t t1 = tau | (1u << (bit - 1)), t2 = tau | (1u << bit), t3 = t1 | t2;
-        uint32_t n = 0;
-#pragma unroll
-        for (int j = 0; j < CPL; ++j)
-          n += (csr[j] >= t1 ? 1u : 0u) + (csr[j] >= t2 ? 1u << 10 : 0u) + (csr[j] >= t3 ? 1u << 20 : 0u);
-        n = __reduce_add_sync(kFull, n);
-        const uint32_t uk = static_cast<uint32_t>(k);
-        tau = (n >> 20) >= uk ? t3 : ((n >> 10) & 1023u) >= uk ? t2 : (n & 1023u) >= uk ? t1 : tau;
-      }
-      if ((tau >> 31) == 0) tau |= (1u << LOW) - 1u;
-    }
-    const uint32_t tlevel = tau >> LOW;
-    const bool fits = (cmax >> LOW) - tlevel < (1u << (32 - idbits)) - 1u;
-    auto put = [&](int pos, uint32_t ord, uint32_t flat) {
-      if (fits) win32[pos] = (((ord >> LOW) - tlevel + 1u) << idbits) | (idmask - flat);
-      else win[pos] = make_key(ord, flat);
-    };
-
-    // emit everything above tau; collect the staircase candidates equal to tau in the tie list
-    int filled = 0, nties = 0;
-    auto emit = [&](int base, uint32_t o) {
-      const unsigned bge = __ballot_sync(kFull, o >= tau);
-      if (bge == 0) return;
-      const unsigned bgt = __ballot_sync(kFull, o > tau);
-      if (o >= tau) {
-        const uint32_t e = pq(base + lane);
-        const uint32_t flat = flat_id(e >> 16, e & 0xFFFFu);
-        if (o > tau) {
-          const int pos = filled + __popc(bgt & below);
-          if (pos < k) put(pos, o, flat);
-        } else {
-          const int pos = nties + __popc((bge & ~bgt) & below);
-          if (pos < kPrunedTieCap) tl[pos] = flat;
-        }
-      }
-      filled += __popc(bgt);
-      nties += __popc(bge & ~bgt);
-    };
-    if constexpr (kUnrollCells) {
-#pragma unroll
-      for (int j = 0; j < CPL; ++j) emit(32 * j, csr[j]);
-    } else {
+    // 3. the sums that reach the bound, or a higher level if those are too many: row counts, then marks at the rows' first
+    //    numbers; lo: at least k sums reach it, hi: fewer do
+    uint32_t lo = level, hi = cmax + 1, step = OrdLowBits<T>::value == 16 ? 1 : 8;
+    int found = 0;
+    bool listed = false;  // the candidates are found and marked
 #pragma unroll 1
-      for (int base = 0; base < C; base += 32) emit(base, base + lane < C ? cs[base + lane] : 0u);
-    }
-    int need = k - filled;
-
-    // 4. ties outside the staircase: runs that continue a row past its last cell, and runs from q = 0 in the rows below
-    //    (all sums there are at most tau and do not increase along a row)
-    for (int base = 0; base < na; base += 32) {
-      const int p = base + lane;
-      const int len = p < k ? (p + 1 < k ? rowstart[p + 1] : C) - rowstart[p] : 0;  // = k / (p + 1)
-      const bool hit = p < na && len < nb && pair_ord(p < na ? p : 0, len < nb ? len : 0) == tau;
-      const unsigned any = __ballot_sync(kFull, hit);
-      if (hit) {
-        for (int q = len; q < nb; ++q) {
-          if (pair_ord(p, q) != tau) break;
-          const int pos = nties + atomicAdd(tcnt, 1);
-          if (pos < kPrunedTieCap) tl[pos] = flat_id(p, q);
-        }
-      }
-      if (base >= k && any == 0u) break;  // rows are sorted: no later row can tie
-    }
-    __syncwarp();
-    nties += *tcnt;
-    __syncwarp();
-    if (nties <= 32) {
-      // the usual case, a handful of ties: one id per lane, its rank among them by a round of shuffles
-      const uint32_t id = lane < nties ? tl[lane] : 0xFFFFFFFFu;
-      int rank = 0;
-      for (int j = 0; j < nties; ++j) rank += (__shfl_sync(kFull, id, j) < id) ? 1 : 0;
-      if (lane < nties && rank < need) put(filled + rank, tau, id);
-      filled += min(nties, need);
-    } else if (nties <= kPrunedTieCap) {
-      uint32_t phi = 0xFFFFFFFFu;  // ids <= phi are taken
-      if (nties > need) {
-        // phi = the need-th smallest id = the largest v with fewer than `need` ids below v
-        uint32_t x = 0;
-        for (int bit = idbits - 1; bit >= 0; --bit) {
-          const uint32_t trial = x | (1u << bit);
-          int under = 0;
-          for (int i = lane; i < nties; i += 32) under += (tl[i] < trial) ? 1 : 0;
-          under = __reduce_add_sync(kFull, under);
-          if (under < need) x = trial;
-        }
-        phi = x;
-      }
-      for (int base = 0; base < nties; base += 32) {
-        const int i = base + lane;
-        const uint32_t id = (i < nties) ? tl[i] : 0xFFFFFFFFu;
-        const bool take = (i < nties) && (id <= phi);
-        const unsigned bal = __ballot_sync(kFull, take);
-        if (take) put(filled + __popc(bal & below), tau, id);
-        filled += __popc(bal);
-      }
-    } else {
-      // more ties than the list holds (e.g. constant inputs): rows in index order, inside a row the lowest column ids
-      int last = -1;
-      while (need > 0) {
-        uint32_t next = 0xFFFFFFFFu;  // (row id << 16) | rank of the next row
-        for (int p = lane; p < na; p += 32)
-          if (static_cast<int>(ia[p]) > last) next = min(next, (static_cast<uint32_t>(ia[p]) << 16) | static_cast<uint32_t>(p));
-        next = __reduce_min_sync(kFull, next);
-        if (next == 0xFFFFFFFFu) break;
-        last = static_cast<int>(next >> 16);
-        const int p = next & 0xFFFFu;
-        int run = 0;
-        for (int q = lane; q < nb; q += 32) run += pair_ord(p, q) == tau ? 1 : 0;
-        run = __reduce_add_sync(kFull, run);
-        if (run == 0) continue;
-        uint32_t phi = 0xFFFFu;  // column ids <= phi are taken
-        if (run > need) {
-          uint32_t x = 0;
-          for (int bit = 10; bit >= 0; --bit) {
-            const uint32_t trial = x | (1u << bit);
-            int under = 0;
-            for (int q = lane; q < nb; q += 32) under += (pair_ord(p, q) == tau && ib[q] < trial) ? 1 : 0;
-            under = __reduce_add_sync(kFull, under);
-            if (under < need) x = trial;
-          }
-          phi = x;
-        }
-        for (int base = 0; base < nb; base += 32) {
-          const int q = base + lane;
-          const bool take = q < nb && pair_ord(p, q < nb ? q : 0) == tau && ib[q < nb ? q : 0] <= phi;
-          const unsigned bal = __ballot_sync(kFull, take);
-          if (take) put(filled + __popc(bal & below), tau, flat_id(p, q));
-          filled += __popc(bal);
-          need -= __popc(bal);
-        }
-      }
-    }
-    __syncwarp();
-
-    // 5. order the winners and write out
-    if (fits) {
-      if (k <= 32) sort_list<T, 1, kUnrollCells>(win32, filled, nullptr, nullptr, lane);
-      else if (k <= 64) sort_list<T, 2, kUnrollCells>(win32, filled, nullptr, nullptr, lane);
-      else sort_list<T, 4, kUnrollCells>(win32, filled, nullptr, nullptr, lane);
-    } else {
-      for (int r = filled + lane; r < kp; r += 32) win[r] = 0;
+    for (level = level != 0 ? level : (lo + hi) >> 1; ordinary; level = max(lo + 1, min(lo + step, (lo + hi) >> 1))) {
+      // a sum rounds to the level or above from `edge` on: half way from the level below, or the next float if that rounds down
+      const float value = HK::value(level << 16), under = HK::value((level == 0x8000u ? 0x7FFEu : level - 1) << 16);  // 0x7FFF: -0
+      if (!(fabsf(value) < INFINITY && fabsf(under) < INFINITY)) break;
+      float edge = 0.5f * value + 0.5f * under;
+      if (sum_level<T>(edge) < level) edge = ord_to_f32(f32_to_ord(edge) + 1u);
+#pragma unroll
+      for (int r = 0; r < R; ++r) win32[32 * r + lane] = 0;
       __syncwarp();
-      bitonic_desc(win, nullptr, kp, lane);
+      found = 0;
+      const int first = 1 << (31 - __clz(nb));
+      auto mark = [&](int p, int n, int start) {
+        if (n > 0 && start < kCap) win32[start] = (static_cast<uint32_t>(p) << 16) | static_cast<uint32_t>(start);
+      };
+      auto up_to = [&](uint32_t v_) {  // inclusive sum over the lanes
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const uint32_t up = __shfl_up_sync(kFull, v_, d);
+          if (lane >= d) v_ += up;
+        }
+        return v_;
+      };
+      if (E <= 16 && na <= 32) {
+        const float a = lane < na ? HK::value(rows[lane]) : -INFINITY;
+        int n = 0;  // sums of the row that reach the edge
+        for (int w = first; w > 0; w >>= 1)
+          if (n + w <= nb && __fadd_rn(a, sb[n + w - 1]) >= edge) n += w;
+        const int incl = up_to(n);
+        found = __shfl_sync(kFull, incl, 31);
+        mark(lane, n, incl - n);
+      } else {
+#pragma unroll 1
+        for (int base = 0; base < na && found <= kCap; base += 64) {  // two rows per lane, both searches at once
+          const int p = base + lane;
+          const float a0 = p < na ? HK::value(rows[p]) : -INFINITY, a1 = p + 32 < na ? HK::value(rows[p + 32]) : -INFINITY;
+          int n0 = 0, n1 = 0;
+          for (int w = first; w > 0; w >>= 1) {
+            if (n0 + w <= nb && __fadd_rn(a0, sb[n0 + w - 1]) >= edge) n0 += w;
+            if (n1 + w <= nb && __fadd_rn(a1, sb[n1 + w - 1]) >= edge) n1 += w;
+          }
+          const uint32_t both = static_cast<uint32_t>(n0) | static_cast<uint32_t>(n1) << 16, incl = up_to(both);
+          const uint32_t total = __shfl_sync(kFull, incl, 31);
+          const int all0 = total & 0xFFFFu, before0 = (incl - both) & 0xFFFFu, before1 = (incl - both) >> 16;
+          mark(p, n0, found + before0);
+          mark(p + 32, n1, found + all0 + before1);
+          found += all0 + static_cast<int>(total >> 16);
+        }
+      }
+      __syncwarp();
+      if (found >= k && found <= kCap) {
+        listed = true;
+        break;
+      }
+      if (found < k) {
+        hi = level;
+      } else {
+        lo = level;
+        step *= 2;
+      }
+      if (hi - lo <= 1) break;
     }
+    const bool few = listed && cmax - level < (1u << (32 - idbits)) - 1u;  // they fit 32-bit keys
+    if (few) {
+      uint32_t cand[R];
+      uint32_t carry = 0;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int i = 32 * r + lane;
+        uint32_t m = win32[i];  // (row << 16) | number of the row's first candidate
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) m = max(m, __shfl_up_sync(kFull, m, d));
+        m = max(m, carry);
+        carry = __shfl_sync(kFull, m, 31);
+        cand[r] = 0;
+        if (i < found) {
+          const int p = m >> 16, q = i - static_cast<int>(m & 0xFFFFu);
+          const uint32_t row = rows[p], flat = HK::id(row) * static_cast<uint32_t>(nk) + ib[q];
+          cand[r] = ((sum_level<T>(__fadd_rn(HK::value(row), sb[q])) - level + 1u) << idbits) | (idmask - flat);
+        }
+      }
+      sort_desc<R, (R <= 4)>(cand, lane);
+      __syncwarp();  // the marks have been read
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (lane * R + r < k) win32[lane * R + r] = cand[r];
+      __syncwarp();
+    } else if (listed) {
+      sort_wide<T, R>(rows, sb, ib, win32, found, nk, k, reinterpret_cast<uint64_t*>(wbase), win, lane);
+    } else {
+      select_exactly<T>(rows, sb, ib, na, nb, nk, k, lo, ordinary ? hi : 0x10000u, reinterpret_cast<uint32_t*>(wbase + L.off_runs),
+                        win, lane);
+    }
+
+    // 4. write out
     float gsum = 0.f;
     for (int r = lane; r < k; r += 32) {
-      uint64_t ky = 0;
-      if (!fits) {
-        ky = win[r];
-      } else if (r < filled) {
+      uint32_t lv, id;
+      if (few) {
         const uint32_t w = win32[r];
-        const uint32_t level = (w >> idbits) - 1u + tlevel;
-        // the low bits of a 16-bit value's order key: zeros for positive values, ones for negative ones
-        ky = make_key((level << LOW) | ((level >> (31 - LOW)) != 0 ? 0u : (1u << LOW) - 1u), idmask - (w & idmask));
+        lv = (w >> idbits) - 1u + level;
+        id = idmask - (w & idmask);
+      } else {
+        const uint64_t ky = win[r];
+        lv = static_cast<uint32_t>(ky >> 32);
+        id = key_id(ky);
       }
-      const float s = key_val(ky);
+      const float s = HK::value(lv << 16);
       scores[t * k + r] = from_f32<T>(s);
-      indices[t * k + r] = static_cast<int64_t>(key_id(ky));
+      indices[t * k + r] = static_cast<int64_t>(id);
       if (gates != nullptr) {
         const T g = from_f32<T>(expf(s));
         gsum += to_f32<T>(g);
@@ -1284,7 +1297,6 @@ router_topk_pruned_kernel(const T* logp, int64_t ntok, int nk, int k, RouterPrun
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) gsum += __shfl_xor_sync(kFull, gsum, d);
       const float denom = round_to<T>(gsum);
-      __syncwarp();
       for (int r = lane; r < k; r += 32) {  // this lane's own scores, written above
         const float g = round_to<T>(expf(to_f32<T>(scores[t * k + r])));
         gates[t * k + r] = from_f32<T>(g / denom);
@@ -1296,27 +1308,18 @@ router_topk_pruned_kernel(const T* logp, int64_t ntok, int nk, int k, RouterPrun
   if ((flags & kTopkLateWait) && blockIdx.x == gridDim.x - 1) pdl_wait();
 }
 
-RouterPrunedLayout make_pruned_layout(int nk, int k) {
+template <typename T, int E, int R>
+int launch_pruned_candidates(const void* logp, int64_t T_, int nk, int k, void* scores, int64_t* indices, void* gates, int norm,
+                             cudaStream_t stream) {
   RouterPrunedLayout L{};
   L.nkp = next_pow2(nk) < 32 ? 32 : next_pow2(nk);
-  L.kp = next_pow2(k);
-  for (int p = 0; p < k; ++p) L.C += k / (p + 1);
-  L.Cp = (L.C + 3) / 4 * 4;
-  L.cta_bytes = static_cast<int>(align_up(static_cast<size_t>(L.Cp) * 2 + static_cast<size_t>(k) * 4, 16));
   L.off_ids = 2 * L.nkp * 4;
-  L.off_win = L.off_ids + 2 * L.nkp * 2;
-  L.off_cs = L.off_win + (L.kp < 32 ? 32 : L.kp) * 8;
-  L.off_tl = L.off_cs + (L.C > 320 ? L.Cp * 4 : 0);  // up to 320 sums live in registers only
-  L.warp_bytes = static_cast<int>(align_up(L.off_tl + (kPrunedTieCap + 4) * 4, 16));
-  return L;
-}
-
-template <typename T, int E, int CPL>
-int launch_pruned_cpl(const void* logp, int64_t T_, int nk, int k, const RouterPrunedLayout& L, void* scores,
-                      int64_t* indices, void* gates, int norm, cudaStream_t stream) {
+  L.off_win = L.off_ids + L.nkp * 2;
+  L.off_runs = L.off_win + 32 * R * 4;
+  L.warp_bytes = L.off_runs + L.nkp * 4;
   const int warps = 4;
-  const int smem = L.cta_bytes + warps * L.warp_bytes;
-  auto kern = router_topk_pruned_kernel<T, E, CPL>;
+  const int smem = warps * L.warp_bytes;
+  auto kern = router_topk_pruned_kernel<T, E, R>;
   FMOE_CUDA_TRY(allow_smem(kern, smem));
   if (norm & kTopkLateWait) FMOE_CUDA_TRY(prefer_smem(kern));
   int per_sm = 1;
@@ -1333,10 +1336,10 @@ int launch_pruned_cpl(const void* logp, int64_t T_, int nk, int k, const RouterP
 template <typename T, int E>
 int launch_pruned(const void* logp, int64_t T_, int nk, int k, void* scores, int64_t* indices, void* gates, int norm,
                   cudaStream_t stream) {
-  const RouterPrunedLayout L = make_pruned_layout(nk, k);
-  if (L.C <= 32 * 4) return launch_pruned_cpl<T, E, 4>(logp, T_, nk, k, L, scores, indices, gates, norm, stream);
-  if (L.C <= 32 * 10) return launch_pruned_cpl<T, E, 10>(logp, T_, nk, k, L, scores, indices, gates, norm, stream);
-  return launch_pruned_cpl<T, E, 22>(logp, T_, nk, k, L, scores, indices, gates, norm, stream);
+  if (k <= 16) return launch_pruned_candidates<T, E, 1>(logp, T_, nk, k, scores, indices, gates, norm, stream);
+  if (k <= 32) return launch_pruned_candidates<T, E, 2>(logp, T_, nk, k, scores, indices, gates, norm, stream);
+  if (k <= 64) return launch_pruned_candidates<T, E, 4>(logp, T_, nk, k, scores, indices, gates, norm, stream);
+  return launch_pruned_candidates<T, E, 8>(logp, T_, nk, k, scores, indices, gates, norm, stream);
 }
 
 template <typename T, int E, int CPL = 0>
@@ -1415,18 +1418,8 @@ int launch_typed(const void* logp, int64_t T_, int nk, int k, void* scores, int6
                  cudaStream_t stream) {
   if constexpr (sizeof(T) == 2) {
     // Not where there is little to drop: one key per lane (20000 x 32 keys top-4: 27 us, 32 pruned), or more than half of a
-    // short row wanted (4096 x 128 top-128: 30 us, 33 pruned; 16384 x 100 top-70 69, 73).
-    // Of rows of 65 to 128 keys with the candidates in registers (k of 35 to 71), the whole sort takes fewer instructions in
-    // all and the pruned one a shorter chain per token, so the first is faster once the tokens are more than one wave of the
-    // pruned one (28 warps per SM): whole and pruned, 16384 x 128 top-64 52.9 and 63.9 us, top-40 52.5 and 57.5; 4700 x 128
-    // top-64 17.8 and 22.3; 4096 17.5 and 17.6, top-40 17.4 and 16.2; 64 tokens 8.1 and 7.8.  Beside a GEMM the pruned one's
-    // smaller shared memory counts whatever the number of tokens (layer of 4096 tokens, 128 keys, top-64: 209.8 and 205.2).
-    bool many = nk > 64 && nk <= 128 && !(norm & kTopkLateWait) && T_ > static_cast<int64_t>(device_sm_count()) * 28;
-    if (many) {
-      const int cells = make_pruned_layout(nk, k).C;
-      many = cells > 128 && cells <= 320;
-    }
-    const bool prune = nk > 32 && (nk > 128 || 2 * k <= nk) && !many;
+    // short row wanted (4096 x 128 top-128: 30 us, 33 pruned; 16384 x 100 top-70 69, 73; both with an earlier form of it).
+    const bool prune = nk > 32 && (nk > 128 || 2 * k <= nk);
     if (nk <= 1024 && k <= kPrunedMaxK && prune) {
       switch ((next_pow2(nk) < 32 ? 32 : next_pow2(nk)) / 32) {
         case 2: return launch_pruned<T, 2>(logp, T_, nk, k, scores, indices, gates, norm, stream);
