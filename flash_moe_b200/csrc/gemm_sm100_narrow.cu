@@ -208,8 +208,58 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
   const bool n_ok = n < ep.n_valid && lane_ok;
   const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
   T* otile = reinterpret_cast<T*>(gen);   // [sh.bn][BLOCK_R]: the ring is free once the accumulator is complete
+  // 16 token columns at a time: the sums of the next batch and their addends are requested before this batch is worked on
+  // (777 tokens, 1000 x 2728 and back: layer 65.5 -> 59.4 us), the first batch's addends while the MMAs still run
+  constexpr int CH = 16;
+  struct Batch {
+    uint32_t a[CH], b[CH];
+    float ad[CH];
+    uint16_t rs[CH];
+  };
+  auto request_addends = [&](int c0, Batch& t) {
+    if (EPI == NARROW_ADD) {
+      const int lim = sh.M - (t0 + c0);
+      const int64_t o = static_cast<int64_t>(t0 + c0) * ep.n_valid + n;
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const bool in = n_ok && i < lim;
+        t.ad[i] = (in && ep.addend != nullptr) ? ld_after_wait(ep.addend + o + static_cast<int64_t>(i) * ep.n_valid) : 0.f;
+        t.rs[i] = (in && ep.residual != nullptr)
+                      ? ld_after_wait(static_cast<const uint16_t*>(ep.residual) + o + static_cast<int64_t>(i) * ep.n_valid) : 0;
+      }
+    }
+  };
+  auto request_sums = [&](int c0, Batch& t) {
+    ptx::tmem_ld_32x16(taddr + c0, t.a);
+    if (NB == 2) ptx::tmem_ld_32x16(taddr + sh.acc_cols + c0, t.b);
+  };
+  auto finish = [&](int c0, const Batch& t) {
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      const float v = __uint_as_float(t.a[i]);
+      float r = v;
+      if (EPI == NARROW_SWIGLU) r = silu_f32(v) * __uint_as_float(t.b[i]);
+      if (EPI == NARROW_ADD) r = v + t.ad[i] + to_f32<T>(*reinterpret_cast<const T*>(&t.rs[i]));
+      if (lane_ok) {
+        if (EPI == NARROW_RAW) reinterpret_cast<float*>(gen)[(c0 + i) * BLOCK_R + row] = v;
+        else otile[(c0 + i) * BLOCK_R + row] = from_f32<T>(r);
+      }
+    }
+    if (EPI == NARROW_SWIGLU && ep.pre_gate != nullptr) {
+      const int64_t o = static_cast<int64_t>(t0 + c0) * ep.n_valid + n;
+#pragma unroll
+      for (int i = 0; i < CH; ++i)
+        if (n_ok && t0 + c0 + i < sh.M) {
+          static_cast<T*>(ep.pre_gate)[o + static_cast<int64_t>(i) * ep.n_valid] = from_f32<T>(__uint_as_float(t.a[i]));
+          static_cast<T*>(ep.pre_up)[o + static_cast<int64_t>(i) * ep.n_valid] = from_f32<T>(__uint_as_float(t.b[i]));
+        }
+    }
+  };
   bool done = true;
   if (epilogue_warp) {
+    Batch even, odd;
+    const int first = turn * CH;
+    if (first < sh.bn) request_addends(first, even);
     done = ptx::mbar_wait_bounded(tfull_bar, 0u, abort_flag);
     done = __all_sync(kFull, done);
     ptx::tc_fence_after();
@@ -217,63 +267,24 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
     if (!done && threadIdx.x == 64)
       for (int j = nkb > sh.stages ? nkb - sh.stages : 0; j < nkb; ++j)
         ptx::mbar_wait_drain(full_bar(j % sh.stages), (j / sh.stages) & 1u);
-  }
-  // COUNT token columns from c0 from their float32 sums.  ad / rs: addend and residual.
-  auto fetch_addends = [&](int c0, auto& ad, auto& rs) {
-    constexpr int COUNT = sizeof(ad) / sizeof(float);
-    if (EPI == NARROW_ADD) {
-      const int lim = min(sh.bn - c0, sh.M - (t0 + c0));
-      const int64_t o = static_cast<int64_t>(t0 + c0) * ep.n_valid + n;
-#pragma unroll
-      for (int i = 0; i < COUNT; ++i) {
-        const bool in = n_ok && i < lim;
-        ad[i] = (in && ep.addend != nullptr) ? ld_after_wait(ep.addend + o + static_cast<int64_t>(i) * ep.n_valid) : 0.f;
-        rs[i] = 0.f;
-        if (in && ep.residual != nullptr) {
-          const uint16_t raw = ld_after_wait(static_cast<const uint16_t*>(ep.residual) + o + static_cast<int64_t>(i) * ep.n_valid);
-          rs[i] = to_f32<T>(*reinterpret_cast<const T*>(&raw));
-        }
-      }
-    }
-  };
-  auto finish = [&](int c0, const auto& v, const auto& u, const auto& ad, const auto& rs) {
-    constexpr int COUNT = sizeof(ad) / sizeof(float);
-    const int lim = sh.bn - c0;
-#pragma unroll
-    for (int i = 0; i < COUNT; ++i) {
-      const float r = EPI == NARROW_SWIGLU ? silu_f32(v[i]) * u[i] : v[i] + ad[i] + rs[i];
-      if (lane_ok && i < lim) {
-        if (EPI == NARROW_RAW) reinterpret_cast<float*>(gen)[(c0 + i) * BLOCK_R + row] = v[i];
-        else otile[(c0 + i) * BLOCK_R + row] = from_f32<T>(r);
-      }
-    }
-    if (EPI == NARROW_SWIGLU && ep.pre_gate != nullptr) {
-      const int64_t o = static_cast<int64_t>(t0 + c0) * ep.n_valid + n;
-#pragma unroll
-      for (int i = 0; i < COUNT; ++i)
-        if (n_ok && i < lim && t0 + c0 + i < sh.M) {
-          static_cast<T*>(ep.pre_gate)[o + static_cast<int64_t>(i) * ep.n_valid] = from_f32<T>(v[i]);
-          static_cast<T*>(ep.pre_up)[o + static_cast<int64_t>(i) * ep.n_valid] = from_f32<T>(u[i]);
-        }
-    }
-  };
-  constexpr int CH = 16;  // token columns per batch
-  if (epilogue_warp && done) {
+    if (done && first < sh.bn) {
+      request_sums(first, even);
 #pragma unroll 1
-    for (int c0 = turn * CH; c0 < sh.bn; c0 += 2 * CH) {
-      float ad[CH], rs[CH];
-      fetch_addends(c0, ad, rs);
-      uint32_t a[CH], b[CH];
-      ptx::tmem_ld_32x16(taddr + c0, a);
-      if (NB == 2) ptx::tmem_ld_32x16(taddr + sh.acc_cols + c0, b);
-      ptx::tmem_ld_wait();
-      float v[CH], u[CH];
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        v[i] = __uint_as_float(a[i]);
-        u[i] = NB == 2 ? __uint_as_float(b[i]) : 0.f;
+      for (int c0 = first; c0 < sh.bn; c0 += 4 * CH) {  // sh.bn is a multiple of CH
+        ptx::tmem_ld_wait();
+        if (c0 + 2 * CH < sh.bn) {
+          request_sums(c0 + 2 * CH, odd);
+          request_addends(c0 + 2 * CH, odd);
+        }
+        finish(c0, even);
+        if (c0 + 2 * CH >= sh.bn) break;
+        ptx::tmem_ld_wait();
+        if (c0 + 4 * CH < sh.bn) {
+          request_sums(c0 + 4 * CH, even);
+          request_addends(c0 + 4 * CH, even);
+        }
+        finish(c0 + 2 * CH, odd);
       }
-      finish(c0, v, u, ad, rs);
     }
   }
 
