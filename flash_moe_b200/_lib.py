@@ -21,6 +21,7 @@ NUM_STAGES = 6
 STAGE_NAMES = ("router_front", "router_topk", "expert_scores", "expert_accum", "mlp_up", "mlp_down")
 
 ERR_UNSUPPORTED = 2  # fmoe_error: a shape/dtype combination no kernel covers
+ERR_ALIGNMENT = 4  # fmoe_error: pointer or row pitch not 16-byte aligned
 STATUS_BAD_EXPERT_ID = 1
 STATUS_WAIT_TIMEOUT = 2
 STATUS_BAD_ROW_INDEX = 4
@@ -78,6 +79,9 @@ assert LAYER_ARGS.size == ctypes.sizeof(LayerArgs)
 # fmoe_train_args: 22 pointers and sizes up to stream, num_tokens, num_experts, six int32
 TRAIN_ARGS = struct.Struct("@22Q2q6i")
 
+# fmoe_dense_backward_args: 17 pointers and the stream, num_tokens, three int32
+DENSE_BACKWARD_ARGS = struct.Struct("@18Qq3i")
+
 _P = ctypes.c_void_p
 _I = ctypes.c_int
 _L = ctypes.c_int64
@@ -108,6 +112,7 @@ SIGNATURES = {
     "fmoe_train_forward": (_I, [ctypes.c_char_p, ctypes.POINTER(_I)]),
     "fmoe_train_backward_workspace_bytes": (_Z, [_L, _I, _L, _I, _I]),
     "fmoe_train_backward": (_I, [ctypes.c_char_p]),
+    "fmoe_dense_backward_f32": (_I, [ctypes.c_char_p]),
     "fmoe_gather_probe": (_I, [_P, _L, _P, _L, _I, _I, _I, _P, _P, _P]),
     "fmoe_rms_norm": (_I, [_P, _P, _P, _I, _L, _I, _F, _P]),
     "fmoe_selftest_wait_timeout": (_I, [ctypes.c_uint64, _P, _P, _P]),

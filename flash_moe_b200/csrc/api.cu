@@ -360,6 +360,11 @@ int fmoe_swiglu_backward_rows(const void* dh, const void* a, const void* b, void
                                 h, dtype, num_rows * intermediate, intermediate, static_cast<cudaStream_t>(stream));
 }
 
+int fmoe_dense_backward_f32(const fmoe_dense_backward_args* args) {
+  if (args == nullptr) return FMOE_ERR_BAD_ARG;
+  return launch_dense_backward_f32(*args);
+}
+
 int fmoe_gather_probe(const void* table, int64_t num_rows, const int32_t* row_ids, int64_t count, int row_bytes,
                       int ctas_per_sm, int mode, float* sink, int32_t* status, fmoe_stream_t stream) {
   return launch_gather_probe(table, num_rows, row_ids, count, row_bytes, ctas_per_sm, mode, sink, status,

@@ -289,6 +289,7 @@ int launch_router_chain_backward(const void* dgates, const void* gates, const in
 // row > 0: da and db are the halves of rows of 2 * row elements (db = da + row)
 int launch_swiglu_backward(const void* dh, const void* a, const void* b, void* da, void* db, void* h, int dtype,
                            int64_t n, int64_t row, cudaStream_t stream);
+int launch_dense_backward_f32(const fmoe_dense_backward_args& args);  // sgemm_grad.cu
 int launch_gather_probe(const void* table, int64_t num_rows, const int32_t* row_ids, int64_t count, int row_bytes,
                         int ctas_per_sm, int mode, float* sink, int32_t* status, cudaStream_t stream);
 int launch_rms_norm(const void* x, const void* weight, void* out, int dtype, int64_t ntok, int H, float eps,

@@ -26,6 +26,14 @@ def _pack(ctx, x, lp, weights, y, pre, extra, ws, stream_dev):
         _lib.status_ptr(stream_dev), _lib.current_stream_ptr(stream_dev), *ctx.dims)
 
 
+def _own_float32_products(T, H, I):
+    """Whether a float32 step takes its dense gradients from fmoe_dense_backward_f32: two launches instead of eight, while the
+    host sets the pace.  500 tokens x 512 x 768: 116 us of kernels and 110 for the library's, a step 613 -> 508; from about
+    2.5e8 multiply-adds a product on the library's larger tiles gain more than its launches cost (1000 x 1024 x 2048: 680 and
+    534 us).  Not where the caller lets torch round the operands to TF32."""
+    return T * H * I <= 250_000_000 and not torch.backends.cuda.matmul.allow_tf32
+
+
 class LayerTrainingStep(torch.autograd.Function):
     """(y [T, H], router_logits [T, 2 nk], indices [T, k], gates [T, k]) from the layer input x, the normalised input xn and
     the weights."""
@@ -95,13 +103,29 @@ class LayerTrainingStep(torch.autograd.Function):
             a, b = rest[8:10]
         else:
             a, b = torch.mm(x, wg.t()), torch.mm(x, wu.t())
-        dh = torch.mm(dy, wd)
+        need = ctx.needs_input_grad
         dab, h = x.new_empty((T, 2 * I)), torch.empty_like(a)
+        if x.dtype == wr.dtype == xn.dtype == torch.float32 and _own_float32_products(T, H, I):
+            xn, wr = xn.contiguous(), wr.contiguous()
+            dxn = torch.empty_like(xn) if need[1] else None
+            dw = x.new_empty((2 * I, H)) if need[3] or need[4] else None
+            dwd = torch.empty_like(wd) if need[5] else None
+            dwr = torch.empty_like(wr) if need[2] else None
+            ptr = _lib.ptr
+            rc = _lib.call_struct("fmoe_dense_backward_f32", dev, _lib.DENSE_BACKWARD_ARGS.pack(
+                dy.data_ptr(), x.data_ptr(), a.data_ptr(), b.data_ptr(), wg.data_ptr(), wu.data_ptr(), wd.data_ptr(),
+                dlogits.data_ptr(), xn.data_ptr(), wr.data_ptr(), dab.data_ptr(), h.data_ptr(), dx.data_ptr() if need[0] else 0,
+                ptr(dxn) or 0, ptr(dw) or 0, ptr(dwd) or 0, ptr(dwr) or 0, _lib.current_stream_ptr(dev), T, H, I, 2 * nk))
+            if rc == 0:
+                dwg, dwu = (dw[:I], dw[I:]) if dw is not None else (None, None)
+                return dx, dxn, dwr, dwg, dwu, dwd, dde, due, None, None, None
+            if rc not in (_lib.ERR_UNSUPPORTED, _lib.ERR_ALIGNMENT):  # those: rows that are not whole aligned 16-byte pieces
+                _lib.check(rc, "fmoe_dense_backward_f32")
+        dh = torch.mm(dy, wd)
         rc = _lib.call("fmoe_swiglu_backward_rows", dev, dh.data_ptr(), a.data_ptr(), b.data_ptr(), dab.data_ptr(),
                        h.data_ptr(), code, T, I)
         if rc:
             _lib.check(rc, "fmoe_swiglu_backward_rows")
-        need = ctx.needs_input_grad
         dwd = torch.mm(dy.t(), h) if need[5] else None
         dwg = dwu = None
         if need[3] or need[4]:

@@ -156,6 +156,25 @@ int fmoe_swiglu_backward_rows(const void* dh, const void* a, const void* b, void
                               int intermediate, fmoe_stream_t stream);
 
 /*
+ * The dense gradients of a float32 layer in two launches (autograd of flash_moe/modules/flash_moe.py:65-66,:95-101 with
+ * flash_mlp.py:52-102 between the products): with dh = dy down_w,
+ *   dab = [dh * up_pre * silu'(gate_pre) | dh * silu(gate_pre)], h = silu(gate_pre) * up_pre       (scratch, [T, 2 I], [T, I])
+ *   dx += dab[:, :I] gate_w + dab[:, I:] up_w,  dgate_up_w [2 I, H] = dab^T x,  ddown_w [H, I] = dy^T h,
+ *   dxn [T, H] = dlogits router_w,  drouter_w [R, H] = dlogits^T xn.
+ * A null output is left out; dlogits, xn and router_w may be null when both router gradients are.  hidden, intermediate and
+ * (with a router gradient) router_rows are multiples of 4, rows contiguous and 16-byte aligned; others are refused.
+ */
+typedef struct fmoe_dense_backward_args {
+  const void *dy, *x, *gate_pre, *up_pre, *gate_w, *up_w, *down_w, *dlogits, *xn, *router_w;
+  void *dab, *h;
+  void *dx, *dxn, *dgate_up_w, *ddown_w, *drouter_w;
+  fmoe_stream_t stream;
+  int64_t num_tokens;
+  int32_t hidden, intermediate, router_rows;
+} fmoe_dense_backward_args;
+int fmoe_dense_backward_f32(const fmoe_dense_backward_args* args);
+
+/*
  * NOT PART OF THE LAYER - a measurement aid with no counterpart in the reference, exported only so that the
  * benchmark can state the ceiling of the expert step on the GPU it runs on.  A load-only kernel with the access
  * pattern of that step: the rows row_ids[count] (each in [0, num_rows); others read row 0 and raise

@@ -347,3 +347,47 @@ def test_autocast_selects_on_float32_log_probabilities():
     assert torch.equal(layer.last_indices.cpu(), idx)
     y.float().sum().backward()
     assert torch.isfinite(layer.router_gate.weight.grad.float()).all()
+
+
+@pytest.mark.parametrize("T,H,I,R", [(1, 4, 4, 4), (2, 8, 260, 68), (65, 64, 128, 64), (64, 132, 68, 36), (500, 512, 768, 128)])
+@pytest.mark.parametrize("leave_out", [(), ("dx", "dwd"), ("dxn", "dwr")])
+def test_dense_backward_float32(T, H, I, R, leave_out):
+    """All dense gradients in two launches: partial tiles of 64 in every direction, steps of k cut off inside (T, H, I and R are
+    each somebody's k), outputs left out; float32 sums against float64 ones (5e-6 as for the other float32 sums here)."""
+    from flash_moe_b200 import _lib
+
+    dev = torch.device("cuda")
+    gen = torch.Generator(device=dev).manual_seed(T + H)
+    sizes = dict(dy=(T, H), x=(T, H), a=(T, I), b=(T, I), wg=(I, H), wu=(I, H), wd=(H, I), dl=(T, R), xn=(T, H), wr=(R, H))
+    t = {n: torch.randn(*s, device=dev, generator=gen) for n, s in sizes.items()}
+    outs = dict(dab=(T, 2 * I), h=(T, I), dx=(T, H), dxn=(T, H), dw=(2 * I, H), dwd=(H, I), dwr=(R, H))
+    o = {n: torch.full(s, float("nan"), device=dev) for n, s in outs.items()}
+    o["dx"].copy_(t["x"])  # added to
+    rc = _lib.call_struct("fmoe_dense_backward_f32", dev, _lib.DENSE_BACKWARD_ARGS.pack(
+        *[v.data_ptr() for v in t.values()], *[0 if n in leave_out else v.data_ptr() for n, v in o.items()],
+        _lib.current_stream_ptr(torch.device("cuda", torch.cuda.current_device())), T, H, I, R))
+    assert rc == 0
+    d = {n: v.double() for n, v in t.items()}
+    sig = torch.sigmoid(d["a"])
+    dh, act = d["dy"] @ d["wd"], d["a"] * sig
+    da, db, h = dh * d["b"] * (sig * (1 + d["a"] * (1 - sig))), dh * act, act * d["b"]
+    dab = torch.cat([da, db], 1)
+    want = dict(dab=dab, h=h, dx=d["x"] + da @ d["wg"] + db @ d["wu"], dxn=d["dl"] @ d["wr"], dw=dab.t() @ d["x"],
+                dwd=d["dy"].t() @ h, dwr=d["dl"].t() @ d["xn"])
+    for n, w in want.items():
+        if n in leave_out:
+            assert n == "dx" or torch.isnan(o[n]).all()
+        else:
+            assert (o[n].double() - w).norm() <= 5e-6 * w.norm(), n
+
+
+def test_dense_backward_float32_refuses_ragged_rows():
+    from flash_moe_b200 import _lib
+
+    dev = torch.device("cuda", torch.cuda.current_device())
+    z = [torch.zeros(64, 64, device=dev).data_ptr()] * 17
+    pack = lambda *n: _lib.DENSE_BACKWARD_ARGS.pack(*z, _lib.current_stream_ptr(dev), *n)
+    assert _lib.call_struct("fmoe_dense_backward_f32", dev, pack(4, 6, 8, 8)) == _lib.ERR_UNSUPPORTED
+    assert _lib.call_struct("fmoe_dense_backward_f32", dev, pack(4, 8, 8, 6)) == _lib.ERR_UNSUPPORTED
+    z[3] += 4
+    assert _lib.call_struct("fmoe_dense_backward_f32", dev, pack(4, 8, 8, 8)) == _lib.ERR_ALIGNMENT
