@@ -120,11 +120,9 @@ __device__ __forceinline__ void store_add_chunk_smem(uint32_t taddr_chunk, T* or
 }
 
 // The accumulator holds NCOLS / 2 gate columns followed by NCOLS / 2 up columns of the same outputs:
-// out[row, col_base .. col_base + NCOLS / 2) = T(silu(gate) * up); grow / urow (nullable, both or neither) receive
-// the two pre-activations rounded to T.
+// out[row, col_base .. col_base + NCOLS / 2) = T(silu(gate) * up).
 template <typename T, int NCOLS>
-__device__ __forceinline__ void store_swiglu_row(uint32_t taddr, T* orow, T* grow, T* urow, int col_base, int n_valid,
-                                                 bool row_ok) {
+__device__ __forceinline__ void store_swiglu_row(uint32_t taddr, T* orow, int col_base, int n_valid, bool row_ok) {
 #pragma unroll 1
   for (int c = 0; c < NCOLS / 64; ++c) {
     uint32_t g[32], u[32];
@@ -138,19 +136,7 @@ __device__ __forceinline__ void store_swiglu_row(uint32_t taddr, T* orow, T* gro
         float f[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] = silu_f32(__uint_as_float(g[v * 8 + i])) * __uint_as_float(u[v * 8 + i]);
-        if (col0 + v * 8 < n_valid) {
-          *reinterpret_cast<uint4*>(orow + col0 + v * 8) = pack16<T>(f);
-          if (grow != nullptr) {
-            float fg[8], fu[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              fg[i] = __uint_as_float(g[v * 8 + i]);
-              fu[i] = __uint_as_float(u[v * 8 + i]);
-            }
-            *reinterpret_cast<uint4*>(grow + col0 + v * 8) = pack16<T>(fg);
-            *reinterpret_cast<uint4*>(urow + col0 + v * 8) = pack16<T>(fu);
-          }
-        }
+        if (col0 + v * 8 < n_valid) *reinterpret_cast<uint4*>(orow + col0 + v * 8) = pack16<T>(f);
       }
     }
   }
@@ -194,9 +180,9 @@ inline int make_tensor_map(CUtensorMap* m, const void* basep, int dtype, uint64_
   return r == CUDA_SUCCESS ? FMOE_OK : FMOE_ERR_BAD_ARG;
 }
 
-// 2-D 16-bit output written by tiled stores: boxes of box_cols x box_rows elements, no swizzle
+// 2-D 16-bit output written by tiled stores: boxes of box_cols x box_rows elements, as a rule without swizzle
 inline int make_tensor_map_out(CUtensorMap* m, const void* basep, int dtype, uint64_t cols, uint64_t rows, uint32_t box_cols,
-                               uint32_t box_rows) {
+                               uint32_t box_rows, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (fn == nullptr) return -static_cast<int>(cudaErrorNotSupported);
   const cuuint64_t dims[2] = {cols, rows};
@@ -206,7 +192,7 @@ inline int make_tensor_map_out(CUtensorMap* m, const void* basep, int dtype, uin
   const CUtensorMapDataType dt = dtype == FMOE_DTYPE_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                  : dtype == FMOE_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const CUresult r = fn(m, dt, 2, const_cast<void*>(basep), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                        swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? FMOE_OK : FMOE_ERR_BAD_ARG;
 }
 

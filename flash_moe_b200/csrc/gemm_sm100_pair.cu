@@ -39,7 +39,17 @@ constexpr int ADDEND_BUFS = 2;  // four (with a five-stage ring) measured the sa
 constexpr int ADDEND_BYTES = ADDEND_BUFS * ADDEND_CHUNK_BYTES;  // chunks on their way while one is being added
 constexpr int smem_bytes(int addend_bytes) { return RING_BYTES + addend_bytes + 256 + 1024; }
 
-enum { PAIR_EPI_ADD = 0, PAIR_EPI_SWIGLU = 1 };
+constexpr int KEEP_BYTES = 4 * 3 * 32 * 64;  // per epilogue warp: 32 rows x 32 columns of three 16-bit outputs
+
+// SWIGLU_KEEP: the two products are stored as well, for the backward pass
+enum { PAIR_EPI_ADD = 0, PAIR_EPI_SWIGLU = 1, PAIR_EPI_SWIGLU_KEEP = 2 };
+// what SWIGLU does not take is for CTAs of a kernel beside this one
+template <int EPI>
+constexpr int kEpilogueBytes = EPI == PAIR_EPI_ADD ? ADDEND_BYTES : EPI == PAIR_EPI_SWIGLU_KEEP ? KEEP_BYTES : 0;
+
+struct PairKeep {  // SWIGLU_KEEP: boxes of 32 rows x 32 columns, 64-byte swizzle
+  CUtensorMap h, gate, up;
+};
 
 struct PairEpi {
   void* out;
@@ -47,8 +57,6 @@ struct PairEpi {
   const void* residual;  // ADD only, nullable: [M, ldo] in the module dtype, added before the single rounding
   int64_t ldo;
   int n_valid;
-  void* pre_gate;  // SWIGLU only, nullable: x Wg^T and x Wu^T rounded to T, kept for the backward pass
-  void* pre_up;
   int release_next;  // the next kernel may become resident at once and run beside this one
 };
 
@@ -72,12 +80,13 @@ template <int EPI, typename T>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB0,
                          const __grid_constant__ CUtensorMap tmB1, PairEpi ep, int M, int num_m_tiles, int num_n_tiles,
-                         int num_k_blocks, int32_t* status) {
+                         int num_k_blocks, int32_t* status, const __grid_constant__ PairKeep keep) {
+  constexpr bool kSwiglu = EPI != PAIR_EPI_ADD;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_u32 = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw_u32 + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - raw_u32);
-  constexpr int kAddend = EPI == PAIR_EPI_ADD ? ADDEND_BYTES : 0;  // the rest is for CTAs of a kernel beside this one
+  constexpr int kAddend = kEpilogueBytes<EPI>;
   const uint32_t bar_base = base + RING_BYTES + kAddend;
   auto a_smem = [&](int s) { return base + s * STAGE_BYTES; };
   auto b_smem = [&](int s) { return base + s * STAGE_BYTES + A_BYTES; };
@@ -110,7 +119,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     ptx::mbar_fence_init();
     ptx::prefetch_tensormap(&tmA);
     ptx::prefetch_tensormap(&tmB0);
-    if (EPI == PAIR_EPI_SWIGLU || ep.addend != nullptr) ptx::prefetch_tensormap(&tmB1);  // ADD: the addend's map
+    if (kSwiglu || ep.addend != nullptr) ptx::prefetch_tensormap(&tmB1);  // ADD: the addend's map
   }
   if (warp == 1) {
     ptx::tmem_alloc_pair(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
@@ -140,7 +149,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           if (rank == 0) ptx::mbar_arrive_expect_tx(full_bar(s), 2 * STAGE_BYTES);
           const uint32_t leader_full = ptx::map_to_cta(full_bar(s), 0);
           ptx::tma_load_2d_pair(a_smem(s), &tmA, leader_full, kb * BLOCK_K, a_row);
-          if (EPI == PAIR_EPI_SWIGLU) {
+          if (kSwiglu) {
             // N columns 0..127 = gate rows (leader), 128..255 = up rows (peer) of the same 128 outputs
             ptx::tma_load_2d_pair(b_smem(s), rank == 0 ? &tmB0 : &tmB1, leader_full, kb * BLOCK_K,
                                   n_tile * (BLOCK_N / 2));
@@ -225,9 +234,47 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       T* orow = static_cast<T*>(ep.out) + row * ep.ldo;
       if constexpr (EPI == PAIR_EPI_SWIGLU) {
         if (!wait_accumulator()) break;
-        T* grow = ep.pre_gate != nullptr ? static_cast<T*>(ep.pre_gate) + row * ep.ldo : nullptr;
-        T* urow = ep.pre_up != nullptr ? static_cast<T*>(ep.pre_up) + row * ep.ldo : nullptr;
-        epi::store_swiglu_row<T, BLOCK_N>(taddr, orow, grow, urow, n_tile * (BLOCK_N / 2), ep.n_valid, row_ok);
+        epi::store_swiglu_row<T, BLOCK_N>(taddr, orow, n_tile * (BLOCK_N / 2), ep.n_valid, row_ok);
+      } else if constexpr (EPI == PAIR_EPI_SWIGLU_KEEP) {
+        // Three outputs stored one row per thread, 16 bytes apart in 32 rows per instruction, take longer than the tile's main
+        // loop (4096 tokens, 1024 x 4096: 83 us, 48 with h alone).  Each warp lays 32 rows x 32 columns of them out in shared
+        // memory (64-byte swizzle: piece j of row r at j xor (r / 2 mod 4), free of conflicts) and TMA stores them: 54 us.
+        if (!wait_accumulator()) break;
+        const int row0 = m_tile * (2 * BLOCK_M) + static_cast<int>(rank) * BLOCK_M + q * 32;
+        uint8_t* boxes = gen + RING_BYTES + (warp - 2) * (KEEP_BYTES / 4);
+        const uint32_t boxes_u32 = base + RING_BYTES + (warp - 2) * (KEEP_BYTES / 4);
+#pragma unroll 1
+        for (int c = 0; c < BLOCK_N / 64; ++c) {
+          uint32_t g[32], u[32];
+          ptx::tmem_ld_32x32(taddr + c * 32, g);
+          ptx::tmem_ld_32x32(taddr + BLOCK_N / 2 + c * 32, u);
+          ptx::tmem_ld_wait();
+          if (lane == 0) ptx::tma_store_wait();  // the boxes of the chunk before have been read
+          __syncwarp();
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            float fh[8], fg[8], fu[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              fg[i] = __uint_as_float(g[v * 8 + i]);
+              fu[i] = __uint_as_float(u[v * 8 + i]);
+              fh[i] = silu_f32(fg[i]) * fu[i];
+            }
+            uint4* at = reinterpret_cast<uint4*>(boxes + lane * 64 + ((v ^ (lane >> 1 & 3)) << 4));
+            at[0] = pack16<T>(fh);
+            at[2048 / 16] = pack16<T>(fg);
+            at[4096 / 16] = pack16<T>(fu);
+          }
+          ptx::fence_async_smem();
+          __syncwarp();
+          const int col0 = n_tile * (BLOCK_N / 2) + c * 32;
+          if (lane == 0 && row0 < M && col0 < ep.n_valid) {
+            ptx::tma_store_2d(&keep.h, boxes_u32, col0, row0);
+            ptx::tma_store_2d(&keep.gate, boxes_u32 + 2048, col0, row0);
+            ptx::tma_store_2d(&keep.up, boxes_u32 + 4096, col0, row0);
+            ptx::tma_store_commit();
+          }
+        }
       } else {
         const T* rrow = (ep.residual != nullptr && row_ok) ? static_cast<const T*>(ep.residual) + row * ep.ldo : nullptr;
         if (ep.addend == nullptr) {
@@ -289,6 +336,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive_cluster(ptx::map_to_cta(tempty_bar(acc), 0));
     }
+    if (EPI == PAIR_EPI_SWIGLU_KEEP && lane == 0) ptx::tma_store_wait();
   }
 
   // ---------------------------------------------------------------- teardown
@@ -309,9 +357,9 @@ int make_map(CUtensorMap* m, const void* basep, int dtype, uint64_t cols, uint64
 
 template <int EPI, typename T>
 int launch_pair(const CUtensorMap& tA, const CUtensorMap& tB0, const CUtensorMap& tB1, const PairEpi& ep, int64_t M,
-                int num_n_tiles, int K, int32_t* status, cudaStream_t stream) {
+                int num_n_tiles, int K, int32_t* status, cudaStream_t stream, const PairKeep& keep = PairKeep{}) {
   auto kern = gemm_tcgen05_pair_kernel<EPI, T>;
-  const int smem = smem_bytes(EPI == PAIR_EPI_ADD ? ADDEND_BYTES : 0);
+  const int smem = smem_bytes(kEpilogueBytes<EPI>);
   FMOE_CUDA_TRY(allow_smem(kern, smem));
   if (ep.release_next) FMOE_CUDA_TRY(prefer_smem(kern));
   const int num_m_tiles = static_cast<int>((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M));
@@ -320,7 +368,7 @@ int launch_pair(const CUtensorMap& tA, const CUtensorMap& tB0, const CUtensorMap
   const int max_pairs = device_sm_count() / 2;
   const int pairs = static_cast<int>(tiles < max_pairs ? tiles : max_pairs);
   FMOE_CUDA_TRY(launch_pdl(16, kern, dim3(2 * pairs), dim3(kThreads), smem, stream, 2, tA, tB0, tB1, ep,
-                           static_cast<int>(M), num_m_tiles, num_n_tiles, num_k_blocks, status));
+                           static_cast<int>(M), num_m_tiles, num_n_tiles, num_k_blocks, status, keep));
   return FMOE_OK;
 }
 
@@ -339,8 +387,18 @@ int launch_gemm_swiglu_pair(const void* x, const void* gate_w, const void* up_w,
   if ((rc = make_map(&tG, gate_w, dtype, K, I, BLOCK_N / 2)) != FMOE_OK) return rc;
   if ((rc = make_map(&tU, up_w, dtype, K, I, BLOCK_N / 2)) != FMOE_OK) return rc;
   if ((pre_gate == nullptr) != (pre_up == nullptr)) return FMOE_ERR_BAD_ARG;
-  PairEpi ep{h, nullptr, nullptr, I, I, pre_gate, pre_up, release_next ? 1 : 0};
+  PairEpi ep{h, nullptr, nullptr, I, I, release_next ? 1 : 0};
   const int n_tiles = (I + 127) / 128;
+  if (pre_gate != nullptr) {
+    PairKeep keep;
+    const void* outs[3] = {h, pre_gate, pre_up};
+    CUtensorMap* maps[3] = {&keep.h, &keep.gate, &keep.up};
+    for (int i = 0; i < 3; ++i)
+      if ((rc = epi::make_tensor_map_out(maps[i], outs[i], dtype, I, M, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B)) != FMOE_OK) return rc;
+    if (dtype == FMOE_DTYPE_BF16)
+      return launch_pair<PAIR_EPI_SWIGLU_KEEP, __nv_bfloat16>(tA, tG, tU, ep, M, n_tiles, K, status, stream, keep);
+    return launch_pair<PAIR_EPI_SWIGLU_KEEP, __half>(tA, tG, tU, ep, M, n_tiles, K, status, stream, keep);
+  }
   if (dtype == FMOE_DTYPE_BF16)
     return launch_pair<PAIR_EPI_SWIGLU, __nv_bfloat16>(tA, tG, tU, ep, M, n_tiles, K, status, stream);
   return launch_pair<PAIR_EPI_SWIGLU, __half>(tA, tG, tU, ep, M, n_tiles, K, status, stream);
@@ -352,7 +410,7 @@ int launch_gemm_add_pair(const void* a, const void* b, const float* addend, void
   int rc;
   if ((rc = make_map(&tA, a, dtype, K, M, BLOCK_M)) != FMOE_OK) return rc;
   if ((rc = make_map(&tB, b, dtype, K, N, BLOCK_N / 2)) != FMOE_OK) return rc;
-  PairEpi ep{out, addend, residual, N, N, nullptr, nullptr, 0};
+  PairEpi ep{out, addend, residual, N, N, 0};
   const int n_tiles = (N + 255) / 256;
   CUtensorMap tC = tB;  // third slot: the float32 addend's map (unused without an addend)
   if (addend != nullptr && (rc = epi::make_tensor_map_f32(&tC, addend, N, M, N, BLOCK_M)) != FMOE_OK) return rc;

@@ -349,6 +349,25 @@ def test_autocast_selects_on_float32_log_probabilities():
     assert torch.isfinite(layer.router_gate.weight.grad.float()).all()
 
 
+@pytest.mark.parametrize("T,H,I", [(512, 256, 256), (515, 264, 264), (545, 256, 392), (2100, 512, 2048)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_kept_products_of_the_pair_gemm(T, H, I, dtype):
+    """Boxes of 32 rows x 32 columns that end inside, at and beyond the last row and column: the output has the bits of the
+    forward that keeps nothing, the products are the float32 ones rounded once (half a step of the type, and the float32 sums'
+    own rounding where it moves a value across: 1e-6 of the sum of magnitudes)."""
+    from flash_moe_b200.ops.flash_mlp import _mlp_forward
+
+    x, wg, wu, wd = (randn(shape, 20 + i, dtype, sc).cuda()
+                     for i, (shape, sc) in enumerate([((T, H), 1.0), ((I, H), 0.05), ((I, H), 0.05), ((H, I), 0.05)]))
+    out, a, b = _mlp_forward(x, wg, wu, wd, save_preacts=True)
+    assert torch.equal(out, _mlp_forward(x, wg, wu, wd))
+    step = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for got, w in ((a, wg), (b, wu)):
+        want = x.double() @ w.double().t()
+        slack = 1e-6 * (x.double().abs() @ w.double().abs().t())
+        assert ((got.double() - want).abs() <= step * want.abs() + slack + 2.0 ** -24).all()
+
+
 @pytest.mark.parametrize("T,H,I,R", [(1, 4, 4, 4), (2, 8, 260, 68), (65, 64, 128, 64), (64, 132, 68, 36), (500, 512, 768, 128)])
 @pytest.mark.parametrize("leave_out", [(), ("dx", "dwd"), ("dxn", "dwr")])
 def test_dense_backward_float32(T, H, I, R, leave_out):
