@@ -14,7 +14,7 @@
 //
 // Bound by the weight bytes, and with the narrowest tiles by the MMAs that follow one another on the same sums: 1 token, hidden
 // 1024, intermediate 4096 (25 MB of weights, both GEMMs inside a forward, us): 33 -> 17; 64 tokens, 2048 x 5632 (69 MB): 48 ->
-// 29; 777 tokens, 1000 x 2728: 43 -> 40 (128-row token tiles in one or two CTAs per row of tiles before).  The set-up runs
+// 29; 777 tokens, 1000 x 2728: 43 -> 35 (128-row token tiles in one or two CTAs per row of tiles before).  The set-up runs
 // ahead of the predecessor's end: barriers and the first ring of weight tiles need nothing from it.
 #include <algorithm>
 
