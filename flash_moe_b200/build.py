@@ -13,7 +13,7 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libfmoe_sm100a.so")
 SOURCES = ["api.cu", "router_topk.cu", "expert.cu", "gemm_sm100.cu", "gemm_sm100_pair.cu", "gemm_sm100_narrow.cu", "gemm_router_bn.cu", "simt_gemm.cu", "sgemm_grad.cu", "elementwise.cu", "gather_probe.cu", "backward.cu", "noalloc.cu", "selftest.cu"]
-HEADERS = ["common.cuh", "ptx_sm100.cuh", "gemm_epilogue.cuh", "warp_sort.cuh", os.path.join("..", "..", "include", "fmoe.h")]
+HEADERS = ["common.cuh", "ptx_sm100.cuh", "gemm_epilogue.cuh", "warp_sort.cuh", "router_ring.h", os.path.join("..", "..", "include", "fmoe.h")]
 
 
 def _sources():

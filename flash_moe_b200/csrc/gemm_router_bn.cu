@@ -13,6 +13,7 @@
 // Columns of x beyond K arrive as zeros from TMA and are normalised with mean 0 / scale 0, so they stay zero.
 // Every wait is bounded; a wait that runs out raises FMOE_STATUS_WAIT_TIMEOUT and the CTA drains and leaves.
 #include "gemm_epilogue.cuh"
+#include "router_ring.h"
 
 namespace fmoe {
 namespace {
@@ -201,6 +202,7 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     // pieces i, i + 128, ... of the BLOCK_M x 128-byte tile: row (i >> 3) + 16 j, position i & 7.  With the 128-byte swizzle position p of row r holds the
     // features 8 * (p ^ (r & 7)) .. + 7 of the k-block, and r & 7 does not depend on j, so one thread always handles the
     // same eight features.
+    using Waits = NormaliseWaits<kStages, kXformGroups>;  // 6 stages: a stage's uses go from group to group
     constexpr int kGroupThreads = (kXformWarps / kXformGroups) * 32;
     constexpr int kGroupPieces = BLOCK_M * 8 / kGroupThreads;
     const int group = (warp - 2) / (kXformWarps / kXformGroups);
@@ -215,7 +217,8 @@ router_gemm_bn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         const float4 v = *reinterpret_cast<const float4*>(&stats[kb * BLOCK_K + (i >> 1) * 16 + (feat0 >> 3) * 2]);
         mm[i] = v.x; ss[i] = v.y; mm[i + 1] = v.z; ss[i + 1] = v.w;
       }
-      ok = ok && ptx::mbar_wait_bounded(full_bar(s), (kb / kStages) & 1u, abort_flag);
+      if (Waits::behind_empty(kb)) ok = ok && ptx::mbar_wait_bounded(empty_bar(s), Waits::empty_parity(kb), abort_flag);
+      ok = ok && ptx::mbar_wait_bounded(full_bar(s), Waits::full_parity(kb), abort_flag);
       uint4* tile = reinterpret_cast<uint4*>(gen + s * STAGE_BYTES);
       uint4 q[kGroupPieces];
 #pragma unroll

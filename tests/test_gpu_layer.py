@@ -366,7 +366,8 @@ def test_pre_norm_stack_matches_torch_composition():
 
 
 @pytest.mark.parametrize("T,H,I,N,k", [(1, 1024, 4096, 16384, 64), (64, 512, 1000, 4096, 16), (300, 256, 512, 1024, 8),
-                                       (777, 1000, 2728, 10000, 24), (2048, 512, 1024, 4096, 32)])
+                                       (777, 1000, 2728, 10000, 24), (2048, 512, 1024, 4096, 32),
+                                       (16384, 2048, 5632, 65536, 32)])  # slabs, pair GEMMs of several waves
 @pytest.mark.parametrize("graph", [False, True])
 def test_kernels_beside_each_other_see_this_forwards_data(T, H, I, N, k, graph):
     """Kernels of one forward run beside each other; with inputs that change from call to call and nothing between the calls,
@@ -388,6 +389,71 @@ def test_kernels_beside_each_other_see_this_forwards_data(T, H, I, N, k, graph):
             got = [[t.clone() for t in run(x)] for x in xs]
             for (y, logits), (y0, logits0) in zip(got, want):
                 assert torch.equal(logits, logits0) and torch.equal(y, y0)
+
+
+@pytest.mark.parametrize("T,H,N", [(16384, 2048, 65536), (9500, 456, 16384), (20000, 1000, 3600)])
+def test_router_tiles_are_normalised_once_they_have_landed(T, H, N):
+    """128 x 128 tiles of the router GEMM, whose ring is six stages deep for four groups of normalising warps: the same logits
+    from every one of some thousand passes over inputs that do not stay in L2."""
+    from flash_moe_b200 import FlashMoE, FlashMoEConfig, check_status
+
+    torch.manual_seed(T)
+    with torch.device("cuda"):
+        layer = FlashMoE(FlashMoEConfig(H, 64, "silu", N, 1, False)).bfloat16().eval()
+        layer.router_norm.running_mean.normal_().mul_(0.1)
+        layer.router_norm.running_var.uniform_(0.5, 2.0)
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    xs = [torch.randn(1, T, H, device="cuda", dtype=torch.bfloat16, generator=gen) for _ in range(3)]
+    wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+    bn = layer.router_norm
+    with torch.no_grad():
+        want = []
+        for x in xs:
+            want.append(layer(x)[1].clone())
+            xn = ((x[0].float() - bn.running_mean.float()) / torch.sqrt(bn.running_var.float() + bn.eps)).bfloat16()
+            exact = xn.double() @ layer.router_gate.weight.double().t()
+            got = want[-1].transpose(0, 1).reshape(T, -1).double()
+            # one rounding of the sum: half a unit of bf16 in the last place, doubled for features of xn at a rounding boundary
+            assert ((got - exact).abs() <= 2.0**-8 * exact.abs() + 2.0**-8 * exact.std()).all()
+        for i in range(1500):
+            wrong += (layer(xs[i % 3])[1] != want[i % 3]).any()
+    assert int(wrong) == 0
+    check_status()
+
+
+def test_stack_of_many_tokens_repeats_itself_and_the_stages_in_order():
+    """Pre-norm blocks over 16384 tokens, nothing between the passes and scratch memory full of NaN before each: the bits of
+    the same blocks run stage by stage."""
+    from flash_moe_b200 import FlashMoEConfig, check_status
+    from flash_moe_b200.modules.flash_moe import StageTimer
+    from flash_moe_b200.modules.stack import FlashMoEStack
+    from flash_moe_b200.ops.rms_norm import rms_norm
+
+    H = 2048
+    torch.manual_seed(3)
+    with torch.device("cuda"):
+        stack = FlashMoEStack(FlashMoEConfig(H, 1024, "silu", 65536, 32, True), 2, pre_norm=True).bfloat16().eval()
+        xs = [torch.randn(8, 2048, H, dtype=torch.bfloat16) for _ in range(2)]
+    wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+    with torch.no_grad():
+        want = []
+        for x in xs:
+            logits = []
+            for layer, weight in zip(stack.layers, stack.norms):
+                xn = rms_norm(x, weight, stack.norm_eps)
+                torch.cuda.synchronize()
+                x, lg = layer(xn, residual=x, stage_timer=StageTimer())
+                logits.append(lg)
+            want.append([x, *logits])
+        assert all(torch.isfinite(t).all() for w in want for t in w)
+        (scratch,) = stack.layers[0]._workspaces.values()
+        for i in range(100):
+            scratch.fill_(255)
+            y, logits = stack(xs[i % 2])
+            for got, w in zip([y, *logits], want[i % 2]):
+                wrong += (got != w).any()
+    assert int(wrong) == 0
+    check_status()
 
 
 @pytest.mark.parametrize("T,H,I,N,k", [(1, 1024, 4096, 16384, 64), (37, 1000, 2728, 10000, 24), (64, 2048, 1000, 4096, 33),
