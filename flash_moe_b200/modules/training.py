@@ -31,7 +31,16 @@ def _own_float32_products(T, H, I):
     host sets the pace.  500 tokens x 512 x 768: 116 us of kernels and 110 for the library's, a step 613 -> 508; from about
     2.5e8 multiply-adds a product on the library's larger tiles gain more than its launches cost (1000 x 1024 x 2048: 680 and
     534 us).  Not where the caller lets torch round the operands to TF32."""
-    return T * H * I <= 250_000_000 and not torch.backends.cuda.matmul.allow_tf32
+    return T * H * I <= 250_000_000 and not _tf32_products()
+
+
+def _tf32_products():
+    """Whether torch may round the operands of a float32 product to TF32.  `fp32_precision` answers for both of torch's
+    interfaces; `allow_tf32` raises once the program has used the other one.  A torch that cannot tell counts as yes."""
+    try:
+        return torch.backends.cuda.matmul.fp32_precision not in ("none", "ieee")
+    except (AttributeError, RuntimeError):
+        return True
 
 
 class LayerTrainingStep(torch.autograd.Function):
