@@ -44,7 +44,7 @@ __device__ __forceinline__ bool store_add_row(uint32_t taddr, T* orow, const flo
     const uint4 (&rcur)[4] = rs[c % DEPTH];
     uint32_t a[32];
     ptx::tmem_ld_32x32(taddr + c * 32, a);
-    ptx::tmem_ld_wait();
+    ptx::tmem_ld_wait(a);
     const int col0 = col_base + c * 32;
     if (row_ok) {
 #pragma unroll
@@ -83,7 +83,7 @@ __device__ __forceinline__ void store_add_chunk_smem(uint32_t taddr_chunk, T* or
                                                      bool row_ok) {
   uint32_t a[32];
   ptx::tmem_ld_32x32(taddr_chunk, a);
-  ptx::tmem_ld_wait();
+  ptx::tmem_ld_wait(a);
   if (!row_ok) return;
   const uint8_t* rowp = achunk + srow * 128;
   uint4 pk[4];
@@ -128,7 +128,8 @@ __device__ __forceinline__ void store_swiglu_row(uint32_t taddr, T* orow, int co
     uint32_t g[32], u[32];
     ptx::tmem_ld_32x32(taddr + c * 32, g);
     ptx::tmem_ld_32x32(taddr + NCOLS / 2 + c * 32, u);
-    ptx::tmem_ld_wait();
+    ptx::tmem_ld_wait(g);
+    ptx::tmem_ld_wait(u);
     const int col0 = col_base + c * 32;
     if (row_ok) {
 #pragma unroll

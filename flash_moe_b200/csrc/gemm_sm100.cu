@@ -192,7 +192,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         for (int c = 0; c < BLOCK_N / 32; ++c) {  // pass 1: round, store logits, row max
           uint32_t a[32];
           ptx::tmem_ld_32x32(taddr + c * 32, a);
-          ptx::tmem_ld_wait();
+          ptx::tmem_ld_wait(a);
           if (row_ok) {
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
@@ -218,7 +218,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         for (int c = 0; c < BLOCK_N / 32; ++c) {  // pass 2: sum of exp
           uint32_t a[32];
           ptx::tmem_ld_32x32(taddr + c * 32, a);
-          ptx::tmem_ld_wait();
+          ptx::tmem_ld_wait(a);
 #pragma unroll
           for (int i = 0; i < 32; ++i)
             if (c * 32 + i < nk) vsum += expf(round_to<T>(__uint_as_float(a[i])) - vmax);
@@ -228,7 +228,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         for (int c = 0; c < BLOCK_N / 32; ++c) {  // pass 3: log-probabilities
           uint32_t a[32];
           ptx::tmem_ld_32x32(taddr + c * 32, a);
-          ptx::tmem_ld_wait();
+          ptx::tmem_ld_wait(a);
           if (row_ok) {
 #pragma unroll
             for (int v = 0; v < 4; ++v) {

@@ -233,6 +233,10 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
     ptx::tmem_ld_32x16(taddr + c0, t.a);
     if (NB == 2) ptx::tmem_ld_32x16(taddr + sh.acc_cols + c0, t.b);
   };
+  auto wait_sums = [&](Batch& t) {
+    ptx::tmem_ld_wait(t.a);
+    if (NB == 2) ptx::tmem_ld_wait(t.b);
+  };
   auto finish = [&](int c0, const Batch& t) {
 #pragma unroll
     for (int i = 0; i < CH; ++i) {
@@ -268,22 +272,22 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_consta
       for (int j = nkb > sh.stages ? nkb - sh.stages : 0; j < nkb; ++j)
         ptx::mbar_wait_drain(full_bar(j % sh.stages), (j / sh.stages) & 1u);
     if (done && first < sh.bn) {
+      // sums are requested and waited for in straight-line code, after the last batch those of that batch again
+      const int last = sh.bn - CH - (sh.bn - CH - first) % (2 * CH);  // sh.bn is a multiple of CH
       request_sums(first, even);
+      wait_sums(even);
 #pragma unroll 1
-      for (int c0 = first; c0 < sh.bn; c0 += 4 * CH) {  // sh.bn is a multiple of CH
-        ptx::tmem_ld_wait();
-        if (c0 + 2 * CH < sh.bn) {
-          request_sums(c0 + 2 * CH, odd);
-          request_addends(c0 + 2 * CH, odd);
-        }
+      for (int c0 = first;; c0 += 4 * CH) {
+        request_sums(min(c0 + 2 * CH, last), odd);
+        if (c0 < last) request_addends(c0 + 2 * CH, odd);
         finish(c0, even);
-        if (c0 + 2 * CH >= sh.bn) break;
-        ptx::tmem_ld_wait();
-        if (c0 + 4 * CH < sh.bn) {
-          request_sums(c0 + 4 * CH, even);
-          request_addends(c0 + 4 * CH, even);
-        }
+        wait_sums(odd);
+        if (c0 >= last) break;
+        request_sums(min(c0 + 4 * CH, last), even);
+        if (c0 + 2 * CH < last) request_addends(c0 + 4 * CH, even);
         finish(c0 + 2 * CH, odd);
+        wait_sums(even);
+        if (c0 + 2 * CH >= last) break;
       }
     }
   }

@@ -248,7 +248,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           uint32_t g[32], u[32];
           ptx::tmem_ld_32x32(taddr + c * 32, g);
           ptx::tmem_ld_32x32(taddr + BLOCK_N / 2 + c * 32, u);
-          ptx::tmem_ld_wait();
+          ptx::tmem_ld_wait(g);
+          ptx::tmem_ld_wait(u);
           if (lane == 0) ptx::tma_store_wait();  // the boxes of the chunk before have been read
           __syncwarp();
 #pragma unroll

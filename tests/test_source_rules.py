@@ -40,3 +40,22 @@ def test_early_kernels_do_not_read_their_predecessors_output_as_constant_memory(
     assert seen >= 10
     with open(os.path.join(CSRC, "gemm_epilogue.cuh")) as f:
         assert "ldg" not in re.sub(r"//[^\n]*", "", f.read())  # addend and residual
+
+
+def test_waits_for_tensor_memory_name_the_registers_that_they_wait_for():
+    """To the compiler the registers of a tcgen05.ld are written at the load.  Every wait takes them as operands, so that nothing
+    is done with them in front of it, and every load has its wait."""
+    loads = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        with open(path) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        if path.endswith("ptx_sm100.cuh"):
+            waits = re.findall(r'asm volatile\("tcgen05\.wait::ld[^;]*;"(.*?)\);\n', text, re.S)
+            assert sorted(w.count('"+r"') for w in waits) == [16, 32]
+            continue
+        assert not re.search(r"tmem_ld_wait\(\s*\)", text), os.path.basename(path)
+        loaded = re.findall(r"tmem_ld_32x\d+\([^;]*,\s*([\w.]+)\);", text)
+        waited = re.findall(r"tmem_ld_wait\(([\w.]+)\);", text)
+        assert sorted(loaded) == sorted(waited), (os.path.basename(path), loaded, waited)
+        loads += len(loaded)
+    assert loads >= 10
