@@ -573,7 +573,7 @@ int fmoe_layer_forward(const fmoe_layer_args* a) {
     }
   }
   rc = launch_expert_forward(a->x, a->down_embed, a->up_embed, indices, gates, w.acc, dtype, FMOE_DTYPE_F32, T, H, N, k,
-                             w.expert, w.expert_bytes, a->status, s, between);
+                             w.expert, w.expert_bytes, a->status, s, between, kActSilu, nullptr, true);
   if (rc != FMOE_OK) return fail(rc);
   FMOE_MARK(FMOE_STAGE_EXPERT_ACCUM, 1, s);
 
@@ -636,7 +636,7 @@ int fmoe_train_forward(const fmoe_train_args* a, int* have_preacts) {
   int rc = launch_router_topk(a->log_probs, dtype, T, nk, k, w.scores, a->indices, a->gates, (a->norm_topk_prob ? kTopkNorm : 0) | kTopkTokenRows, s);
   if (rc != FMOE_OK) return rc;
   rc = launch_expert_forward(a->x, a->down_embed, a->up_embed, a->indices, a->gates, w.acc, dtype, FMOE_DTYPE_F32, T, H, N, k,
-                             w.expert, w.expert_bytes, a->status, s, nullptr, kActSilu, a->expert_scores);
+                             w.expert, w.expert_bytes, a->status, s, nullptr, kActSilu, a->expert_scores, true);
   if (rc != FMOE_OK) return rc;
   *have_preacts = a->pre_gate != nullptr && a->pre_up != nullptr ? 1 : 0;
   rc = mlp_up(a->x, a->gate_proj, a->up_proj, w.h, dtype, T, H, I, a->status, s, a->pre_gate, a->pre_up);

@@ -215,8 +215,9 @@ int launch_expert_forward_adding(const void* x, const void* down, const void* up
 int launch_expert_forward(const void* x, const void* down, const void* up, const int64_t* indices, const void* gates,
                           void* out, int dtype, int out_dtype, int64_t T, int H, int64_t N, int k, void* ws,
                           size_t ws_bytes, int32_t* status, cudaStream_t stream, void* const* between_passes = nullptr,
-                          int act = 0, float* raw_scores = nullptr);
+                          int act = 0, float* raw_scores = nullptr, bool router_ids = false);
 // raw_scores (nullable) [T, k] float32 receives <x[t], down[e]> before the activation, for the backward pass.
+// router_ids: the ids are those of the layer's own router in this call (the same sums; see slab_columns).
 // the same sum with both tables sharded by e % world over the GPUs of a node; *_shards are DEVICE arrays of `world`
 // row-0 pointers (peer pointers for the other GPUs); 16-bit dtypes only
 // hot_down / hot_up (nullable): hot_rows rows replicated on every GPU, addressed by the ids N .. N + hot_rows - 1

@@ -137,15 +137,16 @@ __device__ __forceinline__ const T* table_row(const T* table, const T* const* sh
 // every register that waits for data waits for a gathered down row: batches of 128 columns (8 x 16 B per lane) in two register
 // buffers keep gathers in flight across batches to cover the L2 latency.
 //
-// Tables beyond what L2 keeps are walked in slabs of columns, every task of a slab before the next slab; the sums so far wait
-// in gs, where the thread that stored them takes them up again (same order of columns, same bits).  Gathers from a slab that
-// fits L2 run at up to 18 TB/s, from 256 MiB at 9.7 (loads alone): 131072 tokens x 2048, 2^16 experts, top-32 1945 -> 1560 us.
+// SLABS: the table is walked in slabs of columns (slab_columns), every task of a slab before the next slab; the sums so far
+// wait in gs, where the thread that stored them takes them up again (same order of columns, same bits).  Gathers from a slab that
+// fits L2 run at up to 17 TB/s, from 256 MiB at 9.7 (loads alone).  Without, slab is H, in a kernel of its own: 381 -> 373 us for
+// both passes over 32768 tokens x 1024 float16, top-32 of 2^18 experts by Zipf's law.
 //
 // Bound by the L1's data path: a load takes 64 bytes of each of eight rows, eight of its cycles for 512 bytes, and the x
 // fragments as much again for each fourth load.  Measured and not kept at 4096 x 1024, top-64 (52 us): whole lines per load and
 // an exchange between lanes (56), whole lines and sums handed from lane to lane between the halves of a line (twice the MMAs:
 // 56; rows as B: 71), rows as B and the token as A (twice the MMAs for no register moves: 53.7), 32 rows per fragment (54).
-template <typename T, bool PEER, int COLS, bool LOAD32 = false>
+template <typename T, bool PEER, int COLS, bool LOAD32 = false, bool SLABS = false>
 __global__ void __launch_bounds__(128, 4) expert_scores_mma_kernel(const T* x, const T* __restrict__ down, const int64_t* idx,
                                                                   const T* gates, float* gs, int64_t ntok, int H, int64_t N,
                                                                   int k, int slab, int32_t* status, int act,
@@ -155,6 +156,7 @@ __global__ void __launch_bounds__(128, 4) expert_scores_mma_kernel(const T* x, c
   pdl_wait();  // ids and gates come from the kernel before this one
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, tq = lane & 3;
+  if (!SLABS) slab = H;
   const int xs_stride = (slab + 255) / 256 * 32;  // 16-byte pieces of an x row buffer, two per warp
   uint4* xs_buf = xs_all + (threadIdx.x >> 5) * 2 * xs_stride;
   const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
@@ -252,17 +254,18 @@ __global__ void __launch_bounds__(128, 4) expert_scores_mma_kernel(const T* x, c
   fetch_x(t_first, 0, xs_buf);
   rows_of(0);
   load(b0, 0, min(slab, H));
-  for (int col = 0; col < H; col += slab) {
-    const int cols = min(slab, H - col);
-    const bool last_slab = col + slab >= H;
+  int col = 0;
+  do {
+    const int cols = SLABS ? min(slab, H - col) : H;
+    const bool last_slab = !SLABS || col + slab >= H;
     for (int64_t task = warp_global; task < tasks; task += warps_total) {
       const bool last_task = task + warps_total >= tasks;
       const bool more = !(last_slab && last_task);
       if (!more) pdl_launch_dependents();  // the next kernel may set up
-      const int next_col = last_task ? col + slab : col;
+      const int next_col = SLABS ? (last_task ? col + slab : col) : 0;
       const int64_t t = t_next;
       const int j = G_next * 16;
-      if (last_task) {
+      if (SLABS && last_task) {
         t_next = t_first;
         G_next = G_first;
       } else {
@@ -286,7 +289,7 @@ __global__ void __launch_bounds__(128, 4) expert_scores_mma_kernel(const T* x, c
         fetch_ids(t_next, G_next);
         fetch_x(t_next, next_col, xs_buf + (cur ^ 1) * xs_stride);
         part_next = 0.f;
-        if (next_col > 0 && !lone && tq < 2 && G_next * 16 + own < k) part_next = gs[t_next * k + G_next * 16 + own];
+        if (SLABS && next_col > 0 && !lone && tq < 2 && G_next * 16 + own < k) part_next = gs[t_next * k + G_next * 16 + own];
       }
       for (int c0 = 0; c0 < cols; c0 += 2 * STEP) {
         const bool two = c0 + STEP < cols;
@@ -296,13 +299,13 @@ __global__ void __launch_bounds__(128, 4) expert_scores_mma_kernel(const T* x, c
           load(b0, c0 + 2 * STEP, cols);
         } else if (kCross && more) {
           rows_of(next_col);
-          load(b0, 0, min(slab, H - next_col));
+          load(b0, 0, SLABS ? min(slab, H - next_col) : H);
         }
         if (two) consume(b1, c0 + STEP);
       }
       if (!kCross && more) {
         rows_of(next_col);
-        load(b0, 0, min(slab, H - next_col));
+        load(b0, 0, SLABS ? min(slab, H - next_col) : H);
       }
       cur ^= 1;
       if (tq < 2 && j + own < k) {
@@ -318,7 +321,7 @@ __global__ void __launch_bounds__(128, 4) expert_scores_mma_kernel(const T* x, c
         }
       }
     }
-  }
+  } while (SLABS && (col += slab) < H);
   if (bad && status != nullptr) atomicOr(status, FMOE_STATUS_BAD_EXPERT_ID);
 }
 
@@ -797,21 +800,25 @@ bool whole_lines(int64_t N, int H) {
   return H % 16 == 0 && N * H * static_cast<int64_t>(sizeof(T)) > (384ll << 20);
 }
 
-// Tables that do not stay in L2 (126 MB) are gathered from in slabs of 512 columns, both passes with exactly the CTAs that are
-// resident at once, so that all of them are at the same slab: 16384 tokens, both passes, 65536 experts x 2048 top-32 513 -> 396
-// us, 131072 x 2048 top-16 327 -> 267.  Up to 128 MiB slabs give nothing to the scores pass and cost it a round trip per task
-// (65536 x 1024: 112.3 and 112.7 us; 4096 tokens, 16384 x 1024 top-64: 51.8 and 55.1).  Of 2^20 experts no slab stays, the
-// scores pass only walks a row in two steps (32768 tokens x 2048 top-16: Zipf 1.1 ids 216 us in slabs of 512, 193 of 1024,
-// 187 whole; uniform ids 354, 350, 366).
+// Whether the table does not stay in L2 (126 MB).
 template <typename T>
 bool beyond_l2(int64_t N, int H) {
   return N * H * static_cast<int64_t>(sizeof(T)) > (144ll << 20);
 }
+
+// Columns that the scores pass walks the table in: slabs of 512 for the ids of the layer's own router, which spread over the
+// experts, where the table does not stay in L2, a slab nearly does and its rows come more than once.  Both passes then run with
+// exactly the CTAs that are resident at once, so that all of them are at the same slab.  Layer of 131072 tokens, 2048 x 5632,
+// 65536 experts top-32, whole rows and slabs: 11.6 and 11.1 ms, 16384 tokens 1.40 and 1.37 ms; with a router that sends
+// everything to 5 % of the experts 10.15 and 10.2, 1.32 and 1.32.  Other ids may be skewed, and where the wanted rows stay in L2
+// anyway a slab only costs every task a start and a partial sum: the scores and accumulate passes on ids by Zipf's law (1.1),
+// 32768 tokens x 2048 top-16 of 2^18 experts, 370 us whole and 399 in slabs, 2000 tokens top-33 of 2^17 70 and 80 (uniform ids
+// 621 and 600, 93 and 98).  Up to 128 MiB slabs give nothing (65536 x 1024: 112.3 and 112.7 us).
 template <typename T>
-int slab_columns(int64_t N, int H) {
-  if (!beyond_l2<T>(N, H)) return H;
-  const int slab = N * 512 * static_cast<int64_t>(sizeof(T)) <= (256ll << 20) ? 512 : 1024;
-  return slab < H ? slab : H;
+int slab_columns(int64_t T_, int H, int64_t N, int k, bool router_ids) {
+  constexpr int kSlab = 512;
+  const bool slabs = router_ids && beyond_l2<T>(N, H) && N * kSlab * static_cast<int64_t>(sizeof(T)) <= (256ll << 20) && T_ * k >= N;
+  return slabs && H > kSlab ? kSlab : H;
 }
 
 // the scores pass / accumulate pass for few tokens; false: not the shape for it (or, with `rc`, a launch error)
@@ -865,6 +872,8 @@ void launch_accum(const void* up, const int64_t* idx, const float* gs, void* out
   const int colblocks = (H + 32 * VEC * NCH - 1) / (32 * VEC * NCH);
   const int64_t tasks = T_ * colblocks;
   const int64_t want = (tasks + 3) / 4;
+  // a table beyond L2: the CTAs that are resident at once, all of them at the same columns (32768 tokens x 2048 top-16 of 2^18
+  // experts, both passes: uniform ids 637 -> 620 us, Zipf 1.1 379 -> 373; top-64 of 2^18 x 1024 by Zipf's law 672 -> 681)
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * (beyond_l2<T>(N, H) ? 4 : 16);
   const int grid = static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
   auto kern = expert_accum_kernel<T, OutT, NCH>;
@@ -876,7 +885,8 @@ void launch_accum(const void* up, const int64_t* idx, const float* gs, void* out
 // raw dot product
 template <typename T>
 int run_scores(const void* rows, const void* table, const int64_t* idx, const void* gates, float* out, int64_t T_, int H,
-               int64_t N, int k, int32_t* status, cudaStream_t stream, int act = 0, float* raw_out = nullptr) {
+               int64_t N, int k, int32_t* status, cudaStream_t stream, int act = 0, float* raw_out = nullptr,
+               bool router_ids = false) {
   const int sms = device_sm_count();
   if constexpr (sizeof(T) == 2) {
     cudaError_t rc = cudaSuccess;
@@ -889,11 +899,15 @@ int run_scores(const void* rows, const void* table, const int64_t* idx, const vo
     // the next one's ids and x row already in flight, and the work ends evenly (53.7 vs 55.7 us with 16 per SM)
     const int64_t cap = static_cast<int64_t>(sms) * 4;
     const int grid = static_cast<int>(want < cap ? want : cap);
-    const int slab = slab_columns<T>(N, H);
+    const int slab = slab_columns<T>(T_, H, N, k, router_ids);
     const int smem = 4 * 2 * ((slab + 255) / 256 * 32) * 16;  // two x-row buffers per warp
     const bool aligned32 = (reinterpret_cast<uintptr_t>(table) & 31u) == 0;
-    auto kern = !whole_lines<T>(N, H) ? expert_scores_mma_kernel<T, false, 8>
-                : aligned32 ? expert_scores_mma_kernel<T, false, 16, true> : expert_scores_mma_kernel<T, false, 16>;
+    auto kernel = [&](auto slabs) {
+      constexpr bool S = decltype(slabs)::value;
+      return !whole_lines<T>(N, H) ? expert_scores_mma_kernel<T, false, 8, false, S>
+             : aligned32 ? expert_scores_mma_kernel<T, false, 16, true, S> : expert_scores_mma_kernel<T, false, 16, false, S>;
+    };
+    auto kern = slab < H ? kernel(std::true_type{}) : kernel(std::false_type{});
     FMOE_CUDA_TRY(allow_smem(kern, smem));
     FMOE_CUDA_TRY(launch_pdl(4, kern, dim3(grid), dim3(128), smem, stream, 1, static_cast<const T*>(rows),
                              static_cast<const T*>(table), idx, static_cast<const T*>(gates), out, T_, H, N, k, slab,
@@ -935,7 +949,7 @@ int run_accum(const void* table, const int64_t* idx, const float* coef, void* ou
 template <typename T>
 int run_typed(const void* x, const void* down, const void* up, const int64_t* idx, const void* gates, void* out,
               int out_f32, int64_t T_, int H, int64_t N, int k, const ExpertWs& w, int32_t* status,
-              cudaStream_t stream, void* const* between_passes, int act, float* raw_scores) {
+              cudaStream_t stream, void* const* between_passes, int act, float* raw_scores, bool router_ids) {
   auto mark_between = [&]() -> int {
     if (between_passes != nullptr)
       for (int i = 0; i < 2; ++i)
@@ -943,7 +957,7 @@ int run_typed(const void* x, const void* down, const void* up, const int64_t* id
           FMOE_CUDA_TRY(cudaEventRecord(static_cast<cudaEvent_t>(between_passes[i]), stream));
     return FMOE_OK;
   };
-  int rc = run_scores<T>(x, down, idx, gates, w.gs, T_, H, N, k, status, stream, act, raw_scores);
+  int rc = run_scores<T>(x, down, idx, gates, w.gs, T_, H, N, k, status, stream, act, raw_scores, router_ids);
   if (rc != FMOE_OK) return rc;
   if ((rc = mark_between()) != FMOE_OK) return rc;
   // the accumulate pass may gather rows while the scores pass runs: that pass has waited for the ids (only the kernels
@@ -1539,7 +1553,7 @@ int launch_expert_forward_adding(const void* x, const void* down, const void* up
 int launch_expert_forward(const void* x, const void* down, const void* up, const int64_t* indices, const void* gates,
                           void* out, int dtype, int out_dtype, int64_t T, int H, int64_t N, int k, void* ws,
                           size_t ws_bytes, int32_t* status, cudaStream_t stream, void* const* between_passes, int act,
-                          float* raw_scores) {
+                          float* raw_scores, bool router_ids) {
   if (T < 0 || H <= 0 || N <= 0 || k < 0) return FMOE_ERR_BAD_ARG;
   if (act != kActSilu && act != kActGelu) return FMOE_ERR_BAD_ARG;
   if (out_dtype != dtype && out_dtype != FMOE_DTYPE_F32) return FMOE_ERR_BAD_ARG;
@@ -1560,13 +1574,13 @@ int launch_expert_forward(const void* x, const void* down, const void* up, const
   switch (dtype) {
     case FMOE_DTYPE_F32:
       return run_typed<float>(x, down, up, indices, gates, out, 1, T, H, N, k, w, status, stream, between_passes, act,
-                              raw_scores);
+                              raw_scores, router_ids);
     case FMOE_DTYPE_BF16:
       return run_typed<__nv_bfloat16>(x, down, up, indices, gates, out, out_f32, T, H, N, k, w, status, stream,
-                                      between_passes, act, raw_scores);
+                                      between_passes, act, raw_scores, router_ids);
     case FMOE_DTYPE_F16:
       return run_typed<__half>(x, down, up, indices, gates, out, out_f32, T, H, N, k, w, status, stream, between_passes,
-                               act, raw_scores);
+                               act, raw_scores, router_ids);
     default:
       return FMOE_ERR_BAD_ARG;
   }

@@ -84,10 +84,10 @@ def test_a_token_alone_has_the_bits_it_has_in_a_batch(H, N, dtype):
 
 
 @pytest.mark.parametrize("H,T,k", [(520, 430, 17), (1000, 1500, 17), (1024, 1500, 32), (1544, 801, 16)])
-def test_columns_in_slabs(H, T, k):
-    """Tables of more than 144 MiB are walked in slabs of 512 columns, the sums so far kept in registers (warps with one task)
-    or in memory: last slabs of 8, 488, 512 and 8 columns give the bits of the few-token kernels, which have no slabs, and the
-    float64 sums up to float32 rounding; empty slots stay empty."""
+def test_tables_beyond_l2(H, T, k):
+    """Tables of more than 144 MiB, whose accumulate pass runs with the CTAs that are resident at once: last column blocks of 8,
+    488, 512 and 8 columns give the bits of the few-token kernels and the float64 sums up to float32 rounding; empty slots stay
+    empty."""
     from flash_moe_b200.ops.flash_expert import _expert_forward
 
     N = (150 << 20) // (2 * H)
@@ -107,6 +107,61 @@ def test_columns_in_slabs(H, T, k):
         s = (x.double() * d[e].double()).sum(-1)
         want += (torch.nn.functional.silu(s) * gates[:, j].double() * (idx[:, j] >= 0))[:, None] * u[e].double()
     assert (out.double() - want).norm() <= 5e-6 * want.norm()
+
+
+@pytest.mark.parametrize("H,offset,dtype", [(1040, 0, torch.bfloat16), (1040, 8, torch.float16), (2048, 8, torch.bfloat16)])
+def test_whole_line_loads_over_several_tasks(H, offset, dtype):
+    """Tables of more than 384 MiB with two to four tasks for each warp, the next one's rows fetched behind the present one, at
+    both alignments: the bits of the few-token kernels."""
+    from flash_moe_b200.ops.flash_expert import _expert_forward
+
+    T, k, N = 2500, 33, (400 << 20) // (2 * H)
+    gen = torch.Generator(device="cuda").manual_seed(H + offset)
+
+    def normal(rows, std):
+        flat = torch.empty(rows * H + offset, device="cuda", dtype=dtype).normal_(0, std, generator=gen)
+        return flat[offset:].view(rows, H)
+
+    x, d, u = normal(T, 0.5), normal(N, 0.1), normal(N, 1.0)
+    idx = torch.randint(0, N, (T, k), device="cuda", generator=gen)
+    gates = torch.rand(T, k, device="cuda", generator=gen).to(dtype)
+    out, scores = _expert_forward(x, d, u, idx, gates, torch.float32, save_scores=True)
+    for start in range(0, T, 100):
+        rows = slice(start, start + 100)
+        few, few_scores = _expert_forward(x[rows], d, u, idx[rows], gates[rows], torch.float32, save_scores=True)
+        assert torch.equal(few_scores, scores[rows]) and torch.equal(few, out[rows])
+
+
+@pytest.mark.parametrize(
+    "H,T,k,N,offset,dtype",
+    [(2048, 1184, 32, 37500, 0, torch.bfloat16), (1000, 2500, 33, 78643, 0, torch.float16), (520, 4800, 32, 151233, 0, torch.bfloat16),
+     (1040, 6200, 33, 201649, 0, torch.bfloat16), (2048, 3200, 33, 102400, 8, torch.float16), (1032, 6200, 33, 203212, 0, torch.bfloat16)],
+)
+def test_columns_in_slabs(H, T, k, N, offset, dtype):
+    """A layer's scores pass walks tables of more than 144 MiB, rows wanted more than once, in slabs of 512 columns, the sums so
+    far kept in registers (2048: warps with one task) or in memory: last slabs of 512, 488, 8 and 16 columns, loads of 8 columns,
+    of whole lines (above 384 MiB) and of whole lines in two pieces.  With a down projection of zeros the layer returns the
+    experts' sum, and the op walks whole rows: the same bits."""
+    from flash_moe_b200 import FlashMoE, FlashMoEConfig, check_status
+    from flash_moe_b200.ops.flash_expert import flash_expert_fp32
+
+    gen = torch.Generator(device="cuda").manual_seed(H)
+    with torch.device("cuda"):
+        layer = FlashMoE(FlashMoEConfig(H, 64, "silu", N, k, True)).to(dtype).eval()
+    with torch.no_grad():
+        layer.down_proj.weight.zero_()
+        for table, std in ((layer.down_embed, 0.1), (layer.up_embed, 1.0)):
+            flat = torch.empty(N * H + offset, device="cuda", dtype=dtype).normal_(0, std, generator=gen)
+            table.weight.data = flat[offset:].view(N, H)
+        xs = [torch.empty(1, T, H, device="cuda", dtype=dtype).normal_(0, 0.5, generator=gen) for _ in range(2)]
+        got = []
+        for x in xs:
+            y, _ = layer(x, return_routing=True)
+            got.append((y, layer.last_indices.clone(), layer.last_gates.clone()))
+        for x, (y, idx, gates) in zip(xs, got):
+            want = flash_expert_fp32(x[0], layer.down_embed.weight, layer.up_embed.weight, idx, gates)
+            assert torch.equal(y[0], want.to(dtype)) and bool(want.abs().max() > 0.1)
+    check_status()
 
 
 @pytest.mark.parametrize("T,k", [(5, 3), (64, 20), (1200, 20), (1200, 33)])
