@@ -784,19 +784,20 @@ RouterRegLayout make_reg_layout(int nk, int k) {
 //   2. A key whose sum with the other half's maximum stays below the bound is dropped (a superset is kept where rounding
 //      or a non-finite value blurs the test).  What is left - 25 of 128 keys at top-64, 56 of 512 at top-128 for normal
 //      logits; 41 and 105 with the rectangle alone - is compacted and sorted.
+//      Where that still keeps most keys, raise_level bounds the sums again.
 //   3. Each row of the first half counts its sums at or above the bound by a binary search (they do not increase along a
 //      row).  Where there are at most 2 k in all - raising the bound by bisection if there are more - they are the only
 //      candidates: numbered through a running maximum over marks at the rows' first numbers, formed, and sorted as 32-bit keys
 //      (level of the score above the bound | inverted flat id), which puts ties in the order of their ids as well.
-//   4. Otherwise (long runs of equal sums, non-finite values, a range of levels that does not fit the keys) the level of the
-//      k-th sum is found exactly, the sums above it are taken, and the ties with the lowest flat ids fill the rest.
+//      Levels too far apart for that are sorted as 64-bit keys.
+//   4. Otherwise (long runs of equal sums, non-finite values) the level of the k-th sum is found exactly, the sums above it are
+//      taken, and the ties with the lowest flat ids fill the rest.
 //
 // Bound by one token's chain of dependent instructions and by instruction issue (with all keys kept, a threshold search over the
 // staircase (p + 1)(q + 1) <= k and a separate treatment of ties a token of 512 keys, top-128 took 7100 instructions).  us, that
 // form -> this one: 16384 x 512 keys top-128 217 -> 104, 131072 x 256 top-32 359 -> 262, 16384 x 128 top-64 53.5 -> 39.2,
 // 4096 x 128 top-64 18.7 -> 12.6, 8192 x 1024 top-64 102 -> 78, one token 7.5 -> 6.0; logits 100 times smaller, whose sums tie in
-// long runs, 2000 x 512 top-128 606 -> 60.  Slower only where half the probability is in one key and k is large (2000 x 512
-// top-128, logits 6 x |x|: 44 -> 68).  Measured and not kept: both halves sorted (16384 x 512 top-128 152, 122 with the second
+// long runs, 2000 x 512 top-128 606 -> 60.  Measured and not kept: both halves sorted (16384 x 512 top-128 152, 122 with the second
 // alone), four CTAs per SM for 512 keys instead of six (122, 107), rows counted 32 at a time (108, 104 with 64).
 // ------------------------------------------------------------------------------------------
 struct RouterPrunedLayout {
@@ -844,6 +845,86 @@ __device__ __forceinline__ uint32_t sort_lanes_packed(uint32_t v, int lane) {
 template <typename T>
 __device__ __forceinline__ uint32_t sum_level(float s) {
   return HalfKey<T>::make(round_to<T>(s) + 0.0f, 0) >> 16;
+}
+
+// The lowest key of each half that can be in a sum of order level `level` or above (ta, tb: the halves' largest values); left as
+// it is where there is no such bound.
+template <typename T>
+__device__ __forceinline__ void lowest_keys(uint32_t level, float ta, float tb, uint32_t& thr0, uint32_t& thr1) {
+  using HK = HalfKey<T>;
+  const float bound = HK::value(level << 16);
+  // round(a + b) >= bound needs a + b >= bound less one step of T there; the threshold's key is rounded to T too
+  constexpr float kStep = OrdLowBits<T>::value == 16 ? 0.0078125f : 0.0009765625f;
+  const float low = bound - (fabsf(bound) * kStep + 1e-7f);
+  const float xa = low - tb, xb = low - ta, blur = (fabsf(bound) + fabsf(ta) + fabsf(tb)) * 1e-6f + 1e-7f;
+  const float ya = xa - (fabsf(xa) * kStep + blur), yb = xb - (fabsf(xb) * kStep + blur);
+  if (ya > -INFINITY && yb > -INFINITY) {
+    thr0 = max(HK::make(round_to<T>(ya), 0) & 0xFFFF0000u, 1u);
+    thr1 = max(HK::make(round_to<T>(yb), 0) & 0xFFFF0000u, 1u);
+  }
+}
+
+// Keeps the keys of `list` from `th` on, in their order; returns how many they are.
+__device__ __forceinline__ int keep_from(uint32_t* list, int n, uint32_t th, int lane) {
+  int kept = 0;
+#pragma unroll 2
+  for (int base = 0; base < n; base += 32) {  // in place: a key never moves up
+    const uint32_t kv = base + lane < n ? list[base + lane] : 0u;
+    const unsigned bal = __ballot_sync(kFull, kv >= th);
+    if (kv >= th) list[kept + __popc(bal & ((1u << lane) - 1u))] = kv;
+    kept += __popc(bal);
+    __syncwarp();
+  }
+  return kept;
+}
+
+// Where a key holds nearly all of the probability of its half, the k largest sums are those of its row and of the column of the
+// other half's largest key.  The lane maxima show 32 sums of each, and their bound then keeps most keys of both halves.  Here
+// row and column are counted whole: the level goes up (by bisection) to one that k of their sums reach, the keys below it go.
+// Returns the level and the number of keys kept of each half (16 bits each).
+// us, the kernel of before which dropped fewer keys -> this one without this step -> with it, tokens with 0.99 of the probability
+// in one key of each half: 2000 x 512 keys top-128 43 -> 61 -> 29, 2000 x 1024 top-64 60 -> 119 -> 47, 65536 x 256 top-64 393 ->
+// 463 -> 277; ordinary tokens as before (16384 x 512 top-128 106.5) or up to 2 % slower for this call (65536 x 256 top-64 182, 186).
+template <typename T>
+__device__ __noinline__ uint2 raise_level(uint32_t* rows, uint32_t* cols, int na, int nb, int k, uint32_t level, int lane) {
+  using HK = HalfKey<T>;
+  float top[2], second[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t* list = h == 0 ? rows : cols;
+    uint32_t first = 0, next = 0;
+    for (int i = lane; i < (h == 0 ? na : nb); i += 32) {
+      const uint32_t kv = list[i];
+      next = max(next, min(first, kv));
+      first = max(first, kv);
+    }
+    const uint32_t best = __reduce_max_sync(kFull, first);
+    next = __reduce_max_sync(kFull, first == best ? next : first);
+    top[h] = HK::value(best);
+    second[h] = next != 0 ? HK::value(next) : top[h];
+  }
+  const float from = HK::value(level << 16);
+  float lo = from, hi = fmaxf(__fadd_rn(top[0], second[1]), __fadd_rn(second[0], top[1]));
+#pragma unroll 1
+  for (int step = 0; step < 6; ++step) {
+    const float mid = 0.5f * lo + 0.5f * hi;
+    if (!(mid > from && mid < hi)) break;
+    int n = 0;  // the sum of the two largest keys is counted in the row and in the column
+#pragma unroll 4
+    for (int i = lane; i < na; i += 32) n += __fadd_rn(HK::value(rows[i]), top[1]) >= mid ? 1 : 0;
+#pragma unroll 4
+    for (int i = lane; i < nb; i += 32) n += __fadd_rn(top[0], HK::value(cols[i])) >= mid ? 1 : 0;
+    if (static_cast<int>(__reduce_add_sync(kFull, n)) > k) lo = mid;
+    else hi = mid;
+  }
+  if (lo > from) {
+    level = sum_level<T>(lo);
+    uint32_t thr0 = 1, thr1 = 1;
+    lowest_keys<T>(level, top[0], top[1], thr0, thr1);
+    na = keep_from(rows, na, thr0, lane);
+    nb = keep_from(cols, nb, thr1, lane);
+  }
+  return make_uint2(level, na | nb << 16);
 }
 
 // Step 4 of the kernel below, for the rare rows: exactly k winners as 64-bit keys (level, inverted flat id), in order.  At least k
@@ -1110,16 +1191,7 @@ router_topk_pruned_kernel(const T* logp, int64_t ntok, int nk, int k, RouterPrun
           else hi = mid;
         }
         level = sum_level<T>(lo);
-        const float bound = HK::value(level << 16);
-        // round(a + b) >= bound needs a + b >= bound less one step of T there; the threshold's key is rounded to T too
-        constexpr float kStep = OrdLowBits<T>::value == 16 ? 0.0078125f : 0.0009765625f;
-        const float low = bound - (fabsf(bound) * kStep + 1e-7f);
-        const float xa = low - tb, xb = low - ta, blur = (fabsf(bound) + fabsf(ta) + fabsf(tb)) * 1e-6f + 1e-7f;
-        const float ya = xa - (fabsf(xa) * kStep + blur), yb = xb - (fabsf(xb) * kStep + blur);
-        if (ya > -INFINITY && yb > -INFINITY) {
-          thr0 = max(HK::make(round_to<T>(ya), 0) & 0xFFFF0000u, 1u);
-          thr1 = max(HK::make(round_to<T>(yb), 0) & 0xFFFF0000u, 1u);
-        }
+        lowest_keys<T>(level, ta, tb, thr0, thr1);
       }
     }
     int na = 0, nb = 0;
@@ -1146,24 +1218,17 @@ router_topk_pruned_kernel(const T* logp, int64_t ntok, int nk, int k, RouterPrun
       }
       __syncwarp();
     } else {
-      const unsigned below = (1u << lane) - 1u;
       __syncwarp();
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        uint32_t* list = h == 0 ? rows : cols;
-        const uint32_t th = h == 0 ? thr0 : thr1;
-        int n = 0;
-#pragma unroll 2
-        for (int i = lane; i < nkp; i += 32) {  // in place: a key never moves up
-          const uint32_t kv = list[i];
-          const unsigned bal = __ballot_sync(kFull, kv >= th);
-          if (kv >= th) list[n + __popc(bal & below)] = kv;
-          n += __popc(bal);
-          __syncwarp();
-        }
-        if (h == 0) na = n;
-        else nb = n;
-      }
+      na = keep_from(rows, nkp, thr0, lane);
+      nb = keep_from(cols, nkp, thr1, lane);
+    }
+    // Far more keys than the k sums can need, and not because of ties.  An ordinary row keeps 0.8 k, one in a hundred 3 k; from
+    // 3 k on ordinary tokens took 3 % longer (65536 x 256 top-64: 185 and 190 us).  Up to top-32 the bound above is close enough.
+    if ((R >= 4 || E >= 16) && na + nb > max(min(6 * k, nk + nk / 2), 64) && level != 0 && cmax - level > 8) {
+      const uint2 raised = raise_level<T>(rows, cols, na, nb, k, level, lane);
+      level = raised.x;
+      na = raised.y & 0xFFFFu;
+      nb = raised.y >> 16;
     }
     if (nb <= 32) sort_list<T, 1, true>(cols, nb, sb, ib, lane);
     else if (E <= 2 || nb <= 64) sort_list<T, 2, true>(cols, nb, sb, ib, lane);

@@ -170,10 +170,11 @@ def test_router_pruned_rows(T, nk, k, dtype, scale):
 
 @pytest.mark.parametrize("T,nk,k", [(40, 33, 16), (40, 40, 17), (40, 64, 32), (40, 128, 64), (30, 256, 65), (20, 512, 128), (12, 1000, 33)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("kind", ["masked", "one_hot", "few_values", "infinite", "opposite_signs"])
+@pytest.mark.parametrize("kind", ["masked", "one_hot", "few_values", "infinite", "opposite_signs", "dominant", "half_dominant"])
 def test_router_rare_rows(T, nk, k, dtype, kind):
     """Rows that the usual few candidates do not cover, in one call with rows that they do: keys of -inf (down to fewer finite
-    sums than slots), sums too many levels apart for 32-bit keys, more ties than candidates are kept, +inf, sums around 0."""
+    sums than slots), sums too many levels apart for 32-bit keys, more ties than candidates are kept, +inf, sums around 0, keys that hold most of the
+    probability of their half, or of one half (the k sums are then a row and a column)."""
     x = randn((2, T, nk), T + nk + k, torch.float32)
     if kind == "masked":
         x[torch.rand(x.shape, generator=torch.Generator().manual_seed(nk)) < 0.5] = float("-inf")
@@ -185,9 +186,15 @@ def test_router_rare_rows(T, nk, k, dtype, kind):
         x[:, 1] = 0.0
     elif kind == "infinite":
         x[0, ::3, nk // 2] = float("inf")
+    elif kind == "dominant":
+        x[:, ::2, nk // 3] += 12.0
+        x[0, 1::4, 0] += 7.0
+    elif kind == "half_dominant":
+        x[0, :, nk // 2] += 9.0
+        x[1, ::3, :3] += 9.0
     else:
         x[1] = -x[0].flip(-1)
-    lp = (torch.log_softmax(x, -1) if kind in ("one_hot", "few_values") else x).to(dtype).contiguous()
+    lp = (torch.log_softmax(x, -1) if kind in ("one_hot", "few_values", "dominant", "half_dominant") else x).to(dtype).contiguous()
     want_s, want_i = O.router_topk(lp, nk, k)
     got_s, got_i = run_router(lp, nk, k)
     assert torch.equal(got_s.float(), want_s.float())
