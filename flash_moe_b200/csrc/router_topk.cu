@@ -882,9 +882,9 @@ __device__ __forceinline__ int keep_from(uint32_t* list, int n, uint32_t th, int
 // other half's largest key.  The lane maxima show 32 sums of each, and their bound then keeps most keys of both halves.  Here
 // row and column are counted whole: the level goes up (by bisection) to one that k of their sums reach, the keys below it go.
 // Returns the level and the number of keys kept of each half (16 bits each).
-// us, the kernel of before which dropped fewer keys -> this one without this step -> with it, tokens with 0.99 of the probability
-// in one key of each half: 2000 x 512 keys top-128 43 -> 61 -> 29, 2000 x 1024 top-64 60 -> 119 -> 47, 65536 x 256 top-64 393 ->
-// 463 -> 277; ordinary tokens as before (16384 x 512 top-128 106.5) or up to 2 % slower for this call (65536 x 256 top-64 182, 186).
+// us, the kernel of before, which dropped fewer keys -> this one without this step -> with it, tokens with 0.99 of the probability
+// in one key of each half: 2000 x 512 keys top-128 43 -> 61 -> 29, 2000 x 1024 top-64 60 -> 119 -> 37, 65536 x 256 top-64 393 ->
+// 463 -> 277; ordinary tokens as before (16384 x 512 top-128 106.5) or up to 2 % slower alone (65536 x 256 top-64 182, 186).
 template <typename T>
 __device__ __noinline__ uint2 raise_level(uint32_t* rows, uint32_t* cols, int na, int nb, int k, uint32_t level, int lane) {
   using HK = HalfKey<T>;
@@ -932,7 +932,7 @@ __device__ __noinline__ uint2 raise_level(uint32_t* rows, uint32_t* cols, int na
 // half sorted (nb); runs: scratch, na entries.
 template <typename T>
 __device__ __noinline__ void select_exactly(uint32_t* rows, const float* sb, const uint16_t* ib, int na, int nb, int nk, int k,
-                                            uint32_t lo, uint32_t hi, uint32_t* runs, uint64_t* win, int lane) {
+                                            uint32_t lo, uint32_t hi, uint16_t* runs, uint64_t* win, int lane) {
   using HK = HalfKey<T>;
   auto level = [&](int p, int q) { return sum_level<T>(__fadd_rn(HK::value(rows[p]), sb[q])); };
   const int first = 1 << (31 - __clz(nb));
@@ -960,7 +960,8 @@ __device__ __noinline__ void select_exactly(uint32_t* rows, const float* sb, con
     if (static_cast<int>(__reduce_add_sync(kFull, n)) >= k) lo = mid;
     else hi = mid;
   }
-  // everything above; the runs of ties: (first column rank << 16) | columns
+  // everything above (fewer than k <= 128); the runs of ties: (first column rank << 8) | columns, counted up to 255: a row that is
+  // taken whole has fewer than k
   auto row_id = [&](int p) { return HK::id(rows[p]); };
   auto flat_id = [&](int p, int q) { return row_id(p) * static_cast<uint32_t>(nk) + ib[q]; };
   int filled = 0;
@@ -969,7 +970,7 @@ __device__ __noinline__ void select_exactly(uint32_t* rows, const float* sb, con
     int n = 0;
     if (p < na) {
       n = reach(p, hi);
-      runs[p] = (static_cast<uint32_t>(n) << 16) | static_cast<uint32_t>(max(reach(p, lo) - n, 0));
+      runs[p] = static_cast<uint16_t>(n << 8 | min(max(reach(p, lo) - n, 0), 255));
     }
     int incl = n;
 #pragma unroll
@@ -989,7 +990,7 @@ __device__ __noinline__ void select_exactly(uint32_t* rows, const float* sb, con
   for (int bit = 31 - __clz(nk); bit >= 0; --bit) {
     const uint32_t trial = row | (1u << bit);
     int n = 0;
-    for (int p = lane; p < na; p += 32) n += row_id(p) < trial ? static_cast<int>(runs[p] & 0xFFFFu) : 0;
+    for (int p = lane; p < na; p += 32) n += row_id(p) < trial ? static_cast<int>(runs[p] & 0xFFu) : 0;
     n = __reduce_add_sync(kFull, n);
     if (n < need) {
       row = trial;
@@ -1001,18 +1002,19 @@ __device__ __noinline__ void select_exactly(uint32_t* rows, const float* sb, con
     const int p = base + lane;
     const bool take = p < na && row_id(p) < row;
     const uint32_t run = take ? runs[p] : 0u;
-    const int n = run & 0xFFFFu;
+    const int n = run & 0xFFu;
     int incl = n;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const int up = __shfl_up_sync(kFull, incl, d);
       if (lane >= d) incl += up;
     }
-    for (int q = 0; q < n && at + incl - n + q < k; ++q) win[at + incl - n + q] = make_key(lo, flat_id(p, (run >> 16) + q));
+    for (int q = 0; q < n && at + incl - n + q < k; ++q) win[at + incl - n + q] = make_key(lo, flat_id(p, (run >> 8) + q));
     at += __shfl_sync(kFull, incl, 31);
     const unsigned here = __ballot_sync(kFull, p < na && row_id(p) == row);
     if (here != 0) {
-      const int split = base + __ffs(here) - 1, from = runs[split] >> 16, cols = runs[split] & 0xFFFFu, rest = need - whole;
+      const int split = base + __ffs(here) - 1, from = runs[split] >> 8, cols = max(reach(split, lo) - from, 0);
+      const int rest = need - whole;
       uint32_t phi = 0;  // the largest id with fewer than `rest` column ids of the run below it: those and phi are taken
       for (int bit = 31 - __clz(nk); bit >= 0; --bit) {
         const uint32_t trial = phi | (1u << bit);
@@ -1332,7 +1334,7 @@ router_topk_pruned_kernel(const T* logp, int64_t ntok, int nk, int k, RouterPrun
     } else if (listed) {
       sort_wide<T, R>(rows, sb, ib, win32, found, nk, k, reinterpret_cast<uint64_t*>(wbase), win, lane);
     } else {
-      select_exactly<T>(rows, sb, ib, na, nb, nk, k, lo, ordinary ? hi : 0x10000u, reinterpret_cast<uint32_t*>(wbase + L.off_runs),
+      select_exactly<T>(rows, sb, ib, na, nb, nk, k, lo, ordinary ? hi : 0x10000u, reinterpret_cast<uint16_t*>(wbase + L.off_runs),
                         win, lane);
     }
 
@@ -1381,7 +1383,8 @@ int launch_pruned_candidates(const void* logp, int64_t T_, int nk, int k, void* 
   L.off_ids = 2 * L.nkp * 4;
   L.off_win = L.off_ids + L.nkp * 2;
   L.off_runs = L.off_win + 32 * R * 4;
-  L.warp_bytes = L.off_runs + L.nkp * 4;
+  L.warp_bytes = L.off_runs + L.nkp * 2;  // 1024 keys: four CTAs per SM as the registers allow, top-16 of 2000 tokens 35 -> 27 us
+  static_assert(E < 32 || 4 * (E * 32 * (4 + 4 + 2 + 2) + 32 * R * 4) + 1024 <= 228 * 1024 / 4, "four CTAs per SM");
   const int warps = 4;
   const int smem = warps * L.warp_bytes;
   auto kern = router_topk_pruned_kernel<T, E, R>;
