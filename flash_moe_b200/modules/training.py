@@ -85,7 +85,8 @@ class LayerTrainingStep(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, dy, dlogits_out, _didx, _dgates):
-        x, xn, lp, wr, *rest = ctx.saved_tensors
+        # addresses go to the library: hooks on saved tensors may return them with other strides
+        x, xn, lp, wr, *rest = [t if t.is_contiguous() else t.contiguous() for t in ctx.saved_tensors]
         weights, (idx, gates, scores) = rest[:5], rest[5:8]
         wg, wu, wd, de, ue = weights
         T, N, H, I, nk, k, code, norm = ctx.dims
@@ -115,7 +116,6 @@ class LayerTrainingStep(torch.autograd.Function):
         need = ctx.needs_input_grad
         dab, h = x.new_empty((T, 2 * I)), torch.empty_like(a)
         if x.dtype == wr.dtype == xn.dtype == torch.float32 and _own_float32_products(T, H, I):
-            xn, wr = xn.contiguous(), wr.contiguous()
             dxn = torch.empty_like(xn) if need[1] else None
             dw = x.new_empty((2 * I, H)) if need[3] or need[4] else None
             dwd = torch.empty_like(wd) if need[5] else None

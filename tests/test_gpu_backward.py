@@ -410,3 +410,28 @@ def test_dense_backward_float32_refuses_ragged_rows():
     assert _lib.call_struct("fmoe_dense_backward_f32", dev, pack(4, 8, 8, 6)) == _lib.ERR_UNSUPPORTED
     z[3] += 4
     assert _lib.call_struct("fmoe_dense_backward_f32", dev, pack(4, 8, 8, 8)) == _lib.ERR_ALIGNMENT
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_saved_tensors_may_come_back_with_other_strides(dtype):
+    """Hooks on saved tensors may return them in another layout: the same gradients."""
+    from flash_moe_b200 import FlashMoE, FlashMoEConfig, check_status
+
+    def columns_first(t):
+        return t.t().contiguous().t() if t.dim() == 2 else t
+
+    torch.manual_seed(5)
+    with torch.device("cuda"):
+        layer = FlashMoE(FlashMoEConfig(64, 96, "silu", 400, 8, True)).to(dtype).eval()
+        x, dy = torch.randn(3, 20, 64).to(dtype), torch.randn(3, 20, 64).to(dtype)
+    x.requires_grad_()
+    grads = []
+    for hook in (lambda t: t, columns_first):
+        layer.zero_grad()
+        x.grad = None
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, hook):
+            y, _ = layer(x)
+            y.backward(dy)
+        grads.append([x.grad.clone()] + [p.grad.clone() for p in layer.parameters()])
+    assert all(torch.equal(a, b) for a, b in zip(*grads))
+    check_status()
