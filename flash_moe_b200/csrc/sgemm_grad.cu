@@ -4,7 +4,7 @@
 //        d[a | b] = [dh b silu'(a) | dh silu(a)],  h = silu(a) b              (flash_moe/ops/triton/flash_mlp.py:52-102)
 //   2. dx += da Wg + db Wu,  d[Wg; Wu] = d[a | b]^T x,  dWd = dy^T h,  dxn = dlogits Wr,  dWr = dlogits^T xn, side by side
 // As library calls (and a kernel for the activation between them) they were eight launches, and for a small step the host sets
-// the pace: 500 tokens x 512 x 768, the step 613 -> 508 us, the kernels 110 and 116.
+// the pace: 500 tokens x 512 x 768, the host's part of the step 613 -> 508 us, the step 634 -> 545, the kernels 110 and 116.
 //
 // All have a B operand of rows of k, so one kernel takes them: 64 x 64 outputs per CTA, two groups of 64 threads on alternate
 // halves of each 32-row step of k, 8 x 8 outputs per thread, cp.async ring of three steps.  The A operand lies k-major (rows of

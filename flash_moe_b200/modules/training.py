@@ -28,9 +28,12 @@ def _pack(ctx, x, lp, weights, y, pre, extra, ws, stream_dev):
 
 def _own_float32_products(T, H, I):
     """Whether a float32 step takes its dense gradients from fmoe_dense_backward_f32: two launches instead of eight, while the
-    host sets the pace.  500 tokens x 512 x 768: 116 us of kernels and 110 for the library's, a step 613 -> 508; from about
-    2.5e8 multiply-adds a product on the library's larger tiles gain more than its launches cost (1000 x 1024 x 2048: 680 and
-    534 us).  Not where the caller lets torch round the operands to TF32."""
+    host sets the pace.  500 tokens x 512 x 768: the host's part of a step 613 -> 508 us, the step 634 -> 545.  The gain of the
+    host, 80 to 100 us, is the same at all sizes; the kernels keep pace with the library's larger tiles up to about 2.5e8
+    multiply-adds a product (1000 x 512 x 512 a step from a graph 309 us and 313 with the library's), are 7 to 54 us behind
+    at twice that (4000 x 256 x 512 530 and 524, 1000 x 512 x 1024 452 and 425, 250 x 1024 x 2048 505 and 452), and at 1e9
+    more than the host gains (1000 x 1024 x 1024 eager 773 and 721).  The router's products beside them, up to 5.2e8, changed
+    neither side by more than 1 %.  Not where the caller lets torch round the operands to TF32."""
     return T * H * I <= 250_000_000 and not _tf32_products()
 
 
@@ -115,7 +118,10 @@ class LayerTrainingStep(torch.autograd.Function):
             a, b = torch.mm(x, wg.t()), torch.mm(x, wu.t())
         need = ctx.needs_input_grad
         dab, h = x.new_empty((T, 2 * I)), torch.empty_like(a)
-        if x.dtype == wr.dtype == xn.dtype == torch.float32 and _own_float32_products(T, H, I):
+        # a step that is captured has no host time to gain, and the library's kernels are up to 10 us faster (128 x 256 x 512, from a
+        # graph: 153 and 143 us)
+        if x.dtype == wr.dtype == xn.dtype == torch.float32 and _own_float32_products(T, H, I) \
+                and not torch.cuda.is_current_stream_capturing():
             dxn = torch.empty_like(xn) if need[1] else None
             dw = x.new_empty((2 * I, H)) if need[3] or need[4] else None
             dwd = torch.empty_like(wd) if need[5] else None

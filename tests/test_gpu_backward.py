@@ -435,3 +435,45 @@ def test_saved_tensors_may_come_back_with_other_strides(dtype):
         grads.append([x.grad.clone()] + [p.grad.clone() for p in layer.parameters()])
     assert all(torch.equal(a, b) for a, b in zip(*grads))
     check_status()
+
+
+def test_captured_float32_step_takes_torch_products():
+    """A step replayed from a graph has no host time to gain from fewer launches: torch's products, and the eager step's gradients
+    up to float32 sums in another order."""
+    from flash_moe_b200 import FlashMoE, FlashMoEConfig, _lib, check_status
+
+    torch.manual_seed(6)
+    with torch.device("cuda"):
+        layer = FlashMoE(FlashMoEConfig(64, 96, "silu", 400, 8, True)).eval()
+        x, dy = torch.randn(3, 20, 64), torch.randn(3, 20, 64)
+    called, call_struct = [], _lib.call_struct
+
+    def step():
+        called.clear()
+        layer(x)[0].backward(dy)
+        return set(called)
+
+    _lib.call_struct = lambda name, *args: called.append(name) or call_struct(name, *args)
+    try:
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            for _ in range(2):
+                layer.zero_grad(set_to_none=True)
+                assert "fmoe_dense_backward_f32" in step()
+        torch.cuda.current_stream().wait_stream(side)
+        torch.cuda.synchronize()
+        want = [p.grad.clone() for p in layer.parameters()]
+        layer.zero_grad(set_to_none=True)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            names = step()
+        assert "fmoe_train_backward" in names and "fmoe_dense_backward_f32" not in names
+    finally:
+        _lib.call_struct = call_struct
+    for p in layer.parameters():
+        p.grad.fill_(float("nan"))
+    graph.replay()
+    for p, w in zip(layer.parameters(), want):
+        assert (p.grad.double() - w.double()).norm() <= 5e-6 * w.double().norm()
+    check_status()
