@@ -169,7 +169,7 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
 }
 // The registers of a tmem_ld are written some time before this wait ends, and the compiler takes them for written at the load:
 // it may move arithmetic on them, or a copy of them, in front of a wait that does not name them.  So the wait names them, and no
-// load is in flight across a join of control flow, where the compiler places such copies.
+// load is in flight where a loop closes, at which the compiler places such copies.
 __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
                : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),

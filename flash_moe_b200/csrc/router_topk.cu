@@ -1485,8 +1485,10 @@ template <typename T>
 int launch_typed(const void* logp, int64_t T_, int nk, int k, void* scores, int64_t* indices, void* gates, int norm,
                  cudaStream_t stream) {
   if constexpr (sizeof(T) == 2) {
-    // Not where there is little to drop: one key per lane (20000 x 32 keys top-4: 27 us, 32 pruned), or more than half of a
-    // short row wanted (4096 x 128 top-128: 30 us, 33 pruned; 16384 x 100 top-70 69, 73; both with an earlier form of it).
+    // Not for one key per lane, nor where more than half of a short row is wanted: there the two halves' lists do not hold the
+    // 64-bit keys of all candidates (sort_wide).  With lists of 32 R entries the pruned kernel is the faster one there too (us,
+    // whole rows and pruned: 20000 x 32 top-4 33 and 33, top-16 37 and 33, 16384 x 64 top-48 51 and 39, 16384 x 100 top-70 74
+    // and 61, 4096 x 128 top-128 33 and 25), which no call takes yet.
     const bool prune = nk > 32 && (nk > 128 || 2 * k <= nk);
     if (nk <= 1024 && k <= kPrunedMaxK && prune) {
       switch ((next_pow2(nk) < 32 ? 32 : next_pow2(nk)) / 32) {

@@ -42,3 +42,16 @@ def log_probs(T, nk, seed, dtype):
 
 def num_keys(N):
     return math.floor(math.sqrt(N))
+
+
+def kernels_of(call):
+    """Names of the kernels that `call` launches, in the order of their start."""
+    from torch.profiler import ProfilerActivity, profile
+
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA], acc_events=True) as prof:
+        call()
+        torch.cuda.synchronize()
+    events = [e for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    return [e.name for e in sorted(events, key=lambda e: e.time_range.start)]

@@ -242,7 +242,7 @@ def test_backward_with_no_pairs():
 
 
 def test_mlp_backward_with_kept_preactivations():
-    """A shape the CTA-pair GEMM covers: the forward keeps x Wg^T and x Wu^T, the backward uses them."""
+    """The forward keeps x Wg^T and x Wu^T, the backward uses them."""
     from flash_moe_b200.ops.flash_mlp import FlashMLPFunc, _mlp_forward
 
     dtype = torch.bfloat16
@@ -349,17 +349,32 @@ def test_autocast_selects_on_float32_log_probabilities():
     assert torch.isfinite(layer.router_gate.weight.grad.float()).all()
 
 
-@pytest.mark.parametrize("T,H,I", [(512, 256, 256), (515, 264, 264), (545, 256, 392), (2100, 512, 2048)])
+@pytest.mark.parametrize("T,H,I,pair", [(512, 256, 256, False), (515, 264, 264, False), (545, 256, 392, False),
+                                        (2100, 512, 2048, True), (2100, 512, 1992, True), (2100, 512, 2056, True),
+                                        (1030, 256, 2072, True), (4100, 256, 1064, True)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-def test_kept_products_of_the_pair_gemm(T, H, I, dtype):
-    """Boxes of 32 rows x 32 columns that end inside, at and beyond the last row and column: the output has the bits of the
-    forward that keeps nothing, the products are the float32 ones rounded once (half a step of the type, and the float32 sums'
-    own rounding where it moves a value across: 1e-6 of the sum of magnitudes)."""
+def test_kept_products(T, H, I, pair, dtype):
+    """Both GEMMs that keep the two products, the pair GEMM with boxes of 32 rows x 32 columns that end inside, at and beyond the
+    last row and column: the output has the bits of the forward that keeps nothing, the products are the float32 ones rounded
+    once (half a step of the type, and the float32 sums' own rounding where it moves a value across: 1e-6 of the sum of
+    magnitudes), nothing is written behind them."""
+    from flash_moe_b200 import _lib
     from flash_moe_b200.ops.flash_mlp import _mlp_forward
+    from tests.helpers import kernels_of
 
     x, wg, wu, wd = (randn(shape, 20 + i, dtype, sc).cuda()
                      for i, (shape, sc) in enumerate([((T, H), 1.0), ((I, H), 0.05), ((I, H), 0.05), ((H, I), 0.05)]))
-    out, a, b = _mlp_forward(x, wg, wu, wd, save_preacts=True)
+    dev, code = x.device, _lib.dtype_code(x)
+    ws_bytes = _lib.lib().fmoe_mlp_workspace_bytes(T, H, I, code)
+    sizes = (T * H, T * I, T * I, ws_bytes // 2)
+    bufs = [torch.full((n + 512,), -3.0, dtype=dtype, device=dev) for n in sizes]
+    names = kernels_of(lambda: _lib.check(_lib.call(
+        "fmoe_mlp_forward_saving_preacts", dev, x.data_ptr(), wg.data_ptr(), wu.data_ptr(), wd.data_ptr(),
+        *[t.data_ptr() for t in bufs[:3]], code, T, H, I, bufs[3].data_ptr(), ws_bytes, _lib.status_ptr(dev)), "mlp"))
+    assert "gemm_tcgen05_pair_kernel" in names[0] if pair else "gemm_narrow_kernel" in names[0], names
+    for t, n in zip(bufs, sizes):
+        assert bool((t[n:] == -3.0).all())
+    out, a, b = (t[:n].view(T, -1) for t, n in zip(bufs, sizes[:3]))
     assert torch.equal(out, _mlp_forward(x, wg, wu, wd))
     step = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     for got, w in ((a, wg), (b, wu)):

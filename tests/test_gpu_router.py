@@ -204,8 +204,8 @@ def test_router_rare_rows(T, nk, k, dtype, kind):
 @pytest.mark.parametrize("nk,k", [(65, 36), (72, 60), (100, 50), (100, 71), (128, 40), (128, 64), (128, 72)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_router_in_more_than_one_wave(nk, k, dtype):
-    """The kernel may change with the number of tokens, the result of a token does not: 65 to 128 keys, both sides of the
-    number of candidates that stay in registers, ordinary rows and rows full of ties, more tokens than are resident at once
+    """The result of a token does not depend on the tokens beside it: 65 to 128 keys, both sides of half the keys wanted, where the
+    kernel changes, ordinary rows and rows full of ties, more tokens than are resident at once
     against the same tokens in small batches and, for some of them, against the oracle."""
     T = 6001
     lp = torch.log_softmax(randn((2, T, nk), nk * k, torch.float32), -1)
