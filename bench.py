@@ -57,7 +57,7 @@ PROFILE_OF_STAGE = {
 KERNEL_OF_STAGE = {
     "router_front": "router_gemm_bn_kernel<64, 128> (batch-norm applied to the x tiles in shared memory + sub-key logits, tcgen05)",
     "router_topk": "router_topk_pruned_kernel<bf16, 4, 4> (log-softmax, product-key top-k, gates)",
-    "expert_scores": "expert_scores_mma_kernel<bf16, 4 x 2 buffers> (gathered down rows x token row, silu * gate)",
+    "expert_scores": "expert_scores_mma_kernel<bf16, 8 columns per lane> (gathered down rows x token row, silu * gate)",
     "expert_accum": "expert_accum_kernel<bf16, float, 2> (gate-weighted sum of gathered up rows)",
     "mlp_up": "gemm_tcgen05_pair_kernel<SWIGLU> (shared MLP gate/up GEMM + SiLU*up epilogue, CTA pairs)",
     "mlp_down": "gemm_tcgen05_pair_kernel<ADD> (shared MLP down GEMM + fp32 expert addend, CTA pairs)",
