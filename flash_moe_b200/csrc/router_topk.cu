@@ -1380,6 +1380,7 @@ int launch_pruned_candidates(const void* logp, int64_t T_, int nk, int k, void* 
                              cudaStream_t stream) {
   RouterPrunedLayout L{};
   L.nkp = next_pow2(nk) < 32 ? 32 : next_pow2(nk);
+  if (32 * R > L.nkp) return FMOE_ERR_UNSUPPORTED;  // sort_wide lays 32 R 64-bit keys over the two lists (launch_typed)
   L.off_ids = 2 * L.nkp * 4;
   L.off_win = L.off_ids + L.nkp * 2;
   L.off_runs = L.off_win + 32 * R * 4;
